@@ -2,15 +2,19 @@
 //
 // This is the kernel a new decoder is brought up on, the true-fp32 path of the sequence-step models (no reduced-precision
 // matrix mode anywhere), and the path for shapes the tcgen05 GEMM does not take (dimensions that are not multiples of 8, head
-// slices of a few dozen columns). 64 x 64 output tile per CTA, 256 threads with 4 x 4 outputs each, K walked in slices of 16
-// through shared memory (operands converted to fp32 when they are staged). blockIdx.z walks a batch of independent problems
-// that are column slices of the same buffers (attention heads); an optional tile -> group table turns it into the grouped
-// product of expert-sorted rows. Each output accumulates its K terms in ascending order, whatever the M of the call.
+// slices of a few dozen columns). blockIdx.z walks a batch of independent problems that are column slices of the same buffers
+// (attention heads); an optional tile -> group table turns it into the grouped product of expert-sorted rows.
+//
+// Two kernels share one order of sums, so that a row's result does not depend on the M of the call: K is cut into chunks of 64; in a
+// chunk the even and the odd terms are summed separately in ascending order (one packed fma does both), their sum is the chunk's,
+// and the chunks are added in ascending order.
 #include "seq_common.cuh"
 
 namespace omc {
 
-constexpr int kLinBM = 64, kLinBN = 64, kLinBK = 16;
+constexpr int kLinBM = 64, kLinBN = 64, kLinBK = 32;   // BM: rows per tile, also of the grouped product's tile table
+constexpr int kLinChunk = 64;                          // K terms per partial sum
+constexpr int kLinPitch = kLinBK + 4, kLinStages = 3;
 
 struct LinearArgs {
   const void* X;
@@ -45,10 +49,53 @@ __device__ __forceinline__ float gate_out(float y, const LinearArgs& a, int m, i
   return y / (1.f + expf(-z));
 }
 
-template <typename TX, typename TW, typename TY>
-__global__ void __launch_bounds__(256) linear_tile_kernel(LinearArgs a) {
-  __shared__ float xs[kLinBK][kLinBM + 4];
-  __shared__ float ws[kLinBK][kLinBN + 4];
+__device__ __forceinline__ uint32_t lin_smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+
+typedef unsigned long long f32x2_t;
+__device__ __forceinline__ void fma2(f32x2_t& acc, f32x2_t x, f32x2_t w) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(x), "l"(w)); }
+__device__ __forceinline__ float sum2(f32x2_t v) { return __uint_as_float((uint32_t)v) + __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ void lds_pairs(const float* p, f32x2_t& lo, f32x2_t& hi) {
+  const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
+  lo = v.x, hi = v.y;
+}
+
+// dst[0..3] (shared memory) <- row[k..k+3] as fp32, zero where !valid or past K. VEC: K and the row strides are multiples of four and the
+// rows start on boundaries of four elements; fp32 then goes by cp.async, which the caller commits.
+template <typename T, bool VEC>
+__device__ __forceinline__ void stage4(float* dst, const T* row, int k, int K, bool valid) {
+  if constexpr (VEC && sizeof(T) == 4) {
+    const bool in = valid && k < K;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(lin_smem_u32(dst)), "l"(in ? row + k : row), "r"(in ? 16 : 0) : "memory");
+  } else {
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    if (valid) {
+      if (VEC) {
+        if (k < K) ld4(row + k, v);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (k + j < K) v[j] = ldf(row + k + j);
+      }
+    }
+    st4(dst, v);
+  }
+}
+
+template <typename TW, typename TY>
+__device__ __forceinline__ void finish_output(const LinearArgs& a, TY* Y, float sum, int m, int n) {
+  const float b = a.bias != nullptr ? ldf(static_cast<const TW*>(a.bias) + blockIdx.z * a.sbias + n) : 0.f;
+  stf(Y + (long long)m * a.ldy + n, gate_out(apply_act(sum * a.alpha + b, a.act), a, m, n));
+}
+
+// Many rows: 64 x 64 outputs per CTA of 128 threads, 4 x 8 each, K in slices of 32 that go through a ring of three buffers. A thread
+// reads its rows and columns as 16-byte pieces along K (12 loads for 64 packed fma; a pitch of 36 floats puts eight neighbouring rows on
+// different banks), so what bounds it is the shared-memory pipe behind the fma pipe and, with few tiles, the serial walk over K. Measured in
+// fp32 (the kernel before it, 4 x 4 outputs of 256 threads with scalar loads and one buffer, in brackets): 4096 x 6144 x 2048 2463 us =
+// 42 TFLOP/s (4036), 384 x 1024 x 1024 45 us (93).
+template <typename TX, typename TW, typename TY, bool VEC, int NT>   // NT threads: 128 with 4 x 8 outputs each, 256 with 4 x 4
+__global__ void __launch_bounds__(NT) linear_tile_kernel(LinearArgs a) {
+  extern __shared__ __align__(16) float lin_sm[];   // [stages][64 rows of X | 64 rows of W][pitch]
+  constexpr int kStage = (kLinBM + kLinBN) * kLinPitch;
   const int m0 = blockIdx.y * kLinBM, n0 = blockIdx.x * kLinBN;
   const TX* X = static_cast<const TX*>(a.X) + (long long)blockIdx.z * a.sx;
   const TW* W = static_cast<const TW*>(a.W) + (long long)blockIdx.z * a.sw;
@@ -58,43 +105,145 @@ __global__ void __launch_bounds__(256) linear_tile_kernel(LinearArgs a) {
     if (g < 0) return;
     W += (long long)g * a.group_stride;
   }
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  // staging: thread -> (row = tid / 4, k quarter = tid % 4): 4 consecutive k of one row
-  const int lr = threadIdx.x >> 2, lk = (threadIdx.x & 3) * 4;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < a.K; k0 += kLinBK) {
+  constexpr int NJ = kLinBM * kLinBN / 4 / NT, kTx = kLinBN / NJ, kRowsAtOnce = NT / 8;
+  const int tid = threadIdx.x, tx = tid % kTx, ty = tid / kTx;   // ty < 16
+  const int lk = (tid & 7) * 4, lr = tid >> 3;   // staging: 8 pieces of a row by 8 neighbouring threads
+  auto stage = [&](int kt) {
+    float* xs = lin_sm + (kt % kLinStages) * kStage;
+    float* ws = xs + kLinBM * kLinPitch;
+    const int k = kt * kLinBK + lk;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int k = k0 + lk + j;
-      const int m = m0 + lr, n = n0 + lr;
-      xs[lk + j][lr] = (m < a.M && k < a.K) ? ldf(X + (long long)m * a.ldx + k) : 0.f;
-      ws[lk + j][lr] = (n < a.N && k < a.K) ? ldf(W + (long long)n * a.ldw + k) : 0.f;
+    for (int i = 0; i < kLinBM / kRowsAtOnce; ++i) {
+      const int r = lr + i * kRowsAtOnce;
+      stage4<TX, VEC>(xs + r * kLinPitch + lk, X + (long long)min(m0 + r, a.M - 1) * a.ldx, k, a.K, m0 + r < a.M);
     }
-    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kLinBK; ++k) {
-      const float4 xv = *reinterpret_cast<const float4*>(&xs[k][ty * 4]);
-      const float4 wv = *reinterpret_cast<const float4*>(&ws[k][tx * 4]);
-      const float xr[4] = {xv.x, xv.y, xv.z, xv.w}, wr[4] = {wv.x, wv.y, wv.z, wv.w};
+    for (int i = 0; i < kLinBN / kRowsAtOnce; ++i) {
+      const int r = lr + i * kRowsAtOnce;
+      stage4<TW, VEC>(ws + r * kLinPitch + lk, W + (long long)min(n0 + r, a.N - 1) * a.ldw, k, a.K, n0 + r < a.N);
+    }
+  };
+  f32x2_t acc[4][NJ];
+  float tot[4][NJ];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) acc[i][j] = 0ull, tot[i][j] = 0.f;
+  const int nk = (a.K + kLinBK - 1) / kLinBK;
+#pragma unroll
+  for (int s = 0; s < kLinStages - 1; ++s) {
+    if (s < nk) stage(s);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  for (int kt = 0; kt < nk; ++kt) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kLinStages - 2) : "memory");
+    __syncthreads();   // slice kt is there for everyone, and everyone is done with the buffer that the next load overwrites
+    if (kt + kLinStages - 1 < nk) stage(kt + kLinStages - 1);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    const float* xs = lin_sm + (kt % kLinStages) * kStage + ty * kLinPitch;
+    const float* ws = lin_sm + (kt % kLinStages) * kStage + (kLinBM + tx) * kLinPitch;
+#pragma unroll
+    for (int k = 0; k < kLinBK; k += 4) {
+      f32x2_t xl[4], xh[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) lds_pairs(xs + i * 16 * kLinPitch + k, xl[i], xh[i]);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        f32x2_t wl, wh;
+        lds_pairs(ws + j * kTx * kLinPitch + k, wl, wh);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          fma2(acc[i][j], xl[i], wl);
+          fma2(acc[i][j], xh[i], wh);
+        }
+      }
+    }
+    if ((kt & 1) || kt + 1 == nk) {   // the end of a chunk
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xr[i], wr[j], acc[i][j]);
+        for (int j = 0; j < NJ; ++j) tot[i][j] += sum2(acc[i][j]), acc[i][j] = 0ull;
     }
-    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
+    const int m = m0 + ty + 16 * i;
     if (m >= a.M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n < a.N)
-        stf(Y + (long long)m * a.ldy + n,
-            gate_out(apply_act(acc[i][j] * a.alpha + (a.bias != nullptr ? ldf(static_cast<const TW*>(a.bias) + blockIdx.z * a.sbias + n) : 0.f), a.act), a, m, n));
+    for (int j = 0; j < NJ; ++j) {
+      const int n = n0 + tx + kTx * j;
+      if (n < a.N) finish_output<TW, TY>(a, Y, tot[i][j], m, n);
     }
   }
+}
+
+// Few rows: what counts is how many bytes of W are on their way. A CTA of 64 threads owns 8 columns and up to MR rows and brings K terms
+// 1024 at a time into shared memory, all of them in one go; thread (p, c) sums chunk c of the columns p and p + 4 for every row, and
+// the chunks' sums are added by one thread per output. A pitch of 68 floats per chunk puts the chunks on different
+// banks. 3 x 6144 x 2048 in fp32: 19 us = 2.6 TB/s of W (the tile kernel before: 145), 3 x 4096 x 1024 10 (76).
+constexpr int kRowsCols = 8, kRowsChunks = 16, kRowsPitch = kRowsChunks * (kLinChunk + 4), kRowsThreads = 64;
+
+template <typename TX, typename TW, typename TY, int MR, bool VEC>
+__global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(LinearArgs a) {
+  extern __shared__ __align__(16) float lin_sm[];   // W [8][pitch] | X [MR][pitch] | chunk sums [8][MR][16 + 1]
+  float* ws = lin_sm;
+  float* xs = ws + kRowsCols * kRowsPitch;
+  float* part = xs + MR * kRowsPitch;
+  const int m0 = blockIdx.y * MR, n0 = blockIdx.x * kRowsCols;
+  const TX* X = static_cast<const TX*>(a.X) + (long long)blockIdx.z * a.sx;
+  const TW* W = static_cast<const TW*>(a.W) + (long long)blockIdx.z * a.sw;
+  TY* Y = static_cast<TY*>(a.Y) + (long long)blockIdx.z * a.sy;
+  const int tid = threadIdx.x, c = tid & (kRowsChunks - 1), p = tid >> 4;
+  const int out_n = tid & (kRowsCols - 1), out_m = tid / kRowsCols;   // the output whose chunks this thread adds
+  float total = 0.f;
+  for (int k0 = 0; k0 < a.K; k0 += kRowsChunks * kLinChunk) {
+    const int chunks = min(kRowsChunks, (a.K - k0 + kLinChunk - 1) / kLinChunk);
+    if (k0 > 0) __syncthreads();
+    for (int e = tid; e < chunks * (kLinChunk / 4); e += kRowsThreads) {   // piece e of every row
+      const int k = e * 4, at = k + (k >> 6) * 4;
+#pragma unroll
+      for (int r = 0; r < kRowsCols; ++r)
+        stage4<TW, VEC>(ws + r * kRowsPitch + at, W + (long long)min(n0 + r, a.N - 1) * a.ldw, k0 + k, a.K, n0 + r < a.N);
+#pragma unroll
+      for (int r = 0; r < MR; ++r)
+        stage4<TX, VEC>(xs + r * kRowsPitch + at, X + (long long)min(m0 + r, a.M - 1) * a.ldx, k0 + k, a.K, m0 + r < a.M);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (c < chunks) {
+      f32x2_t acc[2][MR];
+#pragma unroll
+      for (int r = 0; r < MR; ++r) acc[0][r] = acc[1][r] = 0ull;
+      const float* w0 = ws + p * kRowsPitch + c * (kLinChunk + 4);
+      const float* x0 = xs + c * (kLinChunk + 4);
+#pragma unroll 4
+      for (int k = 0; k < kLinChunk; k += 4) {
+        f32x2_t al, ah, bl, bh;
+        lds_pairs(w0 + k, al, ah);
+        lds_pairs(w0 + 4 * kRowsPitch + k, bl, bh);
+#pragma unroll
+        for (int r = 0; r < MR; ++r) {
+          f32x2_t xl, xh;
+          lds_pairs(x0 + r * kRowsPitch + k, xl, xh);
+          fma2(acc[0][r], xl, al);
+          fma2(acc[0][r], xh, ah);
+          fma2(acc[1][r], xl, bl);
+          fma2(acc[1][r], xh, bh);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < MR; ++r) {
+        part[(p * MR + r) * (kRowsChunks + 1) + c] = sum2(acc[0][r]);
+        part[((p + 4) * MR + r) * (kRowsChunks + 1) + c] = sum2(acc[1][r]);
+      }
+    }
+    __syncthreads();
+    if (out_m < MR) {
+      const float* s = part + (out_n * MR + out_m) * (kRowsChunks + 1);
+      for (int i = 0; i < chunks; ++i) total += s[i];
+    }
+  }
+  if (out_m < MR && m0 + out_m < a.M && n0 + out_n < a.N) finish_output<TW, TY>(a, Y, total, m0 + out_m, n0 + out_n);
 }
 
 // ---- a few outputs per row (routers, gates, low-rank factors): the tile kernels would leave such a product to a handful of CTAs
@@ -185,8 +334,6 @@ __global__ void __launch_bounds__(256, 2) linear_narrow_kernel(LinearArgs a) {
 // 128 x 128 output tile, K slices of 32 double-buffered with cp.async, 8 warps of 64 x 32. It serves the batched per-head products
 // of latent attention (absorbing W_uk into the query, W_uv after the attention), whose heads are column slices of one buffer.
 constexpr int kMmaBM = 128, kMmaBN = 128, kMmaBK = 32, kMmaPitch = kMmaBK + 8;
-
-__device__ __forceinline__ uint32_t lin_smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 __device__ __forceinline__ void store_pair(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
 __device__ __forceinline__ void store_pair(bf16_t* p, float x, float y) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y); }
@@ -321,15 +468,72 @@ static int launch_narrow(const LinearArgs& a, int y_dt, int batch, cudaStream_t 
   return set_error(OMC_ERR_ARG, "omc_linear: unknown output dtype");
 }
 
+// Rows kernel or tile kernel: the same results either way. The rows kernel costs 1.7e-7 us per K term of an output, whatever the shape; the
+// tile kernel 0.037 us per K term for a first wave of up to 148 tiles, however few and empty they are, and in proportion above that: they
+// meet at 219,000 outputs per wave, 1480 per SM. Both sides in us at K = 1024 (rows / tile): 8 x 4096 outputs 13 / 37, 32 x 4096 28 / 40,
+// 64 x 4096 48 / 44, 128 x 1024 29 / 44, 256 x 1024 49 / 45.
+static long long lin_tiles(const LinearArgs& a, int batch) {
+  return (long long)((a.N + kLinBN - 1) / kLinBN) * ((a.M + kLinBM - 1) / kLinBM) * batch;
+}
+static bool few_rows(const LinearArgs& a, int batch) {
+  const long long tiles = lin_tiles(a, batch), outputs = (long long)a.M * a.N * batch;
+  return a.tile_group == nullptr && outputs <= 1480 * (tiles > 148 ? tiles : 148) && a.M <= 8 * 65535;
+}
+
+// Dynamic shared memory above 48 KB is asked for once per kernel and device.
+template <typename Kernel>
+static int allow_smem(Kernel* kernel, int smem, bool (&done)[kMaxDevices]) {
+  const int dev = cur_device();
+  if (done[dev]) return OMC_OK;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return set_error(OMC_ERR_CUDA, cudaGetErrorString(e));
+  done[dev] = true;
+  return OMC_OK;
+}
+
+template <typename TX, typename TW, typename TY, int MR, bool VEC>
+static int launch_rows(const LinearArgs& a, int batch, cudaStream_t st) {
+  constexpr int smem = ((kRowsCols + MR) * kRowsPitch + kRowsCols * MR * (kRowsChunks + 1)) * 4;
+  static bool done[kMaxDevices] = {};
+  if (int rc = allow_smem(linear_rows_kernel<TX, TW, TY, MR, VEC>, smem, done); rc != OMC_OK) return rc;
+  const dim3 grid((a.N + kRowsCols - 1) / kRowsCols, (a.M + MR - 1) / MR, batch);
+  linear_rows_kernel<TX, TW, TY, MR, VEC><<<grid, kRowsThreads, smem, st>>>(a);
+  return check_launch("omc_linear");
+}
+
+template <typename TX, typename TW, typename TY, bool VEC, int NT>
+static int launch_tile(const LinearArgs& a, int batch, cudaStream_t st) {
+  constexpr int smem = kLinStages * (kLinBM + kLinBN) * kLinPitch * 4;
+  static bool done[kMaxDevices] = {};
+  if (int rc = allow_smem(linear_tile_kernel<TX, TW, TY, VEC, NT>, smem, done); rc != OMC_OK) return rc;
+  const dim3 grid((a.N + kLinBN - 1) / kLinBN, (a.M + kLinBM - 1) / kLinBM, batch);
+  linear_tile_kernel<TX, TW, TY, VEC, NT><<<grid, NT, smem, st>>>(a);
+  return check_launch("omc_linear");
+}
+
+template <typename TX, typename TW, typename TY, bool VEC>
+static int launch_any(const LinearArgs& a, int batch, cudaStream_t st) {
+  if (few_rows(a, batch)) return a.M <= 4 ? launch_rows<TX, TW, TY, 4, VEC>(a, batch, st) : launch_rows<TX, TW, TY, 8, VEC>(a, batch, st);
+  // with few tiles per SM the smaller tasks of 256 threads hide more (100 x 77, K = 4096 rows: 13 us, 128 threads 17); with many, the better
+  // reuse of 128 counts (4096 x 6144 x 2048: 2463 us, 256 threads 2646)
+  return lin_tiles(a, batch) < 296 ? launch_tile<TX, TW, TY, VEC, 256>(a, batch, st) : launch_tile<TX, TW, TY, VEC, 128>(a, batch, st);
+}
+
+template <typename TX, typename TW, typename TY>
+static int launch_linear_typed(const LinearArgs& a, int batch, cudaStream_t st) {
+  // 16-byte (fp32) / 8-byte (bf16) pieces of rows that start on such boundaries and are a multiple of four long
+  const bool vec = a.K % 4 == 0 && a.ldx % 4 == 0 && a.ldw % 4 == 0 && a.sx % 4 == 0 && a.sw % 4 == 0 && a.group_stride % 4 == 0 &&
+                   reinterpret_cast<uintptr_t>(a.X) % (4 * sizeof(TX)) == 0 && reinterpret_cast<uintptr_t>(a.W) % (4 * sizeof(TW)) == 0;
+  return vec ? launch_any<TX, TW, TY, true>(a, batch, st) : launch_any<TX, TW, TY, false>(a, batch, st);
+}
+
 template <typename TX, typename TW>
 static int launch_linear(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
   // few outputs over a long K: the choice depends on widths only, never on M
   if (a.tile_group == nullptr && a.N <= kNarrowMaxN && a.K >= 4 * a.N) return launch_narrow<TX, TW>(a, y_dt, batch, st);
-  dim3 grid((a.N + kLinBN - 1) / kLinBN, (a.M + kLinBM - 1) / kLinBM, batch);
-  if (y_dt == OMC_DT_F32) linear_tile_kernel<TX, TW, float><<<grid, 256, 0, st>>>(a);
-  else if (y_dt == OMC_DT_BF16) linear_tile_kernel<TX, TW, bf16_t><<<grid, 256, 0, st>>>(a);
-  else return set_error(OMC_ERR_ARG, "omc_linear: unknown output dtype");
-  return check_launch("omc_linear");
+  if (y_dt == OMC_DT_F32) return launch_linear_typed<TX, TW, float>(a, batch, st);
+  if (y_dt == OMC_DT_BF16) return launch_linear_typed<TX, TW, bf16_t>(a, batch, st);
+  return set_error(OMC_ERR_ARG, "omc_linear: unknown output dtype");
 }
 
 }  // namespace omc
