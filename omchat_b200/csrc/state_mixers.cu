@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(256) conv_state_save_kernel(const float* __res
 }
 
 // ---- linear-state recurrence ----------------------------------------------------------------------------------------------
-constexpr int kScanCols = 32, kScanLanes = 8, kScanTok = 16;
+constexpr int kScanLanes = 8, kScanGroups = 16, kScanThreads = kScanLanes * kScanGroups, kScanCpt = 2;
 
 struct ScanArgs {
   const float* q;      // [T, ldq]: head g of kv_heads at columns g * dim
@@ -272,6 +272,7 @@ struct ScanArgs {
   const int32_t* pos;
   const int32_t* slot;
   int H, G, dim, vdim;
+  bool vec_state, vec_out;   // a thread's columns of the state / four outputs as one access
 };
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
@@ -304,77 +305,121 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
 template <int DPT>
 __device__ __forceinline__ int scan_place(int i) { return (i / DPT) * (DPT + 4) + (i % DPT); }
 
-// Two stages of kScanTok tokens each: the raw inputs of the next chunk arrive by cp.async while the current chunk is computed;
+// Two stages of TOK tokens each: the raw inputs of the next chunk arrive by cp.async while the current chunk is computed;
 // after arrival one pass turns them in place into what the recurrence uses (silu, decays, sigmoid). VEC: 16-byte copies
 // (every row starts on a 16-byte boundary and the widths are multiples of four), else 4-byte copies.
 // KIND: what enters the state - v itself, the delta rule's correction, or dt v (decay mode 6).
-// TOK: tokens per stage - kScanTok, or 1 for steps of one-token portions, whose CTAs then need little shared memory (more of them share
+// TOK: tokens per stage; 1 for steps of one-token portions, whose CTAs then need little shared memory (more of them share
 // an SM and keep state loads in flight); any TOK is right for any portion.
+//
+// A thread owns DPT neighbouring key channels of CPT neighbouring columns: a packed register holds two neighbouring CHANNELS of one
+// column, so that keys, queries and per-channel decays are used as they lie in shared memory, and only the numbers that all channels
+// share (the input u of a column, a head's decay) are doubled. What bounds it is the issue of the three (delta: four) packed fma per
+// state pair and token, behind them the latency of a token's chain; so what a token reads first is loaded during the token before it, and
+// the read-out of a chunk is summed over the lanes once at its end, from shared memory, instead of by shuffles in every token. Measured,
+// four portions of 1024, 777, 1024, 301 tokens (before: pairs of columns, a doubled key and a shuffled read-out per token): step sizes, 64
+// heads of 128 x 64: 341 us (501); delta rule, 16 heads of 128 x 128: 368 (513), per-channel decays 435 (560); one token of 32 requests,
+// step sizes: 30 us = 4.5 TB/s (42).
 enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
-template <int DPT, bool VEC, int KIND, int TOK>
-__global__ void __launch_bounds__(kScanCols / 2 * kScanLanes) linear_state_scan_kernel(ScanArgs a) {
+template <int DPT, int TOK>
+__host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
+  return TOK * kScanLanes * (DPT + 4) * (chan ? 3 : 2) + TOK * cols + 2 * (TOK < 4 ? 4 : TOK);
+}
+template <int DPT, bool VEC, int KIND, bool CHAN, int TOK>   // CHAN: one decay per key channel
+__global__ void __launch_bounds__(kScanThreads) linear_state_scan_kernel(ScanArgs a) {
   extern __shared__ __align__(16) float sm[];
-  constexpr int PITCH = kScanLanes * (DPT + 4);
-  const int dim = a.dim;
-  const bool chan = KIND != kScanStep && a.decay_mode >= 2;   // one decay per key channel: computed here (2, 4) or given (3, 5)
-  const bool minus1 = KIND == kScanStep || a.decay_mode >= 4;  // the staged value is the decay minus one
+  constexpr int PITCH = kScanLanes * (DPT + 4), CPT = kScanCpt, COLS = kScanGroups * CPT, DP = DPT / 2;
+  constexpr int OPITCH = COLS + 4;           // a lane's partial read-outs of one token
   constexpr int HEADW = TOK < 4 ? 4 : TOK;   // one number per token, in whole 16-byte pieces
-  const int stage_floats = TOK * PITCH * (chan ? 3 : 2) + TOK * kScanCols + 2 * HEADW;
+  const int dim = a.dim;
+  constexpr bool PRE = TOK > 1 && !CHAN;     // read ahead (per-channel decays fill the registers that this takes)
+  const bool minus1 = KIND == kScanStep || a.decay_mode >= 4;  // the staged value is the decay minus one
+  constexpr int stage_floats = scan_stage_floats<DPT, TOK>(CHAN, COLS);
+  float* po = sm + 2 * stage_floats;         // [TOK][lanes][OPITCH] partial read-outs
   const int h = blockIdx.y, kvh = h / (a.H / a.G);
-  const int col0 = blockIdx.x * kScanCols;
+  const int col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
   if (r1 <= r0) return;
-  // thread = (lane over the key channels, PAIR of neighbouring columns): a packed register holds one key channel of both columns
-  const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cp = tid / kScanLanes, col = col0 + 2 * cp;
-  const bool ok0 = col < a.vdim, ok1 = col + 1 < a.vdim;
+  // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
+  // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
+  const int tid = threadIdx.x, lane = TOK == 1 ? tid / kScanGroups : tid & (kScanLanes - 1), cg = TOK == 1 ? tid % kScanGroups : tid / kScanLanes;
+  const int col = col0 + CPT * cg;
   for (int e = tid; e < 2 * stage_floats; e += blockDim.x) sm[e] = 0.f;   // the pads stay zero: they meet zero state only
   float* S = a.state + (((long long)a.slot[r0] * a.H + h) * dim) * a.vdim;
-  const bool pairs = a.vdim % 2 == 0;   // columns (col, col + 1) lie on an 8-byte boundary
-  f32x2 st[DPT];   // state elements (lane * DPT + r, col) and (lane * DPT + r, col + 1)
+  f32x2 st[CPT][DP];   // state elements (lane * DPT + 2 r, col + c) and (lane * DPT + 2 r + 1, col + c)
   const bool fresh = a.pos[r0] == 0;
 #pragma unroll
-  for (int r = 0; r < DPT; ++r) {
-    const int i = lane * DPT + r;
-    const bool ld = !fresh && i < dim;
-    if (pairs) {   // both columns as one access
-      const float2 e = ld && ok0 ? *reinterpret_cast<const float2*>(S + (long long)i * a.vdim + col) : make_float2(0.f, 0.f);
-      st[r] = pack2(e.x, e.y);
-    } else {
-      st[r] = pack2((ld && ok0) ? S[(long long)i * a.vdim + col] : 0.f, (ld && ok1) ? S[(long long)i * a.vdim + col + 1] : 0.f);
+  for (int r = 0; r < DP; ++r) {
+    float e[2][CPT];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = lane * DPT + 2 * r + j;
+      const float* row = S + (long long)i * a.vdim + col;
+      const bool in = !fresh && i < dim;
+      if (a.vec_state) {   // the columns of a thread as one access (CPT divides vdim)
+        const float2 x = in && col < a.vdim ? *reinterpret_cast<const float2*>(row) : make_float2(0.f, 0.f);
+        e[j][0] = x.x, e[j][1] = x.y;
+      } else {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) e[j][c] = in && col + c < a.vdim ? row[c] : 0.f;
+      }
     }
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) st[c][r] = pack2(e[0][c], e[1][c]);
   }
   const float A = (KIND == kScanStep || a.decay_mode == 1 || a.decay_mode == 2) ? expf(a.A_log[h]) : 0.f;
   const float Dh = (KIND == kScanStep && a.D != nullptr) ? a.D[h] : 0.f;
   const float gconst = a.decay_mode == 0 ? a.decay_const[h] : 1.f;
   __syncthreads();
 
+  // sum of a thread's numbers over the lanes, in the same order either way
+  auto sum_lanes = [&](float (&x)[CPT]) {
+    if constexpr (TOK == 1) {
+      __syncthreads();   // the numbers of the sum before have been read
+      *reinterpret_cast<float2*>(po + lane * OPITCH + CPT * cg) = make_float2(x[0], x[1]);
+      __syncthreads();
+      float2 s[kScanLanes];
+#pragma unroll
+      for (int l = 0; l < kScanLanes; ++l) s[l] = *reinterpret_cast<const float2*>(po + l * OPITCH + CPT * cg);
+#pragma unroll
+      for (int m = 1; m < kScanLanes; m <<= 1)
+#pragma unroll
+        for (int l = 0; l < kScanLanes; l += 2 * m) s[l].x += s[l + m].x, s[l].y += s[l + m].y;
+      x[0] = s[0].x, x[1] = s[0].y;
+    } else {
+#pragma unroll
+      for (int m = 1; m < kScanLanes; m <<= 1)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) x[c] += __shfl_xor_sync(0xffffffffu, x[c], m);
+    }
+  };
   auto issue = [&](int c0, int n, int stage) {
     float* sk = sm + stage * stage_floats;
     float* sq = sk + TOK * PITCH;
     float* sg = sq + TOK * PITCH;                       // [tok][PITCH] (per channel) or [tok]
-    float* sv = sg + (chan ? TOK * PITCH : HEADW);
-    float* sb = sv + TOK * kScanCols;
+    float* sv = sg + (CHAN ? TOK * PITCH : HEADW);
+    float* sb = sv + TOK * COLS;
     if (VEC) {
       const int d4 = dim >> 2;
       for (int e = tid; e < n * d4; e += blockDim.x) {
         const int tt = e / d4, i = (e - tt * d4) << 2, at = tt * PITCH + scan_place<DPT>(i);
         cp_async16(sk + at, a.k + (long long)(c0 + tt) * a.ldk + kvh * dim + i);
         cp_async16(sq + at, a.q + (long long)(c0 + tt) * a.ldq + kvh * dim + i);
-        if (chan) cp_async16(sg + at, a.a + (long long)(c0 + tt) * a.lda + h * dim + i);
+        if (CHAN) cp_async16(sg + at, a.a + (long long)(c0 + tt) * a.lda + h * dim + i);
       }
-      for (int e = tid; e < n * (kScanCols / 4); e += blockDim.x) {
-        const int tt = e / (kScanCols / 4), j = (e - tt * (kScanCols / 4)) << 2;
-        if (col0 + j < a.vdim) cp_async16(sv + tt * kScanCols + j, a.v + (long long)(c0 + tt) * a.ldv + h * a.vdim + col0 + j);
+      for (int e = tid; e < n * (COLS / 4); e += blockDim.x) {
+        const int tt = e / (COLS / 4), j = (e - tt * (COLS / 4)) << 2;
+        if (col0 + j < a.vdim) cp_async16(sv + tt * COLS + j, a.v + (long long)(c0 + tt) * a.ldv + h * a.vdim + col0 + j);
       }
     } else {
       for (int e = tid; e < n * dim; e += blockDim.x) {
         const int tt = e / dim, i = e - tt * dim, at = tt * PITCH + scan_place<DPT>(i);
         cp_async4(sk + at, a.k + (long long)(c0 + tt) * a.ldk + kvh * dim + i);
         cp_async4(sq + at, a.q + (long long)(c0 + tt) * a.ldq + kvh * dim + i);
-        if (chan) cp_async4(sg + at, a.a + (long long)(c0 + tt) * a.lda + h * dim + i);
+        if (CHAN) cp_async4(sg + at, a.a + (long long)(c0 + tt) * a.lda + h * dim + i);
       }
-      for (int e = tid; e < n * kScanCols; e += blockDim.x) {
-        const int tt = e / kScanCols, j = e - tt * kScanCols;
+      for (int e = tid; e < n * COLS; e += blockDim.x) {
+        const int tt = e / COLS, j = e - tt * COLS;
         if (col0 + j < a.vdim) cp_async4(sv + e, a.v + (long long)(c0 + tt) * a.ldv + h * a.vdim + col0 + j);
       }
     }
@@ -399,8 +444,8 @@ __global__ void __launch_bounds__(kScanCols / 2 * kScanLanes) linear_state_scan_
     float* sk = sm + stage * stage_floats;
     float* sq = sk + TOK * PITCH;
     float* sg = sq + TOK * PITCH;
-    float* sv = sg + (chan ? TOK * PITCH : HEADW);
-    float* sb = sv + TOK * kScanCols;
+    float* sv = sg + (CHAN ? TOK * PITCH : HEADW);
+    float* sb = sv + TOK * COLS;
     // raw inputs -> what the recurrence uses
     if (a.silu_in || a.decay_mode == 2 || a.decay_mode == 4) {
       for (int e = tid; e < n * dim; e += blockDim.x) {
@@ -414,7 +459,7 @@ __global__ void __launch_bounds__(kScanCols / 2 * kScanLanes) linear_state_scan_
       }
     }
     if (a.silu_in)
-      for (int e = tid; e < n * kScanCols; e += blockDim.x) sv[e] = silu_f(sv[e]);
+      for (int e = tid; e < n * COLS; e += blockDim.x) sv[e] = silu_f(sv[e]);
     if (KIND == kScanStep) {
       if (tid < n) {
         const float dt = softplus_f(sg[tid] + a.dt_bias[h]);
@@ -427,92 +472,174 @@ __global__ void __launch_bounds__(kScanCols / 2 * kScanLanes) linear_state_scan_
       else if (a.decay_mode == 0) sg[tid] = gconst;
     }
     __syncthreads();
+    // what a token reads first - its key, input and shared numbers - is loaded while the token before it is computed
+    f32x2 k2[DP];
+    float un[CPT], gn, bn;
+    auto fetch_key = [&](int tt) {
+      const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(sk + tt * PITCH + lane * (DPT + 4));
+#pragma unroll
+      for (int r = 0; r < DP; r += 2) {
+        const ulonglong2 x = kr[r / 2];
+        k2[r] = x.x, k2[r + 1] = x.y;
+      }
+    };
+    auto fetch_shared = [&](int tt) {
+#pragma unroll
+      for (int c = 0; c < CPT; c += 2) {
+        const float2 x = *reinterpret_cast<const float2*>(sv + tt * COLS + CPT * cg + c);
+        un[c] = x.x, un[c + 1] = x.y;
+      }
+      gn = CHAN ? 0.f : sg[tt];
+      bn = sb[tt];
+    };
+    if (PRE) fetch_key(0), fetch_shared(0);
     for (int tt = 0; tt < n; ++tt) {
-      const float* kr = sk + tt * PITCH + lane * (DPT + 4);
-      const float* qr = sq + tt * PITCH + lane * (DPT + 4);
-      f32x2 da = 0ull, db = 0ull;   // (column, column + 1) partial dot products, two chains
-      f32x2 k2[DPT];                // the key, each channel doubled: used again by the update
-      const f32x2 gh = pack2(sg[chan ? 0 : tt], sg[chan ? 0 : tt]);
-      const float* gr = sg + tt * PITCH + lane * (DPT + 4);
+      const int next = min(tt + 1, n - 1);
+      if (!PRE) fetch_key(tt), fetch_shared(tt);
+      float u[CPT];
 #pragma unroll
-      for (int r = 0; r < DPT; r += 4) {
-        const float4 kv = *reinterpret_cast<const float4*>(kr + r);
-        k2[r] = pack2(kv.x, kv.x), k2[r + 1] = pack2(kv.y, kv.y), k2[r + 2] = pack2(kv.z, kv.z), k2[r + 3] = pack2(kv.w, kv.w);
-        if (chan) {
-          const float4 gv = *reinterpret_cast<const float4*>(gr + r);
-          if (minus1) {
-            st[r] = fma2(st[r], pack2(gv.x, gv.x), st[r]), st[r + 1] = fma2(st[r + 1], pack2(gv.y, gv.y), st[r + 1]);
-            st[r + 2] = fma2(st[r + 2], pack2(gv.z, gv.z), st[r + 2]), st[r + 3] = fma2(st[r + 3], pack2(gv.w, gv.w), st[r + 3]);
-          } else {
-            st[r] = mul2(st[r], pack2(gv.x, gv.x)), st[r + 1] = mul2(st[r + 1], pack2(gv.y, gv.y));
-            st[r + 2] = mul2(st[r + 2], pack2(gv.z, gv.z)), st[r + 3] = mul2(st[r + 3], pack2(gv.w, gv.w));
+      for (int c = 0; c < CPT; ++c) u[c] = un[c];
+      const float b = bn;
+      if (CHAN) {
+        const ulonglong2* gr = reinterpret_cast<const ulonglong2*>(sg + tt * PITCH + lane * (DPT + 4));
+#pragma unroll
+        for (int r = 0; r < DP; r += 2) {
+          const ulonglong2 g = gr[r / 2];
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) {
+            st[c][r] = minus1 ? fma2(st[c][r], g.x, st[c][r]) : mul2(st[c][r], g.x);
+            st[c][r + 1] = minus1 ? fma2(st[c][r + 1], g.y, st[c][r + 1]) : mul2(st[c][r + 1], g.y);
           }
-        } else if (minus1) {
-          st[r] = fma2(st[r], gh, st[r]), st[r + 1] = fma2(st[r + 1], gh, st[r + 1]);
-          st[r + 2] = fma2(st[r + 2], gh, st[r + 2]), st[r + 3] = fma2(st[r + 3], gh, st[r + 3]);
-        } else {
-          st[r] = mul2(st[r], gh), st[r + 1] = mul2(st[r + 1], gh), st[r + 2] = mul2(st[r + 2], gh), st[r + 3] = mul2(st[r + 3], gh);
         }
-        if (KIND == kScanDelta) {
-          da = fma2(st[r], k2[r], da), db = fma2(st[r + 1], k2[r + 1], db);
-          da = fma2(st[r + 2], k2[r + 2], da), db = fma2(st[r + 3], k2[r + 3], db);
-        }
+      } else {
+        const f32x2 gh = pack2(gn, gn);
+#pragma unroll
+        for (int r = 0; r < DP; ++r)
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) st[c][r] = minus1 ? fma2(st[c][r], gh, st[c][r]) : mul2(st[c][r], gh);
       }
-      const float2 vv = *reinterpret_cast<const float2*>(sv + tt * kScanCols + 2 * cp);
-      float u0 = vv.x, u1 = vv.y;
-      if (KIND == kScanStep) u0 *= sb[tt], u1 *= sb[tt];
+      if (PRE) fetch_shared(next);
+      const ulonglong2* qr = reinterpret_cast<const ulonglong2*>(sq + tt * PITCH + lane * (DPT + 4));
+      f32x2 q2[DP];
+      auto fetch_query = [&] {
+#pragma unroll
+        for (int r = 0; r < DP; r += 2) {
+          const ulonglong2 x = qr[r / 2];
+          q2[r] = x.x, q2[r + 1] = x.y;
+        }
+      };
+      if (PRE) fetch_query();
+      float vin[CPT];   // TOK == 1: what D multiplies
+      if (KIND == kScanStep) {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) vin[c] = u[c], u[c] *= b;
+      }
       if (KIND == kScanDelta) {
-        float a0, a1, b0, b1;
-        unpack2(da, a0, a1);
-        unpack2(db, b0, b1);
-        float dot0 = a0 + b0, dot1 = a1 + b1;
+        float dot[CPT];
 #pragma unroll
-        for (int m = 1; m < kScanLanes; m <<= 1) {
-          dot0 += __shfl_xor_sync(0xffffffffu, dot0, m);
-          dot1 += __shfl_xor_sync(0xffffffffu, dot1, m);
+        for (int c = 0; c < CPT; ++c) {
+          f32x2 d0 = 0ull, d1 = 0ull;   // two chains
+#pragma unroll
+          for (int r = 0; r < DP; r += 2) d0 = fma2(st[c][r], k2[r], d0), d1 = fma2(st[c][r + 1], k2[r + 1], d1);
+          float w, x, y, z;
+          unpack2(d0, w, x);
+          unpack2(d1, y, z);
+          dot[c] = (w + y) + (x + z);
         }
-        u0 = sb[tt] * (u0 - dot0);
-        u1 = sb[tt] * (u1 - dot1);
-      }
-      const f32x2 u2 = pack2(u0, u1);
-      f32x2 oa = 0ull, ob = 0ull;
+        sum_lanes(dot);
 #pragma unroll
-      for (int r = 0; r < DPT; r += 4) {
-        const float4 qv = *reinterpret_cast<const float4*>(qr + r);
-        st[r] = fma2(k2[r], u2, st[r]), st[r + 1] = fma2(k2[r + 1], u2, st[r + 1]);
-        st[r + 2] = fma2(k2[r + 2], u2, st[r + 2]), st[r + 3] = fma2(k2[r + 3], u2, st[r + 3]);
-        oa = fma2(st[r], pack2(qv.x, qv.x), oa), ob = fma2(st[r + 1], pack2(qv.y, qv.y), ob);
-        oa = fma2(st[r + 2], pack2(qv.z, qv.z), oa), ob = fma2(st[r + 3], pack2(qv.w, qv.w), ob);
+        for (int c = 0; c < CPT; ++c) u[c] = b * (u[c] - dot[c]);
       }
-      float o0, o1, p0, p1;
-      unpack2(oa, o0, o1);
-      unpack2(ob, p0, p1);
-      o0 += p0;
-      o1 += p1;
+      f32x2 oa[CPT], ob[CPT];
 #pragma unroll
-      for (int m = 1; m < kScanLanes; m <<= 1) {
-        o0 += __shfl_xor_sync(0xffffffffu, o0, m);
-        o1 += __shfl_xor_sync(0xffffffffu, o1, m);
+      for (int c = 0; c < CPT; ++c) {
+        const f32x2 u2 = pack2(u[c], u[c]);
+        oa[c] = ob[c] = 0ull;
+#pragma unroll
+        for (int r = 0; r < DP; ++r) st[c][r] = fma2(k2[r], u2, st[c][r]);
       }
-      if (lane == 0) {
-        float* dst = a.out + (long long)(c0 + tt) * a.ldo + h * a.vdim + col;
-        if (KIND == kScanStep) o0 = fmaf(Dh, vv.x, o0), o1 = fmaf(Dh, vv.y, o1);
-        if (ok0) dst[0] = o0 * a.out_scale;
-        if (ok1) dst[1] = o1 * a.out_scale;
+      if (PRE) fetch_key(next);
+      else fetch_query();
+#pragma unroll
+      for (int r = 0; r < DP; r += 2)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          oa[c] = fma2(st[c][r], q2[r], oa[c]);
+          ob[c] = fma2(st[c][r + 1], q2[r + 1], ob[c]);
+        }
+      float o[CPT];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        float w, x, y, z;
+        unpack2(oa[c], w, x);
+        unpack2(ob[c], y, z);
+        o[c] = (w + y) + (x + z);
+      }
+      if constexpr (TOK == 1) {
+        sum_lanes(o);
+        if (lane == 0) {
+          float* dst = a.out + (long long)(c0 + tt) * a.ldo + h * a.vdim + col;
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) {
+            if (KIND == kScanStep) o[c] = fmaf(Dh, vin[c], o[c]);
+            if (col + c < a.vdim) dst[c] = o[c] * a.out_scale;
+          }
+        }
+      } else {
+        float* dst = po + (tt * kScanLanes + lane) * OPITCH + CPT * cg;
+#pragma unroll
+        for (int c = 0; c < CPT; c += 2) *reinterpret_cast<float2*>(dst + c) = make_float2(o[c], o[c + 1]);
       }
     }
-    __syncthreads();   // the next iteration's copies overwrite the stage that was just read
+    __syncthreads();   // the partial read-outs are there; the next iteration's copies overwrite the stage that was just read
+    if constexpr (TOK > 1) {
+      for (int e = tid; e < n * (COLS / 4); e += blockDim.x) {
+        const int tt = e / (COLS / 4), j = (e - tt * (COLS / 4)) << 2;
+        if (col0 + j >= a.vdim) continue;
+        const float* src = po + tt * kScanLanes * OPITCH + j;
+        float4 s[kScanLanes];
+#pragma unroll
+        for (int l = 0; l < kScanLanes; ++l) s[l] = *reinterpret_cast<const float4*>(src + l * OPITCH);
+#pragma unroll
+        for (int m = 1; m < kScanLanes; m <<= 1)   // the order of sum_lanes: the same bits
+#pragma unroll
+          for (int l = 0; l < kScanLanes; l += 2 * m) s[l].x += s[l + m].x, s[l].y += s[l + m].y, s[l].z += s[l + m].z, s[l].w += s[l + m].w;
+        float4 o = s[0];
+        if (KIND == kScanStep) {
+          const float4 x = *reinterpret_cast<const float4*>(sv + tt * COLS + j);
+          o.x = fmaf(Dh, x.x, o.x), o.y = fmaf(Dh, x.y, o.y), o.z = fmaf(Dh, x.z, o.z), o.w = fmaf(Dh, x.w, o.w);
+        }
+        o.x *= a.out_scale, o.y *= a.out_scale, o.z *= a.out_scale, o.w *= a.out_scale;
+        float* dst = a.out + (long long)(c0 + tt) * a.ldo + h * a.vdim + col0 + j;
+        if (a.vec_out) {
+          *reinterpret_cast<float4*>(dst) = o;
+        } else {
+          dst[0] = o.x;
+          if (col0 + j + 1 < a.vdim) dst[1] = o.y;
+          if (col0 + j + 2 < a.vdim) dst[2] = o.z;
+          if (col0 + j + 3 < a.vdim) dst[3] = o.w;
+        }
+      }
+      if (KIND == kScanStep) __syncthreads();   // v is read here too
+    }
   }
 #pragma unroll
-  for (int r = 0; r < DPT; ++r) {
-    const int i = lane * DPT + r;
-    float lo, hi;
-    unpack2(st[r], lo, hi);
-    if (pairs) {
-      if (i < dim && ok0) *reinterpret_cast<float2*>(S + (long long)i * a.vdim + col) = make_float2(lo, hi);
-    } else {
-      if (i < dim && ok0) S[(long long)i * a.vdim + col] = lo;
-      if (i < dim && ok1) S[(long long)i * a.vdim + col + 1] = hi;
+  for (int r = 0; r < DP; ++r) {
+    float e[2][CPT];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) unpack2(st[c][r], e[0][c], e[1][c]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = lane * DPT + 2 * r + j;
+      float* row = S + (long long)i * a.vdim + col;
+      if (i >= dim) continue;
+      if (a.vec_state) {
+        if (col < a.vdim) *reinterpret_cast<float2*>(row) = make_float2(e[j][0], e[j][1]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+          if (col + c < a.vdim) row[c] = e[j][c];
+      }
     }
   }
 }
@@ -1113,7 +1240,7 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   if (dim > 256) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: key width above 256");
   if (portions > 65535 || H > 65535) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: more than 65535 portions or heads");
   ScanArgs s{q, k, v, ldq, ldk, ldv, silu_in, decay_mode, decay_pow, out_scale, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo,
-             row_begin, pos, slot, H, G, dim, vdim};
+             row_begin, pos, slot, H, G, dim, vdim, false, false};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int dpt = dim <= 32 ? 4 : (dim <= 64 ? 8 : (dim <= 128 ? 16 : 32));   // key channels per thread: dim / 8 lanes, rounded up to a float4
   const bool chan = decay_mode >= 2 && decay_mode <= 5;
@@ -1121,36 +1248,42 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   const bool vec = dim % 4 == 0 && vdim % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 && al16(q) && al16(k) && al16(v) &&
                    (!chan || (lda % 4 == 0 && al16(a)));
   const bool one = vec && rows <= portions;   // every portion is one token
-  const int tok = one ? 1 : kScanTok;
-  const size_t stage_floats = (size_t)tok * kScanLanes * (dpt + 4) * (chan ? 3 : 2) + tok * kScanCols + 2 * (tok < 4 ? 4 : tok);
-  const size_t smem = 2 * stage_floats * sizeof(float);
-  dim3 grid((vdim + kScanCols - 1) / kScanCols, H, portions);
-  const int threads = kScanCols / 2 * kScanLanes;
-#define OMC_SCAN_LAUNCH(DPT, VEC, KIND, TOK)                                                                                        \
-  do {                                                                                                                              \
-    static bool attr_done[kMaxDevices] = {};                                                                                        \
-    if (!attr_done[cur_device()]) {                                                                                                 \
-      cudaFuncSetAttribute(linear_state_scan_kernel<DPT, VEC, KIND, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024); \
-      attr_done[cur_device()] = true;                                                                                               \
-    }                                                                                                                               \
-    linear_state_scan_kernel<DPT, VEC, KIND, TOK><<<grid, threads, smem, st>>>(s);                                                  \
+  s.vec_state = vdim % kScanCpt == 0 && al16(state);
+  s.vec_out = vdim % 4 == 0 && ldo % 4 == 0 && al16(out);
+  constexpr int cols = kScanGroups * kScanCpt;
+  dim3 grid((vdim + cols - 1) / cols, H, portions);
+  // 16 tokens per stage; with per-channel decays that is 85 KB and two CTAs per SM, so beyond 296 CTAs eight tokens (in us, 16 / 8 tokens,
+  // 32 heads of 128 x 128, portions of 1024, 777, 1024, 301: 713 / 608; 16 heads: 435 / 476)
+  const bool tight = chan && (long long)grid.x * H * portions > 296;
+#define OMC_SCAN_LAUNCH(DPT, VEC, KIND, CHAN, TOK)                                                                                        \
+  do {                                                                                                                                    \
+    static bool attr_done[kMaxDevices] = {};                                                                                              \
+    constexpr int smem = 4 * (2 * scan_stage_floats<DPT, TOK>(CHAN, cols) + TOK * kScanLanes * (cols + 4));                                \
+    if (!attr_done[cur_device()]) {                                                                                                       \
+      cudaFuncSetAttribute(linear_state_scan_kernel<DPT, VEC, KIND, CHAN, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);       \
+      attr_done[cur_device()] = true;                                                                                                     \
+    }                                                                                                                                     \
+    linear_state_scan_kernel<DPT, VEC, KIND, CHAN, TOK><<<grid, kScanThreads, smem, st>>>(s);                                             \
   } while (0)
-#define OMC_SCAN_KIND(DPT, VEC, TOK)                                         \
-  do {                                                                       \
-    if (decay_mode == 6) OMC_SCAN_LAUNCH(DPT, VEC, kScanStep, TOK);          \
-    else if (beta != nullptr) OMC_SCAN_LAUNCH(DPT, VEC, kScanDelta, TOK);    \
-    else OMC_SCAN_LAUNCH(DPT, VEC, kScanPlain, TOK);                         \
+#define OMC_SCAN_KIND(DPT, VEC, TOK)                                                      \
+  do {                                                                                    \
+    if (decay_mode == 6) OMC_SCAN_LAUNCH(DPT, VEC, kScanStep, false, TOK);                \
+    else if (beta != nullptr && chan) OMC_SCAN_LAUNCH(DPT, VEC, kScanDelta, true, TOK);   \
+    else if (beta != nullptr) OMC_SCAN_LAUNCH(DPT, VEC, kScanDelta, false, TOK);          \
+    else if (chan) OMC_SCAN_LAUNCH(DPT, VEC, kScanPlain, true, TOK);                      \
+    else OMC_SCAN_LAUNCH(DPT, VEC, kScanPlain, false, TOK);                               \
   } while (0)
-#define OMC_SCAN_DPT(DPT)                             \
-  do {                                                \
-    if (one) OMC_SCAN_KIND(DPT, true, 1);             \
-    else if (vec) OMC_SCAN_KIND(DPT, true, kScanTok); \
-    else OMC_SCAN_KIND(DPT, false, kScanTok);         \
+#define OMC_SCAN_DPT(DPT, TOK)                  \
+  do {                                          \
+    if (one) OMC_SCAN_KIND(DPT, true, 1);       \
+    else if (vec) OMC_SCAN_KIND(DPT, true, TOK); \
+    else OMC_SCAN_KIND(DPT, false, TOK);        \
   } while (0)
-  if (dpt == 4) OMC_SCAN_DPT(4);
-  else if (dpt == 8) OMC_SCAN_DPT(8);
-  else if (dpt == 16) OMC_SCAN_DPT(16);
-  else OMC_SCAN_DPT(32);
+  if (dpt == 4) OMC_SCAN_DPT(4, 16);
+  else if (dpt == 8) OMC_SCAN_DPT(8, 16);
+  else if (dpt == 16 && tight) OMC_SCAN_DPT(16, 8);
+  else if (dpt == 16) OMC_SCAN_DPT(16, 16);
+  else OMC_SCAN_DPT(32, 8);
 #undef OMC_SCAN_DPT
 #undef OMC_SCAN_KIND
 #undef OMC_SCAN_LAUNCH
