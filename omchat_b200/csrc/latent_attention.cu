@@ -672,6 +672,12 @@ __global__ void latent_decode_items_kernel(const int32_t* __restrict__ pos, cons
   }
 }
 
+// latent_attention_sm100.cu
+bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool);
+int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
+                 int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
+                 float* ws_ml, cudaStream_t st);
+
 template <int VS, int NV, typename TO>
 static int launch_lat_mma_t(const LatMmaArgs& a, int n_items, size_t smem, cudaStream_t st) {
   static bool attr_done[kMaxDevices] = {};
@@ -697,9 +703,17 @@ extern "C" int omc_latent_attn_mma(const void* qcat, int T, int H, int r, int dr
                                    int max_pages, int page_size, const int32_t* items, int n_items, const int32_t* merges,
                                    int n_merges, const float* sink, int window, const float* gate, long long ldg, float scale, void* out,
                                    int out_dt, float* ws_o, float* ws_ml, void* stream) {
+  return omc_latent_attn_mma_rows(qcat, T, H, r, dr, pool, block_table, max_pages, page_size, items, n_items, omc::kMmaRows, merges, n_merges, sink, window, gate,
+                                  ldg, scale, out, out_dt, ws_o, ws_ml, stream);
+}
+
+extern "C" int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, int dr, const void* pool, const int32_t* block_table, int max_pages,
+                                        int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
+                                        const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,
+                                        float* ws_o, float* ws_ml, void* stream) {
   if (window < 1) return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: the window holds at least the row itself");
   if (qcat == nullptr || pool == nullptr || block_table == nullptr || items == nullptr || out == nullptr || T < 0 || H <= 0 ||
-      page_size <= 0 || max_pages <= 0 || n_items < 0 || n_merges < 0 || (n_merges > 0 && (merges == nullptr || ws_o == nullptr || ws_ml == nullptr)))
+      page_size <= 0 || max_pages <= 0 || n_items < 0 || max_rows < 1 || n_merges < 0 || (n_merges > 0 && (merges == nullptr || ws_o == nullptr || ws_ml == nullptr)))
     return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: bad argument");
   if (r <= 0 || r % 16 != 0 || r > 512 || dr < 0 || dr % 16 != 0 || H > kMmaRows)
     return set_error(OMC_ERR_SHAPE, "omc_latent_attn_mma: latent width a multiple of 16 up to 512, rotated width a multiple of 16, at most 64 heads");
@@ -718,7 +732,10 @@ extern "C" int omc_latent_attn_mma(const void* qcat, int T, int H, int r, int dr
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc;
   if (out_dt != OMC_DT_F32 && out_dt != OMC_DT_BF16) return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: unknown output dtype");
-  if (r <= 64) rc = launch_lat_mma<1, 8>(a, out_dt, n_items, smem, st);
+  if (latent_sm100_ok(max_rows, r, dr, page_size, qcat, pool))
+    rc = latent_sm100(qcat, (long long)T * H, H, r, dr, pool, block_table, max_pages, page_size, items, n_items, max_rows, sink, window, gate, ldg, scale,
+                      out, out_dt, ws_o, ws_ml, st);
+  else if (r <= 64) rc = launch_lat_mma<1, 8>(a, out_dt, n_items, smem, st);
   else if (r <= 128) rc = launch_lat_mma<1, 16>(a, out_dt, n_items, smem, st);
   else if (r <= 256) rc = launch_lat_mma<2, 16>(a, out_dt, n_items, smem, st);
   else rc = launch_lat_mma<4, 16>(a, out_dt, n_items, smem, st);  // 16 warps: four per row group, 128 value columns and 16 keys each

@@ -1,0 +1,425 @@
+// Latent attention on tcgen05 / TMEM (bf16; the work list of omc_latent_attn_mma, latent widths that are a multiple of 128 up to 512,
+// pages of a multiple of 64 rows). Everything else stays with the mma.sync kernel of latent_attention.cu.
+//
+// One CTA per item: up to NR = 16 / 32 / 64 rows ((token, head) pairs) against keys in tiles of 128. A key row is 576 numbers wide and its
+// first 512 are the value, so an accumulator with the rows on the 128 lanes of TMEM would need all 512 columns for the output alone.
+// Here both products are TRANSPOSED: keys and value dimensions lie on the lanes, rows on the columns,
+//     S^T [128 keys, NR] = K Q^T          A = the key tile, K-major              B = Q, K-major
+//     O^T [r, NR]       += V^T P^T        A = the SAME shared-memory tile read MN-major (r / 128 accumulators)   B = P^T
+// which needs (r / 128 + 1) NR columns, lets one staged tile serve both products, and lets a decode step (16 heads of one token) run at
+// N = 16 instead of on a mostly empty row tile.
+//   warp 0       TMA: Q once; per tile the 64-column chunks of two 64-key boxes, each chunk on a barrier of its own, so that scores start
+//                with the first and a chunk is refilled as soon as the output products that read it are done
+//   warp 1       MMA issuer (one thread)
+//   warps 2..9   softmax: thread = one key x half the rows. Maxima over keys are maxima over lanes: a transposing butterfly leaves every
+//                lane with one row's maximum. The reference maximum of a row only moves when it grew by more than 2^8 (the sums are scaled by it
+//                consistently, so this is exact), the output accumulators are then rescaled in TMEM; sums stay per thread until the end.
+//                P^T goes to shared memory as the B operand; where Q and the key tile fill it (r = 512) it takes the place of the rotated
+//                chunk, which the scores have consumed.
+// What bounds it: the tensor pipe at N = 64 (68 instructions per tile against one softmax pass over 8192 scores) behind the exposed softmax
+// of a tile and, for decode steps, the 147 KB of a key tile per SM. RATE
+#include <cuda.h>
+
+#include "ptx.cuh"
+#include "seq_common.cuh"
+
+namespace omc {
+
+constexpr int kKT = 128;                    // keys per tile
+constexpr int kChunkBytes = kKT * 128;      // 64 columns of a key tile
+constexpr int kLsThreads = 320, kLsSoftmax = 256, kLsMaxChunks = 10, kLsMaxRows = 64;
+constexpr uint32_t kLsMaxTries = 1u << 22;  // tries of a wait (a few microseconds of work each) before it gives up
+
+__device__ unsigned int g_latent_wait_failures;   // waits that ran out: the launch's outputs are not valid
+
+struct LatSmArgs {
+  const int32_t* bt;
+  const int32_t* items;   // as LatMmaArgs of latent_attention.cu
+  const float* sink;
+  void* out;
+  float* ws_o;
+  float* ws_ml;
+  const float* gate;
+  long long ldg;
+  int window, max_pages, page_size, H, r, D, nc;   // nc: 64-column chunks of a row
+  int p_offset;                                    // of P^T, in bytes behind Q
+  int tmem_cols;
+  float scale_log2;
+};
+
+struct LatSmShared {
+  uint64_t q_full, s_full, p_ready, full[kLsMaxChunks], o_done[4];
+  uint32_t tmem, dead, rescale[2];
+  int lim[kLsMaxRows], low[kLsMaxRows];                     // last and first key a row sees
+  float mref[kLsMaxRows], fac[kLsMaxRows], part[4][kLsMaxRows];   // reference maxima, rescaling factors, the lane quarters' maxima / sums
+};
+
+__device__ __forceinline__ float ls_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// A wait that ends in any case: after kLsMaxTries, or once another wait of the CTA has given up, it returns and the CTA runs on to its end
+// through the same sequence of barriers.
+__device__ __forceinline__ void ls_wait(LatSmShared* sh, uint64_t* bar, uint32_t parity) {
+  for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i) {
+    if (i >= kLsMaxTries) {
+      if (atomicExch(&sh->dead, 1u) == 0u) atomicAdd(&g_latent_wait_failures, 1u);
+    }
+    if (*reinterpret_cast<volatile uint32_t*>(&sh->dead)) return;
+  }
+}
+__device__ __forceinline__ void ls_softmax_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLsSoftmax) : "memory"); }
+
+// v[c]: this lane's value of column c. Returns the reduction over the 32 lanes of column lane / (32 / NC) (v is overwritten).
+template <int NC, typename Op>
+__device__ __forceinline__ float ls_columns(float (&v)[NC], int lane, Op op) {
+  int off = 16;
+#pragma unroll
+  for (int cur = NC; cur > 1; cur >>= 1, off >>= 1) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int i = 0; i < cur / 2; ++i) {
+      const float other = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + cur / 2], off);
+      v[i] = op(up ? v[i + cur / 2] : v[i], other);
+    }
+  }
+#pragma unroll
+  for (; off > 0; off >>= 1) v[0] = op(v[0], __shfl_xor_sync(0xffffffffu, v[0], off));
+  return v[0];
+}
+
+template <int NC>
+__device__ __forceinline__ void ls_tmem_ld(uint32_t addr, uint32_t* v) {
+  if constexpr (NC == 32) tmem_ld32(addr, v);
+  else if constexpr (NC == 16) tmem_ld16(addr, v);
+  else
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(addr)
+                 : "memory");
+}
+template <int NC>
+__device__ __forceinline__ void ls_tmem_st(uint32_t addr, const uint32_t* v) {
+  if constexpr (NC == 32) tmem_st32(addr, v);
+  else if constexpr (NC == 16) tmem_st16(addr, v);
+  else tmem_st8(addr, v);
+}
+
+template <int NR, typename TO>
+__global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
+                                                                          LatSmArgs a) {
+  constexpr int NC = NR / 2;                 // rows per softmax thread
+  constexpr int QCHUNK = NR * 128;           // bytes of a 64-column chunk of Q
+  extern __shared__ uint8_t ls_raw[];
+  __shared__ LatSmShared shared;
+  LatSmShared* sh = &shared;
+  uint8_t* base = ls_raw + ((1024u - (smem_u32(ls_raw) & 1023u)) & 1023u);
+  uint8_t* qs = base;                        // [nc][NR][128 B]
+  uint8_t* ks = base + a.nc * QCHUNK;        // [nc][128][128 B]
+  uint8_t* ps = base + a.p_offset;           // P^T
+  const int32_t* it = a.items + blockIdx.x * 8;
+  const int first_row = it[0], n_tok = it[1], slot = it[2], first_pos = it[3], kb = it[4], part = it[6];
+  const int k_end = min(it[5], first_pos + n_tok), n_rows = n_tok * a.H;
+  const int k0 = kb & ~63;                   // boxes of 64 keys start where pages may
+  const int n_tiles = k_end > kb ? (k_end - k0 + kKT - 1) / kKT : 0;
+  const int nm = a.r >> 7;                   // 128-dimension tiles of the output
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (tid < kLsMaxRows) {
+    const int row_lim = tid < n_rows ? first_pos + tid / a.H : -1;
+    sh->lim[tid] = min(row_lim, k_end - 1);
+    sh->low[tid] = max(row_lim - a.window + 1, kb);
+    sh->mref[tid] = -INFINITY;
+  }
+  if (tid == 0) {
+    mbar_init(&sh->q_full, 1);
+    mbar_init(&sh->s_full, 1);
+    mbar_init(&sh->p_ready, kLsSoftmax / 32);
+    for (int c = 0; c < kLsMaxChunks; ++c) mbar_init(&sh->full[c], 1);
+    for (int m = 0; m < 4; ++m) mbar_init(&sh->o_done[m], 1);
+    sh->dead = 0u;
+    sh->rescale[0] = sh->rescale[1] = 0u;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    __syncwarp();
+    tmem_alloc<1>(&sh->tmem, a.tmem_cols);
+    tmem_relinquish<1>();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sh->tmem, tmem_s = tmem + nm * NR;
+
+  if (warp == 0) {
+    if (elect_one() && n_tiles > 0) {
+      mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
+      for (int c = 0; c < a.nc; ++c) tma_load_2d(qs + c * QCHUNK, &tm_q, &sh->q_full, c * 64, first_row * a.H, kEvictNormal);
+      const int32_t* bt = a.bt + (long long)slot * a.max_pages;
+      for (int t = 0; t < n_tiles; ++t) {
+        const int j0 = k0 + t * kKT, boxes = j0 + 64 < k_end ? 2 : 1;
+        int rows[2];
+        for (int b = 0; b < boxes; ++b) {
+          const int j = j0 + 64 * b;
+          rows[b] = bt[j / a.page_size] * a.page_size + j % a.page_size;
+        }
+        for (int c = 0; c < a.nc; ++c) {
+          if (t > 0) ls_wait(sh, &sh->o_done[min(c >> 1, nm - 1)], (t - 1) & 1);
+          mbar_arrive_expect_tx(&sh->full[c], boxes * (kChunkBytes / 2));
+          for (int b = 0; b < boxes; ++b) tma_load_2d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[c], c * 64, rows[b], kEvictNormal);
+        }
+      }
+      ls_wait(sh, &sh->q_full, 0);           // nothing is on its way any more when this thread leaves
+      for (int c = 0; c < a.nc; ++c) ls_wait(sh, &sh->full[c], (n_tiles - 1) & 1);
+    }
+  } else if (warp == 1) {
+    if (elect_one() && n_tiles > 0) {
+      constexpr uint32_t idesc_s = make_idesc_bf16_major(128, NR, 0, 0);
+      constexpr uint32_t idesc_o = make_idesc_bf16_major(128, NR, 1, NR == 64 ? 1 : 0);
+      const uint32_t q_addr = smem_u32(qs), k_addr = smem_u32(ks), p_addr = smem_u32(ps);
+      ls_wait(sh, &sh->q_full, 0);
+      for (int t = 0; t < n_tiles; ++t) {
+        for (int c = 0; c < a.nc; ++c) {
+          ls_wait(sh, &sh->full[c], t & 1);
+          tc_fence_after();
+          const uint64_t dk = make_sw128_kmajor_desc(k_addr + c * kChunkBytes), dq = make_sw128_kmajor_desc(q_addr + c * QCHUNK);
+          const int steps = min(4, (a.D - c * 64 + 15) >> 4);
+          for (int k = 0; k < steps; ++k) umma_bf16<1>(tmem_s, dk + 2 * k, dq + 2 * k, idesc_s, (c | k) != 0 ? 1u : 0u);
+        }
+        umma_commit(&sh->s_full);            // also: the output products of the tile before are done
+        ls_wait(sh, &sh->p_ready, t & 1);
+        tc_fence_after();
+        for (int m = 0; m < nm; ++m) {
+          const uint64_t dv = make_sw128_mnmajor_desc(k_addr + 2 * m * kChunkBytes, kChunkBytes, 1024);
+#pragma unroll
+          for (int k = 0; k < kKT / 16; ++k) {
+            const uint64_t dp = NR == 64 ? make_sw128_mnmajor_desc(p_addr + k * 2048, 1024, 1024)
+                                         : make_sw128_kmajor_desc(p_addr + (k >> 2) * QCHUNK) + 2 * (k & 3);
+            umma_bf16<1>(tmem + m * NR, dv + (uint64_t)(k * 128), dp, idesc_o, (t | k) != 0 ? 1u : 0u);
+          }
+          umma_commit(&sh->o_done[m]);
+        }
+      }
+    }
+  } else {
+    const int quarter = warp & 3, half = (warp - 2) >> 2,   // TMEM lanes go by warp % 4
+               key_lane = quarter * 32 + lane, c0 = half * NC;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    const int stid = tid - 64;
+    float l[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) l[c] = 0.f;
+    for (int t = 0; t < n_tiles; ++t) {
+      const int j0 = k0 + t * kKT, key = j0 + key_lane;
+      ls_wait(sh, &sh->s_full, t & 1);
+      tc_fence_after();
+      // a tile that every row of the item sees in full needs no mask
+      const bool whole = j0 >= kb && j0 + kKT <= k_end && j0 + kKT - 1 <= first_pos && (long long)j0 >= (long long)first_pos + n_tok - a.window;
+      float s[NC];
+      auto load_scores = [&] {               // twice per tile: the maxima destroy them, and holding both copies would cost 32 registers
+        uint32_t v[NC];
+        ls_tmem_ld<NC>(tmem_s + lanes + c0, v);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          s[c] = whole || (key <= sh->lim[c0 + c] && key >= sh->low[c0 + c]) ? __uint_as_float(v[c]) * a.scale_log2 : -INFINITY;
+      };
+      load_scores();
+      // rows of the tile that are no keys of this item hold whatever the cache holds there: as values they must not meet a product
+      if (!whole && half == 0 && (key < kb || key >= k_end)) {
+        for (int c = 0; c < a.r >> 6; ++c)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(ks + c * kChunkBytes + key_lane * 128 + i * 16) = make_uint4(0, 0, 0, 0);
+      }
+      const float mx = ls_columns<NC>(s, lane, [](float x, float y) { return fmaxf(x, y); });
+      if (lane % (32 / NC) == 0) sh->part[quarter][c0 + lane / (32 / NC)] = mx;
+      ls_softmax_sync();
+      if (stid < NR) {
+        const float now = fmaxf(fmaxf(sh->part[0][stid], sh->part[1][stid]), fmaxf(sh->part[2][stid], sh->part[3][stid]));
+        const float old = sh->mref[stid];
+        if (now > old + 8.f) {               // also the first finite maximum of a row
+          sh->fac[stid] = ls_exp2(old - now);
+          sh->mref[stid] = now;
+          sh->rescale[t & 1] = 1u;
+        } else {
+          sh->fac[stid] = 1.f;
+        }
+      }
+      if (stid == kLsSoftmax - 1) sh->rescale[(t + 1) & 1] = 0u;
+      ls_softmax_sync();
+      if (sh->rescale[t & 1] && t > 0) {
+        float f[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) f[c] = sh->fac[c0 + c], l[c] *= f[c];
+        for (int m = 0; m < nm; ++m) {
+          uint32_t v[NC];
+          ls_tmem_ld<NC>(tmem + lanes + m * NR + c0, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < NC; ++c) v[c] = __float_as_uint(__uint_as_float(v[c]) * f[c]);
+          ls_tmem_st<NC>(tmem + lanes + m * NR + c0, v);
+        }
+        tmem_st_wait();
+      }
+      load_scores();
+      uint32_t p[NC / 2];
+#pragma unroll
+      for (int c = 0; c < NC; c += 2) {
+        const float m0 = sh->mref[c0 + c], m1 = sh->mref[c0 + c + 1];
+        p[c / 2] = pack_bf16(ls_exp2(s[c] - (m0 == -INFINITY ? 0.f : m0)), ls_exp2(s[c + 1] - (m1 == -INFINITY ? 0.f : m1)));
+        const float2 e = unpack_bf16(p[c / 2]);   // the denominator sums the ROUNDED probabilities, the ones the numerator uses
+        l[c] += e.x;
+        l[c + 1] += e.y;
+      }
+      if constexpr (NR == 64) {              // [key][64 rows]: MN-major
+        uint8_t* dst = ps + key_lane * 128;
+#pragma unroll
+        for (int i = 0; i < NC / 8; ++i)
+          *reinterpret_cast<uint4*>(dst + (((half * (NC / 8) + i) ^ (key_lane & 7)) << 4)) = make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
+      } else {                               // [row][64 keys] twice: K-major
+        uint8_t* dst = ps + (key_lane >> 6) * QCHUNK + (key_lane & 7) * 2;
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const int row = c0 + c;
+          *reinterpret_cast<uint16_t*>(dst + row * 128 + ((((key_lane & 63) >> 3) ^ (row & 7)) << 4)) = (uint16_t)(p[c / 2] >> (16 * (c & 1)));
+        }
+      }
+      fence_proxy_async();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sh->p_ready);
+    }
+    // ---- the sums over all keys, then the output
+    const float mine = ls_columns<NC>(l, lane, [](float x, float y) { return x + y; });
+    if (lane % (32 / NC) == 0) sh->part[quarter][c0 + lane / (32 / NC)] = mine;
+    ls_softmax_sync();
+    if (stid < NR) {
+      const float sum = (sh->part[0][stid] + sh->part[1][stid]) + (sh->part[2][stid] + sh->part[3][stid]), m = sh->mref[stid];
+      if (part >= 0) {
+        float* ml = a.ws_ml + ((long long)part * kLsMaxRows + stid) * 2;
+        ml[0] = m, ml[1] = sum;
+        sh->fac[stid] = 1.f;
+      } else if (stid < n_rows) {
+        const int h = stid % a.H;
+        float f = 1.f / (a.sink != nullptr ? sum + exp2f(a.sink[h] * 1.4426950408889634f - m) : sum);
+        if (a.gate != nullptr) f *= 1.f / (1.f + expf(-a.gate[(long long)(first_row + stid / a.H) * a.ldg + h]));
+        sh->fac[stid] = f;
+      }
+    }
+    ls_softmax_sync();
+    if (n_tiles > 0) ls_wait(sh, &sh->o_done[nm - 1], (n_tiles - 1) & 1);
+    tc_fence_after();
+    for (int m = 0; m < nm; ++m) {
+      uint32_t v[NC];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) v[c] = 0u;
+      if (n_tiles > 0) {
+        ls_tmem_ld<NC>(tmem + lanes + m * NR + c0, v);
+        tmem_ld_wait();
+      }
+      const int dim = m * 128 + key_lane;
+      if (part >= 0) {
+        float* dst = a.ws_o + ((long long)part * kLsMaxRows + c0) * a.r + dim;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (c0 + c < n_rows) dst[(long long)c * a.r] = __uint_as_float(v[c]);
+      } else {
+        TO* dst = static_cast<TO*>(a.out) + ((long long)first_row * a.H + c0) * a.r + dim;
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (c0 + c < n_rows) stf(dst + (long long)c * a.r, __uint_as_float(v[c]) * sh->fac[c0 + c]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc<1>(tmem, a.tmem_cols);
+}
+
+typedef CUresult (*LsEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static LsEncodeFn ls_encode_fn() {
+  static LsEncodeFn fn = nullptr;
+  if (fn == nullptr) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
+    fn = reinterpret_cast<LsEncodeFn>(p);
+  }
+  return fn;
+}
+// [rows, D] bf16 rows without gaps, boxes of box_rows x 64 columns
+static int ls_tensor_map(CUtensorMap* tm, const void* p, unsigned long long rows, int D, int box_rows) {
+  LsEncodeFn enc = ls_encode_fn();
+  if (enc == nullptr) return set_error(OMC_ERR_DRIVER, "cuTensorMapEncodeTiled entry point unavailable");
+  cuuint64_t dim[2] = {(cuuint64_t)D, rows}, stride[1] = {(cuuint64_t)D * 2};
+  cuuint32_t box[2] = {64u, (cuuint32_t)box_rows}, one[2] = {1u, 1u};
+  if (enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return set_error(OMC_ERR_DRIVER, "cuTensorMapEncodeTiled failed");
+  return OMC_OK;
+}
+
+constexpr int kLsSmemMax = 227 * 1024;
+static int ls_smem(int nr, int r, int D, int* p_offset) {
+  const int nc = (D + 63) / 64, q = nc * nr * 128, k = nc * kChunkBytes, p = kKT * nr * 2;
+  const int slack = 1024 + (int)sizeof(LatSmShared) + 256;
+  if (q + k + p + slack <= kLsSmemMax) {
+    *p_offset = q + k;
+    return q + k + p + 1024;
+  }
+  if (D > r && q + k + slack <= kLsSmemMax) {   // P^T in the place of the last chunk, which only the scores read
+    *p_offset = q + k - kChunkBytes;
+    return q + k + 1024;
+  }
+  return 0;
+}
+
+// Shapes this kernel takes. max_rows: the most rows an item has.
+bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool) {
+  int at;
+  return max_rows <= kLsMaxRows && r % 128 == 0 && r <= 512 && dr <= 64 && dr % 16 == 0 && page_size % 64 == 0 &&
+         reinterpret_cast<uintptr_t>(q) % 16 == 0 && reinterpret_cast<uintptr_t>(pool) % 16 == 0 && ls_smem(max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64), r, r + dr, &at) > 0;
+}
+
+template <int NR, typename TO>
+static int ls_launch(const CUtensorMap& tq, const CUtensorMap& tk, const LatSmArgs& a, int n_items, int smem, cudaStream_t st) {
+  static bool done[kMaxDevices] = {};
+  const int dev = cur_device();
+  if (!done[dev]) {
+    const cudaError_t e = cudaFuncSetAttribute(latent_attn_sm100_kernel<NR, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLsSmemMax - (int)sizeof(LatSmShared) - 128);
+    if (e != cudaSuccess) return set_error(OMC_ERR_CUDA, cudaGetErrorString(e));
+    done[dev] = true;
+  }
+  latent_attn_sm100_kernel<NR, TO><<<n_items, kLsThreads, smem, st>>>(tq, tk, a);
+  return check_launch("omc_latent_attn_mma");
+}
+
+int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
+                 int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
+                 float* ws_ml, cudaStream_t st) {
+  const int D = r + dr, nr = max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64);
+  LatSmArgs a{bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D, (D + 63) / 64, 0, 0, scale * 1.4426950408889634f};
+  const int smem = ls_smem(nr, r, D, &a.p_offset);
+  const int cols = (r / 128 + 1) * nr;
+  a.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
+  CUtensorMap tq, tk;
+  int rc = ls_tensor_map(&tq, q, q_rows, D, nr);
+  // how many pages the pool has is not known here; rows are only ever addressed through the block table
+  if (rc == OMC_OK) rc = ls_tensor_map(&tk, pool, 1ull << 31, D, 64);
+  if (rc != OMC_OK) return rc;
+  const bool b = out_dt == OMC_DT_BF16;
+  if (nr == 16) return b ? ls_launch<16, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<16, float>(tq, tk, a, n_items, smem, st);
+  if (nr == 32) return b ? ls_launch<32, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<32, float>(tq, tk, a, n_items, smem, st);
+  return b ? ls_launch<64, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<64, float>(tq, tk, a, n_items, smem, st);
+}
+
+}  // namespace omc
+
+extern "C" int omc_latent_wait_failures(unsigned int* count) {
+  if (count == nullptr) return omc::set_error(OMC_ERR_ARG, "omc_latent_wait_failures: bad argument");
+  const cudaError_t e = cudaMemcpyFromSymbol(count, omc::g_latent_wait_failures, sizeof(unsigned int));
+  return e == cudaSuccess ? OMC_OK : omc::set_error(OMC_ERR_CUDA, cudaGetErrorString(e));
+}

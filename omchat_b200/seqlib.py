@@ -61,6 +61,8 @@ SIGNATURES = {
     "omc_moe_plan_scatter_small": (_I, [_P, _I, _I, _I, _P, _P, _P, _I, _L, _I, _I, _P, _I, _P, _P, _L, _P, _P]),
     "omc_rotary_q": (_I, [_P, _I, _L, _I, _I, _I, _I, _P, _I, _P, _P, _I, _I, _P]),
     "omc_latent_attn": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _L, _F, _P, _P]),
+    "omc_latent_attn_mma_rows": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
+    "omc_latent_wait_failures": (_I, [_P]),
     "omc_latent_attn_mma": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_latent_decode_items": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
     "omc_router_topk": (_I, [_P, _L, _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P, _P]),
@@ -298,6 +300,7 @@ class LatentAttnPlan:
                     items.append((fr, nt, slot, p0 + int(starts[i]), lo + j * span, lo + min(k, (j + 1) * span), part, 0))
                     part += 1
         self.n_items, self.n_merges, self.n_parts = len(items), len(merges), part
+        self.max_rows = max((it[1] for it in items), default=1) * H   # (token, head) pairs of the largest item
         flat = torch.tensor(items, dtype=torch.int32).view(-1)
         flat = torch.cat([flat, torch.tensor(merges, dtype=torch.int32).view(-1)]) if merges else flat
         buf = flat.pin_memory().to(device, non_blocking=True)
@@ -313,7 +316,7 @@ class DecodeAttnPlan:
         self.B, self.H, self.parts, self.window = B, H, parts, window
         self.items = torch.zeros(B * parts * 8, device=device, dtype=torch.int32)
         self.merges = torch.zeros(B * 4, device=device, dtype=torch.int32) if parts > 1 else None
-        self.n_items = B * parts
+        self.n_items, self.max_rows = B * parts, H
         self.n_merges = B if parts > 1 else 0
         self.n_parts = B * parts if parts > 1 else 0
 
@@ -351,9 +354,9 @@ def latent_attn_mma(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, blo
             ws = torch.empty(need, device=qcat.device, dtype=torch.float32)
             _mma_ws[key] = ws
         ws_o, ws_ml = ws[:plan.n_parts * MMA_ROWS * r], ws[plan.n_parts * MMA_ROWS * r:]
-    rc = load().omc_latent_attn_mma(_ptr(qcat), T, H, r, dr, _ptr(pool), _ptr(block_table), block_table.shape[1], page_size,
-                                    _ptr(plan.items), plan.n_items, _ptr(plan.merges), plan.n_merges, _ptr(sink), window, _ptr(gate),
-                                    gate.stride(0) if gate is not None else 0, scale, _ptr(out), _dt(out), _ptr(ws_o), _ptr(ws_ml), _stream())
+    rc = load().omc_latent_attn_mma_rows(_ptr(qcat), T, H, r, dr, _ptr(pool), _ptr(block_table), block_table.shape[1], page_size,
+                                         _ptr(plan.items), plan.n_items, plan.max_rows, _ptr(plan.merges), plan.n_merges, _ptr(sink), window, _ptr(gate),
+                                         gate.stride(0) if gate is not None else 0, scale, _ptr(out), _dt(out), _ptr(ws_o), _ptr(ws_ml), _stream())
     _check(rc, "omc_latent_attn_mma")
     if plan.n_merges:
         _core.add_launches(1)

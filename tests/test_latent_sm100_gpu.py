@@ -1,0 +1,85 @@
+"""The tcgen05 latent attention (omc_latent_attn_mma_rows where r is a multiple of 128 and pages of 64 rows) against float64: tile edges, portions
+behind a cached prefix, windows that start inside a box, decode steps in key ranges, sinks, gates, rows of the cache that hold no key."""
+import math
+
+import pytest
+import torch
+
+from omchat_b200 import seqlib
+
+pytestmark = pytest.mark.gpu
+F64 = torch.float64
+
+
+def _reference(q, pool_rows, portions, r, scale, window, sink, gate):
+    """out [T, H, r] and the weighted sums of |latent| that bound the effect of rounded probabilities."""
+    out, mag = torch.zeros(*q.shape[:2], r, dtype=F64), torch.zeros(*q.shape[:2], r, dtype=F64)
+    for row, n, slot, first in portions:
+        keys = pool_rows[slot][:first + n].to(F64)
+        s = torch.einsum("thd,jd->htj", q[row:row + n].to(F64), keys) * scale
+        i, j = first + torch.arange(n)[:, None], torch.arange(first + n)[None, :]
+        s = s.masked_fill((j > i) | (i - j >= window), -math.inf)
+        if sink is not None:
+            s = torch.cat([s, sink.to(F64)[:, None, None].expand(-1, n, 1)], -1)
+        p = torch.softmax(s, -1)[..., :first + n]
+        g = torch.sigmoid(gate[row:row + n].to(F64))[..., None] if gate is not None else 1.0
+        out[row:row + n] = torch.einsum("htj,jr->thr", p, keys[:, :r]) * g
+        mag[row:row + n] = torch.einsum("htj,jr->thr", p, keys[:, :r].abs()) * g
+    return out, mag
+
+
+@pytest.mark.parametrize("H,r,dr,page,window,portions", [
+    (16, 512, 64, 64, 1 << 30, [(5, 0), (4, 123), (9, 124), (1, 127), (1, 128), (133, 60)]),
+    (16, 512, 64, 128, 100, [(70, 0), (64, 300), (1, 511), (3, 190)]),
+    (8, 256, 32, 64, 1 << 30, [(129, 0), (1, 640), (17, 63)]),
+    (32, 512, 48, 64, 64, [(40, 50), (1, 0), (2, 2000)]),
+    (5, 128, 16, 192, 1 << 30, [(13, 0), (30, 100)]),
+    (3, 384, 0, 64, 33, [(50, 0), (1, 200)]),
+    (64, 512, 64, 64, 1 << 30, [(3, 254)]),
+])
+@pytest.mark.parametrize("opt", ["plain", "sink_gate"])
+def test_against_float64(H, r, dr, page, window, portions, opt):
+    gen = torch.Generator().manual_seed(H * r + dr)
+    D, row, slots, plist = r + dr, 0, [], []
+    for s, (n, first) in enumerate(portions):
+        plist.append((row, n, s, first))
+        row += n
+        slots.append(-(-(first + n) // page))
+    T, pages = row, sum(slots) + 1
+    pool = torch.full((pages, page, D), float("nan"), dtype=torch.bfloat16)      # rows that hold no key must not matter
+    order, table, rows = (torch.randperm(pages - 1, generator=gen) + 1).tolist(), torch.zeros(len(slots), max(slots), dtype=torch.int32), []
+    for s, ((_, n, _, first), k) in enumerate(zip(plist, slots)):
+        mine, order = order[:k], order[k:]
+        table[s, :k] = torch.tensor(mine, dtype=torch.int32)
+        lat = torch.randn(first + n, D, generator=gen).to(torch.bfloat16)
+        rows.append(lat)
+        for i in range(k):
+            part = lat[i * page:(i + 1) * page]
+            pool[mine[i], :part.shape[0]] = part
+    q = (torch.randn(T, H, D, generator=gen) * 2).to(torch.bfloat16)
+    scale = 3.0 * D ** -0.5                                                      # scores of some tens: references move, sums are rescaled
+    sink = torch.randn(H, generator=gen) * 3 if opt == "sink_gate" else None
+    gate = torch.randn(T, H, generator=gen) if opt == "sink_gate" else None
+    want, mag = _reference(q, rows, plist, r, scale, window, sink, gate)
+    dev = lambda t: t.cuda() if t is not None else None  # noqa: E731
+    pos = torch.cat([torch.arange(first, first + n) for _, n, _, first in plist]).to(torch.int32).cuda()
+    slot = torch.cat([torch.full((n,), s) for _, n, s, _ in plist]).to(torch.int32).cuda()
+    plans = [seqlib.LatentAttnPlan(plist, H, "cuda", window=window), seqlib.LatentAttnPlan(plist, H, "cuda", target_ctas=2, window=window)]
+    for parts in (1, 3):                                                         # every row on its own, as a decode step addresses them
+        plan = seqlib.DecodeAttnPlan(T, H, parts, "cuda", window=window)
+        plan.fill(pos, slot)
+        plans.append(plan)
+    for plan in plans:
+        for dt in (torch.float32, torch.bfloat16):
+            out = torch.full((T, H, r), float("nan"), dtype=dt, device="cuda")
+            seqlib.latent_attn_mma(q.cuda(), r, dr, pool.cuda(), table.cuda(), page, plan, dev(sink), scale, out, window=window, gate=dev(gate))
+            err = (out.double().cpu() - want).abs()
+            # a probability is rounded to 8 bits (its sum too: 2^-9 each), scores and sums in fp32 over D terms; then the output's own rounding
+            bound = mag * (2.0 ** -8 + 1e-4) + 1e-6 + (want.abs() * 2.0 ** -8 if dt == torch.bfloat16 else 0.0)
+            assert (err <= bound).all(), (plan.n_items, plan.max_rows, dt, float((err - bound).max()))
+
+
+def test_no_wait_ran_out():
+    import ctypes
+    n = ctypes.c_uint(7)
+    assert seqlib.load().omc_latent_wait_failures(ctypes.byref(n)) == 0 and n.value == 0
