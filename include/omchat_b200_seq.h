@@ -99,13 +99,15 @@ int omc_latent_attn_mma(const void* qcat, int T, int H, int r, int dr, const voi
                         int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o, float* ws_ml, void* stream);
 
 /* The same with the most rows (n_tok * H) any item has, which may be fewer than 64 (a decode step: H). On tcgen05 with both products
- * transposed where r is a multiple of 128, dr <= 64 and page_size a multiple of 64; that kernel's waits end by themselves, and
- * omc_latent_wait_failures counts those that ran out (0 on a sound device: after a failure the launch's outputs are not valid). */
+ * transposed where r is a multiple of 128, dr <= 64 and page_size a multiple of 64. */
 int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, int dr, const void* pool, const int32_t* block_table, int max_pages,
                              int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
                              const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,
                              float* ws_o, float* ws_ml, void* stream);
-int omc_latent_wait_failures(unsigned int* count);
+
+/* The waits of the tcgen05 kernels end by themselves; this counts those of the current device that ran out since the library was loaded (0
+ * on a sound device; the outputs of a launch that had one are not valid). Synchronises with the device. */
+int omc_step_wait_failures(unsigned int* count);
 
 /* The work list of a decode-only step, written on the device from pos / slot (one row per request, `parts` <= 64 key ranges each):
  * items int32 [B * parts][8], merges int32 [B][4] (untouched when parts == 1). Lets a CUDA graph replay the step as contexts grow. */

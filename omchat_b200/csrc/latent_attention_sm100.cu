@@ -8,8 +8,9 @@
 //     O^T [r, NR]       += V^T P^T        A = the SAME shared-memory tile read MN-major (r / 128 accumulators)   B = P^T
 // which needs (r / 128 + 1) NR columns, lets one staged tile serve both products, and lets a decode step (16 heads of one token) run at
 // N = 16 instead of on a mostly empty row tile.
-//   warp 0       TMA: Q once; per tile the 64-column chunks of two 64-key boxes, each chunk on a barrier of its own, so that scores start
-//                with the first and a chunk is refilled as soon as the output products that read it are done
+//   warp 0       TMA: Q once; per tile the 64-column chunks of two 64-key boxes. The two chunks (the last time with the rotated one) that hold
+//                128 value dimensions share a barrier: scores start with the first pair, and a pair is refilled as soon as the output
+//                product that reads it is done
 //   warp 1       MMA issuer (one thread)
 //   warps 2..9   softmax: thread = one key x half the rows. Maxima over keys are maxima over lanes: a transposing butterfly leaves every
 //                lane with one row's maximum. The reference maximum of a row only moves when it grew by more than 2^8 (the sums are scaled by it
@@ -18,19 +19,15 @@
 //                chunk, which the scores have consumed.
 // What bounds it: the tensor pipe at N = 64 (68 instructions per tile against one softmax pass over 8192 scores) behind the exposed softmax
 // of a tile and, for decode steps, the 147 KB of a key tile per SM. RATE
-#include <cuda.h>
-
-#include "ptx.cuh"
-#include "seq_common.cuh"
+#include "sm100_step.cuh"
 
 namespace omc {
 
 constexpr int kKT = 128;                    // keys per tile
 constexpr int kChunkBytes = kKT * 128;      // 64 columns of a key tile
-constexpr int kLsThreads = 320, kLsSoftmax = 256, kLsMaxChunks = 10, kLsMaxRows = 64;
-constexpr uint32_t kLsMaxTries = 1u << 22;  // tries of a wait (a few microseconds of work each) before it gives up
+constexpr int kLsThreads = 320, kLsSoftmax = 256, kLsMaxRows = 64;
 
-__device__ unsigned int g_latent_wait_failures;   // waits that ran out: the launch's outputs are not valid
+static __device__ unsigned int g_latent_failures;   // waits that ran out
 
 struct LatSmArgs {
   const int32_t* bt;
@@ -48,10 +45,11 @@ struct LatSmArgs {
 };
 
 struct LatSmShared {
-  uint64_t q_full, s_full, p_ready, full[kLsMaxChunks], o_done[4];
+  uint64_t q_full, s_full, p_ready, full[4], o_done[4];
   uint32_t tmem, dead, rescale[2];
-  int lim[kLsMaxRows], low[kLsMaxRows];                     // last and first key a row sees
-  float mref[kLsMaxRows], fac[kLsMaxRows], part[4][kLsMaxRows];   // reference maxima, rescaling factors, the lane quarters' maxima / sums
+  alignas(16) float mref[kLsMaxRows];
+  alignas(16) float fac[kLsMaxRows];
+  float part[4][kLsMaxRows];   // reference maxima, rescaling factors, the lane quarters' maxima / sums
 };
 
 __device__ __forceinline__ float ls_exp2(float x) {
@@ -59,16 +57,7 @@ __device__ __forceinline__ float ls_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// A wait that ends in any case: after kLsMaxTries, or once another wait of the CTA has given up, it returns and the CTA runs on to its end
-// through the same sequence of barriers.
-__device__ __forceinline__ void ls_wait(LatSmShared* sh, uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i) {
-    if (i >= kLsMaxTries) {
-      if (atomicExch(&sh->dead, 1u) == 0u) atomicAdd(&g_latent_wait_failures, 1u);
-    }
-    if (*reinterpret_cast<volatile uint32_t*>(&sh->dead)) return;
-  }
-}
+__device__ __forceinline__ void ls_wait(LatSmShared* sh, uint64_t* bar, uint32_t parity) { wait_bounded(bar, parity, &sh->dead, &g_latent_failures); }
 __device__ __forceinline__ void ls_softmax_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLsSoftmax) : "memory"); }
 
 // v[c]: this lane's value of column c. Returns the reduction over the 32 lanes of column lane / (32 / NC) (v is overwritten).
@@ -118,6 +107,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   uint8_t* qs = base;                        // [nc][NR][128 B]
   uint8_t* ks = base + a.nc * QCHUNK;        // [nc][128][128 B]
   uint8_t* ps = base + a.p_offset;           // P^T
+  if (threadIdx.x == 32) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_kv);
+  }
   const int32_t* it = a.items + blockIdx.x * 8;
   const int first_row = it[0], n_tok = it[1], slot = it[2], first_pos = it[3], kb = it[4], part = it[6];
   const int k_end = min(it[5], first_pos + n_tok), n_rows = n_tok * a.H;
@@ -126,21 +119,33 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   const int nm = a.r >> 7;                   // 128-dimension tiles of the output
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  if (tid < kLsMaxRows) {
-    const int row_lim = tid < n_rows ? first_pos + tid / a.H : -1;
-    sh->lim[tid] = min(row_lim, k_end - 1);
-    sh->low[tid] = max(row_lim - a.window + 1, kb);
-    sh->mref[tid] = -INFINITY;
-  }
+  const int32_t* bt = a.bt + (long long)slot * a.max_pages;
+  auto load_pair = [&](int t, int g) {       // chunks of barrier g of tile t
+    const int j0 = k0 + t * kKT, boxes = j0 + 64 < k_end ? 2 : 1, c1 = g == nm - 1 ? a.nc : 2 * g + 2;
+    mbar_arrive_expect_tx(&sh->full[g], (c1 - 2 * g) * boxes * (kChunkBytes / 2));
+    for (int b = 0; b < boxes; ++b) {
+      const int j = j0 + 64 * b, row = bt[j / a.page_size] * a.page_size + j % a.page_size;
+      for (int c = 2 * g; c < c1; ++c) tma_load_3d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[g], c * 64, row, 0);
+    }
+  };
+  if (tid >= 64 && tid < 64 + kLsMaxRows) sh->mref[tid - 64] = -INFINITY;
   if (tid == 0) {
     mbar_init(&sh->q_full, 1);
     mbar_init(&sh->s_full, 1);
     mbar_init(&sh->p_ready, kLsSoftmax / 32);
-    for (int c = 0; c < kLsMaxChunks; ++c) mbar_init(&sh->full[c], 1);
-    for (int m = 0; m < 4; ++m) mbar_init(&sh->o_done[m], 1);
+    for (int m = 0; m < 4; ++m) {
+      mbar_init(&sh->full[m], 1);
+      mbar_init(&sh->o_done[m], 1);
+    }
     sh->dead = 0u;
     sh->rescale[0] = sh->rescale[1] = 0u;
     fence_barrier_init();
+    fence_proxy_async();
+    if (n_tiles > 0) {                       // on their way while tensor memory is allocated
+      mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
+      for (int c = 0; c < a.nc; ++c) tma_load_3d(qs + c * QCHUNK, &tm_q, &sh->q_full, c * 64, first_row * a.H, 0);
+      for (int g = 0; g < nm; ++g) load_pair(0, g);
+    }
   }
   if (warp == 1) {
     __syncwarp();
@@ -153,51 +158,47 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   const uint32_t tmem = sh->tmem, tmem_s = tmem + nm * NR;
 
   if (warp == 0) {
-    if (elect_one() && n_tiles > 0) {
-      mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
-      for (int c = 0; c < a.nc; ++c) tma_load_2d(qs + c * QCHUNK, &tm_q, &sh->q_full, c * 64, first_row * a.H, kEvictNormal);
-      const int32_t* bt = a.bt + (long long)slot * a.max_pages;
-      for (int t = 0; t < n_tiles; ++t) {
-        const int j0 = k0 + t * kKT, boxes = j0 + 64 < k_end ? 2 : 1;
-        int rows[2];
-        for (int b = 0; b < boxes; ++b) {
-          const int j = j0 + 64 * b;
-          rows[b] = bt[j / a.page_size] * a.page_size + j % a.page_size;
+    if (lane == 0 && n_tiles > 0) {
+      for (int t = 1; t < n_tiles; ++t)
+        for (int g = 0; g < nm; ++g) {
+          ls_wait(sh, &sh->o_done[g], (t - 1) & 1);
+          load_pair(t, g);
         }
-        for (int c = 0; c < a.nc; ++c) {
-          if (t > 0) ls_wait(sh, &sh->o_done[min(c >> 1, nm - 1)], (t - 1) & 1);
-          mbar_arrive_expect_tx(&sh->full[c], boxes * (kChunkBytes / 2));
-          for (int b = 0; b < boxes; ++b) tma_load_2d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[c], c * 64, rows[b], kEvictNormal);
-        }
-      }
       ls_wait(sh, &sh->q_full, 0);           // nothing is on its way any more when this thread leaves
-      for (int c = 0; c < a.nc; ++c) ls_wait(sh, &sh->full[c], (n_tiles - 1) & 1);
+      for (int g = 0; g < nm; ++g) ls_wait(sh, &sh->full[g], (n_tiles - 1) & 1);
     }
   } else if (warp == 1) {
     if (elect_one() && n_tiles > 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16_major(128, NR, 0, 0);
       constexpr uint32_t idesc_o = make_idesc_bf16_major(128, NR, 1, NR == 64 ? 1 : 0);
-      const uint32_t q_addr = smem_u32(qs), k_addr = smem_u32(ks), p_addr = smem_u32(ps);
+      const uint32_t p_addr = smem_u32(ps);
+      const uint64_t dk0 = make_sw128_kmajor_desc(smem_u32(ks)), dq0 = make_sw128_kmajor_desc(smem_u32(qs));
+      const uint64_t dv0 = make_sw128_mnmajor_desc(smem_u32(ks), kChunkBytes, 1024);
+      const uint64_t dp0 = NR == 64 ? make_sw128_mnmajor_desc(p_addr, 1024, 1024) : make_sw128_kmajor_desc(p_addr);
+      const int tail = (a.D - (a.nc - 1) * 64 + 15) >> 4;   // steps of 16 in the last chunk
       ls_wait(sh, &sh->q_full, 0);
       for (int t = 0; t < n_tiles; ++t) {
-        for (int c = 0; c < a.nc; ++c) {
-          ls_wait(sh, &sh->full[c], t & 1);
+        for (int g = 0; g < nm; ++g) {
+          ls_wait(sh, &sh->full[g], t & 1);
           tc_fence_after();
-          const uint64_t dk = make_sw128_kmajor_desc(k_addr + c * kChunkBytes), dq = make_sw128_kmajor_desc(q_addr + c * QCHUNK);
-          const int steps = min(4, (a.D - c * 64 + 15) >> 4);
-          for (int k = 0; k < steps; ++k) umma_bf16<1>(tmem_s, dk + 2 * k, dq + 2 * k, idesc_s, (c | k) != 0 ? 1u : 0u);
+          const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
+          for (int c = 2 * g; c < c1; ++c) {
+            const uint64_t dk = dk0 + (uint64_t)(c * (kChunkBytes >> 4)), dq = dq0 + (uint64_t)(c * (QCHUNK >> 4));
+            const int steps = c == a.nc - 1 ? tail : 4;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              if (k < steps) umma_bf16<1>(tmem_s, dk + 2 * k, dq + 2 * k, idesc_s, (c | k) != 0 ? 1u : 0u);
+          }
         }
         umma_commit(&sh->s_full);            // also: the output products of the tile before are done
         ls_wait(sh, &sh->p_ready, t & 1);
         tc_fence_after();
         for (int m = 0; m < nm; ++m) {
-          const uint64_t dv = make_sw128_mnmajor_desc(k_addr + 2 * m * kChunkBytes, kChunkBytes, 1024);
+          const uint64_t dv = dv0 + (uint64_t)(m * (2 * kChunkBytes >> 4));
 #pragma unroll
-          for (int k = 0; k < kKT / 16; ++k) {
-            const uint64_t dp = NR == 64 ? make_sw128_mnmajor_desc(p_addr + k * 2048, 1024, 1024)
-                                         : make_sw128_kmajor_desc(p_addr + (k >> 2) * QCHUNK) + 2 * (k & 3);
-            umma_bf16<1>(tmem + m * NR, dv + (uint64_t)(k * 128), dp, idesc_o, (t | k) != 0 ? 1u : 0u);
-          }
+          for (int k = 0; k < kKT / 16; ++k)
+            umma_bf16<1>(tmem + m * NR, dv + (uint64_t)(k * 128), dp0 + (uint64_t)(NR == 64 ? k * 128 : (k >> 2) * (QCHUNK >> 4) + 2 * (k & 3)), idesc_o,
+                         (t | k) != 0 ? 1u : 0u);
           umma_commit(&sh->o_done[m]);
         }
       }
@@ -216,18 +217,26 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       tc_fence_after();
       // a tile that every row of the item sees in full needs no mask
       const bool whole = j0 >= kb && j0 + kKT <= k_end && j0 + kKT - 1 <= first_pos && (long long)j0 >= (long long)first_pos + n_tok - a.window;
+      // the rows that see this thread's key: those of tokens at or behind it, as far as the window reaches
+      const bool is_key = key >= kb && key < k_end;
+      const int see0 = (is_key ? max(key - first_pos, 0) : kLsMaxRows) * a.H - c0;
+      const int see1 = (int)min((long long)kLsMaxRows, (long long)key - first_pos + a.window) * a.H - c0;
       float s[NC];
       auto load_scores = [&] {               // twice per tile: the maxima destroy them, and holding both copies would cost 32 registers
         uint32_t v[NC];
         ls_tmem_ld<NC>(tmem_s + lanes + c0, v);
         tmem_ld_wait();
+        if (whole) {
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
-          s[c] = whole || (key <= sh->lim[c0 + c] && key >= sh->low[c0 + c]) ? __uint_as_float(v[c]) * a.scale_log2 : -INFINITY;
+          for (int c = 0; c < NC; ++c) s[c] = __uint_as_float(v[c]) * a.scale_log2;
+        } else {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) s[c] = c >= see0 && c < see1 ? __uint_as_float(v[c]) * a.scale_log2 : -INFINITY;
+        }
       };
       load_scores();
       // rows of the tile that are no keys of this item hold whatever the cache holds there: as values they must not meet a product
-      if (!whole && half == 0 && (key < kb || key >= k_end)) {
+      if (!whole && half == 0 && !is_key) {
         for (int c = 0; c < a.r >> 6; ++c)
 #pragma unroll
           for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(ks + c * kChunkBytes + key_lane * 128 + i * 16) = make_uint4(0, 0, 0, 0);
@@ -265,12 +274,16 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       load_scores();
       uint32_t p[NC / 2];
 #pragma unroll
-      for (int c = 0; c < NC; c += 2) {
-        const float m0 = sh->mref[c0 + c], m1 = sh->mref[c0 + c + 1];
-        p[c / 2] = pack_bf16(ls_exp2(s[c] - (m0 == -INFINITY ? 0.f : m0)), ls_exp2(s[c + 1] - (m1 == -INFINITY ? 0.f : m1)));
-        const float2 e = unpack_bf16(p[c / 2]);   // the denominator sums the ROUNDED probabilities, the ones the numerator uses
-        l[c] += e.x;
-        l[c + 1] += e.y;
+      for (int c = 0; c < NC; c += 4) {
+        const float4 m4 = *reinterpret_cast<const float4*>(&sh->mref[c0 + c]);
+        const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+          p[(c + i) / 2] = pack_bf16(ls_exp2(s[c + i] - (m[i] == -INFINITY ? 0.f : m[i])), ls_exp2(s[c + i + 1] - (m[i + 1] == -INFINITY ? 0.f : m[i + 1])));
+          const float2 e = unpack_bf16(p[(c + i) / 2]);   // the denominator sums the ROUNDED probabilities, the ones the numerator uses
+          l[c + i] += e.x;
+          l[c + i + 1] += e.y;
+        }
       }
       if constexpr (NR == 64) {              // [key][64 rows]: MN-major
         uint8_t* dst = ps + key_lane * 128;
@@ -338,30 +351,6 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   if (warp == 1) tmem_dealloc<1>(tmem, a.tmem_cols);
 }
 
-typedef CUresult (*LsEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                               CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static LsEncodeFn ls_encode_fn() {
-  static LsEncodeFn fn = nullptr;
-  if (fn == nullptr) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) return nullptr;
-    fn = reinterpret_cast<LsEncodeFn>(p);
-  }
-  return fn;
-}
-// [rows, D] bf16 rows without gaps, boxes of box_rows x 64 columns
-static int ls_tensor_map(CUtensorMap* tm, const void* p, unsigned long long rows, int D, int box_rows) {
-  LsEncodeFn enc = ls_encode_fn();
-  if (enc == nullptr) return set_error(OMC_ERR_DRIVER, "cuTensorMapEncodeTiled entry point unavailable");
-  cuuint64_t dim[2] = {(cuuint64_t)D, rows}, stride[1] = {(cuuint64_t)D * 2};
-  cuuint32_t box[2] = {64u, (cuuint32_t)box_rows}, one[2] = {1u, 1u};
-  if (enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-    return set_error(OMC_ERR_DRIVER, "cuTensorMapEncodeTiled failed");
-  return OMC_OK;
-}
-
 constexpr int kLsSmemMax = 227 * 1024;
 static int ls_smem(int nr, int r, int D, int* p_offset) {
   const int nc = (D + 63) / 64, q = nc * nr * 128, k = nc * kChunkBytes, p = kKT * nr * 2;
@@ -406,9 +395,9 @@ int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const vo
   const int cols = (r / 128 + 1) * nr;
   a.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
   CUtensorMap tq, tk;
-  int rc = ls_tensor_map(&tq, q, q_rows, D, nr);
+  int rc = step_tensor_map(&tq, q, D, q_rows, D, 1, 0, nr);
   // how many pages the pool has is not known here; rows are only ever addressed through the block table
-  if (rc == OMC_OK) rc = ls_tensor_map(&tk, pool, 1ull << 31, D, 64);
+  if (rc == OMC_OK) rc = step_tensor_map(&tk, pool, D, 1ull << 31, D, 1, 0, 64);
   if (rc != OMC_OK) return rc;
   const bool b = out_dt == OMC_DT_BF16;
   if (nr == 16) return b ? ls_launch<16, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<16, float>(tq, tk, a, n_items, smem, st);
@@ -416,10 +405,6 @@ int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const vo
   return b ? ls_launch<64, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<64, float>(tq, tk, a, n_items, smem, st);
 }
 
-}  // namespace omc
+int latent_sm100_failures(unsigned int* n) { return cudaMemcpyFromSymbol(n, g_latent_failures, sizeof(*n)) == cudaSuccess ? OMC_OK : OMC_ERR_CUDA; }
 
-extern "C" int omc_latent_wait_failures(unsigned int* count) {
-  if (count == nullptr) return omc::set_error(OMC_ERR_ARG, "omc_latent_wait_failures: bad argument");
-  const cudaError_t e = cudaMemcpyFromSymbol(count, omc::g_latent_wait_failures, sizeof(unsigned int));
-  return e == cudaSuccess ? OMC_OK : omc::set_error(OMC_ERR_CUDA, cudaGetErrorString(e));
-}
+}  // namespace omc

@@ -8,39 +8,13 @@
 // Two kernels share one order of sums, so that a row's result does not depend on the M of the call: K is cut into chunks of 64; in a
 // chunk the even and the odd terms are summed separately in ascending order (one packed fma does both), their sum is the chunk's,
 // and the chunks are added in ascending order.
-#include "seq_common.cuh"
+#include "linear_args.cuh"
 
 namespace omc {
 
 constexpr int kLinBM = 64, kLinBN = 64, kLinBK = 32;   // BM: rows per tile, also of the grouped product's tile table
 constexpr int kLinChunk = 64;                          // K terms per partial sum
 constexpr int kLinPitch = kLinBK + 4, kLinStages = 3;
-
-struct LinearArgs {
-  const void* X;
-  const void* W;
-  void* Y;
-  long long ldx, sx, ldw, sw, ldy, sy, group_stride;
-  const int32_t* tile_group;
-  int M, N, K;
-  float alpha;
-  int act;
-  const void* bias;  // [N] of the weights' dtype, added before the activation (NULL: none); batch item b reads bias + b * sbias
-  long long sbias;
-  const void* gate;  // [M, .] of gate_dt: outputs are multiplied by sigmoid(gate[m * ldg + b * sg + n]) (NULL: none)
-  int gate_dt;
-  long long ldg, sg;
-};
-
-__device__ __forceinline__ float apply_act(float z, int act) {
-  if (act == OMC_ACT_RELU2) {
-    z = fmaxf(z, 0.f);
-    return z * z;
-  }
-  if (act == OMC_ACT_GELU_TANH) return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-  if (act == OMC_ACT_GELU_ERF) return 0.5f * z * (1.f + erff(z * 0.70710678118654752f));
-  return z;
-}
 
 __device__ __forceinline__ float gate_out(float y, const LinearArgs& a, int m, int n) {
   if (a.gate == nullptr) return y;
@@ -330,123 +304,12 @@ __global__ void __launch_bounds__(256, 2) linear_narrow_kernel(LinearArgs a) {
   }
 }
 
-// ---- bf16 x bf16 on the tensor pipe (mma.sync.m16n8k16): the same interface for operands whose rows start on 16-byte boundaries.
-// 128 x 128 output tile, K slices of 32 double-buffered with cp.async, 8 warps of 64 x 32. It serves the batched per-head products
-// of latent attention (absorbing W_uk into the query, W_uv after the attention), whose heads are column slices of one buffer.
-constexpr int kMmaBM = 128, kMmaBN = 128, kMmaBK = 32, kMmaPitch = kMmaBK + 8;
-
-__device__ __forceinline__ void store_pair(float* p, float x, float y) { *reinterpret_cast<float2*>(p) = make_float2(x, y); }
-__device__ __forceinline__ void store_pair(bf16_t* p, float x, float y) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(x, y); }
-
-template <typename TY>
-__global__ void __launch_bounds__(256) linear_mma_kernel(LinearArgs a) {
-  __shared__ __align__(16) bf16_t As[2][kMmaBM * kMmaPitch];
-  __shared__ __align__(16) bf16_t Bs[2][kMmaBN * kMmaPitch];
-  const int m0 = blockIdx.y * kMmaBM, n0 = blockIdx.x * kMmaBN;
-  const bf16_t* X = static_cast<const bf16_t*>(a.X) + (long long)blockIdx.z * a.sx;
-  const bf16_t* W = static_cast<const bf16_t*>(a.W) + (long long)blockIdx.z * a.sw;
-  TY* Y = static_cast<TY*>(a.Y) + (long long)blockIdx.z * a.sy;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wm = warp >> 2, wn = warp & 3;  // 2 x 4 warps: rows wm * 64, columns wn * 32
-  float acc[4][4][4] = {};
-  auto stage = [&](int buf, int k0) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int idx = tid + i * 256;          // 512 chunks of 8 elements per operand tile
-      const int row = idx >> 2, c = (idx & 3) * 8;
-      const int k = k0 + c;
-      bf16_t* da = &As[buf][row * kMmaPitch + c];
-      bf16_t* db = &Bs[buf][row * kMmaPitch + c];
-      if (m0 + row < a.M && k < a.K)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(lin_smem_u32(da)), "l"(X + (long long)(m0 + row) * a.ldx + k));
-      else *reinterpret_cast<uint4*>(da) = make_uint4(0, 0, 0, 0);
-      if (n0 + row < a.N && k < a.K)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(lin_smem_u32(db)), "l"(W + (long long)(n0 + row) * a.ldw + k));
-      else *reinterpret_cast<uint4*>(db) = make_uint4(0, 0, 0, 0);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-  };
-  const int nk = (a.K + kMmaBK - 1) / kMmaBK;
-  stage(0, 0);
-  for (int kt = 0; kt < nk; ++kt) {
-    const int buf = kt & 1;
-    if (kt + 1 < nk) {
-      stage(buf ^ 1, (kt + 1) * kMmaBK);
-      asm volatile("cp.async.wait_group 1;" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < kMmaBK; kk += 16) {
-      uint32_t bfr[4][2];
-#pragma unroll
-      for (int nn = 0; nn < 2; ++nn) {  // two 8-column tiles per ldmatrix.x4
-        const bf16_t* pb = &Bs[buf][(wn * 32 + nn * 16 + (lane & 7) + 8 * (lane >> 4)) * kMmaPitch + kk + 8 * ((lane >> 3) & 1)];
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(bfr[2 * nn][0]), "=r"(bfr[2 * nn][1]), "=r"(bfr[2 * nn + 1][0]), "=r"(bfr[2 * nn + 1][1])
-                     : "r"(lin_smem_u32(pb)));
-      }
-#pragma unroll
-      for (int mm = 0; mm < 4; ++mm) {
-        uint32_t a0, a1, a2, a3;
-        const bf16_t* pa = &As[buf][(wm * 64 + mm * 16 + (lane & 7) + 8 * ((lane >> 3) & 1)) * kMmaPitch + kk + 8 * (lane >> 4)];
-        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a0), "=r"(a1), "=r"(a2), "=r"(a3) : "r"(lin_smem_u32(pa)));
-#pragma unroll
-        for (int nn = 0; nn < 4; ++nn)
-          asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                       : "+f"(acc[mm][nn][0]), "+f"(acc[mm][nn][1]), "+f"(acc[mm][nn][2]), "+f"(acc[mm][nn][3])
-                       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(bfr[nn][0]), "r"(bfr[nn][1]));
-      }
-    }
-    __syncthreads();
-  }
-  const int g = lane >> 2, t4 = lane & 3;
-  // an accumulator pair (columns n, n + 1) goes out as one 4- or 8-byte store when the row is laid out for it; a gate pair comes in so
-  const bool gate_pair = a.gate != nullptr && a.ldg % 2 == 0 && a.sg % 2 == 0 && reinterpret_cast<uintptr_t>(a.gate) % 8 == 0;
-  const bool pair_ok = (a.ldy % 2 == 0) && (a.sy % 2 == 0) && (reinterpret_cast<uintptr_t>(a.Y) % (2 * sizeof(TY)) == 0);
-#pragma unroll
-  for (int mm = 0; mm < 4; ++mm)
-#pragma unroll
-    for (int nn = 0; nn < 4; ++nn)
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        const int m = m0 + wm * 64 + mm * 16 + g + 8 * hh;
-        const int n = n0 + wn * 32 + nn * 8 + 2 * t4;
-        if (m >= a.M || n >= a.N) continue;
-        const bf16_t* bias = a.bias != nullptr ? static_cast<const bf16_t*>(a.bias) + blockIdx.z * a.sbias : nullptr;
-        const float b0 = bias != nullptr ? ldf(bias + n) : 0.f, b1 = (bias != nullptr && n + 1 < a.N) ? ldf(bias + n + 1) : 0.f;
-        float v0 = apply_act(acc[mm][nn][2 * hh] * a.alpha + b0, a.act), v1 = apply_act(acc[mm][nn][2 * hh + 1] * a.alpha + b1, a.act);
-        if (gate_pair && n + 1 < a.N) {
-          const long long at = (long long)m * a.ldg + (long long)blockIdx.z * a.sg + n;
-          const float2 z = a.gate_dt == OMC_DT_F32 ? *reinterpret_cast<const float2*>(static_cast<const float*>(a.gate) + at)
-                                                   : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(static_cast<const bf16_t*>(a.gate) + at));
-          v0 = v0 / (1.f + __expf(-z.x)), v1 = v1 / (1.f + __expf(-z.y));
-        } else {
-          v0 = gate_out(v0, a, m, n);
-          if (n + 1 < a.N) v1 = gate_out(v1, a, m, n + 1);
-        }
-        TY* dst = Y + (long long)m * a.ldy + n;
-        if (pair_ok && n + 1 < a.N) {
-          store_pair(dst, v0, v1);
-        } else {
-          stf(dst, v0);
-          if (n + 1 < a.N) stf(dst + 1, v1);
-        }
-      }
-}
-
-static bool mma_operands_ok(const LinearArgs& a) {
-  return a.tile_group == nullptr && a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.sx % 8 == 0 && a.sw % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(a.X) % 16 == 0 && reinterpret_cast<uintptr_t>(a.W) % 16 == 0;
-}
-
-static int launch_linear_mma(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
-  dim3 grid((a.N + kMmaBN - 1) / kMmaBN, (a.M + kMmaBM - 1) / kMmaBM, batch);
-  if (y_dt == OMC_DT_F32) linear_mma_kernel<float><<<grid, 256, 0, st>>>(a);
-  else if (y_dt == OMC_DT_BF16) linear_mma_kernel<bf16_t><<<grid, 256, 0, st>>>(a);
-  else return set_error(OMC_ERR_ARG, "omc_linear: unknown output dtype");
-  return check_launch("omc_linear");
+// bf16 operands that the tensor-core kernel (linear_sm100.cu) can fetch: rows and batch items that start on 16-byte boundaries and do not
+// overlap (its tensor maps know no stride of zero; a batch may share an operand).
+int linear_sm100(const LinearArgs& a, int y_dt, int batch, cudaStream_t st);
+static bool sm100_operands_ok(const LinearArgs& a) {
+  return a.tile_group == nullptr && a.K % 8 == 0 && a.ldx % 8 == 0 && a.ldw % 8 == 0 && a.sx % 8 == 0 && a.sw % 8 == 0 && a.ldx >= a.K && a.ldw >= a.K &&
+         a.sx >= 0 && a.sw >= 0 && reinterpret_cast<uintptr_t>(a.X) % 16 == 0 && reinterpret_cast<uintptr_t>(a.W) % 16 == 0;
 }
 
 template <typename TX, typename TW, typename TY>
@@ -557,7 +420,7 @@ static int run_linear(const void* X, int x_dt, long long ldx, long long sx, cons
   if (x_dt == OMC_DT_BF16 && w_dt == OMC_DT_BF16) {
     // the choice depends on layout and widths only, never on M: a row is computed by the same kernel in every batch
     const bool narrow = tile_group == nullptr && N <= kNarrowMaxN && K >= 4 * N;
-    if (!narrow && mma_operands_ok(a) && (long long)N * K >= 4096) return launch_linear_mma(a, y_dt, batch, st);
+    if (!narrow && sm100_operands_ok(a) && (long long)N * K >= 4096) return linear_sm100(a, y_dt, batch, st);
     return launch_linear<bf16_t, bf16_t>(a, y_dt, batch, st);
   }
   return set_error(OMC_ERR_ARG, "omc_linear: operand dtypes must be (f32, f32), (f32, bf16) or (bf16, bf16)");

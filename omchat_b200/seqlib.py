@@ -62,7 +62,7 @@ SIGNATURES = {
     "omc_rotary_q": (_I, [_P, _I, _L, _I, _I, _I, _I, _P, _I, _P, _P, _I, _I, _P]),
     "omc_latent_attn": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _L, _F, _P, _P]),
     "omc_latent_attn_mma_rows": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
-    "omc_latent_wait_failures": (_I, [_P]),
+    "omc_step_wait_failures": (_I, [_P]),
     "omc_latent_attn_mma": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_latent_decode_items": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
     "omc_router_topk": (_I, [_P, _L, _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P, _P]),
@@ -276,36 +276,37 @@ class LatentAttnPlan:
     def __init__(self, portions, H: int, device, target_ctas: int = 296, min_keys: int = 128, window: int = WINDOW_ALL):
         import numpy as np
         tok = max(1, MMA_ROWS // H)
-        base = sum(-(-n // tok) for _, n, _, _ in portions)
-        items, merges, part = [], [], 0
-        for first_row, n, slot, p0 in portions:
-            starts = np.arange(0, n, tok, dtype=np.int64)
-            ntok = np.minimum(tok, n - starts)
-            ends = p0 + starts + ntok                                  # end of the keys the tile's last row sees
-            lows = np.maximum(0, p0 + starts - window + 1)             # first key its first row sees
-            keys = ends - lows
-            parts = np.ones_like(starts)
-            if base < target_ctas // 2:
-                parts = np.clip(np.minimum(-(-keys // min_keys), -(-target_ctas // max(base, 1))), 1, self.MAX_PARTS)
-            for i in range(len(starts)):
-                np_i, k, lo = int(parts[i]), int(keys[i]), int(lows[i])
-                fr, nt = first_row + int(starts[i]), int(ntok[i])
-                if np_i == 1:
-                    items.append((fr, nt, slot, p0 + int(starts[i]), lo, lo + k, -1, 0))
-                    continue
-                span = -(-(-(-k // np_i)) // MMA_ROWS) * MMA_ROWS       # keys per part, a multiple of 64
-                np_i = -(-k // span)
-                merges.append((fr * H, nt * H, part, np_i))
-                for j in range(np_i):
-                    items.append((fr, nt, slot, p0 + int(starts[i]), lo + j * span, lo + min(k, (j + 1) * span), part, 0))
-                    part += 1
-        self.n_items, self.n_merges, self.n_parts = len(items), len(merges), part
-        self.max_rows = max((it[1] for it in items), default=1) * H   # (token, head) pairs of the largest item
-        flat = torch.tensor(items, dtype=torch.int32).view(-1)
-        flat = torch.cat([flat, torch.tensor(merges, dtype=torch.int32).view(-1)]) if merges else flat
-        buf = flat.pin_memory().to(device, non_blocking=True)
+        por = np.array(list(portions), dtype=np.int64).reshape(-1, 4)
+        tiles = -(-por[:, 1] // tok)                                    # row tiles per portion
+        base = int(tiles.sum())
+        of = np.repeat(np.arange(len(por)), tiles)
+        start = (np.arange(base) - np.repeat(np.cumsum(tiles) - tiles, tiles)) * tok
+        ntok, first = np.minimum(tok, por[of, 1] - start), por[of, 3] + start
+        low = np.maximum(0, first - window + 1)                         # first key a tile's first row sees
+        keys = first + ntok - low                                       # ... up to the end of what its last row sees
+        want = np.ones_like(keys)
+        if base < target_ctas // 2:
+            want = np.clip(np.minimum(-(-keys // min_keys), -(-target_ctas // max(base, 1))), 1, self.MAX_PARTS)
+        cut = want > 1
+        span = np.where(cut, -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS, np.maximum(keys, 1))   # keys per part, a multiple of 64
+        n = np.where(cut, -(-keys // span), 1)
+        it = np.repeat(np.arange(base), n)
+        j = np.arange(len(it)) - np.repeat(np.cumsum(n) - n, n)
+        n_cut = np.where(cut, n, 0)
+        part0 = np.cumsum(n_cut) - n_cut
+        items = np.empty((len(it), 8), dtype=np.int32)
+        items[:, 0], items[:, 1], items[:, 2], items[:, 3] = (por[of, 0] + start)[it], ntok[it], por[of, 2][it], first[it]
+        items[:, 4] = low[it] + j * span[it]
+        items[:, 5] = low[it] + np.minimum(keys[it], (j + 1) * span[it])
+        items[:, 6], items[:, 7] = np.where(cut[it], part0[it] + j, -1), 0
+        # the items with the most keys first: with 148 running at a time a long one at the end would run alone
+        items = items[np.argsort(items[:, 4] - items[:, 5], kind="stable")]
+        merges = np.stack([(por[of, 0] + start) * H, ntok * H, part0, n], axis=1)[cut].astype(np.int32)
+        self.n_items, self.n_merges, self.n_parts = len(items), len(merges), int(n_cut.sum())
+        self.max_rows = int(ntok.max(initial=1)) * H                    # (token, head) pairs of the largest item
+        buf = torch.from_numpy(np.concatenate([items.reshape(-1), merges.reshape(-1)])).pin_memory().to(device, non_blocking=True)
         self.items = buf[:self.n_items * 8]
-        self.merges = buf[self.n_items * 8:] if merges else None
+        self.merges = buf[self.n_items * 8:] if self.n_merges else None
 
 
 class DecodeAttnPlan:

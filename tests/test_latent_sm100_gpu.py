@@ -82,4 +82,4 @@ def test_against_float64(H, r, dr, page, window, portions, opt):
 def test_no_wait_ran_out():
     import ctypes
     n = ctypes.c_uint(7)
-    assert seqlib.load().omc_latent_wait_failures(ctypes.byref(n)) == 0 and n.value == 0
+    assert seqlib.load().omc_step_wait_failures(ctypes.byref(n)) == 0 and n.value == 0
