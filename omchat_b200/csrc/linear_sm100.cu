@@ -12,6 +12,7 @@
 namespace omc {
 
 constexpr int kHgThreads = 192, kHgBM = 128, kHgBK = 64, kHgMaxStages = 4;
+constexpr int kHgPitch = 68, kHgSlabs = 4 * 32 * kHgPitch * 4;   // the epilogue's [32 rows][64 columns] fp32 per warp
 
 static __device__ unsigned int g_linear_failures;   // waits that ran out
 
@@ -19,6 +20,29 @@ struct HgShared {
   uint64_t full[kHgMaxStages], empty[kHgMaxStages], done;
   uint32_t tmem, dead;
 };
+
+__device__ __forceinline__ void hg_row(const float* src, float alpha, float (&f)[8]) {
+  const float4 lo = *reinterpret_cast<const float4*>(src), hi = *reinterpret_cast<const float4*>(src + 4);
+  f[0] = lo.x * alpha, f[1] = lo.y * alpha, f[2] = lo.z * alpha, f[3] = lo.w * alpha, f[4] = hi.x * alpha, f[5] = hi.y * alpha, f[6] = hi.z * alpha, f[7] = hi.w * alpha;
+}
+__device__ __forceinline__ void hg_gates(const LinearArgs& a, long long at, float (&z)[8]) {   // eight neighbours from a 16-byte boundary
+  if (a.gate_dt == OMC_DT_F32) {
+    const float4* p = reinterpret_cast<const float4*>(static_cast<const float*>(a.gate) + at);
+    const float4 g0 = p[0], g1 = p[1];
+    z[0] = g0.x, z[1] = g0.y, z[2] = g0.z, z[3] = g0.w, z[4] = g1.x, z[5] = g1.y, z[6] = g1.z, z[7] = g1.w;
+  } else {
+    const uint4 g = *reinterpret_cast<const uint4*>(static_cast<const bf16_t*>(a.gate) + at);
+    const float2 g0 = unpack_bf16(g.x), g1 = unpack_bf16(g.y), g2 = unpack_bf16(g.z), g3 = unpack_bf16(g.w);
+    z[0] = g0.x, z[1] = g0.y, z[2] = g1.x, z[3] = g1.y, z[4] = g2.x, z[5] = g2.y, z[6] = g3.x, z[7] = g3.y;
+  }
+}
+__device__ __forceinline__ void hg_store(float* y, const float (&f)[8]) {
+  reinterpret_cast<float4*>(y)[0] = make_float4(f[0], f[1], f[2], f[3]);
+  reinterpret_cast<float4*>(y)[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+__device__ __forceinline__ void hg_store(bf16_t* y, const float (&f)[8]) {
+  *reinterpret_cast<uint4*>(y) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
 
 template <int BN, typename TY>
 __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, LinearArgs a,
@@ -82,69 +106,90 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
       umma_commit(&sh->done);
     }
   } else {
-    const int quarter = warp & 3, m = m0 + quarter * 32 + lane;
-    const bool row_ok = m < a.M;
-    TY* y = static_cast<TY*>(a.Y) + (long long)b * a.sy + (long long)m * a.ldy;
-    const long long g0 = (long long)m * a.ldg + (long long)b * a.sg;
-    const bf16_t* bias = a.bias != nullptr ? static_cast<const bf16_t*>(a.bias) + b * a.sbias : nullptr;
+    // thread = row while the accumulator is read, eight neighbouring threads = one row of 64 columns while gates come in and outputs go out
+    // (lines of 32 rows per store otherwise); the ring is free by then
+    const int quarter = warp & 3;
+    float* slab = reinterpret_cast<float*>(ring) + quarter * 32 * kHgPitch;
+    const bool plain = vec_out && a.act == OMC_ACT_NONE && a.bias == nullptr && (a.gate == nullptr || vec_gate);
     wait(&sh->done, 0);
     tc_fence_after();
-    for (int c = 0; c < BN && n0 + c < a.N; c += 32) {
-      uint32_t v[32];
-      tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + c, v);
-      tmem_ld_wait();
-      if (!row_ok) continue;
-      const int n = n0 + c, left = min(32, a.N - n);
-      float f[32];
+    for (int c = 0; c < BN && n0 + c < a.N; c += 64) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j)
-        f[j] = apply_act(__uint_as_float(v[j]) * a.alpha + (bias != nullptr && j < left ? __bfloat162float(bias[n + j]) : 0.f), a.act);
-      if (a.gate != nullptr) {
-        if (vec_gate && left == 32) {
-          if (a.gate_dt == OMC_DT_F32) {
-            const float4* g = reinterpret_cast<const float4*>(static_cast<const float*>(a.gate) + g0 + n);
+      for (int part = 0; part < 2; ++part) {
+        uint32_t v[32];
+        tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + c + 32 * part, v);
+        tmem_ld_wait();
+        uint4* dst = reinterpret_cast<uint4*>(slab + lane * kHgPitch + 32 * part);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float4 z = g[j];
-              f[4 * j] /= 1.f + __expf(-z.x), f[4 * j + 1] /= 1.f + __expf(-z.y), f[4 * j + 2] /= 1.f + __expf(-z.z), f[4 * j + 3] /= 1.f + __expf(-z.w);
-            }
-          } else {
-            const uint4* g = reinterpret_cast<const uint4*>(static_cast<const bf16_t*>(a.gate) + g0 + n);
+        for (int j = 0; j < 8; ++j) dst[j] = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      }
+      __syncwarp();
+      const int n = n0 + c + (lane & 7) * 8, left = min(8, a.N - n);
+      const bf16_t* bias = a.bias != nullptr ? static_cast<const bf16_t*>(a.bias) + b * a.sbias : nullptr;
+      if (plain && n0 + c + 64 <= a.N && m0 + quarter * 32 + 32 <= a.M) {
+        // a whole piece without activation or bias: no branch between the loads and the stores of its 8 x 4 rows
+        const long long m = m0 + quarter * 32 + (lane >> 3);
+        const float* src = slab + (lane >> 3) * kHgPitch + (lane & 7) * 8;
+        TY* y = static_cast<TY*>(a.Y) + (long long)b * a.sy + m * a.ldy + n;
+        if (a.gate == nullptr) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint4 z = g[j];
-              const uint32_t w[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float2 e = unpack_bf16(w[i]);
-                f[8 * j + 2 * i] /= 1.f + __expf(-e.x), f[8 * j + 2 * i + 1] /= 1.f + __expf(-e.y);
-              }
-            }
+          for (int i = 0; i < 8; ++i) {
+            float f[8];
+            hg_row(src + i * 4 * kHgPitch, a.alpha, f);
+            hg_store(y + (long long)(i * 4) * a.ldy, f);
           }
         } else {
+          const long long at = m * a.ldg + (long long)b * a.sg + n;
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (j < left) {
-              const float z = a.gate_dt == OMC_DT_F32 ? static_cast<const float*>(a.gate)[g0 + n + j] : ldf(static_cast<const bf16_t*>(a.gate) + g0 + n + j);
-              f[j] /= 1.f + __expf(-z);
+          for (int i0 = 0; i0 < 8; i0 += 4) {
+            float z[4][8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) hg_gates(a, at + (long long)((i0 + i) * 4) * a.ldg, z[i]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              float f[8];
+              hg_row(src + (i0 + i) * 4 * kHgPitch, a.alpha, f);
+#pragma unroll
+              for (int j = 0; j < 8; ++j)   // a bf16 output keeps 8 of the quotient's bits
+                f[j] = sizeof(TY) == 2 ? __fdividef(f[j], 1.f + __expf(-z[i][j])) : f[j] / (1.f + __expf(-z[i][j]));
+              hg_store(y + (long long)((i0 + i) * 4) * a.ldy, f);
             }
+          }
         }
+        __syncwarp();
+        continue;
       }
-      if (vec_out && left == 32) {
-        if constexpr (sizeof(TY) == 4) {
+#pragma unroll 2
+      for (int i = 0; i < 8 && left > 0; ++i) {
+        const int row = i * 4 + (lane >> 3), m = m0 + quarter * 32 + row;
+        if (m >= a.M) break;
+        float f[8];
+        hg_row(slab + row * kHgPitch + (lane & 7) * 8, a.alpha, f);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) reinterpret_cast<float4*>(y + n)[j] = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+        for (int j = 0; j < 8; ++j) f[j] = apply_act(f[j] + (bias != nullptr && j < left ? __bfloat162float(bias[n + j]) : 0.f), a.act);
+        if (a.gate != nullptr) {
+          const long long at = (long long)m * a.ldg + (long long)b * a.sg + n;
+          float z[8];
+          if (vec_gate && left == 8) {
+            hg_gates(a, at, z);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              z[j] = j >= left ? 0.f : (a.gate_dt == OMC_DT_F32 ? static_cast<const float*>(a.gate)[at + j] : ldf(static_cast<const bf16_t*>(a.gate) + at + j));
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] /= 1.f + __expf(-z[j]);
+        }
+        TY* y = static_cast<TY*>(a.Y) + (long long)b * a.sy + (long long)m * a.ldy + n;
+        if (vec_out && left == 8) {
+          hg_store(y, f);
         } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            reinterpret_cast<uint4*>(y + n)[j] = make_uint4(pack_bf16(f[8 * j], f[8 * j + 1]), pack_bf16(f[8 * j + 2], f[8 * j + 3]),
-                                                            pack_bf16(f[8 * j + 4], f[8 * j + 5]), pack_bf16(f[8 * j + 6], f[8 * j + 7]));
+          for (int j = 0; j < 8; ++j)
+            if (j < left) stf(y + j, f[j]);
         }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (j < left) stf(y + n + j, f[j]);
       }
+      __syncwarp();
     }
     tc_fence_before();
   }
@@ -160,6 +205,7 @@ static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
   if (rc == OMC_OK) rc = step_tensor_map(&tw, a.W, a.K, a.N, a.ldw, a.sw > 0 ? batch : 1, a.sw, BN);
   if (rc != OMC_OK) return rc;
   constexpr int stage = (kHgBM + BN) * 128, max_smem = kHgMaxStages * stage + 1024;
+  static_assert(max_smem >= kHgSlabs + 1024, "the ring holds the epilogue's slabs");
   static bool done[kMaxDevices] = {};
   const int dev = cur_device();
   if (!done[dev]) {
@@ -173,7 +219,8 @@ static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
   const int ye = 16 / (int)sizeof(TY), ge = a.gate_dt == OMC_DT_F32 ? 4 : 8;
   const bool vec_out = aligned(a.Y) && a.ldy % ye == 0 && a.sy % ye == 0, vec_gate = aligned(a.gate) && a.ldg % ge == 0 && a.sg % ge == 0;
   const dim3 grid((a.N + BN - 1) / BN, (a.M + kHgBM - 1) / kHgBM, batch);
-  linear_sm100_kernel<BN, TY><<<grid, kHgThreads, stages * stage + 1024, st>>>(tx, tw, a, stages, a.sx == 0, a.sw == 0, vec_out, vec_gate);
+  const int smem = (stages * stage > kHgSlabs ? stages * stage : kHgSlabs) + 1024;
+  linear_sm100_kernel<BN, TY><<<grid, kHgThreads, smem, st>>>(tx, tw, a, stages, a.sx == 0, a.sw == 0, vec_out, vec_gate);
   return check_launch("omc_linear");
 }
 
