@@ -120,13 +120,21 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   const int32_t* bt = a.bt + (long long)slot * a.max_pages;
-  auto load_pair = [&](int t, int g) {       // chunks of barrier g of tile t
-    const int j0 = k0 + t * kKT, boxes = j0 + 64 < k_end ? 2 : 1, c1 = g == nm - 1 ? a.nc : 2 * g + 2;
-    mbar_arrive_expect_tx(&sh->full[g], (c1 - 2 * g) * boxes * (kChunkBytes / 2));
-    for (int b = 0; b < boxes; ++b) {
-      const int j = j0 + 64 * b, row = bt[j / a.page_size] * a.page_size + j % a.page_size;
-      for (int c = 2 * g; c < c1; ++c) tma_load_3d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[g], c * 64, row, 0);
+  // rows of the pool where the two boxes of tile t start (looked up a tile ahead: a lookup takes as long as 20 KB of the copies)
+  auto box_rows = [&](int t, int (&row)[2]) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int j = k0 + t * kKT + 64 * b;
+      row[b] = j < k_end ? bt[j / a.page_size] * a.page_size + j % a.page_size : -1;
     }
+  };
+  auto load_pair = [&](const int (&row)[2], int g) {   // chunks of barrier g
+    const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
+    mbar_arrive_expect_tx(&sh->full[g], (c1 - 2 * g) * (row[1] >= 0 ? 2 : 1) * (kChunkBytes / 2));
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+      if (row[b] >= 0)
+        for (int c = 2 * g; c < c1; ++c) tma_load_3d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[g], c * 64, row[b], 0);
   };
   if (tid >= 64 && tid < 64 + kLsMaxRows) sh->mref[tid - 64] = -INFINITY;
   if (tid == 0) {
@@ -144,7 +152,9 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     if (n_tiles > 0) {                       // on their way while tensor memory is allocated
       mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
       for (int c = 0; c < a.nc; ++c) tma_load_3d(qs + c * QCHUNK, &tm_q, &sh->q_full, c * 64, first_row * a.H, 0);
-      for (int g = 0; g < nm; ++g) load_pair(0, g);
+      int row[2];
+      box_rows(0, row);
+      for (int g = 0; g < nm; ++g) load_pair(row, g);
     }
   }
   if (warp == 1) {
@@ -159,11 +169,14 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
 
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
-      for (int t = 1; t < n_tiles; ++t)
+      for (int t = 1; t < n_tiles; ++t) {
+        int row[2];
+        box_rows(t, row);
         for (int g = 0; g < nm; ++g) {
           ls_wait(sh, &sh->o_done[g], (t - 1) & 1);
-          load_pair(t, g);
+          load_pair(row, g);
         }
+      }
       ls_wait(sh, &sh->q_full, 0);           // nothing is on its way any more when this thread leaves
       for (int g = 0; g < nm; ++g) ls_wait(sh, &sh->full[g], (n_tiles - 1) & 1);
     }

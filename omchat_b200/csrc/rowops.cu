@@ -152,66 +152,65 @@ __global__ void __launch_bounds__(kNormThreads) layernorm_kernel(const bf16* __r
 }
 
 // ------------------------------------------------------------------------------------------------ patch im2col
-template <typename T>
-__global__ void im2col_kernel(const T* __restrict__ pix, bf16* __restrict__ cols, long long ldc, int B, int H, int W) {
-  const int gh = H / 14, gw = W / 14;
-  const long long total = (long long)B * gh * gw * ldc;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int col = (int)(idx % ldc);
-    const long long row = idx / ldc;
-    float val = 0.f;
-    if (col < 588) {
-      const int c = col / 196, r = col % 196, ky = r / 14, kx = r % 14;
-      const int b = (int)(row / (gh * gw)), pr = (int)(row % (gh * gw)), py = pr / gw, px = pr % gw;
-      val = (float)pix[(((long long)b * 3 + c) * H + (py * 14 + ky)) * W + (px * 14 + kx)];
+// One CTA per row of patches (image b, patch row py): its 14 pixel lines of three channels are read from L1 by the 16-byte pieces of the
+// output that need them. HBM-bound: 21 crops 105 us with one 64-bit division chain per element, 22 us so (floor 12).
+// VEC: the output's rows start on 16-byte boundaries.
+template <typename T, bool VEC>
+__global__ void __launch_bounds__(256) im2col_kernel(const T* __restrict__ pix, bf16* __restrict__ cols, long long ldc, int gh, int H, int W) {
+  const int gw = W / 14, b = blockIdx.x / gh, py = blockIdx.x - b * gh, nvec = (int)((ldc + 7) >> 3);
+  const T* img = pix + (long long)b * 3 * H * W + (long long)py * 14 * W;
+  bf16* out = cols + (long long)blockIdx.x * gw * ldc;
+  for (int e = threadIdx.x; e < gw * nvec; e += blockDim.x) {
+    const int px = e / nvec, col0 = (e - px * nvec) << 3;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int col = col0 + j, c = col / 196, r = col - c * 196, ky = r / 14, kx = r - ky * 14;
+      v[j] = col < 588 ? (float)img[(long long)c * H * W + ky * W + px * 14 + kx] : 0.f;
     }
-    cols[idx] = __float2bfloat16(val);
+    bf16* dst = out + (long long)px * ldc + col0;
+    if (VEC) {
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (col0 + j < ldc) dst[j] = __float2bfloat16(v[j]);
+    }
   }
 }
 
 // ------------------------------------------------------------------------------------------------ CLS + pos-embed
-__global__ void vit_assemble_kernel(const bf16* __restrict__ patch, const bf16* __restrict__ cls,
-                                    const bf16* __restrict__ pos, bf16* __restrict__ hidden, int B, int P, int C) {
-  const int nvec = C >> 3;
-  const long long total = (long long)B * (P + 1) * nvec;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int vcol = (int)(idx % nvec);
-    const long long row = idx / nvec;
-    const int tok = (int)(row % (P + 1));
-    const int b = (int)(row / (P + 1));
-    uint4 a = (tok == 0) ? reinterpret_cast<const uint4*>(cls)[vcol]
-                         : reinterpret_cast<const uint4*>(patch + ((long long)b * P + tok - 1) * C)[vcol];
-    uint4 p = reinterpret_cast<const uint4*>(pos + (long long)tok * C)[vcol];
-    uint32_t ai[4] = {a.x, a.y, a.z, a.w}, pi[4] = {p.x, p.y, p.z, p.w}, oo[4];
+// One CTA per row, here and in the next kernel: where a row lies is found once and not per 16 bytes (21 crops of 1025 x 3200: 71 and 111 us
+// before).
+__global__ void __launch_bounds__(128) vit_assemble_kernel(const bf16* __restrict__ patch, const bf16* __restrict__ cls,
+                                                           const bf16* __restrict__ pos, bf16* __restrict__ hidden, int P, int C) {
+  const int b = blockIdx.x / (P + 1), tok = blockIdx.x - b * (P + 1), nvec = C >> 3;
+  const uint4* src = reinterpret_cast<const uint4*>(tok == 0 ? cls : patch + ((long long)b * P + tok - 1) * C);
+  const uint4* add = reinterpret_cast<const uint4*>(pos + (long long)tok * C);
+  uint4* dst = reinterpret_cast<uint4*>(hidden + (long long)blockIdx.x * C);
+#pragma unroll 4
+  for (int i = threadIdx.x; i < nvec; i += 128) {
+    const uint4 a = src[i], p = add[i];
+    const uint32_t ai[4] = {a.x, a.y, a.z, a.w}, pi[4] = {p.x, p.y, p.z, p.w};
+    uint32_t oo[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       float2 x = unpack_bf16(ai[q]), y = unpack_bf16(pi[q]);
       oo[q] = pack_bf16(x.x + y.x, x.y + y.y);
     }
-    reinterpret_cast<uint4*>(hidden + row * C)[vcol] = make_uint4(oo[0], oo[1], oo[2], oo[3]);
+    dst[i] = make_uint4(oo[0], oo[1], oo[2], oo[3]);
   }
 }
 
 // ------------------------------------------------------------------------------------------------ CLS drop + pixel shuffle
 // out[b, (i/d)*(G/d) + j/d, (i%d)*(d*C) + (j%d)*C + c] = hidden[b, 1 + i*G + j, c]
-__global__ void select_pixel_shuffle_kernel(const bf16* __restrict__ hidden, bf16* __restrict__ out, int B, int G,
-                                            int C, int d) {
-  const int nvec = C >> 3;
-  const long long total = (long long)B * G * G * nvec;
-  const int Go = G / d;
-  const long long Co = (long long)C * d * d;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const int vcol = (int)(idx % nvec);
-    const long long t = idx / nvec;
-    const int j = (int)(t % G), i = (int)((t / G) % G), b = (int)(t / ((long long)G * G));
-    uint4 v = reinterpret_cast<const uint4*>(hidden + ((long long)b * (G * G + 1) + 1 + (long long)i * G + j) * C)[vcol];
-    const long long orow = (long long)b * Go * Go + (long long)(i / d) * Go + (j / d);
-    const long long ocol = (long long)(i % d) * d * C + (long long)(j % d) * C + (long long)vcol * 8;
-    *reinterpret_cast<uint4*>(out + orow * Co + ocol) = v;
-  }
+__global__ void __launch_bounds__(128) select_pixel_shuffle_kernel(const bf16* __restrict__ hidden, bf16* __restrict__ out, int G, int C, int d) {
+  const int nvec = C >> 3, Go = G / d, GG = G * G, b = blockIdx.x / GG, t = blockIdx.x - b * GG, i = t / G, j = t - i * G;
+  const uint4* src = reinterpret_cast<const uint4*>(hidden + ((long long)b * (GG + 1) + 1 + t) * C);
+  uint4* dst = reinterpret_cast<uint4*>(out + ((long long)b * Go * Go + (long long)(i / d) * Go + j / d) * ((long long)C * d * d) +
+                                        (long long)(i % d) * d * C + (long long)(j % d) * C);
+#pragma unroll 4
+  for (int v = threadIdx.x; v < nvec; v += 128) dst[v] = src[v];
 }
 
 // ------------------------------------------------------------------------------------------------ embed lookup
@@ -514,12 +513,13 @@ extern "C" int omc_vit_im2col(const void* pixels, int pixels_are_f32, void* cols
                               void* stream) {
   if (B <= 0) return OMC_OK;
   if (H % 14 != 0 || W % 14 != 0 || ldc < 588) return set_error(OMC_ERR_SHAPE, "omc_vit_im2col: H, W must be multiples of 14 and ldc >= 588");
-  long long total = (long long)B * (H / 14) * (W / 14) * ldc;
-  int grid = grid_for(total, 256);
-  if (pixels_are_f32)
-    im2col_kernel<float><<<grid, 256, 0, (cudaStream_t)stream>>>((const float*)pixels, (bf16*)cols, ldc, B, H, W);
-  else
-    im2col_kernel<bf16><<<grid, 256, 0, (cudaStream_t)stream>>>((const bf16*)pixels, (bf16*)cols, ldc, B, H, W);
+  const int gh = H / 14, grid = B * gh;
+  const bool vec = ldc % 8 == 0 && reinterpret_cast<uintptr_t>(cols) % 16 == 0;
+  cudaStream_t st = (cudaStream_t)stream;
+  if (pixels_are_f32 && vec) im2col_kernel<float, true><<<grid, 256, 0, st>>>((const float*)pixels, (bf16*)cols, ldc, gh, H, W);
+  else if (pixels_are_f32) im2col_kernel<float, false><<<grid, 256, 0, st>>>((const float*)pixels, (bf16*)cols, ldc, gh, H, W);
+  else if (vec) im2col_kernel<bf16, true><<<grid, 256, 0, st>>>((const bf16*)pixels, (bf16*)cols, ldc, gh, H, W);
+  else im2col_kernel<bf16, false><<<grid, 256, 0, st>>>((const bf16*)pixels, (bf16*)cols, ldc, gh, H, W);
   return check_launch("im2col");
 }
 
@@ -527,18 +527,14 @@ extern "C" int omc_vit_assemble(const void* patch, const void* cls, const void* 
                                 void* stream) {
   if (B <= 0) return OMC_OK;
   if (C % 8 != 0) return set_error(OMC_ERR_SHAPE, "omc_vit_assemble: C % 8 != 0");
-  long long total = (long long)B * (P + 1) * (C / 8);
-  vit_assemble_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)patch, (const bf16*)cls,
-                                                                              (const bf16*)pos, (bf16*)hidden, B, P, C);
+  vit_assemble_kernel<<<B * (P + 1), 128, 0, (cudaStream_t)stream>>>((const bf16*)patch, (const bf16*)cls, (const bf16*)pos, (bf16*)hidden, P, C);
   return check_launch("vit_assemble");
 }
 
 extern "C" int omc_select_pixel_shuffle(const void* hidden, void* out, int B, int G, int C, int down, void* stream) {
   if (B <= 0) return OMC_OK;
   if (down < 1 || G % down != 0 || C % 8 != 0) return set_error(OMC_ERR_SHAPE, "omc_select_pixel_shuffle: bad G/C/down");
-  long long total = (long long)B * G * G * (C / 8);
-  select_pixel_shuffle_kernel<<<grid_for(total, 256), 256, 0, (cudaStream_t)stream>>>((const bf16*)hidden, (bf16*)out,
-                                                                                      B, G, C, down);
+  select_pixel_shuffle_kernel<<<B * G * G, 128, 0, (cudaStream_t)stream>>>((const bf16*)hidden, (bf16*)out, G, C, down);
   return check_launch("select_pixel_shuffle");
 }
 

@@ -48,19 +48,23 @@ class LatentAttention:
         self.tensor_attention = True    # False: the plain attention kernel for every shape (A/B, tests)
         self._decode_plans = {}         # (rows, heads, parts, window) -> seqlib.DecodeAttnPlan
 
-    def _plan(self, plans: dict, T: int, H: int, window: int, pos, slot):
-        plan = plans.get((H, window))
+    def _plan(self, plans: dict, T: int, H: int, window: int, pos, slot, tcgen05: bool):
+        plan = plans.get((H, window, tcgen05))
         if plan is None:
             if "portions" in plans:
-                plan = seqlib.LatentAttnPlan(plans["portions"], H, self.device, window=window)
+                # the tcgen05 kernel runs one CTA per SM on tiles of 128 keys: contexts are cut only while that leaves half the SMs idle
+                cut = dict(target_ctas=148, min_keys=256) if tcgen05 else {}
+                plan = seqlib.LatentAttnPlan(plans["portions"], H, self.device, window=window, **cut)
             else:
-                parts = plans["decode_parts"] if "decode_parts" in plans else self._decode_parts(T, min(window, plans["decode_keys"]))
+                keys = min(window, plans["decode_keys"]) if "decode_keys" in plans else 0
+                parts = (plans["decode_parts"] if "decode_parts" in plans else
+                         seqlib.DecodeAttnPlan.parts_for_tcgen05(T, keys) if tcgen05 else self._decode_parts(T, keys))
                 key = (T, H, parts, window)
                 plan = self._decode_plans.get(key)
                 if plan is None:
                     plan = self._decode_plans[key] = seqlib.DecodeAttnPlan(T, H, parts, self.device, window=window)
                 plan.fill(pos, slot)
-            plans[(H, window)] = plan
+            plans[(H, window, tcgen05)] = plan
         return plan
 
     @staticmethod
@@ -77,7 +81,8 @@ class LatentAttention:
         window = seqlib.WINDOW_ALL if window is None else min(window, seqlib.WINDOW_ALL)
         if plans is not None and self.tensor_attention and seqlib.latent_attn_mma_ok(H, r, dr, self.dtype):
             out = torch.empty(T, H, r, device=qcat.device, dtype=self.dtype)
-            return seqlib.latent_attn_mma(qcat, r, dr, pool, cache.block_table, cache.page_size, self._plan(plans, T, H, window, pos, slot), sink, scale,
+            tcgen05 = seqlib.latent_attn_tcgen05_ok(H, r, dr, cache.page_size)
+            return seqlib.latent_attn_mma(qcat, r, dr, pool, cache.block_table, cache.page_size, self._plan(plans, T, H, window, pos, slot, tcgen05), sink, scale,
                                           out, window=window, gate=gate)
         out = torch.empty(T, H, r, device=qcat.device, dtype=torch.float32)
         return seqlib.latent_attn(qcat, r, dr, pool, cache.block_table, cache.page_size, pos, slot, sink, scale, out, window=window, gate=gate)

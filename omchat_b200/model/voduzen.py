@@ -348,7 +348,8 @@ class VoduzenDecoder:
         the cache (the attention work list is rebuilt on the device from the positions) and the logits of all B rows.
         Returns fp32 logits [B, vocab] (a static buffer, overwritten by the next call)."""
         B = meta_host.shape[1]
-        parts = seqlib.DecodeAttnPlan.parts_for(B, max_keys)
+        tcgen05 = all(seqlib.latent_attn_tcgen05_ok(l.mixer.heads, l.mixer.kv_rank, l.mixer.rot_dim, cache.page_size) for l in self.cfg.layers)
+        parts = (seqlib.DecodeAttnPlan.parts_for_tcgen05 if tcgen05 else seqlib.DecodeAttnPlan.parts_for)(B, max_keys)
         key = (B, parts, id(cache))
         g = self._graphs.get(key)
         if g is not None and g.cache is not cache:

@@ -265,6 +265,11 @@ def latent_attn_mma_ok(H: int, r: int, dr: int, dtype: torch.dtype) -> bool:
             and 2 * MMA_ROWS * (r + dr + 8) * 2 + exchange <= 227 * 1024)
 
 
+def latent_attn_tcgen05_ok(H: int, r: int, dr: int, page_size: int) -> bool:
+    """Of those, the shapes csrc/latent_attention_sm100.cu takes: key tiles of 128, one CTA per SM."""
+    return H <= MMA_ROWS and r % 128 == 0 and 0 < r <= 512 and dr <= 64 and dr % 16 == 0 and page_size % 64 == 0
+
+
 class LatentAttnPlan:
     """Work list of one step for one head count (omc_latent_attn_mma): items, merge groups and the partial-result workspace.
     portions: host list of (first_row, n_rows, slot, first_pos) - the consecutive rows of each request in the packed batch.
@@ -327,6 +332,14 @@ class DecodeAttnPlan:
         answer - and with it the captured graph - only a few times)."""
         bucket = 1 << max(max_keys - 1, 0).bit_length()
         return max(1, min(bucket // min_keys, -(-target_ctas // B), LatentAttnPlan.MAX_PARTS))
+
+    @staticmethod
+    def parts_for_tcgen05(B: int, max_keys: int) -> int:
+        """The same for the tcgen05 kernel: a key tile of 128 costs 4 us, a CTA 5 us around its tiles and every further range more merging, so
+        ranges of 256 keys or more, and no more of them than one wave of 148 CTAs has. Measured, attention + merge in us at 4 / 5 / 10 ranges:
+        32 rows over 700 to 2100 keys 29 / 34 / 38; at 16 / 32 / 64: 4 rows over 3000 keys 24 / 28 / 49."""
+        bucket = 1 << max(max_keys - 1, 0).bit_length()
+        return max(1, min(bucket // 256, 148 // B, LatentAttnPlan.MAX_PARTS))
 
     def fill(self, pos: torch.Tensor, slot: torch.Tensor):
         rc = load().omc_latent_decode_items(_ptr(pos), _ptr(slot), self.B, self.H, self.parts, self.window, _ptr(self.items),
