@@ -152,15 +152,17 @@ __global__ void __launch_bounds__(kNormThreads) layernorm_kernel(const bf16* __r
 }
 
 // ------------------------------------------------------------------------------------------------ patch im2col
-// One CTA per row of patches (image b, patch row py): its 14 pixel lines of three channels are read from L1 by the 16-byte pieces of the
-// output that need them. HBM-bound: 21 crops 105 us with one 64-bit division chain per element, 22 us so (floor 12).
+// Four CTAs per row of patches (image b, patch row py): its 14 pixel lines of three channels are read from L1 by the 16-byte pieces of the
+// output that need them. HBM-bound: 21 crops took 105 us with one 64-bit division chain per element (floor 12).
+constexpr int kIm2colSplit = 4;
 // VEC: the output's rows start on 16-byte boundaries.
 template <typename T, bool VEC>
 __global__ void __launch_bounds__(256) im2col_kernel(const T* __restrict__ pix, bf16* __restrict__ cols, long long ldc, int gh, int H, int W) {
   const int gw = W / 14, b = blockIdx.x / gh, py = blockIdx.x - b * gh, nvec = (int)((ldc + 7) >> 3);
   const T* img = pix + (long long)b * 3 * H * W + (long long)py * 14 * W;
   bf16* out = cols + (long long)blockIdx.x * gw * ldc;
-  for (int e = threadIdx.x; e < gw * nvec; e += blockDim.x) {
+  const int e0 = (int)((long long)gw * nvec * blockIdx.y / kIm2colSplit), e1 = (int)((long long)gw * nvec * (blockIdx.y + 1) / kIm2colSplit);
+  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
     const int px = e / nvec, col0 = (e - px * nvec) << 3;
     float v[8];
 #pragma unroll
@@ -513,7 +515,8 @@ extern "C" int omc_vit_im2col(const void* pixels, int pixels_are_f32, void* cols
                               void* stream) {
   if (B <= 0) return OMC_OK;
   if (H % 14 != 0 || W % 14 != 0 || ldc < 588) return set_error(OMC_ERR_SHAPE, "omc_vit_im2col: H, W must be multiples of 14 and ldc >= 588");
-  const int gh = H / 14, grid = B * gh;
+  const int gh = H / 14;
+  const dim3 grid(B * gh, kIm2colSplit);
   const bool vec = ldc % 8 == 0 && reinterpret_cast<uintptr_t>(cols) % 16 == 0;
   cudaStream_t st = (cudaStream_t)stream;
   if (pixels_are_f32 && vec) im2col_kernel<float, true><<<grid, 256, 0, st>>>((const float*)pixels, (bf16*)cols, ldc, gh, H, W);

@@ -20,7 +20,7 @@
 
 namespace omc {
 
-constexpr int kWinWarps = 4;
+constexpr int kWinWarps = 8, kWinKeys = 4;   // keys a warp takes at a time
 constexpr int kWinMaxPerLane = 8;  // value width up to 256
 
 // Rotation of the first `dims` dimensions of every `width` consecutive columns by a host-built table of (cos, sin) [position][dims / 2][2]
@@ -242,23 +242,48 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(const TQ* _
   for (int i = 0; i < kWinMaxPerLane; ++i) acc[i] = 0.f;
   // the visible keys in one sequence of indices: 0 .. kept - 1, then first .. p
   const int n_keys = kept + (p - first + 1);
-  for (int i = warp; i < n_keys; i += kWinWarps) {
-    const int j = i < kept ? i : first + (i - kept);
-    const TC* row = pool + ((long long)bt[j / page_size] * page_size + j % page_size) * W;
-    const TC* kr = row + (kvh * maps + mp) * d;
-    const TC* vr = row + G * maps * d + kvh * dv;
-    float s = 0.f;
-    for (int c = lane; c < d; c += 32) s = fmaf(sq[c], ldf(kr + c), s);
-    s = seq_warp_sum(s) * scale;
-    if (softcap > 0.f) s = softcap * tanhf(s * inv_cap);
-    if (dist_bias != nullptr && p - j < window) s += dist_bias[(long long)(p - j) * H + h];
-    const float mn = fmaxf(m, s);
-    const float corr = expf(m - mn), pj = expf(s - mn);  // m = -inf on the first key: corr = 0
-    l = l * corr + pj;
+  for (int i = warp * kWinKeys; i < n_keys; i += kWinWarps * kWinKeys) {
+    const TC* kr[kWinKeys];
+    const TC* vr[kWinKeys];
+    int back[kWinKeys];
+    float s[kWinKeys];
+#pragma unroll
+    for (int u = 0; u < kWinKeys; ++u) {
+      const int iu = min(i + u, n_keys - 1), j = iu < kept ? iu : first + (iu - kept);
+      const TC* row = pool + ((long long)bt[j / page_size] * page_size + j % page_size) * W;
+      kr[u] = row + (kvh * maps + mp) * d;
+      vr[u] = row + G * maps * d + kvh * dv;
+      back[u] = p - j;
+      s[u] = 0.f;
+    }
+    for (int c = lane; c < d; c += 32) {
+      const float qc = sq[c];
+#pragma unroll
+      for (int u = 0; u < kWinKeys; ++u) s[u] = fmaf(qc, ldf(kr[u] + c), s[u]);
+    }
+    float mn = m;
+#pragma unroll
+    for (int u = 0; u < kWinKeys; ++u) {
+      s[u] = seq_warp_sum(s[u]) * scale;
+      if (softcap > 0.f) s[u] = softcap * tanhf(s[u] * inv_cap);
+      if (dist_bias != nullptr && back[u] < window) s[u] += dist_bias[(long long)back[u] * H + h];
+      if (i + u < n_keys) mn = fmaxf(mn, s[u]);
+    }
+    const float corr = expf(m - mn);  // m = -inf on the first group: corr = 0
+    float pj[kWinKeys];
+#pragma unroll
+    for (int u = 0; u < kWinKeys; ++u) pj[u] = i + u < n_keys ? expf(s[u] - mn) : 0.f;
+    l = l * corr + ((pj[0] + pj[1]) + (pj[2] + pj[3]));
 #pragma unroll
     for (int i2 = 0; i2 < kWinMaxPerLane; ++i2) {
       const int c = lane + 32 * i2;
-      if (c < dv) acc[i2] = acc[i2] * corr + pj * ldf(vr + c);
+      if (c < dv) {
+        float x = acc[i2] * corr;
+#pragma unroll
+        for (int u = 0; u < kWinKeys; ++u)
+          if (i + u < n_keys) x = fmaf(pj[u], ldf(vr[u] + c), x);
+        acc[i2] = x;
+      }
     }
     m = mn;
   }
@@ -321,10 +346,16 @@ __device__ __forceinline__ void w_mma_bf16(float (&c)[4], uint32_t a0, uint32_t 
 __device__ __forceinline__ void w_cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
+// 2^x by the hardware exponential alone: exp2f guards results below 2^-126 with three more instructions, which scores have no use for
+__device__ __forceinline__ float w_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // tanh(x) = 1 - 2 / (exp(2x) + 1) through the hardware exponential and reciprocal: an absolute error of a few 1e-7, where the
 // one-instruction tanh.approx has a relative error of 2^-11 - too coarse for scores, which the soft cap multiplies by tens.
 __device__ __forceinline__ float tanh_approx(float x) {
-  const float e = exp2f(fminf(x, 20.f) * 2.8853900817779268f);
+  const float e = w_exp2(fminf(x, 20.f) * 2.8853900817779268f);
   return 1.f - __fdividef(2.f, e + 1.f);
 }
 __device__ __forceinline__ uint32_t w_pack2(float lo, float hi) {
@@ -356,6 +387,182 @@ struct WinMmaArgs {
   int q_rows;             // rows of the query tile held in shared memory: 64, or the next multiple of 16 above H / G when every item is one token
   int bias_in_smem;       // the bias columns of this key/value head's query heads are staged in shared memory ([window][H / G])
 };
+
+// Decode: items of one token whose query heads per key/value head fit one 16-row tile. The keys are dealt to the CTA's eight warps in tiles of
+// 32; every warp stages its own tile, works on it alone and keeps a partial (max, sum, output), and the partials meet in shared memory at the
+// end. One warp walking all tiles was bound by its own instructions, 7 us per 64 keys: 32 rows x 4 key/value heads of 128 + 128 over
+// up to 512 keys 20 us (60).
+constexpr int kWdWarps = 8, kWdKeys = 32, kWdRows = 16;
+template <int NV, typename TO>
+__global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMmaArgs a) {
+  extern __shared__ __align__(16) unsigned char wsm_raw[];
+  __shared__ float s_m[kWdWarps][kWdRows], s_l[kWdWarps][kWdRows];
+  const int d = a.d, dv = a.dv, pq = d + 8, pv = dv + 8;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  bf16_t* Qs = reinterpret_cast<bf16_t*>(wsm_raw);
+  bf16_t* Ks = Qs + kWdRows * pq + warp * kWdKeys * (pq + pv);   // this warp's keys and values
+  bf16_t* Vs = Ks + kWdKeys * pq;
+  const int t = blockIdx.x, slot = a.slot[t], p = a.pos[t];
+  const int kvh = blockIdx.y / a.maps, mp = blockIdx.y - kvh * a.maps, rep = a.H / a.G;
+  const int qchunks = d >> 3, vchunks = dv >> 3, pieces = qchunks + vchunks;
+  for (int i = tid; i < kWdRows * qchunks; i += blockDim.x) {
+    const int row = i / qchunks, c = i - row * qchunks;
+    *reinterpret_cast<uint4*>(Qs + row * pq + c * 8) =
+        row < rep ? *reinterpret_cast<const uint4*>(a.q + (long long)t * a.ldq + ((kvh * rep + row) * a.maps + mp) * d + c * 8) : make_uint4(0, 0, 0, 0);
+  }
+  const int row0 = g, row1 = g + 8, h0 = kvh * rep + row0 % rep, h1 = kvh * rep + row1 % rep;
+  const int32_t* bt = a.bt + (long long)slot * a.max_pages;
+  const int low = max(max(0, p - a.window + 1), p - p % a.chunk), k_end = p + 1;
+  int k_begin = low, kept_end = min(a.keep_first, k_begin);
+  if (kept_end == k_begin) k_begin = 0, kept_end = 0;
+  const int kept_tiles = (kept_end + kWdKeys - 1) / kWdKeys, n_tiles = kept_tiles + (k_end - k_begin + kWdKeys - 1) / kWdKeys;
+  const int roww = a.G * (a.maps * d + dv);
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  float o[NV][4];
+#pragma unroll
+  for (int j = 0; j < NV; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  const int nv = dv >> 3;
+  constexpr float kLog2e = 1.4426950408889634f;
+  const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+  __syncthreads();
+  for (int kt = warp; kt < n_tiles; kt += kWdWarps) {
+    const int j0 = kt < kept_tiles ? kt * kWdKeys : k_begin + (kt - kept_tiles) * kWdKeys, j_end = kt < kept_tiles ? kept_end : k_end;
+    {
+      const int j = j0 + lane;
+      const int mine = j < j_end ? bt[j / a.page_size] * a.page_size + j % a.page_size : -1;   // the row of the pool that lane's key lies in
+      for (int e = lane; e < kWdKeys * pieces; e += 32) {   // the same number of rounds for every lane
+        const int key = e / pieces, c = e - key * pieces, row = __shfl_sync(0xffffffffu, mine, key);
+        bf16_t* dst = c < qchunks ? Ks + key * pq + c * 8 : Vs + key * pv + (c - qchunks) * 8;
+        if (row >= 0) {
+          const bf16_t* src = a.pool + (long long)row * roww + (c < qchunks ? (kvh * a.maps + mp) * d + c * 8 : a.G * a.maps * d + kvh * dv + (c - qchunks) * 8);
+          w_cp_async16(wsmem_u32(dst), src);
+        } else {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+    }
+    float s[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+    const uint32_t q_base = wsmem_u32(Qs + ((lane & 7) + 8 * ((lane >> 3) & 1)) * pq + 8 * (lane >> 4));
+    const uint32_t k_base = wsmem_u32(Ks + ((lane & 7) + 8 * (lane >> 4)) * pq + 8 * ((lane >> 3) & 1));
+    for (int kk = 0; kk < d; kk += 16) {
+      uint32_t a0, a1, a2, a3;
+      w_ldsm_x4(q_base + kk * 2, a0, a1, a2, a3);
+#pragma unroll
+      for (int n2 = 0; n2 < 2; ++n2) {
+        uint32_t b0, b1, b2, b3;
+        w_ldsm_x4(k_base + (n2 * 16 * pq + kk) * 2, b0, b1, b2, b3);
+        w_mma_bf16(s[2 * n2], a0, a1, a2, a3, b0, b1);
+        w_mma_bf16(s[2 * n2 + 1], a0, a1, a2, a3, b2, b3);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int key = j0 + n * 8 + 2 * t4 + (e & 1), dist = p - key;
+        float v = a.softcap > 0.f ? a.softcap * tanh_approx(s[n][e] * a.scale * inv_cap) : s[n][e] * a.scale;
+        if (a.bias != nullptr) {
+          const float bias = __ldg(a.bias + (long long)min(max(dist, 0), a.window - 1) * a.H + (e < 2 ? h0 : h1));
+          v += dist < a.window ? bias : 0.f;
+        }
+        s[n][e] = key < j_end && (key >= low || key < a.keep_first) ? v * kLog2e : -INFINITY;
+      }
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1]));
+      mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
+    }
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
+    const float ms0 = mn0 == -INFINITY ? 0.f : mn0, ms1 = mn1 == -INFINITY ? 0.f : mn1;   // rows that see nothing yet
+    const float c0 = w_exp2(m0 - ms0), c1 = w_exp2(m1 - ms1);
+    m0 = mn0;
+    m1 = mn1;
+    float rs0 = 0.f, rs1 = 0.f;
+    uint32_t pr[4][2];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) {
+      pr[n][0] = w_pack2(w_exp2(s[n][0] - ms0), w_exp2(s[n][1] - ms0));
+      pr[n][1] = w_pack2(w_exp2(s[n][2] - ms1), w_exp2(s[n][3] - ms1));
+      // the denominator sums the ROUNDED probabilities, the ones the numerator uses
+      const float2 f0 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&pr[n][0]));
+      const float2 f1 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&pr[n][1]));
+      rs0 += f0.x + f0.y;
+      rs1 += f1.x + f1.y;
+    }
+    l0 = l0 * c0 + rs0;
+    l1 = l1 * c1 + rs1;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) o[j][0] *= c0, o[j][1] *= c0, o[j][2] *= c1, o[j][3] *= c1;
+    const uint32_t v_base = wsmem_u32(Vs + ((lane & 7) + 8 * ((lane >> 3) & 1)) * pv + 8 * (lane >> 4));
+#pragma unroll
+    for (int kb16 = 0; kb16 < 2; ++kb16) {
+      const uint32_t a0 = pr[2 * kb16][0], a1 = pr[2 * kb16][1], a2 = pr[2 * kb16 + 1][0], a3 = pr[2 * kb16 + 1][1];
+#pragma unroll
+      for (int j = 0; j < NV; j += 2) {
+        if (j < nv) {   // dv is a multiple of 16: tiles come in pairs
+          uint32_t b0, b1, b2, b3;
+          w_ldsm_x4_t(v_base + (kb16 * 16 * pv + j * 8) * 2, b0, b1, b2, b3);
+          w_mma_bf16(o[j], a0, a1, a2, a3, b0, b1);
+          w_mma_bf16(o[j + 1], a0, a1, a2, a3, b2, b3);
+        }
+      }
+    }
+    __syncwarp();   // every lane is done with the tile
+  }
+  l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
+  l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+  l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
+  l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  if (t4 == 0) {
+    s_m[warp][row0] = m0, s_l[warp][row0] = l0;
+    s_m[warp][row1] = m1, s_l[warp][row1] = l1;
+  }
+  __syncthreads();   // the tiles' place is free as well
+  float* part = reinterpret_cast<float*>(wsm_raw);   // [warps][rows][dv]
+#pragma unroll
+  for (int j = 0; j < NV; ++j)
+    if (j < nv) {
+      const int col = j * 8 + 2 * t4;
+      if (row0 < rep) *reinterpret_cast<float2*>(part + (warp * kWdRows + row0) * dv + col) = make_float2(o[j][0], o[j][1]);
+      if (row1 < rep) *reinterpret_cast<float2*>(part + (warp * kWdRows + row1) * dv + col) = make_float2(o[j][2], o[j][3]);
+    }
+  __syncthreads();
+  auto gact = [&](float z) { return a.gate_act == 1 ? z / (1.f + __expf(-z)) : (a.gate_act == 2 ? 1.f / (1.f + __expf(-z)) : z); };
+  for (int e = tid; e < rep * (dv >> 1); e += blockDim.x) {
+    const int row = e / (dv >> 1), col = (e - row * (dv >> 1)) * 2, h = kvh * rep + row;
+    const float sk = a.sink != nullptr ? a.sink[h] * kLog2e : -INFINITY;
+    float mt = sk;
+#pragma unroll
+    for (int w = 0; w < kWdWarps; ++w) mt = fmaxf(mt, s_m[w][row]);
+    float lt = a.sink != nullptr ? w_exp2(sk - mt) : 0.f, x0 = 0.f, x1 = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWdWarps; ++w) {
+      if (s_m[w][row] == -INFINITY) continue;   // a warp without keys
+      const float f = w_exp2(s_m[w][row] - mt);
+      const float2 v = *reinterpret_cast<const float2*>(part + (w * kWdRows + row) * dv + col);
+      lt = fmaf(s_l[w][row], f, lt);
+      x0 = fmaf(v.x, f, x0);
+      x1 = fmaf(v.y, f, x1);
+    }
+    float inv = 1.f / lt;
+    float g0 = 1.f, g1 = 1.f;
+    if (a.gate != nullptr && a.gate_heads) inv *= gact(a.gate[(long long)t * a.ldg + h * a.maps + mp]);
+    else if (a.gate != nullptr) {
+      const float* gp = a.gate + (long long)t * a.ldg + (h * a.maps + mp) * dv + col;
+      g0 = gact(gp[0]), g1 = gact(gp[1]);
+    }
+    w_st_pair(static_cast<TO*>(a.out) + (long long)t * a.ldo + (h * a.maps + mp) * dv + col, x0 * inv * g0, x1 * inv * g1);
+  }
+}
 
 template <int NV, typename TO>  // NV: 8-column output tiles, dv <= 8 * NV
 __global__ void __launch_bounds__(128) window_attn_mma_kernel(WinMmaArgs a) {
@@ -403,7 +610,7 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(WinMmaArgs a) {
   auto stage = [&](int buf, int tile) {
     const int j0 = tile < kept_tiles ? tile * kWmKeys : k_begin + (tile - kept_tiles) * kWmKeys, j_end = tile < kept_tiles ? kept_end : k_end;
     const int half = tid & 1;
-    for (int key = tid >> 1; key < kWmKeys; key += blockDim.x >> 1) {   // one pass with 128 threads, two with the 64 of a one-token item
+    for (int key = tid >> 1; key < kWmKeys; key += blockDim.x >> 1) {
       const int j = j0 + key;
       bf16_t* kd = Ks + (buf * kWmKeys + key) * pq;
       bf16_t* vd = Vs + (buf * kWmKeys + key) * pv;
@@ -457,27 +664,43 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(WinMmaArgs a) {
           w_mma_bf16(s[2 * n2 + 1], a0, a1, a2, a3, b2, b3);
         }
       }
-      // scale, soft cap, distance bias, window: scores in base-2 units
+      // scale, soft cap, distance bias, window: scores in base-2 units. One uniform question at a time over all of a thread's scores (a
+      // branch per score cost more than its arithmetic), and no mask where the whole tile is seen by all of the item's rows
+      if (a.softcap > 0.f) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[n][e] = a.softcap * kLog2e * tanh_approx(s[n][e] * a.scale * inv_cap);
+      } else {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) s[n][e] *= a.scale * kLog2e;
+      }
+      if (a.bias != nullptr) {   // the table has one row per distance inside the window
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int dist = (e < 2 ? p0 : p1) - (j0 + n * 8 + 2 * t4 + (e & 1)), at = min(max(dist, 0), a.window - 1), hh = e < 2 ? h0 : h1;
+            const float v = a.bias_in_smem ? sbias[at * rep + (hh - kvh * rep)] : __ldg(a.bias + (long long)at * a.H + hh);
+            s[n][e] += dist < a.window ? v * kLog2e : 0.f;
+          }
+      }
+      const bool whole = j0 + kWmKeys <= j_end && j0 + kWmKeys - 1 <= first_pos && kt >= kept_tiles && j0 >= k_end - 1 - (k_end - 1) % a.chunk &&
+                         (long long)j0 > (long long)first_pos + n_tok - 1 - a.window;
+      if (!whole) {
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int key = j0 + n * 8 + 2 * t4 + (e & 1), p = e < 2 ? p0 : p1, low = e < 2 ? low0 : low1;
+            s[n][e] = key < j_end && key <= p && (key >= low || key < a.keep_first) ? s[n][e] : -INFINITY;
+          }
+      }
       float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int key = j0 + n * 8 + 2 * t4 + (e & 1);
-          const int p = e < 2 ? p0 : p1, hh = e < 2 ? h0 : h1, low = e < 2 ? low0 : low1;
-          const int dist = p - key;
-          float v = -INFINITY;
-          if (key < j_end && dist >= 0 && (key >= low || key < a.keep_first)) {
-            v = s[n][e] * a.scale;
-            if (a.softcap > 0.f) v = a.softcap * tanh_approx(v * inv_cap);
-            if (dist < a.window) {   // the table has one row per distance inside the window
-              if (a.bias_in_smem) v += sbias[dist * rep + (hh - kvh * rep)];
-              else if (a.bias != nullptr) v += __ldg(a.bias + (long long)dist * a.H + hh);
-            }
-            v *= kLog2e;
-          }
-          s[n][e] = v;
-        }
         mx0 = fmaxf(mx0, fmaxf(s[n][0], s[n][1]));
         mx1 = fmaxf(mx1, fmaxf(s[n][2], s[n][3]));
       }
@@ -487,15 +710,15 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(WinMmaArgs a) {
       mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
       const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
       const float ms0 = mn0 == -INFINITY ? 0.f : mn0, ms1 = mn1 == -INFINITY ? 0.f : mn1;   // rows that see nothing yet
-      const float c0 = exp2f(m0 - ms0), c1 = exp2f(m1 - ms1);
+      const float c0 = w_exp2(m0 - ms0), c1 = w_exp2(m1 - ms1);
       m0 = mn0;
       m1 = mn1;
       float rs0 = 0.f, rs1 = 0.f;
       uint32_t p[8][2];
 #pragma unroll
       for (int n = 0; n < 8; ++n) {
-        p[n][0] = w_pack2(exp2f(s[n][0] - ms0), exp2f(s[n][1] - ms0));
-        p[n][1] = w_pack2(exp2f(s[n][2] - ms1), exp2f(s[n][3] - ms1));
+        p[n][0] = w_pack2(w_exp2(s[n][0] - ms0), w_exp2(s[n][1] - ms0));
+        p[n][1] = w_pack2(w_exp2(s[n][2] - ms1), w_exp2(s[n][3] - ms1));
         // the denominator sums the ROUNDED probabilities, the ones the numerator uses
         const float2 f0 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&p[n][0]));
         const float2 f1 = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&p[n][1]));
@@ -890,6 +1113,7 @@ extern "C" int omc_window_attn(const void* q, long long ldq, int T, int H, int G
   const size_t smem = sizeof(float) * ((size_t)d + (size_t)kWinWarps * dv + 2 * kWinWarps);
   if (smem > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_window_attn: head width too large");
   OMC_DT_SWITCH(dt, TC, OMC_DT_SWITCH(out_dt, TY, {
+    if (smem > 48 * 1024) cudaFuncSetAttribute(window_attn_kernel<TC, TC, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     window_attn_kernel<TC, TC, TY><<<dim3(T, H * maps), kWinWarps * 32, smem, st>>>(static_cast<const TC*>(q), ldq, H, G, d, dv, maps,
                                                                                    static_cast<const TC*>(pool), block_table, max_pages,
                                                                                    page_size, pos, slot, window, chunk, keep_first, scale, softcap,
@@ -928,17 +1152,21 @@ extern "C" int omc_window_attn_mma(const void* q, long long ldq, int T, int H, i
     smem += bias_bytes;
   }
   dim3 grid(n, G * maps);
-  // one token per item and at most 16 rows: one warp computes, a second helps staging - half the registers per CTA, so that
-  // (with the smaller query tile) four CTAs share an SM instead of three
-  const int threads = a.q_rows == 16 ? 64 : 128;
+  // one token per item and at most 16 rows, in tiles of 32 keys per warp that fit shared memory: the warps split the keys
+  const size_t part_bytes = sizeof(float) * kWdWarps * kWdRows * (size_t)dv;
+  size_t dec_smem = sizeof(bf16_t) * ((size_t)kWdRows * (d + 8) + (size_t)kWdWarps * kWdKeys * (d + dv + 16));
+  if (dec_smem < part_bytes) dec_smem = part_bytes;
+  const bool decode = items == nullptr && H / G <= kWdRows && dec_smem <= 220 * 1024;
 #define OMC_WIN_LAUNCH(NV, TO)                                                                                      \
   do {                                                                                                              \
     static bool attr_done[kMaxDevices] = {};                                                                        \
     if (!attr_done[cur_device()]) {                                                                                 \
       cudaFuncSetAttribute(window_attn_mma_kernel<NV, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
+      cudaFuncSetAttribute(window_attn_decode_kernel<NV, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); \
       attr_done[cur_device()] = true;                                                                               \
     }                                                                                                               \
-    window_attn_mma_kernel<NV, TO><<<grid, threads, smem, st>>>(a);                                                     \
+    if (decode) window_attn_decode_kernel<NV, TO><<<grid, kWdWarps * 32, dec_smem, st>>>(a);                        \
+    else window_attn_mma_kernel<NV, TO><<<grid, 128, smem, st>>>(a);                                                \
   } while (0)
   if (out_dt == OMC_DT_BF16) {
     if (dv <= 64) OMC_WIN_LAUNCH(8, bf16_t);
