@@ -2,7 +2,7 @@
 
 Matrices with at least TENSOR_GEMM_MIN_WEIGHT elements go through the tcgen05 GEMM of the core library when the operands are bf16
 and the dimensions are multiples of 8; below it a launch is latency-bound either way and the kernel of the sequence-step library
-(FMA pipe for fp32 or ragged shapes, mma.sync for aligned bf16) needs no second library. Steps of up to 64 rows stream the weights
+(FMA pipe for fp32 or ragged shapes, tcgen05 tiles for aligned bf16) needs no second library. Steps of up to 64 rows stream the weights
 through the skinny GEMM from a much smaller size on: the small-matrix kernel walks K with one row tile per CTA, which leaves a
 decode step waiting on a handful of CTAs. The choice depends on widths, layout and dtypes only, never on what else is in the
 batch beyond the 64-row threshold of the skinny kernel, and every kernel accumulates a row's K terms in an order of its own
