@@ -6,7 +6,7 @@
 // MMA issuer. Warps 2..5: epilogue, thread = row. The K terms of an output are added in one order whatever the tile, so a row's result does
 // not depend on M.
 // What bounds it: the output's and the gate's bytes (51 MB, 1.4 TB/s), behind the set-up and the first load of a tile. 3126 rows x 16 heads, 128 -> 512:
-// 38 us = 690 TFLOP/s; 512 -> 128 with a gate per element 41 us; 32 rows: 6 us each (mma.sync with a two-stage cp.async ring before: 140, 141, 21).
+// 38 us = 690 TFLOP/s; 512 -> 128 with a gate per element 48 us; 32 rows: 6 us each (mma.sync with a two-stage cp.async ring before: 140, 141, 21).
 #include "linear_args.cuh"
 #include "sm100_step.cuh"
 
@@ -151,8 +151,7 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
               float f[8];
               hg_row(src + (i0 + i) * 4 * kHgPitch, a.alpha, f);
 #pragma unroll
-              for (int j = 0; j < 8; ++j)   // a bf16 output keeps 8 of the quotient's bits
-                f[j] = sizeof(TY) == 2 ? __fdividef(f[j], 1.f + __expf(-z[i][j])) : f[j] / (1.f + __expf(-z[i][j]));
+              for (int j = 0; j < 8; ++j) f[j] /= 1.f + __expf(-z[i][j]);   // as at the edges: a row's bits do not depend on its tile
               hg_store(y + (long long)((i0 + i) * 4) * a.ldy, f);
             }
           }
