@@ -13,8 +13,9 @@
 //                product that reads it is done
 //   warp 1       MMA issuer (one thread)
 //   warps 2..9   softmax: thread = one key x half the rows. Maxima over keys are maxima over lanes: a transposing butterfly leaves every
-//                lane with one row's maximum. The reference maximum of a row only moves when it grew by more than 2^8 (the sums are scaled by it
-//                consistently, so this is exact), the output accumulators are then rescaled in TMEM; sums stay per thread until the end.
+//                lane with one row's maximum. The reference of a row is its running maximum, so its largest probability is 1 and takes no
+//                rounding (one that lags behind saves passes over TMEM, but rounds that probability to bf16 as well); where it grew,
+//                the output accumulators are rescaled in TMEM. Sums stay per thread until the end.
 //                P^T goes to shared memory as the B operand; where Q and the key tile fill it (r = 512) it takes the place of the rotated
 //                chunk, which the scores have consumed.
 // What bounds it: shared memory holds one key tile, so a tile of 8300 cycles is a load that only the output products overlap (3100), 68 instructions
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       if (stid < NR) {
         const float now = fmaxf(fmaxf(sh->part[0][stid], sh->part[1][stid]), fmaxf(sh->part[2][stid], sh->part[3][stid]));
         const float old = sh->mref[stid];
-        if (now > old + 8.f) {               // also the first finite maximum of a row
+        if (now > old) {                     // also the first finite maximum of a row
           sh->fac[stid] = ls_exp2(old - now);
           sh->mref[stid] = now;
           sh->rescale[t & 1] = 1u;

@@ -79,6 +79,29 @@ def test_against_float64(H, r, dr, page, window, portions, opt):
             assert (err <= bound).all(), (plan.n_items, plan.max_rows, dt, float((err - bound).max()))
 
 
+@pytest.mark.parametrize("r,dr,page", [(512, 64, 64), (256, 16, 64), (128, 64, 128), (512, 64, 32)])
+@pytest.mark.parametrize("parts", [1, 2])
+def test_the_largest_probability_takes_no_rounding(r, dr, page, parts):
+    """128 keys of one score and, in the next tile, one whose probability is 128.49 times theirs: relative to the row's maximum every number is
+    exact in bf16, relative to the first tile's 128.49 would become 128 (an error of 1e-3 in the output). Page 32: the mma.sync kernel."""
+    H, n, D = 16, 129, r + dr
+    pages = -(-n // page)
+    rows = torch.zeros(pages * page, D)
+    rows[n - 1, :r] = 1.0                                                        # the last key's value; the others' is zero
+    rows[n - 1, r] = 1.0                                                         # its score is the scale, theirs zero
+    q = torch.zeros(1, H, D)
+    q[:, :, r] = 1.0
+    pos, slot = torch.tensor([n - 1], dtype=torch.int32).cuda(), torch.zeros(1, dtype=torch.int32).cuda()
+    plan = seqlib.DecodeAttnPlan(1, H, parts, "cuda")
+    plan.fill(pos, slot)
+    out = torch.empty(1, H, r, device="cuda")
+    table = torch.arange(pages, dtype=torch.int32).view(1, -1).cuda()
+    seqlib.latent_attn_mma(q.to(torch.bfloat16).cuda(), r, dr, rows.to(torch.bfloat16).view(pages, page, D).cuda(), table, page, plan, None, math.log(128.49),
+                           out)
+    # the exponent (7) is known to 2^-21, the hardware exponential to 2^-22, the sums of 129 terms to 2^-17
+    assert (out.double().cpu() - 128.49 / (128.49 + 128)).abs().max() < 1e-5
+
+
 def test_no_wait_ran_out():
     import ctypes
     n = ctypes.c_uint(7)
