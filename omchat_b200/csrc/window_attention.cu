@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
     float lt = a.sink != nullptr ? w_exp2(sk - mt) : 0.f, x0 = 0.f, x1 = 0.f;
 #pragma unroll
     for (int w = 0; w < kWdWarps; ++w) {
-      if (s_m[w][row] == -INFINITY) continue;   // a warp without keys
+      if (w >= n_tiles) break;                  // warps without keys; one whose scores are all NaN has a maximum of -infinity as well, and counts
       const float f = w_exp2(s_m[w][row] - mt);
       const float2 v = *reinterpret_cast<const float2*>(part + (w * kWdRows + row) * dv + col);
       lt = fmaf(s_l[w][row], f, lt);
