@@ -109,6 +109,11 @@ int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, int dr, cons
  * on a sound device; the outputs of a launch that had one are not valid). Synchronises with the device. */
 int omc_step_wait_failures(unsigned int* count);
 
+/* Runs out of a wait on purpose, with nothing under way: out (device, int32 [4]) receives 0 (the wait), 0 (the next one, refused at once), 0 (a
+ * wait for what would still come, refused as well), 1 (the same as a drain of what was issued, which is waited for all the same). Adds one to
+ * the count above. */
+int omc_step_wait_selfcheck(int32_t* out, void* stream);
+
 /* The work list of a decode-only step, written on the device from pos / slot (one row per request, `parts` <= 64 key ranges each):
  * items int32 [B * parts][8], merges int32 [B][4] (untouched when parts == 1). Lets a CUDA graph replay the step as contexts grow. */
 int omc_latent_decode_items(const int32_t* pos, const int32_t* slot, int B, int H, int parts, int window, int32_t* items,

@@ -48,7 +48,7 @@ struct LatSmArgs {
 };
 
 struct LatSmShared {
-  uint64_t q_full, s_full, p_ready, full[4], o_done[4];
+  uint64_t q_full, s_full, p_ready, mma_done, full[4], o_done[4];
   uint32_t tmem, dead, rescale[2];
   alignas(16) float mref[kLsMaxRows];
   alignas(16) float fac[kLsMaxRows];
@@ -60,7 +60,8 @@ __device__ __forceinline__ float ls_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ void ls_wait(LatSmShared* sh, uint64_t* bar, uint32_t parity) { wait_bounded(bar, parity, &sh->dead, &g_latent_failures); }
+__device__ __forceinline__ bool ls_wait(LatSmShared* sh, uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, &sh->dead, &g_latent_failures); }
+__device__ __forceinline__ void ls_drain(LatSmShared* sh, uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, &sh->dead, &g_latent_failures); }
 __device__ __forceinline__ void ls_softmax_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLsSoftmax) : "memory"); }
 
 // v[c]: this lane's value of column c. Returns the reduction over the 32 lanes of column lane / (32 / NC) (v is overwritten).
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     mbar_init(&sh->q_full, 1);
     mbar_init(&sh->s_full, 1);
     mbar_init(&sh->p_ready, kLsSoftmax / 32);
+    mbar_init(&sh->mma_done, 1);
     for (int m = 0; m < 4; ++m) {
       mbar_init(&sh->full[m], 1);
       mbar_init(&sh->o_done[m], 1);
@@ -172,16 +174,14 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
 
   if (warp == 0) {
     if (lane == 0 && n_tiles > 0) {
-      for (int t = 1; t < n_tiles; ++t) {
+      int t = 0, upto = nm;                  // the copies of tile t have been issued for the first `upto` groups, those of the tile before for the others
+      while (upto == nm && t + 1 < n_tiles) {
         int row[2];
-        box_rows(t, row);
-        for (int g = 0; g < nm; ++g) {
-          ls_wait(sh, &sh->o_done[g], (t - 1) & 1);
-          load_pair(row, g);
-        }
+        box_rows(++t, row);
+        for (upto = 0; upto < nm && ls_wait(sh, &sh->o_done[upto], (t - 1) & 1); ++upto) load_pair(row, upto);
       }
-      ls_wait(sh, &sh->q_full, 0);           // nothing is on its way any more when this thread leaves
-      for (int g = 0; g < nm; ++g) ls_wait(sh, &sh->full[g], (n_tiles - 1) & 1);
+      ls_drain(sh, &sh->q_full, 0);          // nothing is on its way any more when this thread leaves
+      for (int g = 0; g < nm; ++g) ls_drain(sh, &sh->full[g], (g < upto ? t : t - 1) & 1);
     }
   } else if (warp == 1) {
     if (elect_one() && n_tiles > 0) {
@@ -192,10 +192,11 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       const uint64_t dv0 = make_sw128_mnmajor_desc(smem_u32(ks), kChunkBytes, 1024);
       const uint64_t dp0 = NR == 64 ? make_sw128_mnmajor_desc(p_addr, 1024, 1024) : make_sw128_kmajor_desc(p_addr);
       const int tail = (a.D - (a.nc - 1) * 64 + 15) >> 4;   // steps of 16 in the last chunk
-      ls_wait(sh, &sh->q_full, 0);
-      for (int t = 0; t < n_tiles; ++t) {
+      bool go = ls_wait(sh, &sh->q_full, 0);
+      for (int t = 0; go && t < n_tiles; ++t) {
         for (int g = 0; g < nm; ++g) {
-          ls_wait(sh, &sh->full[g], t & 1);
+          go = ls_wait(sh, &sh->full[g], t & 1);
+          if (!go) break;
           tc_fence_after();
           const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
           for (int c = 2 * g; c < c1; ++c) {
@@ -206,8 +207,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
               if (k < steps) umma_bf16<1>(tmem_s, dk + 2 * k, dq + 2 * k, idesc_s, (c | k) != 0 ? 1u : 0u);
           }
         }
+        if (!go) break;
         umma_commit(&sh->s_full);            // also: the output products of the tile before are done
-        ls_wait(sh, &sh->p_ready, t & 1);
+        go = ls_wait(sh, &sh->p_ready, t & 1);
+        if (!go) break;
         tc_fence_after();
         for (int m = 0; m < nm; ++m) {
           const uint64_t dv = dv0 + (uint64_t)(m * (2 * kChunkBytes >> 4));
@@ -218,6 +221,8 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
           umma_commit(&sh->o_done[m]);
         }
       }
+      umma_commit(&sh->mma_done);
+      ls_drain(sh, &sh->mma_done, 0);        // every product that was issued is done
     }
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2,   // TMEM lanes go by warp % 4

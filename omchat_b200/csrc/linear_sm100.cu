@@ -55,7 +55,8 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
   uint8_t* ring = hg_raw + ((1024u - (smem_u32(hg_raw) & 1023u)) & 1023u);
   const int m0 = blockIdx.y * kHgBM, n0 = blockIdx.x * BN, b = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nk = (a.K + kHgBK - 1) / kHgBK;
-  auto wait = [&](uint64_t* bar, uint32_t parity) { wait_bounded(bar, parity, &sh->dead, &g_linear_failures); };
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, &sh->dead, &g_linear_failures); };
+  auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, &sh->dead, &g_linear_failures); };
   auto load = [&](int kb) {
     uint8_t* sa = ring + (kb % stages) * kStage;
     uint64_t* bar = &sh->full[kb % stages];
@@ -86,17 +87,15 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
   const uint32_t tmem = sh->tmem;
   if (warp == 0) {
     if (lane == 0) {
-      for (int kb = stages; kb < nk; ++kb) {
-        wait(&sh->empty[kb % stages], (kb / stages - 1) & 1);
-        load(kb);
-      }
-      for (int kb = max(0, nk - stages); kb < nk; ++kb) wait(&sh->full[kb % stages], (kb / stages) & 1);   // nothing is on its way any more
+      int issued = min(stages, nk);
+      for (; issued < nk && wait(&sh->empty[issued % stages], (issued / stages - 1) & 1); ++issued) load(issued);
+      for (int kb = max(0, issued - stages); kb < issued; ++kb) drain(&sh->full[kb % stages], (kb / stages) & 1);   // nothing is on its way any more
     }
   } else if (warp == 1) {
     if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(kHgBM, BN);
       for (int kb = 0; kb < nk; ++kb) {
-        wait(&sh->full[kb % stages], (kb / stages) & 1);
+        if (!wait(&sh->full[kb % stages], (kb / stages) & 1)) break;
         tc_fence_after();
         const uint32_t sa = smem_u32(ring + (kb % stages) * kStage);
         const uint64_t da = make_sw128_kmajor_desc(sa), db = make_sw128_kmajor_desc(sa + kA);
@@ -105,6 +104,7 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
         umma_commit(&sh->empty[kb % stages]);
       }
       umma_commit(&sh->done);
+      drain(&sh->done, 0);   // every product that was issued is done
     }
   } else {
     // thread = row while the accumulator is read, eight neighbouring threads = one row of 64 columns while gates come in and outputs go out
@@ -112,9 +112,9 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
     const int quarter = warp & 3;
     float* slab = reinterpret_cast<float*>(ring) + quarter * 32 * kHgPitch;
     const bool plain = vec_out && a.act == OMC_ACT_NONE && a.bias == nullptr && (a.gate == nullptr || vec_gate);
-    wait(&sh->done, 0);
+    const bool done = wait(&sh->done, 0);
     tc_fence_after();
-    for (int c = 0; c < BN && n0 + c < a.N; c += 64) {
+    for (int c = 0; done && c < BN && n0 + c < a.N; c += 64) {
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         uint32_t v[32];
@@ -242,7 +242,36 @@ int linear_sm100(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
 
 int latent_sm100_failures(unsigned int* n);   // latent_attention_sm100.cu
 
+// out: a wait for a barrier that nothing arrives at; the next one for it; one for a barrier that a later thread arrives at, as a wait and as a drain
+__global__ void step_wait_selfcheck_kernel(int32_t* out) {
+  __shared__ uint64_t never, late;
+  __shared__ uint32_t dead;
+  if (threadIdx.x == 0) {
+    mbar_init(&never, 1);
+    mbar_init(&late, 1);
+    dead = 0u;
+    fence_barrier_init();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    out[0] = wait_bounded(&never, 0, &dead, &g_linear_failures, 8);
+    out[1] = wait_bounded(&never, 0, &dead, &g_linear_failures);
+    out[2] = wait_bounded(&late, 0, &dead, &g_linear_failures);
+    out[3] = drain_bounded(&late, 0, &dead, &g_linear_failures);
+  } else if (threadIdx.x == 32) {
+    for (int i = 0; i < 1000000 && !*reinterpret_cast<volatile uint32_t*>(&dead); ++i) __nanosleep(1000);   // thread 0 sets it after its eight tries
+    __nanosleep(200000);
+    mbar_arrive(&late);
+  }
+}
+
 }  // namespace omc
+
+extern "C" int omc_step_wait_selfcheck(int32_t* out, void* stream) {
+  if (out == nullptr) return omc::set_error(OMC_ERR_ARG, "omc_step_wait_selfcheck: bad argument");
+  omc::step_wait_selfcheck_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(out);
+  return omc::check_launch("omc_step_wait_selfcheck");
+}
 
 extern "C" int omc_step_wait_failures(unsigned int* count) {
   unsigned int linear = 0, latent = 0;

@@ -7,15 +7,24 @@
 
 namespace omc {
 
-// A wait gives up after this many tries (each lets the hardware suspend the thread for a while), or once another wait of the CTA has. The
-// CTA then runs on to its end through the same sequence of barriers, its copies are still waited for (in the same bounded way) and its
-// tensor memory is freed; what it wrote is not valid, and `failures` (a counter in device memory) says so.
-constexpr uint32_t kWaitTries = 1u << 22;
-__device__ __forceinline__ void wait_bounded(uint64_t* bar, uint32_t parity, uint32_t* dead, unsigned int* failures) {
+// A wait gives up after this many tries (each lets the hardware suspend the thread for a while), or at once where another wait of the CTA
+// has, and returns whether its phase has come. Who was refused issues no more copies and no more products; the CTA runs on to its end
+// through the same sequence of block barriers. What it wrote is not valid, and `failures` (a counter in device memory) says so.
+constexpr uint32_t kWaitTries = 1u << 22, kDrainTries = 1u << 20;
+__device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, uint32_t* dead, unsigned int* failures, uint32_t tries = kWaitTries) {
   for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i) {
-    if (i >= kWaitTries && atomicExch(dead, 1u) == 0u) atomicAdd(failures, 1u);
-    if (*reinterpret_cast<volatile uint32_t*>(dead)) return;
+    if (i >= tries && atomicExch(dead, 1u) == 0u) atomicAdd(failures, 1u);
+    if (*reinterpret_cast<volatile uint32_t*>(dead)) return false;
   }
+  return true;
+}
+// For copies and products that have been issued: none may be under way into shared or tensor memory when the CTA gives these back, so these
+// waits have tries of their own whether or not another wait has given up.
+__device__ __forceinline__ bool drain_bounded(uint64_t* bar, uint32_t parity, uint32_t* dead, unsigned int* failures) {
+  for (uint32_t i = 0; i < kDrainTries; ++i)
+    if (mbar_try_wait(bar, parity)) return true;
+  if (atomicExch(dead, 1u) == 0u) atomicAdd(failures, 1u);
+  return false;
 }
 
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
