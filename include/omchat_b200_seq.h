@@ -109,6 +109,10 @@ int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, int dr, cons
  * on a sound device; the outputs of a launch that had one are not valid). Synchronises with the device. */
 int omc_step_wait_failures(unsigned int* count);
 
+/* 1 once that count is not 0 on any device, else 0, without synchronising: for who has waited for a step's results. From then on the launches
+ * of tcgen05 kernels on that device return OMC_ERR_CUDA. */
+int omc_step_wait_failed(void);
+
 /* Runs out of a wait on purpose, with nothing under way: out (device, int32 [4]) receives 0 (the wait), 0 (the next one, refused at once), 0 (a
  * wait for what would still come, refused as well), 1 (the same as a drain of what was issued, which is waited for all the same). Adds one to
  * the count above. */

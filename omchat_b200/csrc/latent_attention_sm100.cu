@@ -45,6 +45,7 @@ struct LatSmArgs {
   int p_offset;                                    // of P^T, in bytes behind Q
   int tmem_cols;
   float scale_log2;
+  unsigned int* failed;
 };
 
 struct LatSmShared {
@@ -60,8 +61,6 @@ __device__ __forceinline__ float ls_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ bool ls_wait(LatSmShared* sh, uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, &sh->dead, &g_latent_failures); }
-__device__ __forceinline__ void ls_drain(LatSmShared* sh, uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, &sh->dead, &g_latent_failures); }
 __device__ __forceinline__ void ls_softmax_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLsSoftmax) : "memory"); }
 
 // v[c]: this lane's value of column c. Returns the reduction over the 32 lanes of column lane / (32 / NC) (v is overwritten).
@@ -123,6 +122,9 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   const int nm = a.r >> 7;                   // 128-dimension tiles of the output
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
+  const WaitReport report{&sh->dead, &g_latent_failures, a.failed};
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, report); };
+  auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, report); };
   const int32_t* bt = a.bt + (long long)slot * a.max_pages;
   // rows of the pool where the two boxes of tile t start (looked up a tile ahead: a lookup takes as long as 20 KB of the copies)
   auto box_rows = [&](int t, int (&row)[2]) {
@@ -178,10 +180,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       while (upto == nm && t + 1 < n_tiles) {
         int row[2];
         box_rows(++t, row);
-        for (upto = 0; upto < nm && ls_wait(sh, &sh->o_done[upto], (t - 1) & 1); ++upto) load_pair(row, upto);
+        for (upto = 0; upto < nm && wait(&sh->o_done[upto], (t - 1) & 1); ++upto) load_pair(row, upto);
       }
-      ls_drain(sh, &sh->q_full, 0);          // nothing is on its way any more when this thread leaves
-      for (int g = 0; g < nm; ++g) ls_drain(sh, &sh->full[g], (g < upto ? t : t - 1) & 1);
+      drain(&sh->q_full, 0);          // nothing is on its way any more when this thread leaves
+      for (int g = 0; g < nm; ++g) drain(&sh->full[g], (g < upto ? t : t - 1) & 1);
     }
   } else if (warp == 1) {
     if (elect_one() && n_tiles > 0) {
@@ -192,10 +194,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       const uint64_t dv0 = make_sw128_mnmajor_desc(smem_u32(ks), kChunkBytes, 1024);
       const uint64_t dp0 = NR == 64 ? make_sw128_mnmajor_desc(p_addr, 1024, 1024) : make_sw128_kmajor_desc(p_addr);
       const int tail = (a.D - (a.nc - 1) * 64 + 15) >> 4;   // steps of 16 in the last chunk
-      bool go = ls_wait(sh, &sh->q_full, 0);
+      bool go = wait(&sh->q_full, 0);
       for (int t = 0; go && t < n_tiles; ++t) {
         for (int g = 0; g < nm; ++g) {
-          go = ls_wait(sh, &sh->full[g], t & 1);
+          go = wait(&sh->full[g], t & 1);
           if (!go) break;
           tc_fence_after();
           const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
@@ -209,7 +211,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
         }
         if (!go) break;
         umma_commit(&sh->s_full);            // also: the output products of the tile before are done
-        go = ls_wait(sh, &sh->p_ready, t & 1);
+        go = wait(&sh->p_ready, t & 1);
         if (!go) break;
         tc_fence_after();
         for (int m = 0; m < nm; ++m) {
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
         }
       }
       umma_commit(&sh->mma_done);
-      ls_drain(sh, &sh->mma_done, 0);        // every product that was issued is done
+      drain(&sh->mma_done, 0);        // every product that was issued is done
     }
   } else {
     const int quarter = warp & 3, half = (warp - 2) >> 2,   // TMEM lanes go by warp % 4
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     for (int c = 0; c < NC; ++c) l[c] = 0.f;
     for (int t = 0; t < n_tiles; ++t) {
       const int j0 = k0 + t * kKT, key = j0 + key_lane;
-      ls_wait(sh, &sh->s_full, t & 1);
+      wait(&sh->s_full, t & 1);
       tc_fence_after();
       // a tile that every row of the item sees in full needs no mask
       const bool whole = j0 >= kb && j0 + kKT <= k_end && j0 + kKT - 1 <= first_pos && (long long)j0 >= (long long)first_pos + n_tok - a.window;
@@ -342,7 +344,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       }
     }
     ls_softmax_sync();
-    if (n_tiles > 0) ls_wait(sh, &sh->o_done[nm - 1], (n_tiles - 1) & 1);
+    if (n_tiles > 0) wait(&sh->o_done[nm - 1], (n_tiles - 1) & 1);
     tc_fence_after();
     for (int m = 0; m < nm; ++m) {
       uint32_t v[NC];
@@ -411,12 +413,13 @@ int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const vo
                  int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
                  float* ws_ml, cudaStream_t st) {
   const int D = r + dr, nr = max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64);
-  LatSmArgs a{bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D, (D + 63) / 64, 0, 0, scale * 1.4426950408889634f};
+  LatSmArgs a{bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D, (D + 63) / 64, 0, 0, scale * 1.4426950408889634f, nullptr};
   const int smem = ls_smem(nr, r, D, &a.p_offset);
   const int cols = (r / 128 + 1) * nr;
   a.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
   CUtensorMap tq, tk;
-  int rc = step_tensor_map(&tq, q, D, q_rows, D, 1, 0, nr);
+  int rc = step_failure_word(&a.failed);
+  if (rc == OMC_OK) rc = step_tensor_map(&tq, q, D, q_rows, D, 1, 0, nr);
   // how many pages the pool has is not known here; rows are only ever addressed through the block table
   if (rc == OMC_OK) rc = step_tensor_map(&tk, pool, D, 1ull << 31, D, 1, 0, 64);
   if (rc != OMC_OK) return rc;

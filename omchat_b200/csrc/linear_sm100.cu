@@ -47,7 +47,7 @@ __device__ __forceinline__ void hg_store(bf16_t* y, const float (&f)[8]) {
 
 template <int BN, typename TY>
 __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, LinearArgs a,
-                                                                  int stages, bool x_shared, bool w_shared, bool vec_out, bool vec_gate) {
+                                                                  int stages, bool x_shared, bool w_shared, bool vec_out, bool vec_gate, unsigned int* failed) {
   constexpr int kA = kHgBM * 128, kStage = kA + BN * 128;
   extern __shared__ uint8_t hg_raw[];
   __shared__ HgShared shared;
@@ -55,8 +55,9 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
   uint8_t* ring = hg_raw + ((1024u - (smem_u32(hg_raw) & 1023u)) & 1023u);
   const int m0 = blockIdx.y * kHgBM, n0 = blockIdx.x * BN, b = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nk = (a.K + kHgBK - 1) / kHgBK;
-  auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, &sh->dead, &g_linear_failures); };
-  auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, &sh->dead, &g_linear_failures); };
+  const WaitReport report{&sh->dead, &g_linear_failures, failed};
+  auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, report); };
+  auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, report); };
   auto load = [&](int kb) {
     uint8_t* sa = ring + (kb % stages) * kStage;
     uint64_t* bar = &sh->full[kb % stages];
@@ -201,7 +202,9 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
 template <int BN, typename TY>
 static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
   CUtensorMap tx, tw;
-  int rc = step_tensor_map(&tx, a.X, a.K, a.M, a.ldx, a.sx > 0 ? batch : 1, a.sx, kHgBM);   // stride 0: the batch shares the operand
+  unsigned int* failed = nullptr;
+  int rc = step_failure_word(&failed);
+  if (rc == OMC_OK) rc = step_tensor_map(&tx, a.X, a.K, a.M, a.ldx, a.sx > 0 ? batch : 1, a.sx, kHgBM);   // stride 0: the batch shares the operand
   if (rc == OMC_OK) rc = step_tensor_map(&tw, a.W, a.K, a.N, a.ldw, a.sw > 0 ? batch : 1, a.sw, BN);
   if (rc != OMC_OK) return rc;
   constexpr int stage = (kHgBM + BN) * 128, max_smem = kHgMaxStages * stage + 1024;
@@ -220,7 +223,7 @@ static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
   const bool vec_out = aligned(a.Y) && a.ldy % ye == 0 && a.sy % ye == 0, vec_gate = aligned(a.gate) && a.ldg % ge == 0 && a.sg % ge == 0;
   const dim3 grid((a.N + BN - 1) / BN, (a.M + kHgBM - 1) / kHgBM, batch);
   const int smem = (stages * stage > kHgSlabs ? stages * stage : kHgSlabs) + 1024;
-  linear_sm100_kernel<BN, TY><<<grid, kHgThreads, smem, st>>>(tx, tw, a, stages, a.sx == 0, a.sw == 0, vec_out, vec_gate);
+  linear_sm100_kernel<BN, TY><<<grid, kHgThreads, smem, st>>>(tx, tw, a, stages, a.sx == 0, a.sw == 0, vec_out, vec_gate, failed);
   return check_launch("omc_linear");
 }
 
@@ -243,7 +246,7 @@ int linear_sm100(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
 int latent_sm100_failures(unsigned int* n);   // latent_attention_sm100.cu
 
 // out: a wait for a barrier that nothing arrives at; the next one for it; one for a barrier that a later thread arrives at, as a wait and as a drain
-__global__ void step_wait_selfcheck_kernel(int32_t* out) {
+__global__ void step_wait_selfcheck_kernel(int32_t* out, unsigned int* failed) {
   __shared__ uint64_t never, late;
   __shared__ uint32_t dead;
   if (threadIdx.x == 0) {
@@ -254,10 +257,11 @@ __global__ void step_wait_selfcheck_kernel(int32_t* out) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    out[0] = wait_bounded(&never, 0, &dead, &g_linear_failures, 8);
-    out[1] = wait_bounded(&never, 0, &dead, &g_linear_failures);
-    out[2] = wait_bounded(&late, 0, &dead, &g_linear_failures);
-    out[3] = drain_bounded(&late, 0, &dead, &g_linear_failures);
+    const WaitReport report{&dead, &g_linear_failures, failed};
+    out[0] = wait_bounded(&never, 0, report, 8);
+    out[1] = wait_bounded(&never, 0, report);
+    out[2] = wait_bounded(&late, 0, report);
+    out[3] = drain_bounded(&late, 0, report);
   } else if (threadIdx.x == 32) {
     for (int i = 0; i < 1000000 && !*reinterpret_cast<volatile uint32_t*>(&dead); ++i) __nanosleep(1000);   // thread 0 sets it after its eight tries
     __nanosleep(200000);
@@ -267,9 +271,18 @@ __global__ void step_wait_selfcheck_kernel(int32_t* out) {
 
 }  // namespace omc
 
+extern "C" int omc_step_wait_failed(void) {
+  const volatile unsigned int* words = omc::step_failure_words();
+  int any = 0;
+  for (int dev = 0; words != nullptr && dev < omc::kMaxDevices; ++dev) any |= words[dev] != 0u;
+  return any;
+}
+
 extern "C" int omc_step_wait_selfcheck(int32_t* out, void* stream) {
   if (out == nullptr) return omc::set_error(OMC_ERR_ARG, "omc_step_wait_selfcheck: bad argument");
-  omc::step_wait_selfcheck_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(out);
+  unsigned int* failed = nullptr;
+  if (const int rc = omc::step_failure_word(&failed); rc != OMC_OK) return rc;
+  omc::step_wait_selfcheck_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(out, failed);
   return omc::check_launch("omc_step_wait_selfcheck");
 }
 

@@ -1,6 +1,7 @@
 // What the tcgen05 kernels of the sequence-step library share: waits that end by themselves, and tensor maps made per launch.
 #pragma once
 #include <cuda.h>
+#include <string.h>
 
 #include "ptx.cuh"
 #include "seq_common.cuh"
@@ -9,22 +10,60 @@ namespace omc {
 
 // A wait gives up after this many tries (each lets the hardware suspend the thread for a while), or at once where another wait of the CTA
 // has, and returns whether its phase has come. Who was refused issues no more copies and no more products; the CTA runs on to its end
-// through the same sequence of block barriers. What it wrote is not valid, and `failures` (a counter in device memory) says so.
+// through the same sequence of block barriers. What it wrote is not valid, and a counter in device memory and a word in host memory say so:
+// the launches of the library refuse while the word is set, and who has waited for a step's results can read it without waiting again.
 constexpr uint32_t kWaitTries = 1u << 22, kDrainTries = 1u << 20;
-__device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, uint32_t* dead, unsigned int* failures, uint32_t tries = kWaitTries) {
+struct WaitReport {
+  uint32_t* dead;         // shared memory: a wait of this CTA has given up
+  unsigned int* count;    // device memory
+  unsigned int* host;     // this device's word of step_failure_words()
+};
+__device__ __forceinline__ void wait_ran_out(const WaitReport& r) {
+  if (atomicExch(r.dead, 1u) != 0u) return;
+  atomicAdd(r.count, 1u);
+  *reinterpret_cast<volatile unsigned int*>(r.host) = 1u;
+  __threadfence_system();
+}
+__device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, const WaitReport& r, uint32_t tries = kWaitTries) {
   for (uint32_t i = 0; !mbar_try_wait(bar, parity); ++i) {
-    if (i >= tries && atomicExch(dead, 1u) == 0u) atomicAdd(failures, 1u);
-    if (*reinterpret_cast<volatile uint32_t*>(dead)) return false;
+    if (i >= tries) wait_ran_out(r);
+    if (*reinterpret_cast<volatile uint32_t*>(r.dead)) return false;
   }
   return true;
 }
 // For copies and products that have been issued: none may be under way into shared or tensor memory when the CTA gives these back, so these
 // waits have tries of their own whether or not another wait has given up.
-__device__ __forceinline__ bool drain_bounded(uint64_t* bar, uint32_t parity, uint32_t* dead, unsigned int* failures) {
+__device__ __forceinline__ bool drain_bounded(uint64_t* bar, uint32_t parity, const WaitReport& r) {
   for (uint32_t i = 0; i < kDrainTries; ++i)
     if (mbar_try_wait(bar, parity)) return true;
-  if (atomicExch(dead, 1u) == 0u) atomicAdd(failures, 1u);
+  wait_ran_out(r);
   return false;
+}
+
+// One word per device, in host memory that every device can write; nullptr where there is none to be had.
+inline unsigned int* step_failure_words() {
+  static unsigned int* words = [] {
+    void* p = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;   // the first launch may be one that is captured
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(&p, kMaxDevices * sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+      memset(p, 0, kMaxDevices * sizeof(unsigned int));
+    } else {
+      cudaGetLastError();
+      p = nullptr;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return static_cast<unsigned int*>(p);
+  }();
+  return words;
+}
+// The current device's word, for a launch; an error where there is none or it is set.
+inline int step_failure_word(unsigned int** word) {
+  unsigned int* words = step_failure_words();
+  if (words == nullptr) return set_error(OMC_ERR_CUDA, "no host memory for the step kernels' failure words");
+  *word = words + cur_device();
+  if (*reinterpret_cast<volatile unsigned int*>(*word) != 0u) return set_error(OMC_ERR_CUDA, "a wait of an earlier step kernel ran out on this device; what was computed since is not valid");
+  return OMC_OK;
 }
 
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,

@@ -63,6 +63,7 @@ SIGNATURES = {
     "omc_latent_attn": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _L, _F, _P, _P]),
     "omc_latent_attn_mma_rows": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_step_wait_failures": (_I, [_P]),
+    "omc_step_wait_failed": (_I, []),
     "omc_step_wait_selfcheck": (_I, [_P, _P]),
     "omc_latent_attn_mma": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_latent_decode_items": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
@@ -98,6 +99,13 @@ def _check(rc: int, what: str):
     _core.add_launches(1)
     if rc != 0:
         raise OmcError(f"{what} failed ({rc}): {load().omc_last_error().decode(errors='replace')}")
+
+
+def check_waits():
+    """Raises if a wait of a step kernel has run out: what was computed since is not valid. Does not synchronise - call it behind whatever
+    waited for the results."""
+    if _lib is not None and _lib.omc_step_wait_failed():
+        raise OmcError("a wait of a step kernel ran out; what was computed since is not valid")
 
 
 def dt_code(dtype: torch.dtype) -> int:

@@ -26,7 +26,7 @@ from typing import Dict, List, Optional, Sequence
 
 import torch
 
-from . import lib
+from . import lib, seqlib
 from .model.decoder import PagedKVCache
 from .model.paged_cache import PageAllocator
 
@@ -262,6 +262,7 @@ class StepScheduler:
         """entries: [(request key, token ids, wanted offsets among these tokens)]; a key seen for the first time is admitted.
         Runs them as one batch and returns fp32 logits [total wanted, vocab] in the order of the entries (None if nothing is
         wanted); then releases the requests named in `end`."""
+        seqlib.check_waits()                               # of the steps before, as far as they have run
         toks: List[int] = []
         pos: List[int] = []
         slot: List[int] = []
@@ -354,6 +355,7 @@ class StepScheduler:
             done = []
             if order:
                 nxt = lib.argmax(logits).tolist()          # greedy: lowest index on ties
+                seqlib.check_waits()                       # a replayed step passes no launch that would refuse
                 for g, t in zip(order, nxt):
                     g.out.append(int(t))
                     if (g.eos is not None and t == g.eos) or len(g.out) >= g.max_new:

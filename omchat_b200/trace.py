@@ -31,6 +31,7 @@ def main(argv=None) -> int:
     a = ap.parse_args(argv)
 
     import torch
+    from . import seqlib
     from .model import registry
     from .serving import StepScheduler
     dtype = getattr(torch, a.dtype)
@@ -55,12 +56,14 @@ def main(argv=None) -> int:
         logits = sched.run_step(entries, st.get("end", []))
         if logits is not None:
             data = logits.to(torch.float32).contiguous().cpu().numpy().astype("<f4", copy=False)
+            seqlib.check_waits()
             tmp = os.path.join(a.out, f".{st['step']}.f32.part")
             with open(tmp, "wb") as fh:
                 fh.write(data.tobytes())
             os.replace(tmp, os.path.join(a.out, f"{st['step']}.f32"))
         else:
             torch.cuda.synchronize()
+            seqlib.check_waits()
         print(f"done {st['step']}", flush=True)
     return 0
 

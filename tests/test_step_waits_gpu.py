@@ -22,3 +22,18 @@ def test_a_wait_that_runs_out_refuses_the_next_and_lets_drains_finish():
                "print(L.omc_step_wait_failures(ctypes.byref(n)), n.value)\n"
                "print(torch.ones(3, device='cuda').sum().item())")
     assert got[:4] == ["0 0", "0 [0, 0, 0, 1]", "0 1", "3.0"]
+
+
+def test_a_wait_that_ran_out_is_reported():
+    """By the next launch of a kernel that has such waits, and to who replays a graph by seqlib.check_waits; kernels without them still run."""
+    got = _run("x, y = torch.ones(64, 128, dtype=torch.bfloat16, device='cuda'), torch.zeros(64, 64, device='cuda')\n"
+               "g = torch.cuda.CUDAGraph()\n"
+               "with torch.cuda.graph(g):\n    seqlib.linear(x, x, y)\n"       # the first launch of the process: captured
+               "g.replay(); torch.cuda.synchronize(); seqlib.check_waits(); print(L.omc_step_wait_failed(), y[0, 0].item())\n"
+               "L.omc_step_wait_selfcheck(out.data_ptr(), torch.cuda.current_stream().cuda_stream); torch.cuda.synchronize()\n"
+               "print(L.omc_step_wait_failed())\n"
+               "for f in (seqlib.check_waits, lambda: seqlib.linear(x, x, y)):\n"
+               "    try:\n        f(); print('no error')\n"
+               "    except seqlib.OmcError as e:\n        print('ran out' in str(e))\n"
+               "z = torch.ones(64, 64, device='cuda'); seqlib.linear(z, z, y); print(y[0, 0].item())\n")
+    assert got[:5] == ["0 128.0", "1", "True", "True", "64.0"]

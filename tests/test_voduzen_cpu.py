@@ -8,6 +8,7 @@ import torch
 from omchat_b200.config import RotarySpec, VoduzenConfig
 from omchat_b200.model.checkpoint import config_from_dict
 from omchat_b200.model.paged_cache import PageAllocator, PagedLatentCache
+from omchat_b200 import seqlib
 from omchat_b200.model import registry
 from omchat_b200.serving import StepScheduler
 from oracle import voduzen_oracle as O
@@ -85,6 +86,30 @@ class _Recorder:
         if want_rows is None:
             return None
         return torch.stack([pos[want_rows].float(), slot[want_rows].float()], dim=1)
+
+
+def test_scheduler_raises_when_a_wait_of_a_kernel_ran_out(monkeypatch):
+    """The library says so after the step it happened in: a step's logits are not handed on as tokens, and no further step runs."""
+    class Lib:
+        failed = 0
+
+        def omc_step_wait_failed(self):
+            return self.failed
+
+    fake, m = Lib(), _Recorder(page=4)
+    monkeypatch.setattr(seqlib, "_lib", fake)
+    s = StepScheduler(m, max_tokens=24, slots=2)
+    s.run_step([("a", [7, 8], [1])])
+    fake.failed = 1
+    with pytest.raises(seqlib.OmcError, match="ran out"):
+        s.run_step([("a", [9], [0])])
+    assert len(m.batches) == 1
+    fake.failed = 0
+    monkeypatch.setattr("omchat_b200.serving.lib.argmax", lambda logits: setattr(fake, "failed", 1) or torch.zeros(len(logits), dtype=torch.int64))
+    s.submit([1, 2, 3], max_new_tokens=2)
+    with pytest.raises(seqlib.OmcError, match="ran out"):
+        s.run()
+    assert not s.results
 
 
 def test_scheduler_positions_slots_and_page_reuse():
