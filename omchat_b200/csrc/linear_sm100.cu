@@ -47,7 +47,7 @@ __device__ __forceinline__ void hg_store(bf16_t* y, const float (&f)[8]) {
 
 template <int BN, typename TY>
 __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w, LinearArgs a,
-                                                                  int stages, bool x_shared, bool w_shared, bool vec_out, bool vec_gate, unsigned int* failed) {
+                                                                  int stages, bool x_shared, bool w_shared, bool vec_out, bool vec_gate, bool pair_gate, unsigned int* failed) {
   constexpr int kA = kHgBM * 128, kStage = kA + BN * 128;
   extern __shared__ uint8_t hg_raw[];
   __shared__ HgShared shared;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
               float f[8];
               hg_row(src + (i0 + i) * 4 * kHgPitch, a.alpha, f);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] /= 1.f + __expf(-z[i][j]);   // as at the edges: a row's bits do not depend on its tile
+              for (int j = 0; j < 8; ++j) f[j] /= 1.f + __expf(-z[i][j]);   // as at the edges: bits do not depend on the tile
               hg_store(y + (long long)((i0 + i) * 4) * a.ldy, f);
             }
           }
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
               z[j] = j >= left ? 0.f : (a.gate_dt == OMC_DT_F32 ? static_cast<const float*>(a.gate)[at + j] : ldf(static_cast<const bf16_t*>(a.gate) + at + j));
           }
 #pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] /= 1.f + __expf(-z[j]);
+          for (int j = 0; j < 8; ++j) f[j] /= 1.f + (pair_gate && n + (j | 1) < a.N ? __expf(-z[j]) : expf(-z[j]));
         }
         TY* y = static_cast<TY*>(a.Y) + (long long)b * a.sy + (long long)m * a.ldy + n;
         if (vec_out && left == 8) {
@@ -221,9 +221,11 @@ static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const int ye = 16 / (int)sizeof(TY), ge = a.gate_dt == OMC_DT_F32 ? 4 : 8;
   const bool vec_out = aligned(a.Y) && a.ldy % ye == 0 && a.sy % ye == 0, vec_gate = aligned(a.gate) && a.ldg % ge == 0 && a.sg % ge == 0;
+  // the hardware exponential for gates that come in pairs on 8-byte boundaries, the precise one for those at odd strides and an odd last column
+  const bool pair_gate = a.ldg % 2 == 0 && a.sg % 2 == 0 && reinterpret_cast<uintptr_t>(a.gate) % 8 == 0;
   const dim3 grid((a.N + BN - 1) / BN, (a.M + kHgBM - 1) / kHgBM, batch);
   const int smem = (stages * stage > kHgSlabs ? stages * stage : kHgSlabs) + 1024;
-  linear_sm100_kernel<BN, TY><<<grid, kHgThreads, smem, st>>>(tx, tw, a, stages, a.sx == 0, a.sw == 0, vec_out, vec_gate, failed);
+  linear_sm100_kernel<BN, TY><<<grid, kHgThreads, smem, st>>>(tx, tw, a, stages, a.sx == 0, a.sw == 0, vec_out, vec_gate, pair_gate, failed);
   return check_launch("omc_linear");
 }
 

@@ -45,3 +45,17 @@ def test_a_batch_may_share_an_operand():
     assert torch.allclose(y.double(), torch.einsum("mk,bnk->mbn", x.double(), w.double()).reshape(40, 320), atol=1e-4)
     seqlib.linear(w.view(4, 80, 96)[0], x, z := torch.empty(80, 40, device="cuda"))
     assert torch.allclose(z.double(), w[0].double() @ x.double().T, atol=1e-4)
+
+
+@pytest.mark.parametrize("N,pad,gate", [(72, 3, F32), (72, 1, BF16), (73, 7, F32)])   # odd strides of rows; of batch items
+def test_gates_that_do_not_come_in_pairs_use_the_precise_exponential(N, pad, gate):
+    M, K = 150, 64
+    g = torch.linspace(-34, -10, M * N).view(M, N)
+    buf = torch.zeros(M, N + pad)
+    buf[:, :N] = g
+    g = buf.to(gate).cuda()[:, :N]
+    x, w, y = torch.ones(M, K, dtype=BF16, device="cuda"), torch.ones(N, K, dtype=BF16, device="cuda"), torch.empty(M, N, device="cuda")
+    seqlib.linear(x, w, y, gate=g)
+    err = (y.double() / (K * torch.sigmoid(g.double())) - 1).abs()
+    # the product is exact; two units of the last place for the exponential, half of one for the sum, the quotient and their effect on it
+    assert err.max() <= 4 * 2.0 ** -23, float(err.max())
