@@ -292,8 +292,11 @@ extern "C" int omc_latent_attn(const void* qcat, int q_dt, int T, int H, int r, 
   if (T == 0) return OMC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t smem = sizeof(float) * ((size_t)r + dr + (size_t)kLatWarps * r + 2 * kLatWarps);
+  // the widths whose query and four partial outputs fit 48 KB; the eight partial outputs of the widest take up to 64 KB
+  if (sizeof(float) * (5 * (size_t)r + dr + 8) > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_latent_attn: rows too wide");
   OMC_DT_SWITCH(q_dt, TQ, OMC_DT_SWITCH(pool_dt, TC, {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(latent_attn_kernel<TQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(latent_attn_kernel<TQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return check_launch("omc_latent_attn");
     latent_attn_kernel<TQ, TC><<<dim3(T, H), kLatWarps * 32, smem, st>>>(static_cast<const TQ*>(qcat), H, r, dr,
                                                                          static_cast<const TC*>(pool), block_table, max_pages,
                                                                          page_size, pos, slot, sink, window, gate, ldg, scale, out);

@@ -1111,9 +1111,11 @@ extern "C" int omc_window_attn(const void* q, long long ldq, int T, int H, int G
   if ((long long)H * maps > 65535) return set_error(OMC_ERR_SHAPE, "omc_window_attn: more than 65535 heads");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const size_t smem = sizeof(float) * ((size_t)d + (size_t)kWinWarps * dv + 2 * kWinWarps);
-  if (smem > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_window_attn: head width too large");
+  // the widths whose query and four partial outputs fit 48 KB; the eight partial outputs of the widest take up to 52 KB
+  if (sizeof(float) * ((size_t)d + 4 * (size_t)dv + 8) > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_window_attn: head width too large");
   OMC_DT_SWITCH(dt, TC, OMC_DT_SWITCH(out_dt, TY, {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(window_attn_kernel<TC, TC, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024 && cudaFuncSetAttribute(window_attn_kernel<TC, TC, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return check_launch("omc_window_attn");
     window_attn_kernel<TC, TC, TY><<<dim3(T, H * maps), kWinWarps * 32, smem, st>>>(static_cast<const TC*>(q), ldq, H, G, d, dv, maps,
                                                                                    static_cast<const TC*>(pool), block_table, max_pages,
                                                                                    page_size, pos, slot, window, chunk, keep_first, scale, softcap,
