@@ -515,6 +515,7 @@ extern "C" int omc_vit_im2col(const void* pixels, int pixels_are_f32, void* cols
                               void* stream) {
   if (B <= 0) return OMC_OK;
   if (H % 14 != 0 || W % 14 != 0 || ldc < 588) return set_error(OMC_ERR_SHAPE, "omc_vit_im2col: H, W must be multiples of 14 and ldc >= 588");
+  if (H == 0 || W == 0) return OMC_OK;
   const int gh = H / 14;
   const dim3 grid(B * gh, kIm2colSplit);
   const bool vec = ldc % 8 == 0 && reinterpret_cast<uintptr_t>(cols) % 16 == 0;
@@ -537,6 +538,7 @@ extern "C" int omc_vit_assemble(const void* patch, const void* cls, const void* 
 extern "C" int omc_select_pixel_shuffle(const void* hidden, void* out, int B, int G, int C, int down, void* stream) {
   if (B <= 0) return OMC_OK;
   if (down < 1 || G % down != 0 || C % 8 != 0) return set_error(OMC_ERR_SHAPE, "omc_select_pixel_shuffle: bad G/C/down");
+  if (G == 0) return OMC_OK;
   select_pixel_shuffle_kernel<<<B * G * G, 128, 0, (cudaStream_t)stream>>>((const bf16*)hidden, (bf16*)out, G, C, down);
   return check_launch("select_pixel_shuffle");
 }

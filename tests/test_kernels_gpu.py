@@ -286,6 +286,17 @@ def test_vit_embeddings(L):
     assert_close(hidden.view(3, 257, C).flatten(0, 1), want.flatten(0, 1), rel=2 ** -6, what="vit embeddings")
 
 
+def test_vision_row_kernels_take_empty_images(L):
+    C, buf = L.load(), torch.full((64,), 7.0, dtype=torch.bfloat16, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    for H, W in ((0, 28), (28, 0), (0, 0)):
+        assert C.omc_vit_im2col(buf.data_ptr(), 0, buf.data_ptr(), 592, 2, H, W, st) == 0
+    assert C.omc_vit_im2col(buf.data_ptr(), 0, buf.data_ptr(), 592, 2, 0, 13, st) != 0
+    assert C.omc_select_pixel_shuffle(buf.data_ptr(), buf.data_ptr(), 2, 0, 64, 2, st) == 0
+    torch.cuda.synchronize()
+    assert (buf == 7.0).all()
+
+
 @pytest.mark.parametrize("down", [1, 2, 4])
 def test_select_pixel_shuffle_bit_exact(L, down):
     B, G, C = 3, 16, 64
