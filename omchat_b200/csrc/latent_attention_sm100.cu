@@ -126,6 +126,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, report); };
   auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, report); };
   const int32_t* bt = a.bt + (long long)slot * a.max_pages;
+  // The last chunk ends where the row does: its box starts at D - 64 and repeats columns of the chunk before where D is no multiple of 64. A
+  // box that reached past the row would have its columns filled with zeros, but the pool's map knows no last row (see latent_sm100), and a
+  // copy of the last row of a pool that ends with its mapping then faulted.
+  auto chunk_col = [&](int c) { return c == a.nc - 1 ? a.D - 64 : c * 64; };
   // rows of the pool where the two boxes of tile t start (looked up a tile ahead: a lookup takes as long as 20 KB of the copies)
   auto box_rows = [&](int t, int (&row)[2]) {
 #pragma unroll
@@ -140,7 +144,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
 #pragma unroll
     for (int b = 0; b < 2; ++b)
       if (row[b] >= 0)
-        for (int c = 2 * g; c < c1; ++c) tma_load_3d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[g], c * 64, row[b], 0);
+        for (int c = 2 * g; c < c1; ++c) tma_load_3d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[g], chunk_col(c), row[b], 0);
   };
   if (tid >= 64 && tid < 64 + kLsMaxRows) sh->mref[tid - 64] = -INFINITY;
   if (tid == 0) {
@@ -158,7 +162,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     fence_proxy_async();
     if (n_tiles > 0) {                       // on their way while tensor memory is allocated
       mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
-      for (int c = 0; c < a.nc; ++c) tma_load_3d(qs + c * QCHUNK, &tm_q, &sh->q_full, c * 64, first_row * a.H, 0);
+      for (int c = 0; c < a.nc; ++c) tma_load_3d(qs + c * QCHUNK, &tm_q, &sh->q_full, chunk_col(c), first_row * a.H, 0);
       int row[2];
       box_rows(0, row);
       for (int g = 0; g < nm; ++g) load_pair(row, g);
@@ -193,7 +197,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       const uint64_t dk0 = make_sw128_kmajor_desc(smem_u32(ks)), dq0 = make_sw128_kmajor_desc(smem_u32(qs));
       const uint64_t dv0 = make_sw128_mnmajor_desc(smem_u32(ks), kChunkBytes, 1024);
       const uint64_t dp0 = NR == 64 ? make_sw128_mnmajor_desc(p_addr, 1024, 1024) : make_sw128_kmajor_desc(p_addr);
-      const int tail = (a.D - (a.nc - 1) * 64 + 15) >> 4;   // steps of 16 in the last chunk
+      const int repeated = (a.nc * 64 - a.D) >> 4;   // steps of 16 that the last chunk has in common with the one before
       bool go = wait(&sh->q_full, 0);
       for (int t = 0; go && t < n_tiles; ++t) {
         for (int g = 0; g < nm; ++g) {
@@ -203,10 +207,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
           const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
           for (int c = 2 * g; c < c1; ++c) {
             const uint64_t dk = dk0 + (uint64_t)(c * (kChunkBytes >> 4)), dq = dq0 + (uint64_t)(c * (QCHUNK >> 4));
-            const int steps = c == a.nc - 1 ? tail : 4;
+            const int first = c == a.nc - 1 ? repeated : 0;
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              if (k < steps) umma_bf16<1>(tmem_s, dk + 2 * k, dq + 2 * k, idesc_s, (c | k) != 0 ? 1u : 0u);
+              if (k >= first) umma_bf16<1>(tmem_s, dk + 2 * k, dq + 2 * k, idesc_s, (c | k) != 0 ? 1u : 0u);
           }
         }
         if (!go) break;
@@ -420,7 +424,7 @@ int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const vo
   CUtensorMap tq, tk;
   int rc = step_failure_word(&a.failed);
   if (rc == OMC_OK) rc = step_tensor_map(&tq, q, D, q_rows, D, 1, 0, nr);
-  // how many pages the pool has is not known here; rows are only ever addressed through the block table
+  // how many pages the pool has is not known here; boxes lie wholly inside pages that the block table names
   if (rc == OMC_OK) rc = step_tensor_map(&tk, pool, D, 1ull << 31, D, 1, 0, 64);
   if (rc != OMC_OK) return rc;
   const bool b = out_dt == OMC_DT_BF16;

@@ -106,3 +106,28 @@ def test_no_wait_ran_out():
     import ctypes
     n = ctypes.c_uint(7)
     assert seqlib.load().omc_step_wait_failures(ctypes.byref(n)) == 0 and n.value == 0
+
+
+@pytest.mark.parametrize("r,dr", [(128, 32), (256, 16), (512, 64)])
+def test_a_pool_that_ends_with_its_mapping(r, dr):
+    """The last row of the pool is the last of an allocation of whole 2 MB pages, and nothing is kept behind it: every copy stays inside the rows."""
+    H, D, pages = 4, r + dr, 1024
+    gen = torch.Generator().manual_seed(D)
+    torch.cuda.empty_cache()
+    pool = torch.zeros(pages, 64, D, dtype=torch.bfloat16, device="cuda")
+    assert pool.numel() * 2 % (2 << 20) == 0
+    rows, q = torch.randn(192, D, generator=gen).to(torch.bfloat16), torch.randn(3, H, D, generator=gen).to(torch.bfloat16)
+    pool[-3:] = rows.view(3, 64, D).cuda()
+    table = torch.arange(pages - 3, pages, dtype=torch.int32).view(1, 3).cuda()
+    qd, out = q.cuda(), torch.empty(3, H, r, device="cuda")
+    plist = [(0, 3, 0, 192 - 3)]                                                 # the last three positions: their rows end where the pool does
+    plans = [seqlib.LatentAttnPlan(plist, H, "cuda", **cut) for cut in ({}, dict(target_ctas=148, min_keys=64))]
+    pos = torch.arange(192 - 3, 192, dtype=torch.int32).cuda()
+    plans.append(seqlib.DecodeAttnPlan(3, H, 2, "cuda"))
+    plans[-1].fill(pos, torch.zeros(3, dtype=torch.int32, device="cuda"))
+    want, mag = _reference(q, [rows], plist, r, D ** -0.5, 1 << 30, None, None)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    for plan in plans:
+        seqlib.latent_attn_mma(qd, r, dr, pool, table, 64, plan, None, D ** -0.5, out)
+        assert ((out.double().cpu() - want).abs() <= mag * (2.0 ** -8 + 1e-4) + 1e-6).all()
