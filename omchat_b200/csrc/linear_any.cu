@@ -331,16 +331,21 @@ static int launch_narrow(const LinearArgs& a, int y_dt, int batch, cudaStream_t 
   return set_error(OMC_ERR_ARG, "omc_linear: unknown output dtype");
 }
 
-// Rows kernel or tile kernel: the same results either way. The rows kernel costs 1.7e-7 us per K term of an output, whatever the shape; the
-// tile kernel 0.037 us per K term for a first wave of up to 148 tiles, however few and empty they are, and in proportion above that: they
-// meet at 219,000 outputs per wave, 1480 per SM. Both sides in us at K = 1024 (rows / tile): 8 x 4096 outputs 13 / 37, 32 x 4096 28 / 40,
-// 64 x 4096 48 / 44, 128 x 1024 29 / 44, 256 x 1024 49 / 45.
+// Rows kernel or tile kernel: the same results either way. Both were measured at K from 16 to 2048 (in us, rows / tile):
+//   K =   64: 16 x 2048 outputs 5.9 / 4.6, 64 x 512 5.3 / 6.6, 100 x 2048 20.6 / 7.5, 32 x 4096 13.5 / 5.5
+//   K =  256: 32 x 1024 7 / 14, 100 x 1024 14.5 / 14.1, 100 x 2048 26 / 14, 200 x 1024 25 / 14
+//   K = 1024: 8 x 4096 13 / 37, 32 x 4096 28 / 40, 64 x 4096 48 / 44, 128 x 1024 29 / 44, 256 x 1024 49 / 45
+// The tile kernel's time goes with K alone up to a first wave of 148 tiles, however few and empty they are, and in proportion above that. The rows
+// kernel's goes with the outputs, and falls only slowly with K below its stage of 1024 terms (K / 64 of a CTA's 16 sums are at work, and its shared
+// memory is the same): they meet at some 20,000 outputs plus 195 per K term and wave. Rows that its vector loads do not take cost it four times
+// as much (63 terms, 90 x 2048 outputs: 39 / 9).
 static long long lin_tiles(const LinearArgs& a, int batch) {
   return (long long)((a.N + kLinBN - 1) / kLinBN) * ((a.M + kLinBM - 1) / kLinBM) * batch;
 }
-static bool few_rows(const LinearArgs& a, int batch) {
+static bool few_rows(const LinearArgs& a, int batch, bool vec) {
   const long long tiles = lin_tiles(a, batch), outputs = (long long)a.M * a.N * batch;
-  return a.tile_group == nullptr && outputs <= 1480 * (tiles > 148 ? tiles : 148) && a.M <= 8 * 65535;
+  const long long meet = (20000 + 195LL * (a.K < 1024 ? a.K : 1024)) / (vec ? 1 : 4);
+  return a.tile_group == nullptr && 148 * outputs <= meet * (tiles > 148 ? tiles : 148) && a.M <= 8 * 65535;
 }
 
 // Dynamic shared memory above 48 KB is asked for once per kernel and device.
@@ -376,7 +381,7 @@ static int launch_tile(const LinearArgs& a, int batch, cudaStream_t st) {
 
 template <typename TX, typename TW, typename TY, bool VEC>
 static int launch_any(const LinearArgs& a, int batch, cudaStream_t st) {
-  if (few_rows(a, batch)) return a.M <= 4 ? launch_rows<TX, TW, TY, 4, VEC>(a, batch, st) : launch_rows<TX, TW, TY, 8, VEC>(a, batch, st);
+  if (few_rows(a, batch, VEC)) return a.M <= 4 ? launch_rows<TX, TW, TY, 4, VEC>(a, batch, st) : launch_rows<TX, TW, TY, 8, VEC>(a, batch, st);
   // with few tiles per SM the smaller tasks of 256 threads hide more (100 x 77, K = 4096 rows: 13 us, 128 threads 17); with many, the better
   // reuse of 128 counts (4096 x 6144 x 2048: 2463 us, 256 threads 2646)
   return lin_tiles(a, batch) < 296 ? launch_tile<TX, TW, TY, VEC, 256>(a, batch, st) : launch_tile<TX, TW, TY, VEC, 128>(a, batch, st);
