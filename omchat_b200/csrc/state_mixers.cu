@@ -326,7 +326,9 @@ __device__ __forceinline__ int scan_place(int i) { return (i / DPT) * (DPT + 4) 
 // (every row starts on a 16-byte boundary and the widths are multiples of four), else 4-byte copies.
 // KIND: what enters the state - v itself, the delta rule's correction, or dt v (decay mode 6).
 // TOK: tokens per stage; 1 for steps of one-token portions, whose CTAs then need little shared memory (more of them share
-// an SM and keep state loads in flight); any TOK is right for any portion.
+// an SM and keep state loads in flight: seven at 128 key channels, four at 256, which the launch bounds hold the registers to; with the 94 and
+// 156 that the compiler took by itself, 256 requests of 64 heads of 128 x 64 took 385 us and of 4 heads of 256 x 256 271, now 306 and 158);
+// any TOK is right for any portion.
 //
 // A thread owns DPT neighbouring key channels of CPT neighbouring columns: a packed register holds two neighbouring CHANNELS of one
 // column, so that keys, queries and per-channel decays are used as they lie in shared memory, and only the numbers that all channels
@@ -342,12 +344,13 @@ __host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
   return TOK * kScanLanes * (DPT + 4) * (chan ? 3 : 2) + TOK * cols + 2 * (TOK < 4 ? 4 : TOK);
 }
 template <int DPT, bool VEC, int KIND, bool CHAN, int TOK>   // CHAN: one decay per key channel
-__global__ void __launch_bounds__(kScanThreads) linear_state_scan_kernel(ScanArgs a) {
+__global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 32 ? 4 : 7) : 0) linear_state_scan_kernel(ScanArgs a) {
   extern __shared__ __align__(16) float sm[];
   constexpr int PITCH = kScanLanes * (DPT + 4), CPT = kScanCpt, COLS = kScanGroups * CPT, DP = DPT / 2;
   constexpr int OPITCH = COLS + 4;           // a lane's partial read-outs of one token
   constexpr int HEADW = TOK < 4 ? 4 : TOK;   // one number per token, in whole 16-byte pieces
   const int dim = a.dim;
+  constexpr bool WIDE = TOK == 1 && DPT <= 16;
   constexpr bool PRE = TOK > 1 && !CHAN;     // read ahead (per-channel decays fill the registers that this takes)
   const bool minus1 = KIND == kScanStep || a.decay_mode >= 4;  // the staged value is the decay minus one
   constexpr int stage_floats = scan_stage_floats<DPT, TOK>(CHAN, COLS);
@@ -358,7 +361,7 @@ __global__ void __launch_bounds__(kScanThreads) linear_state_scan_kernel(ScanArg
   if (r1 <= r0) return;
   // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
   // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
-  const int tid = threadIdx.x, lane = TOK == 1 ? tid / kScanGroups : tid & (kScanLanes - 1), cg = TOK == 1 ? tid % kScanGroups : tid / kScanLanes;
+  const int tid = threadIdx.x, lane = WIDE ? tid / kScanGroups : tid & (kScanLanes - 1), cg = WIDE ? tid % kScanGroups : tid / kScanLanes;
   const int col = col0 + CPT * cg;
   for (int e = tid; e < 2 * stage_floats; e += blockDim.x) sm[e] = 0.f;   // the pads stay zero: they meet zero state only
   float* S = a.state + (((long long)a.slot[r0] * a.H + h) * dim) * a.vdim;
@@ -372,7 +375,9 @@ __global__ void __launch_bounds__(kScanThreads) linear_state_scan_kernel(ScanArg
       const int i = lane * DPT + 2 * r + j;
       const float* row = S + (long long)i * a.vdim + col;
       const bool in = !fresh && i < dim;
-      if (a.vec_state) {   // the columns of a thread as one access (CPT divides vdim)
+      // the columns of a thread as one access (CPT divides vdim); not where 32 of them per thread are all that is on its way: they would have to
+      // be taken apart before the next could be asked for
+      if (a.vec_state && !(TOK == 1 && DPT == 32)) {
         const float2 x = in && col < a.vdim ? *reinterpret_cast<const float2*>(row) : make_float2(0.f, 0.f);
         e[j][0] = x.x, e[j][1] = x.y;
       } else {
@@ -390,7 +395,7 @@ __global__ void __launch_bounds__(kScanThreads) linear_state_scan_kernel(ScanArg
 
   // sum of a thread's numbers over the lanes, in the same order either way
   auto sum_lanes = [&](float (&x)[CPT]) {
-    if constexpr (TOK == 1) {
+    if constexpr (WIDE) {
       __syncthreads();   // the numbers of the sum before have been read
       *reinterpret_cast<float2*>(po + lane * OPITCH + CPT * cg) = make_float2(x[0], x[1]);
       __syncthreads();
@@ -1274,8 +1279,10 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   constexpr int cols = kScanGroups * kScanCpt;
   dim3 grid((vdim + cols - 1) / cols, H, portions);
   // 16 tokens per stage; with per-channel decays that is 85 KB and two CTAs per SM, so beyond 296 CTAs eight tokens (in us, 16 / 8 tokens,
-  // 32 heads of 128 x 128, portions of 1024, 777, 1024, 301: 713 / 608; 16 heads: 435 / 476)
+  // 32 heads of 128 x 128, portions of 1024, 777, 1024, 301: 713 / 608; 16 heads: 435 / 476). Portions of few tokens have no use for 16, whose 63 KB
+  // (39 at 32 channels) leave three CTAs to an SM: eight portions of three tokens, 16 heads of 128 x 128, 15.4 / 10.3
   const bool tight = chan && (long long)grid.x * H * portions > 296;
+  const bool brief = rows <= 16LL * portions;
 #define OMC_SCAN_LAUNCH(DPT, VEC, KIND, CHAN, TOK)                                                                                        \
   do {                                                                                                                                    \
     static bool attr_done[kMaxDevices] = {};                                                                                              \
@@ -1300,9 +1307,11 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
     else if (vec) OMC_SCAN_KIND(DPT, true, TOK); \
     else OMC_SCAN_KIND(DPT, false, TOK);        \
   } while (0)
-  if (dpt == 4) OMC_SCAN_DPT(4, 16);
+  if (dpt == 4 && brief) OMC_SCAN_DPT(4, 8);
+  else if (dpt == 4) OMC_SCAN_DPT(4, 16);
+  else if (dpt == 8 && brief) OMC_SCAN_DPT(8, 8);
   else if (dpt == 8) OMC_SCAN_DPT(8, 16);
-  else if (dpt == 16 && tight) OMC_SCAN_DPT(16, 8);
+  else if (dpt == 16 && (tight || brief)) OMC_SCAN_DPT(16, 8);
   else if (dpt == 16) OMC_SCAN_DPT(16, 16);
   else OMC_SCAN_DPT(32, 8);
 #undef OMC_SCAN_DPT

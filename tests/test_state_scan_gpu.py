@@ -1,5 +1,5 @@
-"""omc_linear_state_scan: token by token (the kernel that shares a sum through shared memory) and whole portions (the one that defers the
-read-out) give the same bits, at every number of key channels per thread, ragged widths and both stage lengths of per-channel decays."""
+"""omc_linear_state_scan: token by token (the kernel that shares a sum through shared memory), a few tokens at a time and whole portions (the one that
+defers the read-out) give the same bits, at every number of key channels per thread, ragged widths and both stage lengths."""
 import pytest
 import torch
 
@@ -13,7 +13,7 @@ def _i32(x):
 
 
 @pytest.mark.parametrize("kind", ["steps", "delta", "delta_channel", "const"])
-@pytest.mark.parametrize("H,G,dim,vdim", [(2, 1, 32, 36), (3, 3, 60, 34), (2, 2, 64, 64), (4, 2, 128, 96), (2, 1, 136, 33), (200, 1, 128, 64)])
+@pytest.mark.parametrize("H,G,dim,vdim", [(2, 1, 32, 36), (3, 3, 60, 34), (2, 2, 64, 64), (4, 2, 128, 96), (2, 1, 136, 33), (2, 1, 256, 64), (200, 1, 128, 64)])
 def test_one_token_at_a_time_gives_the_bits_of_the_whole(H, G, dim, vdim, kind):
     gen = torch.Generator().manual_seed(H * dim + vdim)
     rn = lambda *s: torch.randn(*s, generator=gen).cuda()  # noqa: E731
@@ -34,10 +34,13 @@ def test_one_token_at_a_time_gives_the_bits_of_the_whole(H, G, dim, vdim, kind):
     whole, S = torch.empty(T, H * vdim, device="cuda"), torch.full((P, H, dim, vdim), float("nan"), device="cuda")
     scan(slice(None), S, whole, _i32(starts), P, pos, slot)
     assert torch.isfinite(whole).all() and torch.isfinite(S).all()
-    S1 = torch.full_like(S, float("nan"))
-    for t in range(max(lens)):
-        rows = [starts[i] + t for i, n in enumerate(lens) if t < n]
-        out = torch.empty(len(rows), H * vdim, device="cuda")
-        scan(torch.tensor(rows, device="cuda"), S1, out, _i32(list(range(len(rows) + 1))), len(rows), pos[rows].contiguous(), slot[rows].contiguous())
-        assert torch.equal(out, whole[rows]), t
-    assert torch.equal(S1, S)
+    for step in (1, 3):                    # 3: portions of few tokens, which take shorter stages
+        S1 = torch.full_like(S, float("nan"))
+        for t in range(0, max(lens), step):
+            pieces = [list(range(starts[i] + t, starts[i] + min(t + step, n))) for i, n in enumerate(lens) if t < n]
+            rows = sum(pieces, [])
+            out = torch.empty(len(rows), H * vdim, device="cuda")
+            begin = _i32([sum(map(len, pieces[:i])) for i in range(len(pieces) + 1)])
+            scan(torch.tensor(rows, device="cuda"), S1, out, begin, len(pieces), pos[rows].contiguous(), slot[rows].contiguous())
+            assert torch.equal(out, whole[rows]), (step, t)
+        assert torch.equal(S1, S), step
