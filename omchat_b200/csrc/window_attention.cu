@@ -388,17 +388,17 @@ struct WinMmaArgs {
   int bias_in_smem;       // the bias columns of this key/value head's query heads are staged in shared memory ([window][H / G])
 };
 
-// Decode: items of one token whose query heads per key/value head fit one 16-row tile. The keys are dealt to the CTA's eight warps in tiles of
+// Decode: items of one token whose query heads per key/value head fit one 16-row tile. The keys are dealt to the CTA's warps in tiles of
 // 32; every warp stages its own tile, works on it alone and keeps a partial (max, sum, output), and the partials meet in shared memory at the
 // end. One warp walking all tiles was bound by its own instructions, 7 us per 64 keys: 32 rows x 4 key/value heads of 128 + 128 over
-// up to 512 keys 20 us (60).
+// up to 512 keys 20 us (60). How many warps: win_decode_warps.
 constexpr int kWdWarps = 8, kWdKeys = 32, kWdRows = 16;
 template <int NV, typename TO>
 __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMmaArgs a) {
   extern __shared__ __align__(16) unsigned char wsm_raw[];
   __shared__ float s_m[kWdWarps][kWdRows], s_l[kWdWarps][kWdRows];
   const int d = a.d, dv = a.dv, pq = d + 8, pv = dv + 8;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3, warps = blockDim.x >> 5;
   bf16_t* Qs = reinterpret_cast<bf16_t*>(wsm_raw);
   bf16_t* Ks = Qs + kWdRows * pq + warp * kWdKeys * (pq + pv);   // this warp's keys and values
   bf16_t* Vs = Ks + kWdKeys * pq;
@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
   constexpr float kLog2e = 1.4426950408889634f;
   const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
   __syncthreads();
-  for (int kt = warp; kt < n_tiles; kt += kWdWarps) {
+  for (int kt = warp; kt < n_tiles; kt += warps) {
     const int j0 = kt < kept_tiles ? kt * kWdKeys : k_begin + (kt - kept_tiles) * kWdKeys, j_end = kt < kept_tiles ? kept_end : k_end;
     {
       const int j = j0 + lane;
@@ -541,12 +541,9 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
     const int row = e / (dv >> 1), col = (e - row * (dv >> 1)) * 2, h = kvh * rep + row;
     const float sk = a.sink != nullptr ? a.sink[h] * kLog2e : -INFINITY;
     float mt = sk;
-#pragma unroll
-    for (int w = 0; w < kWdWarps; ++w) mt = fmaxf(mt, s_m[w][row]);
+    for (int w = 0; w < warps; ++w) mt = fmaxf(mt, s_m[w][row]);
     float lt = a.sink != nullptr ? w_exp2(sk - mt) : 0.f, x0 = 0.f, x1 = 0.f;
-#pragma unroll
-    for (int w = 0; w < kWdWarps; ++w) {
-      if (w >= n_tiles) break;                  // warps without keys; one whose scores are all NaN has a maximum of -infinity as well, and counts
+    for (int w = 0; w < min(warps, n_tiles); ++w) {   // one whose scores are all NaN has a maximum of -infinity as well, and counts
       const float f = w_exp2(s_m[w][row] - mt);
       const float2 v = *reinterpret_cast<const float2*>(part + (w * kWdRows + row) * dv + col);
       lt = fmaf(s_l[w][row], f, lt);
@@ -1124,6 +1121,16 @@ extern "C" int omc_window_attn(const void* q, long long ldq, int T, int H, int G
   return check_launch("omc_window_attn");
 }
 
+// Warps of a decode CTA. Eight finish a CTA soonest, and take more than half an SM's shared memory at widths of 128 (two such CTAs fit at 64): right
+// while every CTA runs in the first wave. Beyond that four, of which three CTAs share an SM: short contexts are then a matter of CTAs, each some
+// 9 us from its first load to its last store. 128 + 128 columns, us at 8 / 4 / 2 warps (one warp of 64 threads per CTA in brackets): 256 CTAs over
+// 16 keys 19 / 11 / 12 (12), over 512 37 / 35 / 59 (104); 2048 CTAs over 16 keys 123 / 45 / 30 (49), over 512 257 / 176 / 199 (301); 128 CTAs over
+// 512 20 / 32 / 58 (55).
+static int win_decode_warps(long long ctas, size_t smem_of_eight) {
+  const int fit = smem_of_eight + 2048 <= 113 * 1024 ? 2 : 1;   // 1 KB of its own and 1 KB of the system's per CTA; 128 registers allow two as well
+  return ctas <= 148LL * fit ? 8 : 4;
+}
+
 extern "C" int omc_window_attn_mma_ok(int H, int G, int d, int dv) {
   if (H <= 0 || G <= 0 || H % G) return 0;
   const int rep = H / G;
@@ -1154,11 +1161,11 @@ extern "C" int omc_window_attn_mma(const void* q, long long ldq, int T, int H, i
     smem += bias_bytes;
   }
   dim3 grid(n, G * maps);
-  // one token per item and at most 16 rows, in tiles of 32 keys per warp that fit shared memory: the warps split the keys
-  const size_t part_bytes = sizeof(float) * kWdWarps * kWdRows * (size_t)dv;
-  size_t dec_smem = sizeof(bf16_t) * ((size_t)kWdRows * (d + 8) + (size_t)kWdWarps * kWdKeys * (d + dv + 16));
-  if (dec_smem < part_bytes) dec_smem = part_bytes;
-  const bool decode = items == nullptr && H / G <= kWdRows && dec_smem <= 220 * 1024;
+  // one token per item and at most 16 rows: the warps split the keys. At most 208 KB (d = 256, dv = 128), and the partial outputs always fit
+  const bool decode = items == nullptr && H / G <= kWdRows;
+  auto dec_bytes = [&](int warps) { return sizeof(bf16_t) * ((size_t)kWdRows * (d + 8) + (size_t)warps * kWdKeys * (d + dv + 16)); };
+  const int dec_warps = win_decode_warps((long long)n * G * maps, dec_bytes(kWdWarps));
+  const size_t dec_smem = dec_bytes(dec_warps);
 #define OMC_WIN_LAUNCH(NV, TO)                                                                                      \
   do {                                                                                                              \
     static bool attr_done[kMaxDevices] = {};                                                                        \
@@ -1167,7 +1174,7 @@ extern "C" int omc_window_attn_mma(const void* q, long long ldq, int T, int H, i
       cudaFuncSetAttribute(window_attn_decode_kernel<NV, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); \
       attr_done[cur_device()] = true;                                                                               \
     }                                                                                                               \
-    if (decode) window_attn_decode_kernel<NV, TO><<<grid, kWdWarps * 32, dec_smem, st>>>(a);                        \
+    if (decode) window_attn_decode_kernel<NV, TO><<<grid, dec_warps * 32, dec_smem, st>>>(a);                        \
     else window_attn_mma_kernel<NV, TO><<<grid, 128, smem, st>>>(a);                                                \
   } while (0)
   if (out_dt == OMC_DT_BF16) {
