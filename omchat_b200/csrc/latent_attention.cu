@@ -9,7 +9,7 @@
 //                        row's page (fused norm + rotation + cache write)
 //   omc_rotary_q         the rotated query parts, written behind the absorbed part of each head
 //   omc_latent_rope_store  both of these in one launch, the pairs of a rotation being (2i, 2i + 1) or (i, i + dims / 2)
-//   omc_latent_attn      plain kernel, any sizes, fp32 arithmetic: one CTA per (row, head), one warp per key, online softmax with
+//   omc_latent_attn      plain kernel, any sizes, fp32 arithmetic: one CTA per (row, head), four keys per warp at a time, online softmax with
 //                        an optional sink term exp(sink_h) that only enlarges the denominator
 // Rows of a step are addressed by (slot, position): a row sees cache entries 0..position of its slot, whether they were written
 // by this step or by earlier ones, so portions of prompts and single decoded tokens are the same case.
@@ -127,16 +127,20 @@ __device__ __forceinline__ float head_gate_f(const float* gate, long long ldg, l
   return gate != nullptr ? 1.f / (1.f + expf(-gate[t * ldg + h])) : 1.f;
 }
 
-constexpr int kLatWarps = 8, kLatKeys = 4;   // keys a warp takes at a time
+constexpr int kLatParts = 8;        // partial sums of a row
 constexpr int kLatMaxPerLane = 32;  // r <= 1024
 
-// One CTA per (row, head). The warps take groups of four keys in turn: lanes split the r + dr columns of the key rows for the dot products,
-// every lane keeps its share (columns lane, lane + 32, ...) of the running weighted sum of latents. The warps' partial (max, sum, accumulator)
-// triples are merged through shared memory at the end. Bound by the latency of a group's chain (page, rows, sum over lanes, exponential): four
-// keys share it, and eight warps overlap it. Eight heads in fp32 over rows of 320: a step of 376 prompt rows and six of three rows over some 130
-// keys together 437 us (one key at a time by four warps: 848).
-template <typename TQ, typename TC>
-__global__ void __launch_bounds__(kLatWarps * 32) latent_attn_kernel(const TQ* __restrict__ qcat, int H, int r, int dr,
+// One CTA per (row, head). Groups of KEYS keys go to eight partial sums in turn: the lanes of a warp split the r + dr columns of the key rows for
+// the dot products, and every lane keeps its share (columns lane, lane + 32, ... of up to PER_LANE) of the running weighted sum of latents. The
+// partial (max, sum, accumulator) triples that have keys are merged through shared memory at the end. Bound by the latency of a group's chain
+// (page, rows, sum over lanes, exponential): the keys of a group share it, and the warps overlap it. Eight warps where a step has few rows, one
+// partial sum each; four where CTAs abound, which then take two one after the other: the same bits. Four keys where rows are short; one where they
+// are wider than 256 latents: every row is read twice, and the rows of all groups under way have to stay in L1 in between. In us, in fp32, one key
+// at a time by four warps with registers for 1024 columns in brackets: 376 rows x 8 heads over rows of 256 + 64, all keys 206 (341), a window
+// of 16 24 (33); 16 heads over rows of 512 + 64 550 (836; four keys at a time 893), 67 (84; 174); 3 rows x 8 heads over 130 keys of 256 + 64
+// 14 (50).
+template <typename TQ, typename TC, int PER_LANE, int KEYS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 && PER_LANE == 32 ? 6 : 0) latent_attn_kernel(const TQ* __restrict__ qcat, int H, int r, int dr,
                                                                      const TC* __restrict__ pool,
                                                                      const int32_t* __restrict__ block_table, int max_pages,
                                                                      int page_size, const int32_t* __restrict__ pos,
@@ -144,88 +148,90 @@ __global__ void __launch_bounds__(kLatWarps * 32) latent_attn_kernel(const TQ* _
                                                                      const float* __restrict__ sink, int window,
                                                                      const float* __restrict__ gate, long long ldg, float scale,
                                                                      float* __restrict__ out) {
-  extern __shared__ float sm[];  // q [r + dr] | acc [kLatWarps][r] | m [kLatWarps] | l [kLatWarps]
+  extern __shared__ float sm[];  // q [r + dr] | acc [kLatParts][r] | m [kLatParts] | l [kLatParts]
   const int t = blockIdx.x, h = blockIdx.y;
   const int D = r + dr;
   float* sq = sm;
   float* sacc = sm + D;
-  float* s_m = sacc + kLatWarps * r;
-  float* s_l = s_m + kLatWarps;
+  float* s_m = sacc + kLatParts * r;
+  float* s_l = s_m + kLatParts;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const TQ* q = qcat + ((long long)t * H + h) * D;
   for (int c = threadIdx.x; c < D; c += blockDim.x) sq[c] = ldf(q + c);
   __syncthreads();
-  const int n_keys = pos[t] + 1;
+  const int n_keys = pos[t] + 1, low = max(0, n_keys - window), parts = min(kLatParts, (n_keys - low + KEYS - 1) / KEYS);
   const int32_t* bt = block_table + (long long)slot[t] * max_pages;
-  float m = -INFINITY, l = 0.f;
-  float acc[kLatMaxPerLane];
+  for (int part = warp; part < parts; part += WARPS) {
+    float m = -INFINITY, l = 0.f;
+    float acc[PER_LANE];
 #pragma unroll
-  for (int i = 0; i < kLatMaxPerLane; ++i) acc[i] = 0.f;
-  for (int j = max(0, n_keys - window) + warp * kLatKeys; j < n_keys; j += kLatWarps * kLatKeys) {
-    const TC* kr[kLatKeys];
-    float d[kLatKeys];
+    for (int i = 0; i < PER_LANE; ++i) acc[i] = 0.f;
+    for (int j = low + part * KEYS; j < n_keys; j += kLatParts * KEYS) {
+      const TC* kr[KEYS];
+      float d[KEYS];
 #pragma unroll
-    for (int u = 0; u < kLatKeys; ++u) {
-      const int ju = min(j + u, n_keys - 1);
-      kr[u] = pool + ((long long)bt[ju / page_size] * page_size + ju % page_size) * D;
-      d[u] = 0.f;
-    }
-    for (int c = lane; c < D; c += 32) {
-      const float qc = sq[c];
-#pragma unroll
-      for (int u = 0; u < kLatKeys; ++u) d[u] = fmaf(qc, ldf(kr[u] + c), d[u]);
-    }
-    float mn = m;
-#pragma unroll
-    for (int u = 0; u < kLatKeys; ++u) {
-      d[u] = seq_warp_sum(d[u]) * scale;
-      if (j + u < n_keys) mn = fmaxf(mn, d[u]);
-    }
-    const float corr = expf(m - mn);  // m = -inf on the first group: corr = 0
-    float pj[kLatKeys];
-#pragma unroll
-    for (int u = 0; u < kLatKeys; ++u) pj[u] = j + u < n_keys ? expf(d[u] - mn) : 0.f;
-    l = l * corr + ((pj[0] + pj[1]) + (pj[2] + pj[3]));
-#pragma unroll
-    for (int i = 0; i < kLatMaxPerLane; ++i) {
-      const int c = lane + 32 * i;
-      if (c < r) {
-        float s = acc[i] * corr;
-#pragma unroll
-        for (int u = 0; u < kLatKeys; ++u)
-          if (j + u < n_keys) s = fmaf(pj[u], ldf(kr[u] + c), s);
-        acc[i] = s;
+      for (int u = 0; u < KEYS; ++u) {
+        const int ju = min(j + u, n_keys - 1);
+        kr[u] = pool + ((long long)bt[ju / page_size] * page_size + ju % page_size) * D;
+        d[u] = 0.f;
       }
-    }
-    m = mn;
-  }
+      for (int c = lane; c < D; c += 32) {
+        const float qc = sq[c];
 #pragma unroll
-  for (int i = 0; i < kLatMaxPerLane; ++i) {
-    const int c = lane + 32 * i;
-    if (c < r) sacc[warp * r + c] = acc[i];
-  }
-  if (lane == 0) {
-    s_m[warp] = m;
-    s_l[warp] = l;
+        for (int u = 0; u < KEYS; ++u) d[u] = fmaf(qc, ldf(kr[u] + c), d[u]);
+      }
+      float mn = m;
+#pragma unroll
+      for (int u = 0; u < KEYS; ++u) {
+        d[u] = seq_warp_sum(d[u]) * scale;
+        if (j + u < n_keys) mn = fmaxf(mn, d[u]);
+      }
+      const float corr = expf(m - mn);  // m = -inf on the first group: corr = 0
+      float pj[KEYS];
+#pragma unroll
+      for (int u = 0; u < KEYS; ++u) pj[u] = j + u < n_keys ? expf(d[u] - mn) : 0.f;
+      l = l * corr + (KEYS == 4 ? (pj[0] + pj[1]) + (pj[KEYS / 2] + pj[KEYS - 1]) : KEYS == 2 ? pj[0] + pj[KEYS - 1] : pj[0]);
+#pragma unroll
+      for (int i = 0; i < PER_LANE; ++i) {
+        const int c = lane + 32 * i;
+        if (c < r) {
+          float s = acc[i] * corr;
+#pragma unroll
+          for (int u = 0; u < KEYS; ++u)
+            if (j + u < n_keys) s = fmaf(pj[u], ldf(kr[u] + c), s);
+          acc[i] = s;
+        }
+      }
+      m = mn;
+    }
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      const int c = lane + 32 * i;
+      if (c < r) sacc[part * r + c] = acc[i];
+    }
+    if (lane == 0) {
+      s_m[part] = m;
+      s_l[part] = l;
+    }
   }
   __syncthreads();
   float mt = -INFINITY;
-#pragma unroll
-  for (int w = 0; w < kLatWarps; ++w) mt = fmaxf(mt, s_m[w]);
+  for (int w = 0; w < parts; ++w) mt = fmaxf(mt, s_m[w]);
   if (sink != nullptr) mt = fmaxf(mt, sink[h]);
   float lt = sink != nullptr ? expf(sink[h] - mt) : 0.f;
-  float f[kLatWarps];
+  float f[kLatParts];
 #pragma unroll
-  for (int w = 0; w < kLatWarps; ++w) {
-    f[w] = s_m[w] == -INFINITY ? 0.f : expf(s_m[w] - mt);
-    lt += s_l[w] * f[w];
+  for (int w = 0; w < kLatParts; ++w) {
+    f[w] = w >= parts || s_m[w] == -INFINITY ? 0.f : expf(s_m[w] - mt);
+    if (w < parts) lt += s_l[w] * f[w];
   }
   const float inv = head_gate_f(gate, ldg, t, h) / lt;
   float* o = out + ((long long)t * H + h) * r;
   for (int c = threadIdx.x; c < r; c += blockDim.x) {
     float v = 0.f;
 #pragma unroll
-    for (int w = 0; w < kLatWarps; ++w) v += sacc[w * r + c] * f[w];
+    for (int w = 0; w < kLatParts; ++w)
+      if (w < parts) v += sacc[w * r + c] * f[w];
     o[c] = v * inv;
   }
 }
@@ -291,17 +297,21 @@ extern "C" int omc_latent_attn(const void* qcat, int q_dt, int T, int H, int r, 
   if (H > 65535) return set_error(OMC_ERR_SHAPE, "omc_latent_attn: more than 65535 heads");
   if (T == 0) return OMC_OK;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t smem = sizeof(float) * ((size_t)r + dr + (size_t)kLatWarps * r + 2 * kLatWarps);
+  const size_t smem = sizeof(float) * ((size_t)r + dr + (size_t)kLatParts * r + 2 * kLatParts);
   // the widths whose query and four partial outputs fit 48 KB; the eight partial outputs of the widest take up to 64 KB
   if (sizeof(float) * (5 * (size_t)r + dr + 8) > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_latent_attn: rows too wide");
   OMC_DT_SWITCH(q_dt, TQ, OMC_DT_SWITCH(pool_dt, TC, {
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(latent_attn_kernel<TQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    auto go = [&](auto kernel, int warps) {
+      if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return check_launch("omc_latent_attn");
+      kernel<<<dim3(T, H), warps * 32, smem, st>>>(static_cast<const TQ*>(qcat), H, r, dr, static_cast<const TC*>(pool), block_table, max_pages, page_size, pos, slot,
+                                                   sink, window, gate, ldg, scale, out);
       return check_launch("omc_latent_attn");
-    latent_attn_kernel<TQ, TC><<<dim3(T, H), kLatWarps * 32, smem, st>>>(static_cast<const TQ*>(qcat), H, r, dr,
-                                                                         static_cast<const TC*>(pool), block_table, max_pages,
-                                                                         page_size, pos, slot, sink, window, gate, ldg, scale, out);
+    };
+    const bool many = (long long)T * H > 4 * 148;
+    if (r <= 256) return many ? go(latent_attn_kernel<TQ, TC, 8, 4, 4>, 4) : go(latent_attn_kernel<TQ, TC, 8, 4, 8>, 8);
+    if (r <= 512) return many ? go(latent_attn_kernel<TQ, TC, 16, 1, 4>, 4) : go(latent_attn_kernel<TQ, TC, 16, 1, 8>, 8);
+    return many ? go(latent_attn_kernel<TQ, TC, kLatMaxPerLane, 1, 4>, 4) : go(latent_attn_kernel<TQ, TC, kLatMaxPerLane, 1, 8>, 8);
   }))
-  return check_launch("omc_latent_attn");
 }
 
 // ---------------------------------------------------------------------------------------------------------------------------

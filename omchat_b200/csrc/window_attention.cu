@@ -13,14 +13,14 @@
 // The distance bias arrives as a table [window, heads] that the host builds (here from a bucketed learned table; any function of
 // the distance fits). Prompt portions and decoded tokens are one case: row t at position pos[t] of slot[t] reads the cached
 // entries max(0, pos - window + 1, pos - pos % chunk) .. pos of its slot, which the store kernel of the same step has written.
-// The plain kernel: fp32 arithmetic, one CTA per (row, head), a warp per key, lanes across the head dimension.
+// The plain kernel: fp32 arithmetic, one CTA per (row, head), four keys per warp at a time, lanes across the head dimension.
 #include <math.h>
 
 #include "seq_common.cuh"
 
 namespace omc {
 
-constexpr int kWinWarps = 8, kWinKeys = 4;   // keys a warp takes at a time
+constexpr int kWinParts = 8, kWinKeys = 4;   // partial sums of a row; keys a warp takes at a time
 constexpr int kWinMaxPerLane = 8;  // value width up to 256
 
 // Rotation of the first `dims` dimensions of every `width` consecutive columns by a host-built table of (cos, sin) [position][dims / 2][2]
@@ -210,8 +210,10 @@ __global__ void __launch_bounds__(256) pos_qkv_store_kernel(const float* __restr
   }
 }
 
-template <typename TQ, typename TC, typename TY>
-__global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(const TQ* __restrict__ q, long long ldq, int H, int G, int d,
+// Groups of four keys go to eight partial sums in turn, those that have keys are merged at the end: as latent_attn_kernel, with up to PER_LANE
+// values per lane.
+template <typename TQ, typename TC, typename TY, int PER_LANE, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) window_attn_kernel(const TQ* __restrict__ q, long long ldq, int H, int G, int d,
                                                                      int dv, int maps, const TC* __restrict__ pool,
                                                                      const int32_t* __restrict__ block_table, int max_pages,
                                                                      int page_size, const int32_t* __restrict__ pos,
@@ -220,13 +222,13 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(const TQ* _
                                                                      const float* __restrict__ sink, const float* __restrict__ gate,
                                                                      long long ldg, int gate_act, int gate_heads, TY* __restrict__ out,
                                                                      long long ldo) {
-  extern __shared__ float sm[];  // q [d] | acc [warps][dv] | m [warps] | l [warps]
+  extern __shared__ float sm[];  // q [d] | acc [parts][dv] | m [parts] | l [parts]
   // blockIdx.y = head * maps + map: queries and outputs are laid out [head][map][.], keys [key/value head][map][d]
   const int t = blockIdx.x, hm = blockIdx.y, h = hm / maps, mp = hm - h * maps, kvh = h / (H / G);
   float* sq = sm;
   float* sacc = sm + d;
-  float* s_m = sacc + kWinWarps * dv;
-  float* s_l = s_m + kWinWarps;
+  float* s_m = sacc + kWinParts * dv;
+  float* s_l = s_m + kWinParts;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int c = threadIdx.x; c < d; c += blockDim.x) sq[c] = ldf(q + (long long)t * ldq + hm * d + c);
   __syncthreads();
@@ -236,83 +238,85 @@ __global__ void __launch_bounds__(kWinWarps * 32) window_attn_kernel(const TQ* _
   const int32_t* bt = block_table + (long long)slot[t] * max_pages;
   const int W = G * (maps * d + dv);
   const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
-  float m = -INFINITY, l = 0.f;
-  float acc[kWinMaxPerLane];
-#pragma unroll
-  for (int i = 0; i < kWinMaxPerLane; ++i) acc[i] = 0.f;
   // the visible keys in one sequence of indices: 0 .. kept - 1, then first .. p
-  const int n_keys = kept + (p - first + 1);
-  for (int i = warp * kWinKeys; i < n_keys; i += kWinWarps * kWinKeys) {
-    const TC* kr[kWinKeys];
-    const TC* vr[kWinKeys];
-    int back[kWinKeys];
-    float s[kWinKeys];
+  const int n_keys = kept + (p - first + 1), parts = min(kWinParts, (n_keys + kWinKeys - 1) / kWinKeys);
+  for (int part = warp; part < parts; part += WARPS) {
+    float m = -INFINITY, l = 0.f;
+    float acc[PER_LANE];
 #pragma unroll
-    for (int u = 0; u < kWinKeys; ++u) {
-      const int iu = min(i + u, n_keys - 1), j = iu < kept ? iu : first + (iu - kept);
-      const TC* row = pool + ((long long)bt[j / page_size] * page_size + j % page_size) * W;
-      kr[u] = row + (kvh * maps + mp) * d;
-      vr[u] = row + G * maps * d + kvh * dv;
-      back[u] = p - j;
-      s[u] = 0.f;
-    }
-    for (int c = lane; c < d; c += 32) {
-      const float qc = sq[c];
+    for (int i = 0; i < PER_LANE; ++i) acc[i] = 0.f;
+    for (int i = part * kWinKeys; i < n_keys; i += kWinParts * kWinKeys) {
+      const TC* kr[kWinKeys];
+      const TC* vr[kWinKeys];
+      int back[kWinKeys];
+      float s[kWinKeys];
 #pragma unroll
-      for (int u = 0; u < kWinKeys; ++u) s[u] = fmaf(qc, ldf(kr[u] + c), s[u]);
-    }
-    float mn = m;
-#pragma unroll
-    for (int u = 0; u < kWinKeys; ++u) {
-      s[u] = seq_warp_sum(s[u]) * scale;
-      if (softcap > 0.f) s[u] = softcap * tanhf(s[u] * inv_cap);
-      if (dist_bias != nullptr && back[u] < window) s[u] += dist_bias[(long long)back[u] * H + h];
-      if (i + u < n_keys) mn = fmaxf(mn, s[u]);
-    }
-    const float corr = expf(m - mn);  // m = -inf on the first group: corr = 0
-    float pj[kWinKeys];
-#pragma unroll
-    for (int u = 0; u < kWinKeys; ++u) pj[u] = i + u < n_keys ? expf(s[u] - mn) : 0.f;
-    l = l * corr + ((pj[0] + pj[1]) + (pj[2] + pj[3]));
-#pragma unroll
-    for (int i2 = 0; i2 < kWinMaxPerLane; ++i2) {
-      const int c = lane + 32 * i2;
-      if (c < dv) {
-        float x = acc[i2] * corr;
-#pragma unroll
-        for (int u = 0; u < kWinKeys; ++u)
-          if (i + u < n_keys) x = fmaf(pj[u], ldf(vr[u] + c), x);
-        acc[i2] = x;
+      for (int u = 0; u < kWinKeys; ++u) {
+        const int iu = min(i + u, n_keys - 1), j = iu < kept ? iu : first + (iu - kept);
+        const TC* row = pool + ((long long)bt[j / page_size] * page_size + j % page_size) * W;
+        kr[u] = row + (kvh * maps + mp) * d;
+        vr[u] = row + G * maps * d + kvh * dv;
+        back[u] = p - j;
+        s[u] = 0.f;
       }
-    }
-    m = mn;
-  }
+      for (int c = lane; c < d; c += 32) {
+        const float qc = sq[c];
 #pragma unroll
-  for (int i = 0; i < kWinMaxPerLane; ++i) {
-    const int c = lane + 32 * i;
-    if (c < dv) sacc[warp * dv + c] = acc[i];
-  }
-  if (lane == 0) {
-    s_m[warp] = m;
-    s_l[warp] = l;
+        for (int u = 0; u < kWinKeys; ++u) s[u] = fmaf(qc, ldf(kr[u] + c), s[u]);
+      }
+      float mn = m;
+#pragma unroll
+      for (int u = 0; u < kWinKeys; ++u) {
+        s[u] = seq_warp_sum(s[u]) * scale;
+        if (softcap > 0.f) s[u] = softcap * tanhf(s[u] * inv_cap);
+        if (dist_bias != nullptr && back[u] < window) s[u] += dist_bias[(long long)back[u] * H + h];
+        if (i + u < n_keys) mn = fmaxf(mn, s[u]);
+      }
+      const float corr = expf(m - mn);  // m = -inf on the first group: corr = 0
+      float pj[kWinKeys];
+#pragma unroll
+      for (int u = 0; u < kWinKeys; ++u) pj[u] = i + u < n_keys ? expf(s[u] - mn) : 0.f;
+      l = l * corr + ((pj[0] + pj[1]) + (pj[2] + pj[3]));
+#pragma unroll
+      for (int i2 = 0; i2 < PER_LANE; ++i2) {
+        const int c = lane + 32 * i2;
+        if (c < dv) {
+          float x = acc[i2] * corr;
+#pragma unroll
+          for (int u = 0; u < kWinKeys; ++u)
+            if (i + u < n_keys) x = fmaf(pj[u], ldf(vr[u] + c), x);
+          acc[i2] = x;
+        }
+      }
+      m = mn;
+    }
+#pragma unroll
+    for (int i = 0; i < PER_LANE; ++i) {
+      const int c = lane + 32 * i;
+      if (c < dv) sacc[part * dv + c] = acc[i];
+    }
+    if (lane == 0) {
+      s_m[part] = m;
+      s_l[part] = l;
+    }
   }
   __syncthreads();
   // the sink: one more term exp(sink[h]) in the denominator, without a key or a value
   float mt = sink != nullptr ? sink[h] : -INFINITY;
-#pragma unroll
-  for (int w = 0; w < kWinWarps; ++w) mt = fmaxf(mt, s_m[w]);
+  for (int w = 0; w < parts; ++w) mt = fmaxf(mt, s_m[w]);
   float lt = sink != nullptr ? expf(sink[h] - mt) : 0.f;
-  float f[kWinWarps];
+  float f[kWinParts];
 #pragma unroll
-  for (int w = 0; w < kWinWarps; ++w) {
-    f[w] = s_m[w] == -INFINITY ? 0.f : expf(s_m[w] - mt);
-    lt += s_l[w] * f[w];
+  for (int w = 0; w < kWinParts; ++w) {
+    f[w] = w >= parts || s_m[w] == -INFINITY ? 0.f : expf(s_m[w] - mt);
+    if (w < parts) lt += s_l[w] * f[w];
   }
   const float inv = 1.f / lt;
   for (int c = threadIdx.x; c < dv; c += blockDim.x) {
     float o = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWinWarps; ++w) o += sacc[w * dv + c] * f[w];
+    for (int w = 0; w < kWinParts; ++w)
+      if (w < parts) o += sacc[w * dv + c] * f[w];
     o *= inv;
     if (gate != nullptr) {
       const float z = gate[(long long)t * ldg + (gate_heads ? hm : hm * dv + c)];
@@ -1107,18 +1111,22 @@ extern "C" int omc_window_attn(const void* q, long long ldq, int T, int H, int G
   if (dv > 32 * kWinMaxPerLane) return set_error(OMC_ERR_SHAPE, "omc_window_attn: value width above 256");
   if ((long long)H * maps > 65535) return set_error(OMC_ERR_SHAPE, "omc_window_attn: more than 65535 heads");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const size_t smem = sizeof(float) * ((size_t)d + (size_t)kWinWarps * dv + 2 * kWinWarps);
+  const size_t smem = sizeof(float) * ((size_t)d + (size_t)kWinParts * dv + 2 * kWinParts);
   // the widths whose query and four partial outputs fit 48 KB; the eight partial outputs of the widest take up to 52 KB
   if (sizeof(float) * ((size_t)d + 4 * (size_t)dv + 8) > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_window_attn: head width too large");
   OMC_DT_SWITCH(dt, TC, OMC_DT_SWITCH(out_dt, TY, {
-    if (smem > 48 * 1024 && cudaFuncSetAttribute(window_attn_kernel<TC, TC, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    auto go = [&](auto kernel, int warps) {
+      if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return check_launch("omc_window_attn");
+      kernel<<<dim3(T, H * maps), warps * 32, smem, st>>>(static_cast<const TC*>(q), ldq, H, G, d, dv, maps, static_cast<const TC*>(pool), block_table, max_pages,
+                                                          page_size, pos, slot, window, chunk, keep_first, scale, softcap, dist_bias, sink, gate, ldg, gate_act,
+                                                          gate_heads, static_cast<TY*>(out), ldo);
       return check_launch("omc_window_attn");
-    window_attn_kernel<TC, TC, TY><<<dim3(T, H * maps), kWinWarps * 32, smem, st>>>(static_cast<const TC*>(q), ldq, H, G, d, dv, maps,
-                                                                                   static_cast<const TC*>(pool), block_table, max_pages,
-                                                                                   page_size, pos, slot, window, chunk, keep_first, scale, softcap,
-                                                                                   dist_bias, sink, gate, ldg, gate_act, gate_heads, static_cast<TY*>(out), ldo);
+    };
+    const bool many = (long long)T * H * maps > 4 * 148;
+    if (dv <= 64) return many ? go(window_attn_kernel<TC, TC, TY, 2, 4>, 4) : go(window_attn_kernel<TC, TC, TY, 2, 8>, 8);
+    if (dv <= 128) return many ? go(window_attn_kernel<TC, TC, TY, 4, 4>, 4) : go(window_attn_kernel<TC, TC, TY, 4, 8>, 8);
+    return many ? go(window_attn_kernel<TC, TC, TY, kWinMaxPerLane, 4>, 4) : go(window_attn_kernel<TC, TC, TY, kWinMaxPerLane, 8>, 8);
   }))
-  return check_launch("omc_window_attn");
 }
 
 // Warps of a decode CTA. Eight finish a CTA soonest, and take more than half an SM's shared memory at widths of 128 (two such CTAs fit at 64): right
