@@ -52,13 +52,10 @@ class LatentAttention:
         plan = plans.get((H, window, tcgen05))
         if plan is None:
             if "portions" in plans:
-                # the tcgen05 kernel runs one CTA per SM on tiles of 128 keys: contexts are cut only while that leaves half the SMs idle
-                cut = dict(target_ctas=148, min_keys=256) if tcgen05 else {}
-                plan = seqlib.LatentAttnPlan(plans["portions"], H, self.device, window=window, **cut)
+                plan = self._prompt_plan(plans["portions"], H, self.device, window, tcgen05)
             else:
                 keys = min(window, plans["decode_keys"]) if "decode_keys" in plans else 0
-                parts = (plans["decode_parts"] if "decode_parts" in plans else
-                         seqlib.DecodeAttnPlan.parts_for_tcgen05(T, keys) if tcgen05 else self._decode_parts(T, keys))
+                parts = plans["decode_parts"] if "decode_parts" in plans else self._decode_parts(T, keys, tcgen05)
                 key = (T, H, parts, window)
                 plan = self._decode_plans.get(key)
                 if plan is None:
@@ -68,8 +65,15 @@ class LatentAttention:
         return plan
 
     @staticmethod
-    def _decode_parts(T: int, keys: int) -> int:
-        """Key ranges per row of a decode-only step: of 128 keys or more, of 64 where a short window would leave SMs without a CTA."""
+    def _prompt_plan(portions, H: int, device, window: int, tcgen05: bool) -> seqlib.LatentAttnPlan:
+        # the tcgen05 kernel runs one CTA per SM on tiles of 128 keys: contexts are cut only while that leaves half the SMs idle
+        return seqlib.LatentAttnPlan(portions, H, device, window=window, **(dict(target_ctas=148, min_keys=256) if tcgen05 else {}))
+
+    @staticmethod
+    def _decode_parts(T: int, keys: int, tcgen05: bool) -> int:
+        """Key ranges per row of a decode-only step; of the mma.sync kernel 128 keys or more, 64 where a short window would leave SMs without a CTA."""
+        if tcgen05:
+            return seqlib.DecodeAttnPlan.parts_for_tcgen05(T, keys)
         parts = seqlib.DecodeAttnPlan.parts_for(T, keys)
         return parts if T * parts >= 148 else seqlib.DecodeAttnPlan.parts_for(T, keys, min_keys=64)
 

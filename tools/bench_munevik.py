@@ -176,7 +176,7 @@ def kernels(z, n_seq, L, B, ctx):
     portions = [(s * L, L, s, 0) for s in range(n_seq)]
     for name, win, gt in (("voduzen_latent_attn_prefill", seqlib.WINDOW_ALL, None), ("latent_attn_window_gate_prefill", z["win"], gate),
                           ("latent_attn_window256_gate_prefill", 256, gate)):
-        plan = seqlib.LatentAttnPlan(portions, H, dev, window=win)
+        plan = LatentAttention._prompt_plan(portions, H, dev, win, seqlib.latent_attn_tcgen05_ok(H, r, dr, page))
         ms = timed(lambda: seqlib.latent_attn_mma(q, r, dr, pool, table, page, plan, None, 0.07, o, window=win, gate=gt))
         vis = n_seq * sum(min(i + 1, win) for i in range(L))
         out[name] = rate(ms, flops=vis * H * 2.0 * (2 * r + dr), ctas=plan.n_items)
@@ -189,7 +189,7 @@ def kernels(z, n_seq, L, B, ctx):
     for name, win, gt in (("voduzen_latent_attn_decode", seqlib.WINDOW_ALL, None), ("latent_attn_window_gate_decode", z["win"], gate[:B]),
                           ("latent_attn_window256_gate_decode", 256, gate[:B])):
         keys = min(win, ctx + 1)
-        plan = seqlib.DecodeAttnPlan(B, H, LatentAttention._decode_parts(B, keys), dev, window=win)
+        plan = seqlib.DecodeAttnPlan(B, H, LatentAttention._decode_parts(B, keys, seqlib.latent_attn_tcgen05_ok(H, r, dr, page)), dev, window=win)
         plan.fill(posd, slotd)
         ms = timed(lambda: seqlib.latent_attn_mma(q, r, dr, pool, table, page, plan, None, 0.07, o, window=win, gate=gt))
         out[name] = rate(ms, B * keys * D * 2, batch=B, keys=keys, ctas=plan.n_items)

@@ -180,7 +180,8 @@ def kernels(z, n_seq, L, B, ctx):
         out[name] = rate(ms, T * (D * 6 + H * dr * 4))
     q.normal_(std=0.3)
     o, sink = torch.empty(T, H, r, device=dev, dtype=bf), torch.zeros(H, device=dev)
-    plan = seqlib.LatentAttnPlan(portions, H, dev)
+    tcgen05 = seqlib.latent_attn_tcgen05_ok(H, r, dr, page)
+    plan = LatentAttention._prompt_plan(portions, H, dev, seqlib.WINDOW_ALL, tcgen05)
     for name, sk in (("latent_attn_sink", sink), ("voduzen_latent_attn", None)):
         ms = timed(lambda: seqlib.latent_attn_mma(q, r, dr, lpool, table, page, plan, sk, 0.07, o))
         out[name + "_prefill"] = rate(ms, flops=n_seq * L * (L + 1) / 2 * H * 2.0 * (2 * r + dr), ctas=plan.n_items)
@@ -192,7 +193,7 @@ def kernels(z, n_seq, L, B, ctx):
     del lpool, q, o
     lpool = (torch.randn(B * pages_d + 1, page, D, device=dev) * 0.3).to(bf)
     q, o = (torch.randn(B, H, D, device=dev) * 0.3).to(bf), torch.empty(B, H, r, device=dev, dtype=bf)
-    plan = seqlib.DecodeAttnPlan(B, H, LatentAttention._decode_parts(B, ctx + 1), dev)
+    plan = seqlib.DecodeAttnPlan(B, H, LatentAttention._decode_parts(B, ctx + 1, tcgen05), dev)
     plan.fill(posd, slotd)
     for name, sk in (("latent_attn_sink", sink), ("voduzen_latent_attn", None)):
         ms = timed(lambda: seqlib.latent_attn_mma(q, r, dr, lpool, tabled, page, plan, sk, 0.07, o))

@@ -23,6 +23,7 @@ import torch  # noqa: E402
 
 from omchat_b200 import lib, seqlib  # noqa: E402
 from omchat_b200.config import VoduzenConfig  # noqa: E402
+from omchat_b200.model.seq_latent import LatentAttention  # noqa: E402
 from omchat_b200.model.voduzen import VoduzenForCausalLM, random_state_dict  # noqa: E402
 from omchat_b200.serving import StepScheduler  # noqa: E402
 
@@ -96,7 +97,8 @@ def kernels(z, n_seq, L, B, ctx):
     table = (torch.arange(n_seq * pages_per, dtype=i32, device=dev) + 1).view(n_seq, pages_per).contiguous()
     q = (torch.randn(T, H, D, device=dev) * 0.3).to(bf)
     o = torch.empty(T, H, r, device=dev, dtype=f32)
-    plan = seqlib.LatentAttnPlan([(s * L, L, s, 0) for s in range(n_seq)], H, dev)
+    tcgen05 = seqlib.latent_attn_tcgen05_ok(H, r, dr, page)
+    plan = LatentAttention._prompt_plan([(s * L, L, s, 0) for s in range(n_seq)], H, dev, seqlib.WINDOW_ALL, tcgen05)
     ms = timed(lambda: seqlib.latent_attn_mma(q, r, dr, pool, table, page, plan, None, 0.07, o))
     flops = n_seq * H * (L * (L + 1) / 2) * 2 * (2 * r + dr)
     out["latent_attn_prefill"] = {"ms": ms, "tflops": flops / ms / 1e9, "frac_tensor": flops / ms / 1e9 / tf}
@@ -113,7 +115,8 @@ def kernels(z, n_seq, L, B, ctx):
     table = (torch.arange(B * pages_per, dtype=i32, device=dev) + 1).view(B, pages_per).contiguous()
     q = (torch.randn(B, H, D, device=dev) * 0.3).to(bf)
     o = torch.empty(B, H, r, device=dev, dtype=f32)
-    plan = seqlib.LatentAttnPlan([(b, 1, b, ctx) for b in range(B)], H, dev)
+    plan = seqlib.DecodeAttnPlan(B, H, LatentAttention._decode_parts(B, ctx + 1, tcgen05), dev)
+    plan.fill(torch.full((B,), ctx, dtype=i32, device=dev), torch.arange(B, dtype=i32, device=dev))
     ms = timed(lambda: seqlib.latent_attn_mma(q, r, dr, pool, table, page, plan, None, 0.07, o))
     nbytes = B * (ctx + 1) * D * 2
     out["latent_attn_decode"] = {"batch": B, "ctx": ctx, "ms": ms, "gbs": nbytes / ms / 1e6, "frac_hbm": nbytes / ms / 1e6 / hbm,
