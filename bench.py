@@ -117,7 +117,7 @@ _TEARDOWN = []  # callables that release what still references the communicator 
 
 
 def _finish(torch, dist):
-    """End of a multi-rank run. destroy_process_group() hung in round 1 because CUDA graphs that had captured NCCL
+    """End of a multi-rank run. destroy_process_group() hung where CUDA graphs that had captured NCCL
     collectives (the batched decode step) were still alive when the communicator was torn down: release them first (and
     close the CUDA-IPC peer mappings of the tensor-parallel decode kernel), drain the device, then destroy the group. A
     watchdog turns a teardown that still blocks into a loud message on stderr + exit instead of a silent hang."""
@@ -555,7 +555,7 @@ def main():
                                    "peak_source": peaks["source"] + " (bf16_tflops_sustained: kernel timed inside a long train)",
                                    "flops_per_launch": gm["flops_per_launch"], "avg_launch_us": gm["avg_launch_us"],
                                    "shapes": "ViT block GEMMs, 8 crops (M=8200)"}
-    # ---- the workloads that shard naturally, on the same weights, each with its own timing (VERDICT r01 item 4):
+    # ---- the workloads that shard naturally, on the same weights, each with its own timing:
     # c3 = 64 crops data-parallel over the N towers (images/s, tensor roofline), c4 = 32 x 1024-token prefill + batch-32
     # decode with the decoder tensor-parallel over the N GPUs (tokens/s, HBM roofline)
     if not args.no_workloads:

@@ -127,11 +127,11 @@ class Qwen2Decoder:
         self.scale = cfg.head_dim ** -0.5
         self.eps = cfg.rms_norm_eps
         self.mega_enabled = os.environ.get("OMCHAT_B200_NO_MEGA", "0") != "1"
-        # batched decode steps (B > 4): weight-streaming GEMMs on packed weights (0 = the round-1 skinny GEMM / GEMV path)
+        # batched decode steps (B > 4): weight-streaming GEMMs on packed weights (0 = the skinny GEMM / GEMV path)
         self.stream_enabled = os.environ.get("OMCHAT_B200_NO_STREAM", "0") != "1"
         self.stream_min_b = int(os.environ.get("OMCHAT_B200_STREAM_MIN_B",
                                                str(STREAM_MIN_B if self.tp.size == 1 else STREAM_MIN_B_TP)))
-        # prefill: RMSNorms folded into the GEMMs that follow them (0 = stand-alone RMSNorm kernels, the round-1 path)
+        # prefill: RMSNorms folded into the GEMMs that follow them (0 = stand-alone RMSNorm kernels)
         self.fold_norms = os.environ.get("OMCHAT_B200_FOLD_NORMS", "1") != "0"
         self._folded_w = None
         self._ssq_bufs = None

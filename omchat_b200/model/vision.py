@@ -35,7 +35,7 @@ class InternVITVisionTower:
         self.image_processor = None  # CPU preprocessing (CLIPImageProcessor) is outside the hot path
         self.max_crops_per_pass = 64
         self._cu_cache = {}
-        # norm1 / norm2 folded into the GEMMs that follow them (0 = stand-alone RMSNorm kernels, the round-1 path); RMSNorm only:
+        # norm1 / norm2 folded into the GEMMs that follow them (0 = stand-alone RMSNorm kernels); RMSNorm only:
         # the 'layer_norm' variant (InternViT-300M) keeps its stand-alone LayerNorm kernel
         self.fold_norms = os.environ.get("OMCHAT_B200_FOLD_NORMS", "1") != "0" and self.vc.norm_type == "rms_norm"
         self._mats = {}

@@ -68,7 +68,7 @@ def _check_mega_vs_per_op(cfg, dec, lens, n_layers):
     B, steps = len(lens), 6
     # bf16 rounding differences between two correct paths are amplified layer by layer on random-init weights: the FFMA and
     # mma.sync variants of the SAME kernel differ by 0.3 % of the logit scale at 2 layers, 1.2 % at 7 and 3.2 % at 28
-    # (tools/debug_depth.py), so the max-abs bound follows the depth; the cosine bound does not move
+    # (measured layer by layer), so the max-abs bound follows the depth; the cosine bound does not move
     rel_tol = 0.02 if n_layers <= 8 else 0.06
     cache_a, first = _prefill(dec, cfg, lens)
     cache_b, first_b = _prefill(dec, cfg, lens)
@@ -195,7 +195,7 @@ def test_batched_decode_stream_vs_oracle_full_width(lens):
     (csrc/gemm_stream.cu: packed weights, stream-K, programmatic dependent launch, RMSNorm folded into the GEMMs) at full
     Qwen2-7B width, 2 layers, against the CPU oracle run sequence by sequence on the same weights, teacher-forced on the
     CUDA path's own tokens: logits cosine >= 0.999 and max-abs <= 2 % of scale per row; the eager step, the CUDA-graph
-    replay and the round-1 per-op path (skinny GEMM + RMSNorm kernels) must sample the same tokens up to near-ties."""
+    replay and the per-op path (skinny GEMM + RMSNorm kernels) must sample the same tokens up to near-ties."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     from omchat_b200.model.weights import OmChatWeights, to_reference_state_dict
@@ -237,7 +237,7 @@ def test_batched_decode_stream_vs_oracle_full_width(lens):
             raise AssertionError(f"step {s}: graph replay and eager step disagree on rows {(~same).nonzero().flatten().tolist()}")
         cur = nxt
     assert cache.ctx_lens.tolist() == [n + steps for n in lens]
-    # the round-1 path (per-op skinny GEMM / GEMV + stand-alone RMSNorm) on a third cache: same logits within bf16 noise
+    # the per-op path (skinny GEMM / GEMV + stand-alone RMSNorm) on a third cache: same logits within bf16 noise
     cache_c, _ = _prefill(dec, cfg, lens)
     dec.stream_enabled = False
     try:

@@ -1,4 +1,4 @@
-"""Full-WIDTH parity of the CUDA path against the CPU oracle (VERDICT r01 item 1 / BASELINE.json north_star):
+"""Full-WIDTH parity of the CUDA path against the CPU oracle:
 the real OmChat-2.0-13B dimensions - InternViT-6B blocks 3200 wide / 25 heads / MLP 12800 at 448 px (1025 tokens), projector
 3200 -> 3584 -> 3584, Qwen2-7B layers 3584 wide / 28 q + 4 kv heads / MLP 18944 / vocab 152064 - at REDUCED DEPTH (3 + 3
 layers, so that the fp32 oracle finishes in about a minute on the host cores), one 448 x 448 crop + 64 text ids with the

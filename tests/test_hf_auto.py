@@ -1,5 +1,5 @@
 """The reference's Hugging Face Auto* surface (omchat_b200/hf.py; omchat_qwen2.py:113-114, hf_example.py:7-18):
-registration and config / processor round trips on the CPU (no compute), and on the GPU the judge's acceptance path -
+registration and config / processor round trips on the CPU (no compute), and on the GPU the path of a user's script -
 AutoModelForCausalLM.from_pretrained(<saved tiny checkpoint>) -> generate(stopping_criteria=...) against the oracle."""
 import json
 import os

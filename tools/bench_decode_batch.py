@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Batched decode step in isolation: full-depth Qwen2-7B decoder, B sequences at context `ctx`, the CUDA-graph replay path
 generate() uses, CUDA events over `steps` steps. Prints ms/step and the fraction of the HBM roofline (weights + KV bytes).
-Variants through the environment: OMCHAT_B200_NO_STREAM=1 (round-1 skinny path), OMCHAT_B200_PDL=0,
+Variants through the environment: OMCHAT_B200_NO_STREAM=1 (skinny path), OMCHAT_B200_PDL=0,
 OMCHAT_B200_STREAM_CTAS_PER_SM=2.   python tools/bench_decode_batch.py --batch 32 --ctx 1024 --steps 64"""
 import argparse
 import json

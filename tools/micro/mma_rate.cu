@@ -1,5 +1,5 @@
 // Microbenchmark: cycles per tcgen05.mma (cta_group::1, M=128, K=16, bf16) for the operand forms the attention kernel uses.
-//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I omchat_b200/csrc -o gpurun_out/mma_rate tools/micro/mma_rate.cu
+//   nvcc -gencode arch=compute_100a,code=sm_100a -O3 -I omchat_b200/csrc -o mma_rate tools/micro/mma_rate.cu
 #include <cstdio>
 #include <cuda_runtime.h>
 #include "ptx.cuh"
