@@ -6,7 +6,7 @@
 // MMA issuer. Warps 2..5: epilogue, thread = row. The K terms of an output are added in one order whatever the tile, so a row's result does
 // not depend on M.
 // What bounds it: the output's and the gate's bytes (51 MB, 1.4 TB/s), behind the set-up and the first load of a tile. 3126 rows x 16 heads, 128 -> 512:
-// 38 us = 690 TFLOP/s; 512 -> 128 with a gate per element 48 us; 32 rows: 6 us each (mma.sync with a two-stage cp.async ring before: 140, 141, 21).
+// 38 us = 172 TFLOP/s; 512 -> 128 with a gate per element 48 us; 32 rows: 6 us each (mma.sync with a two-stage cp.async ring before: 140, 141, 21).
 #include "linear_args.cuh"
 #include "sm100_step.cuh"
 
@@ -238,7 +238,7 @@ static int hg_launch_typed(const LinearArgs& a, int batch, cudaStream_t st) {
   return hg_launch<64, TY>(a, batch, st);
 }
 
-// X and W bf16 with rows and batch items on 16-byte boundaries (mma_operands_ok of linear_any.cu)
+// X and W bf16 with rows and batch items on 16-byte boundaries (sm100_operands_ok of linear_any.cu)
 int linear_sm100(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
   if (y_dt == OMC_DT_F32) return hg_launch_typed<float>(a, batch, st);
   if (y_dt == OMC_DT_BF16) return hg_launch_typed<bf16_t>(a, batch, st);
@@ -247,14 +247,15 @@ int linear_sm100(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
 
 int latent_sm100_failures(unsigned int* n);   // latent_attention_sm100.cu
 
-// out: a wait for a barrier that nothing arrives at; the next one for it; one for a barrier that a later thread arrives at, as a wait and as a drain
+// out: a wait for a barrier that nothing arrives at; the next one for it; one for a barrier that another thread arrives at only behind it; a drain of
+// that one
 __global__ void step_wait_selfcheck_kernel(int32_t* out, unsigned int* failed) {
   __shared__ uint64_t never, late;
-  __shared__ uint32_t dead;
+  __shared__ uint32_t dead, refused;
   if (threadIdx.x == 0) {
     mbar_init(&never, 1);
     mbar_init(&late, 1);
-    dead = 0u;
+    dead = refused = 0u;
     fence_barrier_init();
   }
   __syncthreads();
@@ -263,10 +264,11 @@ __global__ void step_wait_selfcheck_kernel(int32_t* out, unsigned int* failed) {
     out[0] = wait_bounded(&never, 0, report, 8);
     out[1] = wait_bounded(&never, 0, report);
     out[2] = wait_bounded(&late, 0, report);
+    *reinterpret_cast<volatile uint32_t*>(&refused) = 1u;
     out[3] = drain_bounded(&late, 0, report);
   } else if (threadIdx.x == 32) {
-    for (int i = 0; i < 1000000 && !*reinterpret_cast<volatile uint32_t*>(&dead); ++i) __nanosleep(1000);   // thread 0 sets it after its eight tries
-    __nanosleep(200000);
+    for (int i = 0; i < 1000000 && !*reinterpret_cast<volatile uint32_t*>(&refused); ++i) __nanosleep(1000);   // thread 0 sets it after its eight tries
+    __nanosleep(20000);
     mbar_arrive(&late);
   }
 }
