@@ -287,22 +287,58 @@ class LatentAttnPlan:
 
     MAX_PARTS = 64  # key ranges one merge group may have (csrc/latent_attention.cu: kMergeMaxParts)
 
+    FEW_TILES = 24  # up to here a loop builds the lists sooner than array arithmetic, some 60 calls of a microsecond or two: 5 rows 18 us (120)
+
     def __init__(self, portions, H: int, device, target_ctas: int = 296, min_keys: int = 128, window: int = WINDOW_ALL):
+        portions, tok = list(portions), max(1, MMA_ROWS // H)
+        base = sum(-(-n // tok) for _, n, _, _ in portions)                 # row tiles
+        build = self._by_loop if base <= self.FEW_TILES else self._by_arrays
+        numbers, self.n_items, self.n_merges, self.n_parts = build(portions, H, tok, base, target_ctas, min_keys, window)
+        self.max_rows = max((min(tok, n) for _, n, _, _ in portions), default=1) * H   # (token, head) pairs of the largest item
+        buf = torch.as_tensor(numbers, dtype=torch.int32).pin_memory().to(device, non_blocking=True)
+        self.items = buf[:self.n_items * 8]
+        self.merges = buf[self.n_items * 8:] if self.n_merges else None
+
+    @classmethod
+    def _by_loop(cls, portions, H, tok, base, target_ctas, min_keys, window):
+        items, merges, part = [], [], 0
+        for first_row, n, slot, p0 in portions:
+            for start in range(0, n, tok):
+                ntok, first = min(tok, n - start), p0 + start
+                low = max(0, first - window + 1)                            # first key the tile's first row sees
+                keys = first + ntok - low                                   # ... up to the end of what its last row sees
+                want = 1
+                if base < target_ctas // 2:
+                    want = max(1, min(-(-keys // min_keys), -(-target_ctas // base), cls.MAX_PARTS))
+                if want == 1:
+                    items.append((first_row + start, ntok, slot, first, low, low + keys, -1, 0))
+                    continue
+                span = -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS        # keys per part, a multiple of 64
+                ends = [min(keys, at + span) for at in range(0, keys, span)]
+                merges += [(first_row + start) * H, ntok * H, part, len(ends)]
+                for i, end in enumerate(ends):
+                    items.append((first_row + start, ntok, slot, first, low + i * span, low + end, part + i, 0))
+                part += len(ends)
+        # the items with the most keys first: with 148 running at a time a long one at the end would run alone
+        items.sort(key=lambda it: it[4] - it[5])
+        return [x for it in items for x in it] + merges, len(items), len(merges) // 4, part
+
+    @classmethod
+    def _by_arrays(cls, portions, H, tok, base, target_ctas, min_keys, window):
+        """The same lists."""
         import numpy as np
-        tok = max(1, MMA_ROWS // H)
-        por = np.array(list(portions), dtype=np.int64).reshape(-1, 4)
+        por = np.array(portions, dtype=np.int64).reshape(-1, 4)
         tiles = -(-por[:, 1] // tok)                                    # row tiles per portion
-        base = int(tiles.sum())
         of = np.repeat(np.arange(len(por)), tiles)
         start = (np.arange(base) - np.repeat(np.cumsum(tiles) - tiles, tiles)) * tok
         ntok, first = np.minimum(tok, por[of, 1] - start), por[of, 3] + start
-        low = np.maximum(0, first - window + 1)                         # first key a tile's first row sees
-        keys = first + ntok - low                                       # ... up to the end of what its last row sees
+        low = np.maximum(0, first - window + 1)
+        keys = first + ntok - low
         want = np.ones_like(keys)
         if base < target_ctas // 2:
-            want = np.clip(np.minimum(-(-keys // min_keys), -(-target_ctas // max(base, 1))), 1, self.MAX_PARTS)
+            want = np.clip(np.minimum(-(-keys // min_keys), -(-target_ctas // max(base, 1))), 1, cls.MAX_PARTS)
         cut = want > 1
-        span = np.where(cut, -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS, np.maximum(keys, 1))   # keys per part, a multiple of 64
+        span = np.where(cut, -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS, np.maximum(keys, 1))
         n = np.where(cut, -(-keys // span), 1)
         it = np.repeat(np.arange(base), n)
         j = np.arange(len(it)) - np.repeat(np.cumsum(n) - n, n)
@@ -313,14 +349,9 @@ class LatentAttnPlan:
         items[:, 4] = low[it] + j * span[it]
         items[:, 5] = low[it] + np.minimum(keys[it], (j + 1) * span[it])
         items[:, 6], items[:, 7] = np.where(cut[it], part0[it] + j, -1), 0
-        # the items with the most keys first: with 148 running at a time a long one at the end would run alone
         items = items[np.argsort(items[:, 4] - items[:, 5], kind="stable")]
         merges = np.stack([(por[of, 0] + start) * H, ntok * H, part0, n], axis=1)[cut].astype(np.int32)
-        self.n_items, self.n_merges, self.n_parts = len(items), len(merges), int(n_cut.sum())
-        self.max_rows = int(ntok.max(initial=1)) * H                    # (token, head) pairs of the largest item
-        buf = torch.from_numpy(np.concatenate([items.reshape(-1), merges.reshape(-1)])).pin_memory().to(device, non_blocking=True)
-        self.items = buf[:self.n_items * 8]
-        self.merges = buf[self.n_items * 8:] if self.n_merges else None
+        return np.concatenate([items.reshape(-1), merges.reshape(-1)]), len(items), len(merges), int(n_cut.sum())
 
 
 class DecodeAttnPlan:

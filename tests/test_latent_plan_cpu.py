@@ -1,0 +1,46 @@
+"""The work lists of omc_latent_attn_mma: the loop and the array arithmetic build the same numbers, and these cover every key of every row once."""
+import random
+
+import pytest
+
+from omchat_b200.seqlib import MMA_ROWS, WINDOW_ALL, LatentAttnPlan
+
+
+def _portions(rng):
+    out, row = [], 0
+    for slot in range(rng.choice([0, 1, 2, 5])):
+        n = rng.choice([0, 1, 3, 64, rng.randint(1, 300)])
+        out.append((row, n, slot, rng.choice([0, 1, 63, 64, rng.randint(0, 5000)])))
+        row += n
+    return out
+
+
+@pytest.mark.parametrize("seed", range(60))
+def test_the_loop_and_the_arrays_build_the_same_lists(seed):
+    rng = random.Random(seed)
+    portions, H = _portions(rng), rng.choice([1, 3, 8, 16, 33, 64])
+    target, min_keys, window = rng.choice([2, 148, 296]), rng.choice([64, 128, 256]), rng.choice([1, 33, 256, 1024, WINDOW_ALL])
+    tok = MMA_ROWS // H
+    base = sum(-(-n // tok) for _, n, _, _ in portions)
+    a = LatentAttnPlan._by_loop(portions, H, tok, base, target, min_keys, window)
+    b = LatentAttnPlan._by_arrays(portions, H, tok, base, target, min_keys, window)
+    assert list(a[0]) == b[0].tolist() and a[1:] == b[1:]
+    numbers, n_items, n_merges, n_parts = a
+    seen, parts = {}, {}
+    for i in range(n_items):
+        row, ntok, slot, first, lo, hi, part, zero = numbers[8 * i:8 * i + 8]
+        assert 1 <= ntok <= tok and lo < hi and zero == 0
+        seen.setdefault((row, ntok, slot, first), []).append((lo, hi))
+        if part >= 0:
+            assert part not in parts
+            parts[part] = row
+    assert sorted(parts) == list(range(n_parts))
+    want = {(r + s, min(tok, n - s), slot, p0 + s) for r, n, slot, p0 in portions for s in range(0, n, tok)}
+    assert set(seen) == want
+    for (row, ntok, slot, first), ranges in seen.items():
+        ranges.sort()
+        assert ranges[0][0] == max(0, first - window + 1) and ranges[-1][1] == first + ntok
+        assert all(x[1] == y[0] for x, y in zip(ranges, ranges[1:]))
+    for i in range(n_merges):
+        qrow, rows, part, n = numbers[8 * n_items + 4 * i:8 * n_items + 4 * i + 4]
+        assert rows <= MMA_ROWS and 1 <= n <= LatentAttnPlan.MAX_PARTS and all(parts[part + j] * H == qrow for j in range(n))
