@@ -13,15 +13,16 @@
 //                product that reads it is done
 //   warp 1       MMA issuer (one thread)
 //   warps 2..9   softmax: thread = one key x half the rows. Maxima over keys are maxima over lanes: a transposing butterfly leaves every
-//                lane with one row's maximum. The reference of a row is its running maximum, so its largest probability is 1 and takes no
-//                rounding (one that lags behind saves passes over TMEM, but rounds that probability to bf16 as well); where it grew,
-//                the output accumulators are rescaled in TMEM. Sums stay per thread until the end.
-//                P^T goes to shared memory as the B operand; where Q and the key tile fill it (r = 512) it takes the place of the rotated
-//                chunk, which the scores have consumed.
-// What bounds it: shared memory holds one key tile, so a tile of 8300 cycles is a load that only the output products overlap (3100), 68 instructions
-// on the tensor pipe at 50 to 70 cycles each, and one softmax pass over 8192 scores (2200). 16 heads, latents of 512 + 64 (the mma.sync kernel in
-// brackets): portions of 1024, 777, 1024 behind 1024 and 301 rows 249 us = 341 TFLOP/s (721); 4 x 1024 rows of 32 heads 482 us (1134); 2048 rows 191 us
-// (651); a decode step of 32 rows over 700 to 2100 keys, merge included, 29 us (77).
+//                lane with one row's maximum. The reference maximum of a row only moves when it grew by more than 2^8; the output
+//                accumulators are then rescaled in TMEM. Sums stay per thread until the end.
+//                P^T goes to shared memory as the B operand, as two bf16 numbers per probability (its rounding and what that left, 2^-18 of it
+//                together): with one, tiles of 128 keys and longer key ranges gave 1 to 44 % more error than the mma.sync kernel's tiles of 64. Where
+//                Q and the key tile fill shared memory (64 rows, r = 512) half of it takes the places of the rotated chunks, which the scores
+//                have consumed.
+// What bounds it: shared memory holds one key tile, so a tile of 8300 cycles is a load that only the output products overlap (3100), 100 instructions
+// on the tensor pipe (36 for the scores), and one softmax pass over 8192 scores (2200). 16 heads, latents of 512 + 64 (the mma.sync kernel in
+// brackets): portions of 1024, 777, 1024 behind 1024 and 301 rows 253 us = 336 TFLOP/s without the second half of the probabilities (722); 4 x 1024
+// rows of 32 heads 483 us (1136); 2048 rows 196 us (653); a decode step of 32 rows over 700 to 2100 keys, merge included, 31 us (79).
 #include "sm100_step.cuh"
 
 namespace omc {
@@ -42,7 +43,8 @@ struct LatSmArgs {
   const float* gate;
   long long ldg;
   int window, max_pages, page_size, H, r, D, nc;   // nc: 64-column chunks of a row
-  int p_offset;                                    // of P^T, in bytes behind Q
+  int p_at[4];                                     // P^T behind Q, in bytes: its upper and its lower numbers, 64 keys each
+  bool reload_q;                                   // P^T lies where the last chunk of Q does
   int tmem_cols;
   float scale_log2;
   unsigned int* failed;
@@ -109,7 +111,6 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   uint8_t* base = ls_raw + ((1024u - (smem_u32(ls_raw) & 1023u)) & 1023u);
   uint8_t* qs = base;                        // [nc][NR][128 B]
   uint8_t* ks = base + a.nc * QCHUNK;        // [nc][128][128 B]
-  uint8_t* ps = base + a.p_offset;           // P^T
   if (threadIdx.x == 32) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_kv);
@@ -138,9 +139,12 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       row[b] = j < k_end ? bt[j / a.page_size] * a.page_size + j % a.page_size : -1;
     }
   };
-  auto load_pair = [&](const int (&row)[2], int g) {   // chunks of barrier g
+  auto load_q = [&](int c, uint64_t* bar) { tma_load_3d(qs + c * QCHUNK, &tm_q, bar, chunk_col(c), first_row * a.H, 0); };
+  auto load_pair = [&](const int (&row)[2], int g, bool again) {   // chunks of barrier g
     const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
-    mbar_arrive_expect_tx(&sh->full[g], (c1 - 2 * g) * (row[1] >= 0 ? 2 : 1) * (kChunkBytes / 2));
+    const bool q_too = again && a.reload_q && g == nm - 1;
+    mbar_arrive_expect_tx(&sh->full[g], (c1 - 2 * g) * (row[1] >= 0 ? 2 : 1) * (kChunkBytes / 2) + (q_too ? QCHUNK : 0));
+    if (q_too) load_q(a.nc - 1, &sh->full[g]);
 #pragma unroll
     for (int b = 0; b < 2; ++b)
       if (row[b] >= 0)
@@ -162,10 +166,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     fence_proxy_async();
     if (n_tiles > 0) {                       // on their way while tensor memory is allocated
       mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
-      for (int c = 0; c < a.nc; ++c) tma_load_3d(qs + c * QCHUNK, &tm_q, &sh->q_full, chunk_col(c), first_row * a.H, 0);
+      for (int c = 0; c < a.nc; ++c) load_q(c, &sh->q_full);
       int row[2];
       box_rows(0, row);
-      for (int g = 0; g < nm; ++g) load_pair(row, g);
+      for (int g = 0; g < nm; ++g) load_pair(row, g, false);
     }
   }
   if (warp == 1) {
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       while (upto == nm && t + 1 < n_tiles) {
         int row[2];
         box_rows(++t, row);
-        for (upto = 0; upto < nm && wait(&sh->o_done[upto], (t - 1) & 1); ++upto) load_pair(row, upto);
+        for (upto = 0; upto < nm && wait(&sh->o_done[upto], (t - 1) & 1); ++upto) load_pair(row, upto, true);
       }
       drain(&sh->q_full, 0);          // nothing is on its way any more when this thread leaves
       for (int g = 0; g < nm; ++g) drain(&sh->full[g], (g < upto ? t : t - 1) & 1);
@@ -193,10 +197,14 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     if (elect_one() && n_tiles > 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16_major(128, NR, 0, 0);
       constexpr uint32_t idesc_o = make_idesc_bf16_major(128, NR, 1, NR == 64 ? 1 : 0);
-      const uint32_t p_addr = smem_u32(ps);
       const uint64_t dk0 = make_sw128_kmajor_desc(smem_u32(ks)), dq0 = make_sw128_kmajor_desc(smem_u32(qs));
       const uint64_t dv0 = make_sw128_mnmajor_desc(smem_u32(ks), kChunkBytes, 1024);
-      const uint64_t dp0 = NR == 64 ? make_sw128_mnmajor_desc(p_addr, 1024, 1024) : make_sw128_kmajor_desc(p_addr);
+      uint64_t dp[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t at = smem_u32(base) + a.p_at[i];
+        dp[i] = NR == 64 ? make_sw128_mnmajor_desc(at, 1024, 1024) : make_sw128_kmajor_desc(at);
+      }
       const int repeated = (a.nc * 64 - a.D) >> 4;   // steps of 16 that the last chunk has in common with the one before
       bool go = wait(&sh->q_full, 0);
       for (int t = 0; go && t < n_tiles; ++t) {
@@ -222,8 +230,10 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
           const uint64_t dv = dv0 + (uint64_t)(m * (2 * kChunkBytes >> 4));
 #pragma unroll
           for (int k = 0; k < kKT / 16; ++k)
-            umma_bf16<1>(tmem + m * NR, dv + (uint64_t)(k * 128), dp0 + (uint64_t)(NR == 64 ? k * 128 : (k >> 2) * (QCHUNK >> 4) + 2 * (k & 3)), idesc_o,
-                         (t | k) != 0 ? 1u : 0u);
+#pragma unroll
+            for (int low = 0; low < 2; ++low)
+              umma_bf16<1>(tmem + m * NR, dv + (uint64_t)(k * 128), dp[2 * low + (k >> 2)] + (uint64_t)((NR == 64 ? 128 : 2) * (k & 3)), idesc_o,
+                           (t | k | low) != 0 ? 1u : 0u);
           umma_commit(&sh->o_done[m]);
         }
       }
@@ -274,7 +284,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       if (stid < NR) {
         const float now = fmaxf(fmaxf(sh->part[0][stid], sh->part[1][stid]), fmaxf(sh->part[2][stid], sh->part[3][stid]));
         const float old = sh->mref[stid];
-        if (now > old) {                     // also the first finite maximum of a row
+        if (now > old + 8.f) {               // also the first finite maximum of a row
           sh->fac[stid] = ls_exp2(old - now);
           sh->mref[stid] = now;
           sh->rescale[t & 1] = 1u;
@@ -299,30 +309,37 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
         tmem_st_wait();
       }
       load_scores();
-      uint32_t p[NC / 2];
+      uint8_t* const hi_at = base + (quarter < 2 ? a.p_at[0] : a.p_at[1]);
+      uint8_t* const lo_at = base + (quarter < 2 ? a.p_at[2] : a.p_at[3]);
 #pragma unroll
-      for (int c = 0; c < NC; c += 4) {
-        const float4 m4 = *reinterpret_cast<const float4*>(&sh->mref[c0 + c]);
-        const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+      for (int c = 0; c < NC; c += 8) {
+        uint32_t hi[4], lo[4];
 #pragma unroll
-        for (int i = 0; i < 4; i += 2) {
-          p[(c + i) / 2] = pack_bf16(ls_exp2(s[c + i] - (m[i] == -INFINITY ? 0.f : m[i])), ls_exp2(s[c + i + 1] - (m[i + 1] == -INFINITY ? 0.f : m[i + 1])));
-          const float2 e = unpack_bf16(p[(c + i) / 2]);   // the denominator sums the ROUNDED probabilities, the ones the numerator uses
-          l[c + i] += e.x;
-          l[c + i + 1] += e.y;
+        for (int i = 0; i < 8; i += 4) {
+          const float4 m4 = *reinterpret_cast<const float4*>(&sh->mref[c0 + c + i]);
+          const float m[4] = {m4.x, m4.y, m4.z, m4.w};
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            const float p0 = ls_exp2(s[c + i + e] - (m[e] == -INFINITY ? 0.f : m[e])), p1 = ls_exp2(s[c + i + e + 1] - (m[e + 1] == -INFINITY ? 0.f : m[e + 1]));
+            const uint32_t h = pack_bf16(p0, p1);
+            const float2 up = unpack_bf16(h);
+            hi[(i + e) / 2] = h;
+            lo[(i + e) / 2] = pack_bf16(p0 - up.x, p1 - up.y);
+            l[c + i + e] += p0;
+            l[c + i + e + 1] += p1;
+          }
         }
-      }
-      if constexpr (NR == 64) {              // [key][64 rows]: MN-major
-        uint8_t* dst = ps + key_lane * 128;
+        if constexpr (NR == 64) {            // [key][64 rows]: MN-major
+          const int at = (key_lane & 63) * 128 + (((half * (NC / 8) + c / 8) ^ (key_lane & 7)) << 4);
+          *reinterpret_cast<uint4*>(hi_at + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(lo_at + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        } else {                             // [row][64 keys] twice: K-major
 #pragma unroll
-        for (int i = 0; i < NC / 8; ++i)
-          *reinterpret_cast<uint4*>(dst + (((half * (NC / 8) + i) ^ (key_lane & 7)) << 4)) = make_uint4(p[4 * i], p[4 * i + 1], p[4 * i + 2], p[4 * i + 3]);
-      } else {                               // [row][64 keys] twice: K-major
-        uint8_t* dst = ps + (key_lane >> 6) * QCHUNK + (key_lane & 7) * 2;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          const int row = c0 + c;
-          *reinterpret_cast<uint16_t*>(dst + row * 128 + ((((key_lane & 63) >> 3) ^ (row & 7)) << 4)) = (uint16_t)(p[c / 2] >> (16 * (c & 1)));
+          for (int i = 0; i < 8; ++i) {
+            const int row = c0 + c + i, at = (key_lane & 7) * 2 + row * 128 + ((((key_lane & 63) >> 3) ^ (row & 7)) << 4);
+            *reinterpret_cast<uint16_t*>(hi_at + at) = (uint16_t)(hi[i / 2] >> (16 * (i & 1)));
+            *reinterpret_cast<uint16_t*>(lo_at + at) = (uint16_t)(lo[i / 2] >> (16 * (i & 1)));
+          }
         }
       }
       fence_proxy_async();
@@ -379,25 +396,29 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
 }
 
 constexpr int kLsSmemMax = 227 * 1024;
-static int ls_smem(int nr, int r, int D, int* p_offset) {
-  const int nc = (D + 63) / 64, q = nc * nr * 128, k = nc * kChunkBytes, p = kKT * nr * 2;
+// Shared memory of a launch (0: none fits) and where P^T lies: behind the key tile, or, where that fills it, half of it in the places of the last
+// chunks of the key tile and of Q, which only the scores read (Q's is then loaded again with the next tile).
+static int ls_smem(int nr, int r, int D, LatSmArgs* a) {
+  const int nc = (D + 63) / 64, qc = nr * 128, q = nc * qc, k = nc * kChunkBytes;
   const int slack = 1024 + (int)sizeof(LatSmShared) + 256;
-  if (q + k + p + slack <= kLsSmemMax) {
-    *p_offset = q + k;
-    return q + k + p + 1024;
+  if (q + k + 4 * qc + slack <= kLsSmemMax) {
+    for (int i = 0; i < 4; ++i) a->p_at[i] = q + k + i * qc;
+    a->reload_q = false;
+    return q + k + 4 * qc + 1024;
   }
-  if (D > r && q + k + slack <= kLsSmemMax) {   // P^T in the place of the last chunk, which only the scores read
-    *p_offset = q + k - kChunkBytes;
-    return q + k + 1024;
+  if (D > r && 2 * qc <= kChunkBytes && q + k + qc + slack <= kLsSmemMax) {
+    a->p_at[0] = q + k - kChunkBytes, a->p_at[1] = a->p_at[0] + qc, a->p_at[2] = q + k, a->p_at[3] = q - qc;
+    a->reload_q = true;
+    return q + k + qc + 1024;
   }
   return 0;
 }
 
 // Shapes this kernel takes. max_rows: the most rows an item has.
 bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool) {
-  int at;
+  LatSmArgs a;
   return max_rows <= kLsMaxRows && r % 128 == 0 && r <= 512 && dr <= 64 && dr % 16 == 0 && page_size % 64 == 0 &&
-         reinterpret_cast<uintptr_t>(q) % 16 == 0 && reinterpret_cast<uintptr_t>(pool) % 16 == 0 && ls_smem(max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64), r, r + dr, &at) > 0;
+         reinterpret_cast<uintptr_t>(q) % 16 == 0 && reinterpret_cast<uintptr_t>(pool) % 16 == 0 && ls_smem(max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64), r, r + dr, &a) > 0;
 }
 
 template <int NR, typename TO>
@@ -417,8 +438,8 @@ int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const vo
                  int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
                  float* ws_ml, cudaStream_t st) {
   const int D = r + dr, nr = max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64);
-  LatSmArgs a{bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D, (D + 63) / 64, 0, 0, scale * 1.4426950408889634f, nullptr};
-  const int smem = ls_smem(nr, r, D, &a.p_offset);
+  LatSmArgs a{bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D, (D + 63) / 64, {}, false, 0, scale * 1.4426950408889634f, nullptr};
+  const int smem = ls_smem(nr, r, D, &a);
   const int cols = (r / 128 + 1) * nr;
   a.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
   CUtensorMap tq, tk;

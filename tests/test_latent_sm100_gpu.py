@@ -131,3 +131,23 @@ def test_a_pool_that_ends_with_its_mapping(r, dr):
     for plan in plans:
         seqlib.latent_attn_mma(qd, r, dr, pool, table, 64, plan, None, D ** -0.5, out)
         assert ((out.double().cpu() - want).abs() <= mag * (2.0 ** -8 + 1e-4) + 1e-6).all()
+
+
+@pytest.mark.parametrize("H,r,dr,n,first", [(16, 512, 64, 9, 500), (16, 512, 0, 70, 300), (32, 512, 32, 40, 129), (16, 384, 64, 33, 60), (8, 128, 32, 20, 700)])
+@pytest.mark.parametrize("decode", [0, 1, 3])
+def test_probabilities_are_not_rounded_to_8_bits(H, r, dr, n, first, decode):
+    """Two bf16 numbers per probability, in every place that shared memory has for them; whole contexts, key ranges and decode steps."""
+    gen = torch.Generator().manual_seed(r + dr + n)
+    D, pages = r + dr, -(-(n + first) // 64)
+    rows, q = torch.randn(pages * 64, D, generator=gen).to(torch.bfloat16), torch.randn(n, H, D, generator=gen).to(torch.bfloat16)
+    plist, scale = [(0, n, 0, first)], 3.0 * D ** -0.5
+    if decode:
+        plan = seqlib.DecodeAttnPlan(n, H, decode, "cuda")
+        plan.fill(torch.arange(first, first + n, dtype=torch.int32).cuda(), torch.zeros(n, dtype=torch.int32).cuda())
+    else:
+        plan = seqlib.LatentAttnPlan(plist, H, "cuda", target_ctas=2)
+    out = torch.empty(n, H, r, device="cuda")
+    seqlib.latent_attn_mma(q.cuda(), r, dr, rows.view(pages, 64, D).cuda(), torch.arange(pages, dtype=torch.int32).view(1, -1).cuda(), 64, plan, None, scale, out)
+    want, mag = _reference(q, [rows], plist, r, scale, 1 << 30, None, None)
+    # 2^-18 per probability; scores of up to some 15 from fp32 sums of D products, exponentials and sums of up to 720 keys in fp32
+    assert ((out.double().cpu() - want).abs() <= mag * (2.0 ** -17 + 6e-5) + 1e-6).all()
