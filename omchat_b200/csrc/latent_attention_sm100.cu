@@ -273,10 +273,12 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       };
       load_scores();
       // rows of the tile that are no keys of this item hold whatever the cache holds there: as values they must not meet a product
-      if (!whole && half == 0 && !is_key) {
-        for (int c = 0; c < a.r >> 6; ++c)
-#pragma unroll
-          for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(ks + c * kChunkBytes + key_lane * 128 + i * 16) = make_uint4(0, 0, 0, 0);
+      if (!whole) {                          // eight lanes per row of 128 bytes: a lane per row would meet one bank with all 32
+        for (int i = 0; i < 32; i += 4) {
+          const int row = quarter * 32 + i + (lane >> 3);
+          if (j0 + row < kb || j0 + row >= k_end)
+            for (int c = half; c < a.r >> 6; c += 2) *reinterpret_cast<uint4*>(ks + c * kChunkBytes + row * 128 + (lane & 7) * 16) = make_uint4(0, 0, 0, 0);
+        }
       }
       const float mx = ls_columns<NC>(s, lane, [](float x, float y) { return fmaxf(x, y); });
       if (lane % (32 / NC) == 0) sh->part[quarter][c0 + lane / (32 / NC)] = mx;

@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(128) window_attn_mma_kernel(WinMmaArgs a) {
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-    if (warp * 16 < n_rows) {   // a warp without rows (decode: H / G of the 64 rows) only helps staging
+    if (warp * 16 < n_rows) {   // a warp without rows (the last rows of a portion; decode steps of 17 to 48 heads per key/value head) only helps staging
       const bf16_t* Kc = Ks + buf * kWmKeys * pq;
       const bf16_t* Vc = Vs + buf * kWmKeys * pv;
       float s[8][4];

@@ -48,7 +48,12 @@ class LatentAttention:
         self.tensor_attention = True    # False: the plain attention kernel for every shape (A/B, tests)
         self._decode_plans = {}         # (rows, heads, parts, window) -> seqlib.DecodeAttnPlan
 
-    def _plan(self, plans: dict, T: int, H: int, window: int, pos, slot, tcgen05: bool):
+    def _plan(self, plans: dict, T: int, H: int, r: int, window: int, pos, slot, tcgen05: bool):
+        if tcgen05 and "portions" in plans:
+            key = ("tcgen05", H, r, window)
+            if key not in plans:
+                plans[key] = self._tcgen05_pays(plans["portions"], H, r, window)
+            tcgen05 = plans[key]
         plan = plans.get((H, window, tcgen05))
         if plan is None:
             if "portions" in plans:
@@ -65,9 +70,21 @@ class LatentAttention:
         return plan
 
     @staticmethod
+    def _tcgen05_pays(portions, H: int, r: int, window: int) -> bool:
+        """Not where no row tile meets more than 64 keys: a tile of 128 is half empty then, and the mma.sync kernel starts on one of 64 sooner (64
+        rows of 16 heads, latents of 512 / 256 / 128: 18 / 11.9 / 10.0 us there, 14.4 / 10.9 / 9.0; 100 keys: 18.2, 22.0). Nor for latents of 128,
+        whose few products per key do not hide a tile's softmax, in steps of many tiles over short windows (1564 tiles, a window of 256: 160 us,
+        134; 196 tiles: 48, 38; without a window 75, 187)."""
+        tok = max(1, seqlib.MMA_ROWS // H)
+        longest = max((min(p0 + n, window + tok - 1) for _, n, _, p0 in portions), default=0)
+        return longest > (320 if r == 128 and sum(-(-n // tok) for _, n, _, _ in portions) >= 148 else 64)
+
+    @staticmethod
     def _prompt_plan(portions, H: int, device, window: int, tcgen05: bool) -> seqlib.LatentAttnPlan:
+        if not tcgen05:
+            return seqlib.LatentAttnPlan(portions, H, device, window=window, mma_sync=True)
         # the tcgen05 kernel runs one CTA per SM on tiles of 128 keys: contexts are cut only while that leaves half the SMs idle
-        return seqlib.LatentAttnPlan(portions, H, device, window=window, **(dict(target_ctas=148, min_keys=256) if tcgen05 else {}))
+        return seqlib.LatentAttnPlan(portions, H, device, window=window, target_ctas=148, min_keys=128)
 
     @staticmethod
     def _decode_parts(T: int, keys: int, tcgen05: bool) -> int:
@@ -86,7 +103,7 @@ class LatentAttention:
         if plans is not None and self.tensor_attention and seqlib.latent_attn_mma_ok(H, r, dr, self.dtype):
             out = torch.empty(T, H, r, device=qcat.device, dtype=self.dtype)
             tcgen05 = seqlib.latent_attn_tcgen05_ok(H, r, dr, cache.page_size)
-            return seqlib.latent_attn_mma(qcat, r, dr, pool, cache.block_table, cache.page_size, self._plan(plans, T, H, window, pos, slot, tcgen05), sink, scale,
+            return seqlib.latent_attn_mma(qcat, r, dr, pool, cache.block_table, cache.page_size, self._plan(plans, T, H, r, window, pos, slot, tcgen05), sink, scale,
                                           out, window=window, gate=gate)
         out = torch.empty(T, H, r, device=qcat.device, dtype=torch.float32)
         return seqlib.latent_attn(qcat, r, dr, pool, cache.block_table, cache.page_size, pos, slot, sink, scale, out, window=window, gate=gate)

@@ -289,12 +289,14 @@ class LatentAttnPlan:
 
     FEW_TILES = 24  # up to here a loop builds the lists sooner than array arithmetic, some 60 calls of a microsecond or two: 5 rows 18 us (120)
 
-    def __init__(self, portions, H: int, device, target_ctas: int = 296, min_keys: int = 128, window: int = WINDOW_ALL):
+    def __init__(self, portions, H: int, device, target_ctas: int = 296, min_keys: int = 128, window: int = WINDOW_ALL, mma_sync: bool = False):
         portions, tok = list(portions), max(1, MMA_ROWS // H)
         base = sum(-(-n // tok) for _, n, _, _ in portions)                 # row tiles
         build = self._by_loop if base <= self.FEW_TILES else self._by_arrays
         numbers, self.n_items, self.n_merges, self.n_parts = build(portions, H, tok, base, target_ctas, min_keys, window)
         self.max_rows = max((min(tok, n) for _, n, _, _ in portions), default=1) * H   # (token, head) pairs of the largest item
+        if mma_sync:    # whatever the shapes
+            self.max_rows = MMA_ROWS + 1
         buf = torch.as_tensor(numbers, dtype=torch.int32).pin_memory().to(device, non_blocking=True)
         self.items = buf[:self.n_items * 8]
         self.merges = buf[self.n_items * 8:] if self.n_merges else None

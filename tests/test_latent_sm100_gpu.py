@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from omchat_b200 import seqlib
+from omchat_b200.model.seq_latent import LatentAttention
 
 pytestmark = pytest.mark.gpu
 F64 = torch.float64
@@ -151,3 +152,24 @@ def test_probabilities_are_not_rounded_to_8_bits(H, r, dr, n, first, decode):
     want, mag = _reference(q, [rows], plist, r, scale, 1 << 30, None, None)
     # 2^-18 per probability; scores of up to some 15 from fp32 sums of D products, exponentials and sums of up to 720 keys in fp32
     assert ((out.double().cpu() - want).abs() <= mag * (2.0 ** -17 + 6e-5) + 1e-6).all()
+
+
+@pytest.mark.parametrize("H,r,portions,window", [(16, 512, [(40, 0), (3, 60)], 1 << 30), (32, 128, [(150, 0), (200, 40)], 70), (8, 256, [(5, 300)], 20)])
+def test_steps_of_few_keys_take_the_other_kernel(H, r, portions, window):
+    """_tcgen05_pays: no more than 64 keys per tile, or latents of 128 over short windows. Both kernels give the same within their rounding."""
+    gen = torch.Generator().manual_seed(r)
+    D, plist, row = r + 32, [], 0
+    for s, (n, first) in enumerate(portions):
+        plist.append((row, n, s, first))
+        row += n
+    assert not LatentAttention._tcgen05_pays(plist, H, r, window) and LatentAttention._tcgen05_pays(plist, H, 256, 1 << 30) == (max(n + f for n, f in portions) > 64)
+    pages = max(-(-(n + f) // 64) for n, f in portions)
+    lat = [torch.randn(pages * 64, D, generator=gen).to(torch.bfloat16) for _ in portions]
+    q = torch.randn(row, H, D, generator=gen).to(torch.bfloat16)
+    want, mag = _reference(q, lat, plist, r, D ** -0.5, window, None, None)
+    table = torch.arange(pages * len(portions), dtype=torch.int32).view(len(portions), -1).cuda()
+    for tcgen05 in (True, False):
+        out = torch.empty(row, H, r, device="cuda")
+        plan = LatentAttention._prompt_plan(plist, H, "cuda", window, tcgen05)
+        seqlib.latent_attn_mma(q.cuda(), r, 32, torch.cat(lat).view(-1, 64, D).cuda(), table, 64, plan, None, D ** -0.5, out, window=window)
+        assert ((out.double().cpu() - want).abs() <= mag * (2.0 ** (-17 if tcgen05 else -8) + 6e-5) + 1e-6).all(), tcgen05
