@@ -34,12 +34,18 @@ __device__ __forceinline__ void lds_pairs(const float* p, f32x2_t& lo, f32x2_t& 
 }
 
 // dst[0..3] (shared memory) <- row[k..k+3] as fp32, zero where !valid or past K. VEC: K and the row strides are multiples of four and the
-// rows start on boundaries of four elements; fp32 then goes by cp.async, which the caller commits.
+// rows start on boundaries of four elements. fp32 goes by cp.async, which the caller commits: as one piece with VEC, as four without.
 template <typename T, bool VEC>
 __device__ __forceinline__ void stage4(float* dst, const T* row, int k, int K, bool valid) {
   if constexpr (VEC && sizeof(T) == 4) {
     const bool in = valid && k < K;
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(lin_smem_u32(dst)), "l"(in ? row + k : row), "r"(in ? 16 : 0) : "memory");
+  } else if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const bool in = valid && k + j < K;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(lin_smem_u32(dst + j)), "l"(in ? row + k + j : row), "r"(in ? 4 : 0) : "memory");
+    }
   } else {
     float v[4] = {0.f, 0.f, 0.f, 0.f};
     if (valid) {
@@ -337,14 +343,14 @@ static int launch_narrow(const LinearArgs& a, int y_dt, int batch, cudaStream_t 
 //   K = 1024: 8 x 4096 13 / 37, 32 x 4096 28 / 40, 64 x 4096 48 / 44, 128 x 1024 29 / 44, 256 x 1024 49 / 45
 // The tile kernel's time goes with K alone up to a first wave of 148 tiles, however few and empty they are, and in proportion above that. The rows
 // kernel's goes with the outputs, and falls only slowly with K below its stage of 1024 terms (K / 64 of a CTA's 16 sums are at work, and its shared
-// memory is the same): they meet at some 20,000 outputs plus 195 per K term and wave. Rows that its vector loads do not take cost it four times
-// as much (63 terms, 90 x 2048 outputs: 39 / 9).
+// memory is the same): they meet at some 20,000 outputs plus 195 per K term and wave, whether the vector loads take the rows or not, and sooner where
+// bf16 is converted on its way (K = 1001: 196,000 outputs in fp32, 150,000 with bf16 weights, 110,000 with bf16 rows too).
 static long long lin_tiles(const LinearArgs& a, int batch) {
   return (long long)((a.N + kLinBN - 1) / kLinBN) * ((a.M + kLinBM - 1) / kLinBM) * batch;
 }
-static bool few_rows(const LinearArgs& a, int batch, bool vec) {
+static bool few_rows(const LinearArgs& a, int batch, int bf16_operands) {
   const long long tiles = lin_tiles(a, batch), outputs = (long long)a.M * a.N * batch;
-  const long long meet = (20000 + 195LL * (a.K < 1024 ? a.K : 1024)) / (vec ? 1 : 4);
+  const long long meet = (20000 + 195LL * (a.K < 1024 ? a.K : 1024)) * (4 - bf16_operands) / 4;
   return a.tile_group == nullptr && 148 * outputs <= meet * (tiles > 148 ? tiles : 148) && a.M <= 8 * 65535;
 }
 
@@ -381,10 +387,14 @@ static int launch_tile(const LinearArgs& a, int batch, cudaStream_t st) {
 
 template <typename TX, typename TW, typename TY, bool VEC>
 static int launch_any(const LinearArgs& a, int batch, cudaStream_t st) {
-  if (few_rows(a, batch, VEC)) return a.M <= 4 ? launch_rows<TX, TW, TY, 4, VEC>(a, batch, st) : launch_rows<TX, TW, TY, 8, VEC>(a, batch, st);
-  // with few tiles per SM the smaller tasks of 256 threads hide more (100 x 77, K = 4096 rows: 13 us, 128 threads 17); with many, the better
-  // reuse of 128 counts (4096 x 6144 x 2048: 2463 us, 256 threads 2646)
-  return lin_tiles(a, batch) < 296 ? launch_tile<TX, TW, TY, VEC, 256>(a, batch, st) : launch_tile<TX, TW, TY, VEC, 128>(a, batch, st);
+  constexpr int bf16_operands = (sizeof(TX) == 2) + (sizeof(TW) == 2);
+  if (few_rows(a, batch, bf16_operands)) return a.M <= 4 ? launch_rows<TX, TW, TY, 4, VEC>(a, batch, st) : launch_rows<TX, TW, TY, 8, VEC>(a, batch, st);
+  // the better reuse of 128 threads counts where a long sum over many tiles of fp32 leaves nothing else to wait for (in us, 128 / 256 threads: 4096 x
+  // 6144 x 2048 2463 / 2646, 4096 x 2048 x 1024 432 / 454); the smaller tasks of 256 hide more elsewhere (the same at K = 256 142 / 127, at 64
+  // 76 / 52, with bf16 weights at 257 244 / 189; 700 x 2000 x 256 43 / 32; 100 x 77 x 4096 17 / 13)
+  if constexpr (bf16_operands == 0)
+    if (a.K >= 768 && lin_tiles(a, batch) >= 296) return launch_tile<TX, TW, TY, VEC, 128>(a, batch, st);
+  return launch_tile<TX, TW, TY, VEC, 256>(a, batch, st);
 }
 
 template <typename TX, typename TW, typename TY>

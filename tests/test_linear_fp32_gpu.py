@@ -40,9 +40,9 @@ def test_rows_do_not_depend_on_the_kernel_that_takes_them(N, K, xdt, wdt):
 
 
 @pytest.mark.parametrize("xdt,wdt", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
-@pytest.mark.parametrize("K", [196, 203])
-def test_tiles_of_128_threads(K, xdt, wdt):
-    """296 tiles or more: 4 x 8 outputs per thread. The same bits as in calls of fewer rows."""
+@pytest.mark.parametrize("K", [196, 203, 900, 901])
+def test_many_tiles(K, xdt, wdt):
+    """336 tiles: 4 x 8 outputs per thread for long sums in fp32, 4 x 4 otherwise. The same bits as in calls of fewer rows."""
     M, N = 1300, 1000
     x, w = _operands(M, N, K, xdt, wdt, torch.Generator().manual_seed(K))
     y = torch.empty(M, N, device="cuda")
@@ -55,8 +55,8 @@ def test_tiles_of_128_threads(K, xdt, wdt):
 
 
 @pytest.mark.parametrize("wdt", [torch.float32, torch.bfloat16])
-@pytest.mark.parametrize("K", [68, 131])
-@pytest.mark.parametrize("tiles", [4, 33])             # 40 tiles of 256 threads, 330 of 128
+@pytest.mark.parametrize("K", [68, 131, 801])
+@pytest.mark.parametrize("tiles", [4, 33])             # 40 tiles, 330
 def test_grouped_rows(tiles, K, wdt):
     """Row tiles of 64 that each name the matrix they meet; -1: rows that nobody asks for stay as they were."""
     N, G = 600, 5
