@@ -326,8 +326,7 @@ __device__ __forceinline__ int scan_place(int i) { return (i / DPT) * (DPT + 4) 
 // (every row starts on a 16-byte boundary and the widths are multiples of four), else 4-byte copies.
 // KIND: what enters the state - v itself, the delta rule's correction, or dt v (decay mode 6).
 // TOK: tokens per stage; 1 for steps of one-token portions, whose CTAs then need little shared memory (more of them share
-// an SM and keep state loads in flight: seven at 128 key channels, four at 256, which the launch bounds hold the registers to; with the 94 and
-// 156 that the compiler took by itself, 256 requests of 64 heads of 128 x 64 took 385 us and of 4 heads of 256 x 256 271, now 306 and 158);
+// an SM and keep state loads in flight: seven at 128 key channels, four at 256, which the launch bounds hold the registers to);
 // any TOK is right for any portion.
 //
 // A thread owns DPT neighbouring key channels of CPT neighbouring columns: a packed register holds two neighbouring CHANNELS of one
@@ -337,7 +336,7 @@ __device__ __forceinline__ int scan_place(int i) { return (i / DPT) * (DPT + 4) 
 // the read-out of a chunk is summed over the lanes once at its end, from shared memory, instead of by shuffles in every token. Measured,
 // four portions of 1024, 777, 1024, 301 tokens (before: pairs of columns, a doubled key and a shuffled read-out per token): step sizes, 64
 // heads of 128 x 64: 341 us (501); delta rule, 16 heads of 128 x 128: 368 (513), per-channel decays 435 (560); one token of 32 requests,
-// step sizes: 30 us = 4.5 TB/s (42).
+// step sizes: 22 us = 6.1 TB/s (42).
 enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
 template <int DPT, int TOK>
 __host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
@@ -375,9 +374,9 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
       const int i = lane * DPT + 2 * r + j;
       const float* row = S + (long long)i * a.vdim + col;
       const bool in = !fresh && i < dim;
-      // the columns of a thread as one access (CPT divides vdim); not where 32 of them per thread are all that is on its way: they would have to
-      // be taken apart before the next could be asked for
-      if (a.vec_state && !(TOK == 1 && DPT == 32)) {
+      // the columns of a thread as one access (CPT divides vdim); one by one in a decode step, whose time is these loads: two columns at once have to
+      // be taken apart into the registers that keep them, and fewer loads are on their way (256 requests, 64 heads of 128 x 64: 190 us, 307)
+      if (a.vec_state && TOK != 1) {
         const float2 x = in && col < a.vdim ? *reinterpret_cast<const float2*>(row) : make_float2(0.f, 0.f);
         e[j][0] = x.x, e[j][1] = x.y;
       } else {
