@@ -246,6 +246,7 @@ int linear_sm100(const LinearArgs& a, int y_dt, int batch, cudaStream_t st) {
 }
 
 int latent_sm100_failures(unsigned int* n);   // latent_attention_sm100.cu
+int window_sm100_failures(unsigned int* n);   // window_attention_sm100.cu
 
 // out: a wait for a barrier that nothing arrives at; the next one for it; one for a barrier that another thread arrives at only behind it; a drain of
 // that one
@@ -291,10 +292,11 @@ extern "C" int omc_step_wait_selfcheck(int32_t* out, void* stream) {
 }
 
 extern "C" int omc_step_wait_failures(unsigned int* count) {
-  unsigned int linear = 0, latent = 0;
+  unsigned int linear = 0, latent = 0, window = 0;
   if (count == nullptr) return omc::set_error(OMC_ERR_ARG, "omc_step_wait_failures: bad argument");
-  if (cudaMemcpyFromSymbol(&linear, omc::g_linear_failures, sizeof(linear)) != cudaSuccess || omc::latent_sm100_failures(&latent) != OMC_OK)
+  if (cudaMemcpyFromSymbol(&linear, omc::g_linear_failures, sizeof(linear)) != cudaSuccess || omc::latent_sm100_failures(&latent) != OMC_OK ||
+      omc::window_sm100_failures(&window) != OMC_OK)
     return omc::set_error(OMC_ERR_CUDA, "omc_step_wait_failures: the counters could not be read");
-  *count = linear + latent;
+  *count = linear + latent + window;
   return OMC_OK;
 }
