@@ -337,13 +337,6 @@ int omc_window_attn_mma(const void* q, long long ldq, int T, int H, int G, int d
                         const int32_t* slot, int window, int chunk, int keep_first, float scale, float softcap, const float* dist_bias,
                         const float* sink, const float* gate, long long ldg, int gate_act, int gate_heads, void* out, int out_dt, long long ldo, void* stream);
 
-/* The same, told how many rows (pages * page_size) the pool has: items then run on tcgen05 where d = dv is 64 or 128, maps is 1, keep_first 0, page_size a
- * multiple of 64, out on 16 bytes with ldo a multiple of 8, and the bias of a key/value head's heads fits shared memory. pool_rows 0: not known. */
-int omc_window_attn_mma_rows(const void* q, long long ldq, int T, int H, int G, int d, int dv, int maps, const void* pool, long long pool_rows,
-                        const int32_t* block_table, int max_pages, int page_size, const int32_t* items, int n_items, const int32_t* pos,
-                        const int32_t* slot, int window, int chunk, int keep_first, float scale, float softcap, const float* dist_bias,
-                        const float* sink, const float* gate, long long ldg, int gate_act, int gate_heads, void* out, int out_dt, long long ldo, void* stream);
-
 /* Differential heads: a fp32 [T, H, 2, dv] (two score maps per head) -> o = a1 - lambda * a2; o / sqrt(mean(o^2) + eps) over the
  * head's dv values; times mult; times act(gate[t, h * dv + c]) (gate fp32 or NULL; gate_act 0: as is, 1: silu, 2: sigmoid)
  * -> y [T, H * dv] of y_dt. */

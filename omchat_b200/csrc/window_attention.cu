@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(WARPS * 32) window_attn_kernel(const TQ* __res
 
 // ---------------------------------------------------------------------------------------------------------------------------
 // Tensor-core kernel (bf16; head widths multiples of 16, values up to 128 wide, up to 64 heads per key/value head). Prompt portions with heads of 64 or
-// 128 run on tcgen05 instead (window_attention_sm100.cu), which was never the slower one from a portion of one row to 4 x 2048.
+// 128 run on tcgen05 instead where that is the faster one (window_attention_sm100.cu).
 // mma.sync.m16n8k16 over 64-key tiles staged by cp.async straight out of the pages, two buffers. The 64 rows of a tile are
 // (token, query head) pairs of ONE key/value head - up to floor(64 / (H / G)) consecutive tokens of one request - so the heads of a group share
 // the staged keys and values. Four warps of 16 rows; S = Q K^T, then scale, soft cap (tanh.approx), distance bias and window
@@ -1057,10 +1057,10 @@ __global__ void __launch_bounds__(256) diff_heads_gate_kernel(const float* __res
   }
 }
 
-bool window_sm100_ok(int H, int G, int d, int dv, int maps, int keep_first, long long pool_rows, int page_size, int window, const float* bias, const void* out, long long ldo,
-                     const void* pool);
-int window_sm100(const void* q, long long ldq, int T, int H, int G, int d, const void* pool, long long pool_rows, const int32_t* bt, int max_pages, int page_size,
-                 const int32_t* items, int n_items, int window, int chunk, float scale, float softcap, const float* bias, const float* sink, const float* gate, long long ldg, int gate_act,
+bool window_sm100_ok(int H, int G, int d, int dv, int maps, int keep_first, int page_size, int n_items, int window, int chunk, const float* bias, const void* out,
+                     long long ldo);
+int window_sm100(const void* q, long long ldq, int T, int H, int G, int d, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
+                 int n_items, int window, int chunk, float scale, float softcap, const float* bias, const float* sink, const float* gate, long long ldg, int gate_act,
                  int gate_heads, void* out, int out_dt, long long ldo, cudaStream_t st);
 
 }  // namespace omc
@@ -1152,11 +1152,11 @@ extern "C" int omc_window_attn_mma_ok(int H, int G, int d, int dv) {
   return (d % 16 == 0 && dv % 16 == 0 && d >= 16 && d <= 256 && dv >= 16 && dv <= 128 && rep <= 64) ? 1 : 0;
 }
 
-extern "C" int omc_window_attn_mma_rows(const void* q, long long ldq, int T, int H, int G, int d, int dv, int maps, const void* pool, long long pool_rows,
-                                        const int32_t* block_table, int max_pages, int page_size, const int32_t* items, int n_items,
-                                        const int32_t* pos, const int32_t* slot, int window, int chunk, int keep_first, float scale, float softcap,
-                                        const float* dist_bias, const float* sink, const float* gate, long long ldg, int gate_act, int gate_heads, void* out,
-                                        int out_dt, long long ldo, void* stream) {
+extern "C" int omc_window_attn_mma(const void* q, long long ldq, int T, int H, int G, int d, int dv, int maps, const void* pool,
+                                   const int32_t* block_table, int max_pages, int page_size, const int32_t* items, int n_items,
+                                   const int32_t* pos, const int32_t* slot, int window, int chunk, int keep_first, float scale, float softcap,
+                                   const float* dist_bias, const float* sink, const float* gate, long long ldg, int gate_act, int gate_heads, void* out,
+                                   int out_dt, long long ldo, void* stream) {
   if (q == nullptr || pool == nullptr || block_table == nullptr || out == nullptr || T < 0 || window < 1 || chunk < 1 || maps < 1 || keep_first < 0 || page_size <= 0 ||
       gate_act < 0 || gate_act > 2 || max_pages <= 0 || (items == nullptr && (pos == nullptr || slot == nullptr)) || n_items < 0)
     return set_error(OMC_ERR_ARG, "omc_window_attn_mma: bad argument");
@@ -1166,8 +1166,8 @@ extern "C" int omc_window_attn_mma_rows(const void* q, long long ldq, int T, int
   if (n == 0) return OMC_OK;
   if ((long long)G * maps > 65535) return set_error(OMC_ERR_SHAPE, "omc_window_attn_mma: more than 65535 key/value heads");
   if (items != nullptr && (out_dt == OMC_DT_BF16 || out_dt == OMC_DT_F32) &&
-      window_sm100_ok(H, G, d, dv, maps, keep_first, pool_rows, page_size, window, dist_bias, out, ldo, pool))
-    return window_sm100(q, ldq, T, H, G, d, pool, pool_rows, block_table, max_pages, page_size, items, n_items, window, chunk, scale, softcap, dist_bias, sink, gate, ldg,
+      window_sm100_ok(H, G, d, dv, maps, keep_first, page_size, n_items, window, chunk, dist_bias, out, ldo))
+    return window_sm100(q, ldq, T, H, G, d, pool, block_table, max_pages, page_size, items, n_items, window, chunk, scale, softcap, dist_bias, sink, gate, ldg,
                         gate_act, gate_heads, out, out_dt, ldo, static_cast<cudaStream_t>(stream));
   WinMmaArgs a{static_cast<const bf16_t*>(q), ldq, static_cast<const bf16_t*>(pool), block_table, items, pos, slot, dist_bias, sink, gate, ldg,
                gate_act, gate_heads, out, ldo, max_pages, page_size, H, G, d, dv, window, chunk, maps, keep_first, scale, softcap, kWmRows, 0};
@@ -1207,15 +1207,6 @@ extern "C" int omc_window_attn_mma_rows(const void* q, long long ldq, int T, int
   }
 #undef OMC_WIN_LAUNCH
   return check_launch("omc_window_attn_mma");
-}
-
-extern "C" int omc_window_attn_mma(const void* q, long long ldq, int T, int H, int G, int d, int dv, int maps, const void* pool,
-                                   const int32_t* block_table, int max_pages, int page_size, const int32_t* items, int n_items,
-                                   const int32_t* pos, const int32_t* slot, int window, int chunk, int keep_first, float scale, float softcap,
-                                   const float* dist_bias, const float* sink, const float* gate, long long ldg, int gate_act, int gate_heads, void* out,
-                                   int out_dt, long long ldo, void* stream) {
-  return omc_window_attn_mma_rows(q, ldq, T, H, G, d, dv, maps, pool, 0, block_table, max_pages, page_size, items, n_items, pos, slot, window, chunk, keep_first, scale,
-                                  softcap, dist_bias, sink, gate, ldg, gate_act, gate_heads, out, out_dt, ldo, stream);
 }
 
 static size_t diff_pair_smem(int d, int dv) {

@@ -5,28 +5,35 @@
 // The 128 rows of a CTA are the (token, query head) pairs of one key/value head: one item of the list, or two that follow one another in the same
 // request (each takes half of the rows). Rows lie on the 128 lanes of TMEM, so a softmax thread owns one row: no shuffles, and its 64 scores
 // of a key tile stay in registers.
-//   warp 0       TMA: Q once, 64 keys and 64 values per tile in rings of kStages
-//   warp 1       MMA issuer (one thread): S = Q K^T of the next tile before O += P V of this one, so scores wait in a second buffer of TMEM
-//   warps 2..5   softmax, one thread per row: scale, soft cap, distance bias, mask, maximum, probabilities. P goes back to TMEM over its scores as
+//   warps 0..3   Q; softmax, one thread per row: scale, soft cap, distance bias, mask, maximum, probabilities. P goes back to TMEM over its scores as
 //                two bf16 numbers (its rounding and what that left), which is the A operand of the output product. The reference maximum of a row
 //                moves only when it grew by more than 2^8; O is then rescaled in TMEM.
+//   warp 4       MMA issuer (one thread): S = Q K^T of the next tile before O += P V of this one, so scores wait in a second buffer of TMEM
+//   warps 5, 6   keys and values by cp.async, two tiles each
 // The bias lies in shared memory by head and distance, in base-2 units with the soft cap's constant added: a row walks its tile at fixed offsets
 // from one address, and the rows of a warp (consecutive tokens, heads a bank offset apart) meet different banks.
 // Two CTAs share an SM and hide each other's waits. What bounds it with a soft cap is the exponential unit (three operations per score, 16 per cycle and SM:
 // 1536 cycles per tile) and the chain of a tile behind it; two threads per row were slower without a cap (12 to 27 %: one more barrier per tile) and no
 // faster with one. Head fastest and the later items first in the grid: portions end with their items of few keys (103 us with the items fastest).
 // Measured, mma.sync kernel in brackets: 32 heads on 8 key/value heads of 128, portions of 1024, 777, 1024 behind 1024 and 301 rows, window 512, cap and
-// bias: 90 us (270); 4 x 2048 rows behind 2048, causal: 531 us = 777 TFLOP/s (2880); 64-key portions: 6 us (8).
+// bias: 89 us (270); 4 x 2048 rows behind 2048, causal: 667 us = 618 TFLOP/s (2880).
+// Keys and values come by cp.async and not by TMA: boxes addressed through a block table, every one of them inside the pool, gave illegal accesses with
+// a tensor map that claimed more rows than the pool has, and once with one that did not, for no reason that was found.
+#include <type_traits>
+
 #include "sm100_step.cuh"
 
 namespace omc {
 
-constexpr int kWsKeys = 64, kWsRows = 128, kWsSoftmax = 128, kWsThreads = 64 + kWsSoftmax, kWsMaxStages = 4;
+constexpr int kWsKeys = 64, kWsRows = 128, kWsSoftmax = 128, kWsLoad = 64, kWsThreads = kWsSoftmax + 32 + kWsLoad;
 constexpr int kWsBox = kWsKeys * 128;            // bytes of 64 columns x 64 keys
 
 static __device__ unsigned int g_window_failures;   // waits that ran out
 
 struct WinSmArgs {
+  const bf16_t* q;
+  long long ldq;
+  const bf16_t* pool;
   const int32_t* bt;
   const int32_t* items;   // int32[n][4]: first row, tokens, slot, first position
   const float* bias;      // [window][H] or NULL
@@ -42,7 +49,7 @@ struct WinSmArgs {
 };
 
 struct WinSmBars {
-  uint64_t q_full, k_full[kWsMaxStages], k_empty[kWsMaxStages], v_full[kWsMaxStages], v_empty[kWsMaxStages], s_full[2], p_ready[2], o_done, mma_done;
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2], s_full[2], p_ready[2], o_done, mma_done;
   uint32_t tmem, dead;
 };
 constexpr int kWsTail = 768;                     // bytes behind the bias table: the barriers, and what hidden scores read over its end
@@ -68,8 +75,8 @@ __device__ __forceinline__ bool ws_follows(const int4& a, const int4& b, int tok
 }
 
 template <int D, bool CAP, bool BIAS>
-__global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv, WinSmArgs a) {
-  constexpr int kStages = D == 128 ? 2 : 4, kChunks = D / 64, kTile = kChunks * kWsBox, kQChunk = kWsRows * 128;
+__global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(WinSmArgs a) {
+  constexpr int kChunks = D / 64, kTile = kChunks * kWsBox, kQChunk = kWsRows * 128;
   constexpr float kLog2e = 1.4426950408889634f;
   // Two items of a run become one CTA. The items of a portion are `tok` tokens apart, so the parity of position / tok alternates along it
   // and says which of two neighbours leads, without a look at more than one item on either side.
@@ -84,9 +91,9 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
     if (!ws_follows(it, next, a.tok, a.chunk)) next.y = 0;
   }
   extern __shared__ __align__(1024) uint8_t ws_raw[];
-  uint8_t* const ks = ws_raw;                              // [stages][chunk][64 keys][128 B]
-  uint8_t* const vs = ks + kStages * kTile;
-  uint8_t* const qs = vs + kStages * kTile;                // [chunk][128 rows][128 B]
+  uint8_t* const ks = ws_raw;                              // [2 stages][chunk][64 keys][128 B]
+  uint8_t* const vs = ks + 2 * kTile;
+  uint8_t* const qs = vs + 2 * kTile;                      // [chunk][128 rows][128 B]
   float* const table = reinterpret_cast<float*>(qs + kChunks * kQChunk);   // hidden scores read up to 190 floats over its ends: Q in front, kWsTail behind
   WinSmBars* const sh = reinterpret_cast<WinSmBars*>(qs + kChunks * kQChunk + a.table);
   const int rep = a.H / a.G, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -96,18 +103,13 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
 
   const WaitReport report{&sh->dead, &g_window_failures, a.failed};
   auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, report); };
-  auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, report); };
   if (tid == 0) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_kv);
-    mbar_init(&sh->q_full, 1);
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(&sh->k_full[s], 1);
-      mbar_init(&sh->k_empty[s], 1);
-      mbar_init(&sh->v_full[s], 1);
-      mbar_init(&sh->v_empty[s], 1);
-    }
+    mbar_init(&sh->q_full, kWsSoftmax / 32);
     for (int b = 0; b < 2; ++b) {
+      mbar_init(&sh->k_full[b], kWsLoad / 32);
+      mbar_init(&sh->k_empty[b], 1);
+      mbar_init(&sh->v_full[b], kWsLoad / 32);
+      mbar_init(&sh->v_empty[b], 1);
       mbar_init(&sh->s_full[b], 1);
       mbar_init(&sh->p_ready[b], kWsSoftmax / 32);
     }
@@ -115,11 +117,26 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
     mbar_init(&sh->mma_done, 1);
     sh->dead = 0u;
     fence_barrier_init();
-    fence_proxy_async();
   }
-  if (warp == 1) {
+  if (warp == 4) {
     tmem_alloc<1>(&sh->tmem, 256);
     tmem_relinquish<1>();
+  }
+  // loads: eight lanes per 128 bytes of a row, as the 128-byte swizzle has them
+  if (tid < kWsSoftmax) {
+    const int c = tid & 7;
+    for (int r = tid >> 3; r < kWsRows; r += kWsSoftmax / 8) {
+      const int4 mine = r < 64 ? it : next;
+      const int row = r & 63, token = row / rep, h = row - token * rep;
+      const bf16_t* src = a.q + (long long)(mine.x + token) * a.ldq + (long long)(kvh * rep + h) * D + c * 8;
+      uint8_t* at = qs + r * 128 + ((c ^ (r & 7)) << 4);
+#pragma unroll
+      for (int b = 0; b < kChunks; ++b) {
+        if (token < mine.y) cp_async16(at + b * kQChunk, src + b * 64, true);
+        else *reinterpret_cast<uint4*>(at + b * kQChunk) = make_uint4(0, 0, 0, 0);
+      }
+    }
+    cp_async_commit();
   }
   if constexpr (BIAS) {
     const int pitch = ws_bias_pitch(a.window, rep);
@@ -133,75 +150,91 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
   tc_fence_after();
   const uint32_t tmem = sh->tmem, tmem_o = tmem + 2 * kWsKeys;   // scores: two buffers of 64 columns
 
-  if (warp == 0) {
-    if (elect_one()) {
-      const int32_t* bt = a.bt + (long long)it.z * a.max_pages;
-      mbar_arrive_expect_tx(&sh->q_full, (next.y > 0 ? 2 : 1) * kChunks * a.tok * rep * 128);
-      for (int c = 0; c < kChunks; ++c) {
-        tma_load_3d(qs + c * kQChunk, &tm_q, &sh->q_full, c * 64, kvh * rep, it.x);
-        if (next.y > 0) tma_load_3d(qs + c * kQChunk + 64 * 128, &tm_q, &sh->q_full, c * 64, kvh * rep, next.x);
-      }
-      int nk = 0, nv = 0;                                  // tiles whose keys / values have been asked for
-      for (int t = 0; t < n_tiles; ++t) {
-        const int s = t % kStages, j = k0 + t * kWsKeys;
-        const uint32_t before = ((uint32_t)(t / kStages) & 1u) ^ 1u;
-        const int row = bt[j / a.page_size] * a.page_size + j % a.page_size;
-        if (!wait(&sh->k_empty[s], before)) break;
-        mbar_arrive_expect_tx(&sh->k_full[s], kTile);
-        for (int c = 0; c < kChunks; ++c) tma_load_3d(ks + s * kTile + c * kWsBox, &tm_kv, &sh->k_full[s], kvh * D + c * 64, row, 0);
-        ++nk;
-        if (!wait(&sh->v_empty[s], before)) break;
-        mbar_arrive_expect_tx(&sh->v_full[s], kTile);
-        for (int c = 0; c < kChunks; ++c) tma_load_3d(vs + s * kTile + c * kWsBox, &tm_kv, &sh->v_full[s], (a.G + kvh) * D + c * 64, row, 0);
-        ++nv;
-      }
-      drain(&sh->q_full, 0);                               // nothing is on its way any more when this thread leaves
-      for (int t = max(0, nk - kStages); t < nk; ++t) drain(&sh->k_full[t % kStages], (uint32_t)(t / kStages) & 1u);
-      for (int t = max(0, nv - kStages); t < nv; ++t) drain(&sh->v_full[t % kStages], (uint32_t)(t / kStages) & 1u);
-    }
-  } else if (warp == 1) {
+  if (warp == 4) {
     if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16_major(kWsRows, kWsKeys, 0, 0), idesc_o = make_idesc_bf16_major(kWsRows, D, 0, 1);
       const uint64_t dq = make_sw128_kmajor_desc(smem_u32(qs)), dk0 = make_sw128_kmajor_desc(smem_u32(ks));
       const uint64_t dv0 = make_sw128_mnmajor_desc(smem_u32(vs), kWsBox, 1024);
       auto scores = [&](int t) {
-        const uint64_t dk = dk0 + (uint64_t)((t % kStages) * (kTile >> 4));
+        const uint64_t dk = dk0 + (uint64_t)((t & 1) * (kTile >> 4));
 #pragma unroll
         for (int k = 0; k < D / 16; ++k)
           umma_bf16<1>(tmem + (uint32_t)(t & 1) * kWsKeys, dq + (uint64_t)((k >> 2) * (kQChunk >> 4) + 2 * (k & 3)), dk + (uint64_t)((k >> 2) * (kWsBox >> 4) + 2 * (k & 3)),
                        idesc_s, k != 0 ? 1u : 0u);
         umma_commit(&sh->s_full[t & 1]);
-        umma_commit(&sh->k_empty[t % kStages]);
+        umma_commit(&sh->k_empty[t & 1]);
       };
       bool go = wait(&sh->q_full, 0) && wait(&sh->k_full[0], 0);
       tc_fence_after();
       if (go) scores(0);
       for (int t = 0; go && t < n_tiles; ++t) {
+        const uint32_t phase = (uint32_t)(t >> 1) & 1u;
         if (t + 1 < n_tiles) {
-          // into the buffer that holds the probabilities of the tile before: the order of products is only promised for one accumulator,
-          // so the one that reads them has to be done, not only issued
-          go = (t == 0 || wait(&sh->o_done, (uint32_t)(t - 1) & 1u)) && wait(&sh->k_full[(t + 1) % kStages], (uint32_t)((t + 1) / kStages) & 1u);
+          // over the probabilities of the tile before: the order of products is only promised for one accumulator, so the one that reads them has
+          // to be done, not only issued
+          go = (t == 0 || wait(&sh->o_done, (uint32_t)(t - 1) & 1u)) && wait(&sh->k_full[(t + 1) & 1], (uint32_t)((t + 1) >> 1) & 1u);
           if (!go) break;
           tc_fence_after();
           scores(t + 1);
         }
-        go = wait(&sh->v_full[t % kStages], (uint32_t)(t / kStages) & 1u) && wait(&sh->p_ready[t & 1], (uint32_t)(t >> 1) & 1u);
+        go = wait(&sh->v_full[t & 1], phase) && wait(&sh->p_ready[t & 1], phase);
         if (!go) break;
         tc_fence_after();
-        const uint64_t dv = dv0 + (uint64_t)((t % kStages) * (kTile >> 4));
+        const uint64_t dv = dv0 + (uint64_t)((t & 1) * (kTile >> 4));
         const uint32_t p = tmem + (uint32_t)(t & 1) * kWsKeys;   // columns 0..31: upper numbers, 32..63: lower ones
 #pragma unroll
         for (int k = 0; k < kWsKeys / 16; ++k)
 #pragma unroll
           for (int low = 0; low < 2; ++low) umma_bf16_ts(tmem_o, p + 32u * low + 8u * k, dv + (uint64_t)(k * 128), idesc_o, (t | k | low) != 0 ? 1u : 0u);
         umma_commit(&sh->o_done);
-        umma_commit(&sh->v_empty[t % kStages]);
+        umma_commit(&sh->v_empty[t & 1]);
       }
       umma_commit(&sh->mma_done);
-      drain(&sh->mma_done, 0);                             // every product that was issued is done
+      drain_bounded(&sh->mma_done, 0, report);             // every product that was issued is done
     }
+  } else if (warp > 4) {
+    // keys and values of the tiles in turn, two copies ahead of the one that is waited for
+    const int32_t* bt = a.bt + (long long)it.z * a.max_pages;
+    const long long W = 2LL * a.G * D;
+    const int c = tid & 7, key0 = (tid - kWsSoftmax - 32) >> 3;
+    auto arrive = [&](int i, auto ahead) {                 // copy i is there, and visible to the products
+      cp_async_wait<decltype(ahead)::value>();
+      fence_proxy_async();
+      __syncwarp();
+      if (lane == 0) mbar_arrive((i & 1) ? &sh->v_full[(i >> 1) & 1] : &sh->k_full[(i >> 1) & 1]);
+    };
+    long long first = 0;                                   // the tile's first row of the pool: a tile starts at a multiple of 64 keys, as pages do
+    int i = 0;
+    for (; i < 2 * n_tiles; ++i) {
+      const int t = i >> 1, j0 = k0 + t * kWsKeys;
+      const bool values = i & 1;
+      if (!values) first = (long long)bt[j0 / a.page_size] * a.page_size + j0 % a.page_size;
+      const bool free = wait(values ? &sh->v_empty[t & 1] : &sh->k_empty[t & 1], ((uint32_t)(t >> 1) & 1u) ^ 1u);
+      if (!free) break;
+      uint8_t* dst = (values ? vs : ks) + (t & 1) * kTile;
+      const bf16_t* src = a.pool + first * W + (values ? a.G + kvh : kvh) * D + c * 8;
+#pragma unroll
+      for (int k = 0; k < kWsKeys; k += kWsLoad / 8) {
+        const int key = k + key0;
+        uint8_t* at = dst + key * 128 + ((c ^ (key & 7)) << 4);
+        // rows that are no keys of this CTA hold whatever the cache holds there: as values they must not meet a product
+        const bool is_key = j0 + key >= k_begin && j0 + key < k_end;
+#pragma unroll
+        for (int b = 0; b < kChunks; ++b) {
+          if (is_key) cp_async16(at + b * kWsBox, src + key * W + b * 64, true);
+          else *reinterpret_cast<uint4*>(at + b * kWsBox) = make_uint4(0, 0, 0, 0);
+        }
+      }
+      cp_async_commit();
+      if (i >= 2) arrive(i - 2, std::integral_constant<int, 2>());
+    }
+    if (i == 2 * n_tiles) {
+      arrive(i - 2, std::integral_constant<int, 1>());
+      arrive(i - 1, std::integral_constant<int, 0>());
+    }
+    cp_async_wait<0>();
   } else {
-    const int quarter = warp & 3, row = (quarter & 1) * 32 + lane;   // TMEM lanes go by warp % 4
+    const int quarter = warp, row = (quarter & 1) * 32 + lane;   // TMEM lanes go by warp % 4
     const int4 mine = quarter < 2 ? it : next;
     const int n_rows = mine.y * rep, token = row / rep, h = row - token * rep;
     const bool any = (quarter & 1) * 32 < n_rows, is_row = row < n_rows;
@@ -222,6 +255,10 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
     auto o_before = [&](int t) {
       if (t > 0) wait_together(&sh->o_done, (uint32_t)(t - 1) & 1u);
     };
+    cp_async_wait<0>();                                    // this thread's part of Q is there, and visible to the products
+    fence_proxy_async();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sh->q_full);
     for (int t = 0; t < n_tiles; ++t) {
       const uint32_t ts = tmem + lanes + (uint32_t)(t & 1) * kWsKeys;
       const int j0 = k0 + t * kWsKeys;
@@ -295,18 +332,6 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
         }
         tmem_st_wait();
       }
-      // rows of the tile that are no keys of this CTA hold whatever the cache holds there: as values they must not meet a product
-      if (j0 < k_begin || j0 + kWsKeys > k_end) {
-        if (wait_together(&sh->v_full[t % kStages], (uint32_t)(t / kStages) & 1u)) {
-          uint8_t* v = vs + (t % kStages) * kTile;
-          for (int e = tid - 64; e < kWsKeys * 8; e += kWsSoftmax) {
-            const int key = e >> 3;
-            if (j0 + key < k_begin || j0 + key >= k_end)
-              for (int c = 0; c < kChunks; ++c) *reinterpret_cast<uint4*>(v + c * kWsBox + key * 128 + (e & 7) * 16) = make_uint4(0, 0, 0, 0);
-          }
-        }
-        fence_proxy_async();
-      }
       o_before(t);
       tc_fence_before();
       __syncwarp();
@@ -357,24 +382,26 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(const 
   }
   __syncwarp();
   __syncthreads();
-  if (warp == 1) tmem_dealloc<1>(tmem, 256);
+  if (warp == 4) tmem_dealloc<1>(tmem, 256);
 }
 
-static int ws_smem(int d, int table) { return (d == 128 ? 2 : 4) * 2 * (d / 64) * kWsBox + (d / 64) * kWsRows * 128 + table + kWsTail; }
+static int ws_smem(int d, int table) { return 4 * (d / 64) * kWsBox + (d / 64) * kWsRows * 128 + table + kWsTail; }
 static int ws_table(bool bias, int window, int rep) { return bias ? (ws_bias_pitch(window, rep) * rep * 4 + 15) / 16 * 16 : 0; }
 
-// Shapes this kernel takes; the widths of rows and the alignment of the output are what its 16-byte accesses want.
-bool window_sm100_ok(int H, int G, int d, int dv, int maps, int keep_first, long long pool_rows, int page_size, int window, const float* bias, const void* out, long long ldo,
-                     const void* pool) {
-  const int rep = H / G;
-  return (d == 64 || d == 128) && dv == d && maps == 1 && keep_first == 0 && pool_rows >= kWsKeys && pool_rows <= (1ll << 31) &&
-         page_size % kWsKeys == 0 && rep <= 64 && ldo % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(out) % 16 == 0 && reinterpret_cast<uintptr_t>(pool) % 16 == 0 &&
-         (bias == nullptr || (window <= 16384 && ws_smem(d, ws_table(true, window, rep)) <= 220 * 1024));
+// Shapes this kernel takes (the alignment of the output is what its 16-byte accesses want), where it is the faster one. A CTA of it costs some 5 us before
+// its first tile, so a row has to see enough keys: at widths of 128 from 64 keys on (64 keys 0.52 to 0.93 of the mma.sync kernel's time, 32 keys up to
+// 1.34), at widths of 64, whose tiles are shorter, from 192 on (0.54 to 1.03; 128 keys up to 1.20) or from 64 on where CTAs come in several waves
+// (0.65 to 0.85).
+bool window_sm100_ok(int H, int G, int d, int dv, int maps, int keep_first, int page_size, int n_items, int window, int chunk, const float* bias, const void* out,
+                     long long ldo) {
+  const int rep = H / G, reach = window < chunk ? window : chunk;
+  return (d == 64 || d == 128) && dv == d && maps == 1 && keep_first == 0 && page_size % kWsKeys == 0 && rep <= 64 && ldo % 8 == 0 &&
+         reinterpret_cast<uintptr_t>(out) % 16 == 0 && reach >= 64 && (d == 128 || reach >= 192 || (long long)n_items * G >= 4 * 148) &&
+         (long long)n_items * G < (1ll << 31) && (bias == nullptr || (window <= 16384 && ws_smem(d, ws_table(true, window, rep)) <= 220 * 1024));
 }
 
 template <int D, bool CAP, bool BIAS>
-static int ws_launch(const CUtensorMap& tq, const CUtensorMap& tk, const WinSmArgs& a, cudaStream_t st) {
+static int ws_launch(const WinSmArgs& a, cudaStream_t st) {
   static bool done[kMaxDevices] = {};
   const int dev = cur_device();
   if (!done[dev]) {
@@ -382,32 +409,19 @@ static int ws_launch(const CUtensorMap& tq, const CUtensorMap& tk, const WinSmAr
     if (e != cudaSuccess) return set_error(OMC_ERR_CUDA, cudaGetErrorString(e));
     done[dev] = true;
   }
-  window_attn_sm100_kernel<D, CAP, BIAS><<<(unsigned)a.n_items * a.G, kWsThreads, ws_smem(D, a.table), st>>>(tq, tk, a);
+  window_attn_sm100_kernel<D, CAP, BIAS><<<(unsigned)a.n_items * a.G, kWsThreads, ws_smem(D, a.table), st>>>(a);
   return check_launch("omc_window_attn_mma");
 }
 
-int window_sm100(const void* q, long long ldq, int T, int H, int G, int d, const void* pool, long long pool_rows, const int32_t* bt, int max_pages, int page_size,
-                 const int32_t* items, int n_items, int window, int chunk, float scale, float softcap, const float* bias, const float* sink, const float* gate, long long ldg, int gate_act,
+int window_sm100(const void* q, long long ldq, int T, int H, int G, int d, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
+                 int n_items, int window, int chunk, float scale, float softcap, const float* bias, const float* sink, const float* gate, long long ldg, int gate_act,
                  int gate_heads, void* out, int out_dt, long long ldo, cudaStream_t st) {
   const int rep = H / G;
-  WinSmArgs a{bt, items, bias, sink, gate, ldg, gate_act, gate_heads, out, ldo, out_dt == OMC_DT_BF16, n_items, max_pages, page_size, H, G, window, chunk, 64 / rep,
+  WinSmArgs a{static_cast<const bf16_t*>(q), ldq, static_cast<const bf16_t*>(pool), bt, items, bias, sink, gate, ldg, gate_act, gate_heads, out, ldo, out_dt == OMC_DT_BF16, n_items, max_pages, page_size, H, G, window, chunk, 64 / rep,
               ws_table(bias != nullptr, window, rep), scale, softcap, nullptr};
   int rc = step_failure_word(&a.failed);
   if (rc != OMC_OK) return rc;
-  TensorMapEncodeFn enc = tensor_map_encode_fn();
-  if (enc == nullptr) return set_error(OMC_ERR_DRIVER, "cuTensorMapEncodeTiled entry point unavailable");
-  CUtensorMap tq, tk;
-  {   // [tokens][heads][d]: a box is 64 columns of the query heads of one key/value head, of as many tokens as an item has
-    cuuint64_t dim[3] = {(cuuint64_t)d, (cuuint64_t)H, (cuuint64_t)T}, stride[2] = {(cuuint64_t)d * 2, (cuuint64_t)ldq * 2};
-    cuuint32_t box[3] = {64u, (cuuint32_t)rep, (cuuint32_t)a.tok}, one[3] = {1u, 1u, 1u};
-    if (enc(&tq, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(q), dim, stride, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return set_error(OMC_ERR_DRIVER, "cuTensorMapEncodeTiled failed");
-  }
-  const long long W = 2LL * G * d;
-  rc = step_tensor_map(&tk, pool, W, pool_rows, W, 1, 0, kWsKeys);   // the rows that there are: whatever a copy asks for, it stays inside the pool
-  if (rc != OMC_OK) return rc;
-#define OMC_WS(CAP, BIAS) (d == 64 ? ws_launch<64, CAP, BIAS>(tq, tk, a, st) : ws_launch<128, CAP, BIAS>(tq, tk, a, st))
+#define OMC_WS(CAP, BIAS) (d == 64 ? ws_launch<64, CAP, BIAS>(a, st) : ws_launch<128, CAP, BIAS>(a, st))
   if (softcap > 0.f) return bias != nullptr ? OMC_WS(true, true) : OMC_WS(true, false);
   return bias != nullptr ? OMC_WS(false, true) : OMC_WS(false, false);
 #undef OMC_WS

@@ -47,7 +47,6 @@ SIGNATURES = {
     "omc_window_attn": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P, _I, _I, _I, _F, _F, _P, _P, _P, _L, _I, _I, _P, _I, _L, _P]),
     "omc_window_attn_mma_ok": (_I, [_I, _I, _I, _I]),
     "omc_window_attn_mma": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _F, _F, _P, _P, _P, _L, _I, _I, _P, _I, _L, _P]),
-    "omc_window_attn_mma_rows": (_I, [_P, _L, _I, _I, _I, _I, _I, _I, _P, _L, _P, _I, _I, _P, _I, _P, _P, _I, _I, _I, _F, _F, _P, _P, _P, _L, _I, _I, _P, _I, _L, _P]),
     "omc_diff_attn_pair_ok": (_I, [_I, _I, _I, _I]),
     "omc_diff_attn_pair": (_I, [_P, _L, _I, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _I, _I, _F, _F, _F, _F, _P, _L, _I, _P, _I, _L, _P]),
     "omc_ln_residual": (_I, [_P, _L, _F, _P, _L, _P, _L, _P, _P, _I, _P, _P, _I, _F, _P, _L, _P, _I, _L, _I, _I, _P]),
@@ -759,11 +758,10 @@ def window_attn_mma(q: torch.Tensor, H: int, G: int, d: int, dv: int, pool: torc
     assert pool.is_contiguous() and pool.shape[-1] == G * (maps * d + dv) and block_table.is_contiguous()
     assert items is None or (items.dtype == torch.int32 and items.is_contiguous() and items.shape[1] == 4)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape == (window, H))
-    rc = load().omc_window_attn_mma_rows(_ptr(q), q.stride(0), q.shape[0], H, G, d, dv, maps, _ptr(pool), pool.numel() // pool.shape[-1], _ptr(block_table),
-                                         block_table.shape[1], page_size, _ptr(items), items.shape[0] if items is not None else 0, _ptr(pos), _ptr(slot),
-                                         window, chunk, keep_first, scale, softcap, _ptr(dist_bias), _ptr(sink), _ptr(gate),
-                                         gate.stride(0) if gate is not None else 0, gate_act, 1 if gate_heads else 0, _ptr(out), _dt(out), out.stride(0),
-                                         _stream())
+    rc = load().omc_window_attn_mma(_ptr(q), q.stride(0), q.shape[0], H, G, d, dv, maps, _ptr(pool), _ptr(block_table), block_table.shape[1],
+                                    page_size, _ptr(items), items.shape[0] if items is not None else 0, _ptr(pos), _ptr(slot), window, chunk,
+                                    keep_first, scale, softcap, _ptr(dist_bias), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
+                                    gate_act, 1 if gate_heads else 0, _ptr(out), _dt(out), out.stride(0), _stream())
     _check(rc, "omc_window_attn_mma")
     return out
 

@@ -77,13 +77,13 @@ def test_against_float64(portions, H, G, d, page, opt):
     rows, pool, table, q, plan = _inputs(PORTIONS[portions], H, G, d, page, gen)
     T, scale, window, chunk, cap, bias, sink, gate, act = q.shape[0], 8.0 / d ** 0.5, seqlib.WINDOW_ALL, seqlib.WINDOW_ALL, 0.0, None, None, None, 0
     if opt == "window_cap_bias":
-        window, cap = 150, 50.0
+        window, cap = 200, 50.0
         bias = torch.randn(window, H, generator=gen) * 3
     elif opt == "window_bias_sink":
-        window = 64
+        window = 64 if d == 128 else 192                                 # the least this kernel takes
         bias, sink = torch.randn(window, H, generator=gen) * 3, torch.randn(H, generator=gen) * 10
     elif opt == "chunk_cap_sink_heads_gate":
-        chunk, cap, sink, gate, act = 96, 30.0, torch.randn(H, generator=gen) * 10, torch.randn(T, H, generator=gen), 2
+        chunk, cap, sink, gate, act = 96 if d == 128 else 200, 30.0, torch.randn(H, generator=gen) * 10, torch.randn(T, H, generator=gen), 2
     elif opt == "short_chunk_gate":
         chunk, gate, act = 24, torch.randn(T, H * d, generator=gen), 1
     cu = lambda t: t.cuda() if t is not None else None
@@ -94,9 +94,10 @@ def test_against_float64(portions, H, G, d, page, opt):
         seqlib.window_attn_mma(q.cuda(), H, G, d, d, pool.cuda(), table.cuda(), page, items, None, None, window, scale, cap, cu(bias), out, sink=cu(sink), gate=cu(gate),
                                gate_act=act, chunk=chunk, gate_heads=opt == "chunk_cap_sink_heads_gate")
         # fp32 scores of up to some tens (in base 2: 2^7) after some eight roundings and a soft cap of a few 2^-23 of the cap: 2^-14; probabilities as
-        # two bf16 numbers: 2^-17; the gate through the fast exponential: 2^-20. A bf16 output adds its own rounding
+        # two bf16 numbers: 2^-17 (chunks too short for this kernel, on mma.sync: one, in the sums above and below the line, 2^-8); the gate through the
+        # fast exponential: 2^-20. A bf16 output adds its own rounding
         err = (out.double() - want).abs()
-        assert (err <= mag * 2.0 ** -13 + (want.abs() * 2.0 ** -8 if dt == BF16 else 0.0) + 1e-30).all(), (dt, float((err / (mag + 1e-30)).max()))
+        assert (err <= mag * (2.0 ** -13 + (2.0 ** -8 if opt == "short_chunk_gate" else 0.0)) + (want.abs() * 2.0 ** -8 if dt == BF16 else 0.0) + 1e-30).all(), (dt, float((err / (mag + 1e-30)).max()))
 
 
 def test_requests_do_not_meet():
