@@ -127,9 +127,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, report); };
   auto drain = [&](uint64_t* bar, uint32_t parity) { drain_bounded(bar, parity, report); };
   const int32_t* bt = a.bt + (long long)slot * a.max_pages;
-  // The last chunk ends where the row does: its box starts at D - 64 and repeats columns of the chunk before where D is no multiple of 64. A
-  // box that reached past the row would have its columns filled with zeros, but the pool's map knows no last row (see latent_sm100), and a
-  // copy of the last row of a pool that ends with its mapping then faulted.
+  // The last chunk ends where the row does: its box starts at D - 64 and repeats columns of the chunk before where D is no multiple of 64.
   auto chunk_col = [&](int c) { return c == a.nc - 1 ? a.D - 64 : c * 64; };
   // rows of the pool where the two boxes of tile t start (looked up a tile ahead: a lookup takes as long as 20 KB of the copies)
   auto box_rows = [&](int t, int (&row)[2]) {
@@ -417,9 +415,9 @@ static int ls_smem(int nr, int r, int D, LatSmArgs* a) {
 }
 
 // Shapes this kernel takes. max_rows: the most rows an item has.
-bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool) {
+bool latent_sm100_ok(int max_rows, int r, int dr, long long pool_rows, int page_size, const void* q, const void* pool) {
   LatSmArgs a;
-  return max_rows <= kLsMaxRows && r % 128 == 0 && r <= 512 && dr <= 64 && dr % 16 == 0 && page_size % 64 == 0 &&
+  return pool_rows >= 64 && pool_rows <= (1ll << 31) && max_rows <= kLsMaxRows && r % 128 == 0 && r <= 512 && dr <= 64 && dr % 16 == 0 && page_size % 64 == 0 &&
          reinterpret_cast<uintptr_t>(q) % 16 == 0 && reinterpret_cast<uintptr_t>(pool) % 16 == 0 && ls_smem(max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64), r, r + dr, &a) > 0;
 }
 
@@ -436,7 +434,7 @@ static int ls_launch(const CUtensorMap& tq, const CUtensorMap& tk, const LatSmAr
   return check_launch("omc_latent_attn_mma");
 }
 
-int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
+int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, long long pool_rows, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
                  int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
                  float* ws_ml, cudaStream_t st) {
   const int D = r + dr, nr = max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64);
@@ -447,8 +445,8 @@ int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const vo
   CUtensorMap tq, tk;
   int rc = step_failure_word(&a.failed);
   if (rc == OMC_OK) rc = step_tensor_map(&tq, q, D, q_rows, D, 1, 0, nr);
-  // how many pages the pool has is not known here; boxes lie wholly inside pages that the block table names
-  if (rc == OMC_OK) rc = step_tensor_map(&tk, pool, D, 1ull << 31, D, 1, 0, 64);
+  // the rows that there are and no more: a map of 2^31 rows let copies of a pool's last rows touch what lies behind the pool
+  if (rc == OMC_OK) rc = step_tensor_map(&tk, pool, D, pool_rows, D, 1, 0, 64);
   if (rc != OMC_OK) return rc;
   const bool b = out_dt == OMC_DT_BF16;
   if (nr == 16) return b ? ls_launch<16, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<16, float>(tq, tk, a, n_items, smem, st);

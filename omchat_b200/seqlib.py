@@ -62,6 +62,7 @@ SIGNATURES = {
     "omc_rotary_q": (_I, [_P, _I, _L, _I, _I, _I, _I, _P, _I, _P, _P, _I, _I, _P]),
     "omc_latent_attn": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _P, _I, _I, _P, _P, _P, _I, _P, _L, _F, _P, _P]),
     "omc_latent_attn_mma_rows": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
+    "omc_latent_attn_mma_pool": (_I, [_P, _I, _I, _I, _I, _P, _L, _P, _I, _I, _P, _I, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_step_wait_failures": (_I, [_P]),
     "omc_step_wait_failed": (_I, []),
     "omc_step_wait_selfcheck": (_I, [_P, _P]),
@@ -410,7 +411,7 @@ def latent_attn_mma(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, blo
             ws = torch.empty(need, device=qcat.device, dtype=torch.float32)
             _mma_ws[key] = ws
         ws_o, ws_ml = ws[:plan.n_parts * MMA_ROWS * r], ws[plan.n_parts * MMA_ROWS * r:]
-    rc = load().omc_latent_attn_mma_rows(_ptr(qcat), T, H, r, dr, _ptr(pool), _ptr(block_table), block_table.shape[1], page_size,
+    rc = load().omc_latent_attn_mma_pool(_ptr(qcat), T, H, r, dr, _ptr(pool), pool.numel() // (r + dr), _ptr(block_table), block_table.shape[1], page_size,
                                          _ptr(plan.items), plan.n_items, plan.max_rows, _ptr(plan.merges), plan.n_merges, _ptr(sink), window, _ptr(gate),
                                          gate.stride(0) if gate is not None else 0, scale, _ptr(out), _dt(out), _ptr(ws_o), _ptr(ws_ml), _stream())
     _check(rc, "omc_latent_attn_mma")
