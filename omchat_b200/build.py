@@ -9,6 +9,7 @@ Separate libraries, so that a process compiles only what its model needs:
                                                 (include/omchat_b200_seq.h); built with IEEE division / square root / exp
   dense omchat_b200/_lib/libomchat_b200_dense.so  the GEMM / row-kernel / sampling subset of core, for a process that has no core
                                                 library (lib.load_dense() prefers a built core library, which has the same symbols)
+  calls omchat_b200/_lib/omc_call.so            how Python calls the entries of these (csrc/call.cpp; ctypes does where it cannot be built)
 `python -m omchat_b200.build [core|seq ...]` or `__graft_entry__.build()` builds both; nvcc cross-compiles without a GPU. The
 libraries are git-ignored but travel to the GPU box with the repo snapshot. `ensure(name)` builds one library on demand (first
 use in a fresh checkout).
@@ -17,6 +18,7 @@ from __future__ import annotations
 
 import hashlib
 import os
+import shutil
 import subprocess
 import sys
 from concurrent.futures import ThreadPoolExecutor
@@ -97,13 +99,44 @@ def build_component(name: str, force: bool = False, verbose: bool = False) -> Pa
     return lib
 
 
+CALL_LIB, CALL_SOURCE = LIBDIR / "omc_call.so", CSRC / "call.cpp"
+
+
+def ensure_call(force: bool = False) -> Path | None:
+    """The compiled calls of native.py (host code, a few seconds of g++), built first if missing, older than the source or made for another interpreter or torch; None
+    where there is neither a built one nor a compiler with Python's headers."""
+    import sysconfig
+
+    import torch
+    include = sysconfig.get_paths()["include"]
+    root = Path(torch.__file__).resolve().parent
+    flags = ["-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    digest = _digest([CALL_SOURCE], [*flags, sys.version, torch.__version__])
+    stamp = LIBDIR / "build_call.sha256"
+    if not force and CALL_LIB.exists() and stamp.exists() and stamp.read_text() == digest:
+        return CALL_LIB
+    gxx = shutil.which("g++")
+    if gxx is None or not os.path.exists(os.path.join(include, "Python.h")):
+        return None
+    LIBDIR.mkdir(exist_ok=True)
+    tmp = CALL_LIB.with_suffix(f".so.tmp{os.getpid()}")
+    r = subprocess.run([gxx, *flags, str(CALL_SOURCE), "-o", str(tmp), f"-I{include}", f"-I{root}/include", f"-I{root}/include/torch/csrc/api/include", f"-L{root}/lib",
+                        "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10"], capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for {CALL_SOURCE.name}:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, CALL_LIB)  # a concurrent process never sees a half-written library
+    stamp.write_text(digest)
+    return CALL_LIB
+
+
 def ensure(name: str) -> Path:
     """The library of component `name`, built first if it is missing or older than its sources."""
     return build_component(name)
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
-    """Builds the seq and the core library (the dense subset is built on demand only); returns the core library's path."""
+    """Builds the seq and the core library and the compiled calls (the dense subset is built on demand only); returns the core library's path."""
+    ensure_call(force)
     build_component("seq", force, verbose)
     return build_component("core", force, verbose)
 

@@ -12,6 +12,8 @@ from typing import Optional
 
 import torch
 
+from . import native
+
 _PKG = Path(__file__).resolve().parent
 LIB_PATH = _PKG / "_lib" / "libomchat_b200.so"
 
@@ -98,7 +100,7 @@ class OmcError(RuntimeError):
     pass
 
 
-def load() -> ctypes.CDLL:
+def load() -> native.Entries:
     """Load the shared library (building is __graft_entry__.build()'s job; a missing library is a hard error)."""
     global _lib
     if _lib is not None:
@@ -106,19 +108,14 @@ def load() -> ctypes.CDLL:
     path = os.environ.get("OMCHAT_B200_LIB", str(LIB_PATH))
     if not os.path.exists(path):
         raise OmcError(f"{path} not found: run `python -m omchat_b200.build` (there is no CPU fallback)")
-    lib = ctypes.CDLL(path)
-    for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)  # AttributeError if the library does not export a declared symbol
-        fn.restype = res
-        fn.argtypes = args
-    _lib = lib
-    return lib
+    _lib = native.Entries(ctypes.CDLL(path), SIGNATURES)
+    return _lib
 
 
 _dense = None
 
 
-def load_dense() -> ctypes.CDLL:
+def load_dense() -> native.Entries:
     """The library that holds the GEMMs (tcgen05, skinny, grouped), the row kernels and omc_argmax: the full core library when it
     is loaded or has been built; else its `dense` subset, compiled on first use (build.ensure("dense")). Models that need nothing
     else of the core library (model/voduzen.py) call their GEMMs and the sampler through this."""
@@ -130,14 +127,8 @@ def load_dense() -> ctypes.CDLL:
     if os.environ.get("OMCHAT_B200_LIB") or LIB_PATH.exists():
         return load()
     from . import build
-    lib = ctypes.CDLL(str(build.ensure("dense")))
-    for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name, None)
-        if fn is not None:
-            fn.restype = res
-            fn.argtypes = args
-    _dense = lib
-    return lib
+    _dense = native.Entries(ctypes.CDLL(str(build.ensure("dense"))), SIGNATURES, missing_ok=True)
+    return _dense
 
 
 _KERNELS_PER_CALL = {"omc_splice": 2, "omc_argmax": 2}
@@ -151,28 +142,8 @@ def _check(rc: int, what: str):
         raise OmcError(f"{what} failed ({rc}): {msg}")
 
 
-def _ptr(t: Optional[torch.Tensor]):
-    return None if t is None else t.data_ptr()
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
-
-
-def _need_cuda(*ts):
-    """Every kernel is launched on torch.cuda.current_stream() of the CURRENT device: a tensor living on another GPU would
-    be dereferenced there (illegal access or silent peer traffic), so that is an error, not a convention."""
-    cur = None
-    for t in ts:
-        if t is None:
-            continue
-        if not t.is_cuda:
-            raise OmcError("omchat_b200 kernels need CUDA tensors (no CPU fallback)")
-        if cur is None:
-            cur = torch.cuda.current_device()
-        if t.device.index != cur:
-            raise OmcError(f"tensor on cuda:{t.device.index} but the current device is cuda:{cur}: run the call under "
-                           f"`with torch.cuda.device({t.device.index}):` (the model classes do this themselves)")
+_stream = native.raw_stream
+_need_cuda = native.need_cuda(OmcError)
 
 
 SKINNY_MAX_M = 64  # rows up to which gemm() streams the weights through the swapped-operand skinny kernel
@@ -225,8 +196,8 @@ def _gemm_autotune(x, w, out, bias, scale, res, epi, out_f32) -> int:
             _l2_flush.zero_()
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
-            rc = load_dense().omc_gemm_bf16(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(scratch), scratch.stride(0), M, N, K,
-                                      _ptr(bias), _ptr(scale), _ptr(res), res.stride(0) if res is not None else 0, epi,
+            rc = load_dense().omc_gemm_bf16(x, x.stride(0), w, w.stride(0), scratch, scratch.stride(0), M, N, K,
+                                      bias, scale, res, res.stride(0) if res is not None else 0, epi,
                                       1 if out_f32 else 0, c, _stream())
             e1.record()
             if rc != 0:
@@ -262,7 +233,7 @@ class RowSsq:
         """Rows no GEMM produced (embeddings, all-reduced rows): one warp per row."""
         _need_cuda(x)
         assert x.dim() == 2 and x.stride(1) == 1 and x.shape[0] <= self.rows
-        rc = load().omc_row_ssq_rows(_ptr(x), x.stride(0), x.shape[0], x.shape[1], self.buf.data_ptr(), _stream())
+        rc = load().omc_row_ssq_rows(x, x.stride(0), x.shape[0], x.shape[1], self.buf.data_ptr(), _stream())
         _check(rc, "omc_row_ssq_rows")
         self.parts = 1
         return self
@@ -292,8 +263,8 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
         if ssq_out is not None:
             assert ssq_out.rows >= M
             nf.ssq_out, nf.ssq_out_ld, nf.ssq_out_max_parts = ssq_out.buf.data_ptr(), ssq_out.rows, RowSsq.MAX_PARTS
-        rc = load_dense().omc_gemm_bf16_norm(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K,
-                                       _ptr(bias), _ptr(scale), _ptr(res), res.stride(0) if res is not None else 0, epi,
+        rc = load_dense().omc_gemm_bf16_norm(x, x.stride(0), w, w.stride(0), out, out.stride(0), M, N, K,
+                                       bias, scale, res, res.stride(0) if res is not None else 0, epi,
                                        1 if out_f32 else 0, tile_cfg, ctypes.byref(nf), _stream())
         _check(rc, "omc_gemm_bf16_norm")
         if ssq_out is not None:
@@ -301,15 +272,15 @@ def gemm(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
         return out
     if M <= SKINNY_MAX_M and tile_cfg == 0 and SKINNY_ENABLED:
         ws = _skinny_workspace(x.device, N)
-        rc = load_dense().omc_gemm_skinny_bf16(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K,
-                                         _ptr(bias), _ptr(scale), _ptr(res), res.stride(0) if res is not None else 0, epi,
+        rc = load_dense().omc_gemm_skinny_bf16(x, x.stride(0), w, w.stride(0), out, out.stride(0), M, N, K,
+                                         bias, scale, res, res.stride(0) if res is not None else 0, epi,
                                          1 if out_f32 else 0, ws.data_ptr(), ws.numel(), _stream())
         _check(rc, "omc_gemm_skinny_bf16")
         return out
     if tile_cfg == 0 and GEMM_AUTOTUNE and M <= GEMM_AUTOTUNE_MAX_M:
         tile_cfg = _gemm_autotune(x, w, out, bias, scale, res, epi, out_f32)
-    rc = load_dense().omc_gemm_bf16(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), M, N, K,
-                              _ptr(bias), _ptr(scale), _ptr(res), res.stride(0) if res is not None else 0, epi,
+    rc = load_dense().omc_gemm_bf16(x, x.stride(0), w, w.stride(0), out, out.stride(0), M, N, K,
+                              bias, scale, res, res.stride(0) if res is not None else 0, epi,
                               1 if out_f32 else 0, tile_cfg, _stream())
     _check(rc, "omc_gemm_bf16")
     return out
@@ -323,7 +294,7 @@ def gemm_grouped(x: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor, ou
     assert x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.dim() == 3 and w.is_contiguous() and x.stride(1) == 1
     E, N, K = w.shape
     fn = load_dense().omc_gemm_bf16_grouped_f32 if out.dtype == torch.float32 else load_dense().omc_gemm_bf16_grouped
-    rc = fn(_ptr(x), x.stride(0), x.shape[0], _ptr(w), K, E, N, K, _ptr(tile_expert), active_tiles_hint, _ptr(out), out.stride(0),
+    rc = fn(x, x.stride(0), x.shape[0], w, K, E, N, K, tile_expert, active_tiles_hint, out, out.stride(0),
             epi, _stream())
     _check(rc, "omc_gemm_bf16_grouped")
     return out
@@ -345,7 +316,7 @@ class PackedWeight:
         self._buf = torch.empty(nbytes + 1024, device=w.device, dtype=torch.uint8)
         off = (-self._buf.data_ptr()) % 1024
         self.data = self._buf[off:off + nbytes]
-        rc = load().omc_pack_weight(_ptr(w), w.stride(0), self.N, self.K, _ptr(col_scale), self.data.data_ptr(), _stream())
+        rc = load().omc_pack_weight(w, w.stride(0), self.N, self.K, col_scale, self.data.data_ptr(), _stream())
         _check(rc, "omc_pack_weight")
 
 
@@ -403,9 +374,9 @@ def gemm_stream(x: torch.Tensor, wp: PackedWeight, out: Optional[torch.Tensor] =
     if ssq_out is not None:
         assert ssq_out.dtype == torch.float32 and ssq_out.numel() >= ssq_parts(N) * 64
     ws = _stream_workspace(x.device)
-    rc = load().omc_gemm_stream(_ptr(x), x.stride(0), M, wp.data.data_ptr(), N, K, _ptr(out), out.stride(0), 1 if out_f32 else 0,
-                                _ptr(bias), _ptr(res), res.stride(0) if res is not None else 0, epi, _ptr(ssq_in),
-                                ssq_in_parts, norm_dim, eps, _ptr(ssq_out), ws.data_ptr(),
+    rc = load().omc_gemm_stream(x, x.stride(0), M, wp.data.data_ptr(), N, K, out, out.stride(0), 1 if out_f32 else 0,
+                                bias, res, res.stride(0) if res is not None else 0, epi, ssq_in,
+                                ssq_in_parts, norm_dim, eps, ssq_out, ws.data_ptr(),
                                 1 if (PDL_ENABLED if pdl is None else pdl) else 0, ctypes.byref(tp) if tp is not None else None,
                                 _stream())
     _check(rc, "omc_gemm_stream")
@@ -415,7 +386,7 @@ def gemm_stream(x: torch.Tensor, wp: PackedWeight, out: Optional[torch.Tensor] =
 def row_ssq(x: torch.Tensor, ssq: torch.Tensor, parts: int = 1, pdl: Optional[bool] = None):
     _need_cuda(x, ssq)
     assert x.dim() == 2 and x.stride(1) == 1 and ssq.dtype == torch.float32 and ssq.numel() >= parts * 64
-    rc = load().omc_row_ssq(_ptr(x), x.stride(0), x.shape[0], x.shape[1], _ptr(ssq), parts,
+    rc = load().omc_row_ssq(x, x.stride(0), x.shape[0], x.shape[1], ssq, parts,
                             1 if (PDL_ENABLED if pdl is None else pdl) else 0, _stream())
     _check(rc, "omc_row_ssq")
     return ssq
@@ -429,8 +400,8 @@ def gemv(x: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor] = None, *
     n_out = N // 2 if epi == EPI_SWIGLU else N
     if out is None:
         out = torch.empty(B, n_out, device=x.device, dtype=torch.float32 if out_f32 else torch.bfloat16)
-    rc = load().omc_gemv_bf16(_ptr(x), x.stride(0), _ptr(w), w.stride(0), _ptr(out), out.stride(0), B, N, K,
-                              _ptr(norm_w), eps, _ptr(bias), _ptr(res), res.stride(0) if res is not None else 0, epi,
+    rc = load().omc_gemv_bf16(x, x.stride(0), w, w.stride(0), out, out.stride(0), B, N, K,
+                              norm_w, eps, bias, res, res.stride(0) if res is not None else 0, epi,
                               1 if out_f32 else 0, _stream())
     _check(rc, "omc_gemv_bf16")
     return out
@@ -441,7 +412,7 @@ def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float, out: Optional[torch.Te
     assert x.dim() == 2 and x.stride(1) == 1
     if out is None:
         out = torch.empty(x.shape, device=x.device, dtype=torch.bfloat16)
-    rc = load().omc_rmsnorm(_ptr(x), x.stride(0), _ptr(w), _ptr(out), out.stride(0), x.shape[0], x.shape[1], eps,
+    rc = load().omc_rmsnorm(x, x.stride(0), w, out, out.stride(0), x.shape[0], x.shape[1], eps,
                             _stream())
     _check(rc, "omc_rmsnorm")
     return out
@@ -454,7 +425,7 @@ def layernorm(x: torch.Tensor, w: torch.Tensor, b: Optional[torch.Tensor], eps: 
     assert x.dim() == 2 and x.stride(1) == 1
     if out is None:
         out = torch.empty(x.shape, device=x.device, dtype=torch.bfloat16)
-    rc = load().omc_layernorm(_ptr(x), x.stride(0), _ptr(w), _ptr(b) if b is not None else None, _ptr(out), out.stride(0),
+    rc = load().omc_layernorm(x, x.stride(0), w, b if b is not None else None, out, out.stride(0),
                               x.shape[0], x.shape[1], eps, _stream())
     _check(rc, "omc_layernorm")
     return out
@@ -464,7 +435,7 @@ def rmsnorm_pair(x: torch.Tensor, w_a: torch.Tensor, w_b: torch.Tensor, C: int, 
     """In place: x[:, :C] normalised with w_a, x[:, C:2C] with w_b (q_norm / k_norm on packed qkv rows), one launch."""
     _need_cuda(x, w_a, w_b)
     assert x.dim() == 2 and x.stride(1) == 1 and x.shape[1] >= 2 * C
-    rc = load().omc_rmsnorm_pair(_ptr(x), x.stride(0), _ptr(w_a), _ptr(w_b), x.shape[0], C, eps, _stream())
+    rc = load().omc_rmsnorm_pair(x, x.stride(0), w_a, w_b, x.shape[0], C, eps, _stream())
     _check(rc, "omc_rmsnorm_pair")
     return x
 
@@ -475,7 +446,7 @@ def vit_im2col(pixels: torch.Tensor, ldc: int = 640) -> torch.Tensor:
     assert pixels.dtype in (torch.float32, torch.bfloat16)
     B, _, H, W = pixels.shape
     cols = torch.empty(B * (H // 14) * (W // 14), ldc, device=pixels.device, dtype=torch.bfloat16)
-    rc = load().omc_vit_im2col(_ptr(pixels), 1 if pixels.dtype == torch.float32 else 0, _ptr(cols), ldc, B, H, W,
+    rc = load().omc_vit_im2col(pixels, 1 if pixels.dtype == torch.float32 else 0, cols, ldc, B, H, W,
                                _stream())
     _check(rc, "omc_vit_im2col")
     return cols
@@ -486,7 +457,7 @@ def vit_assemble(patch: torch.Tensor, cls: torch.Tensor, pos: torch.Tensor, B: i
     P = patch.shape[0] // B
     C = patch.shape[1]
     hidden = torch.empty(B * (P + 1), C, device=patch.device, dtype=torch.bfloat16)
-    rc = load().omc_vit_assemble(_ptr(patch), _ptr(cls), _ptr(pos), _ptr(hidden), B, P, C, _stream())
+    rc = load().omc_vit_assemble(patch, cls, pos, hidden, B, P, C, _stream())
     _check(rc, "omc_vit_assemble")
     return hidden
 
@@ -495,7 +466,7 @@ def select_pixel_shuffle(hidden: torch.Tensor, B: int, G: int, down: int) -> tor
     _need_cuda(hidden)
     C = hidden.shape[-1]
     out = torch.empty(B * (G // down) ** 2, C * down * down, device=hidden.device, dtype=torch.bfloat16)
-    rc = load().omc_select_pixel_shuffle(_ptr(hidden), _ptr(out), B, G, C, down, _stream())
+    rc = load().omc_select_pixel_shuffle(hidden, out, B, G, C, down, _stream())
     _check(rc, "omc_select_pixel_shuffle")
     return out
 
@@ -506,7 +477,7 @@ def resample_u8(src: torch.Tensor, dst_h: int, dst_w: int, coefs: torch.Tensor, 
     assert src.dtype == torch.uint8 and src.dim() == 3 and src.shape[2] == 3 and src.is_contiguous()
     assert coefs.dtype == torch.int32 and bounds.dtype == torch.int32 and coefs.is_contiguous() and bounds.is_contiguous()
     dst = torch.empty(dst_h, dst_w, 3, device=src.device, dtype=torch.uint8)
-    rc = load().omc_resample_u8(_ptr(src), src.shape[0], src.shape[1], _ptr(dst), dst_h, dst_w, _ptr(coefs), _ptr(bounds),
+    rc = load().omc_resample_u8(src, src.shape[0], src.shape[1], dst, dst_h, dst_w, coefs, bounds,
                                 coefs.shape[1], 1 if vertical else 0, _stream())
     _check(rc, "omc_resample_u8")
     return dst
@@ -517,8 +488,8 @@ def anyres_pack(thumb, resized, target_w, target_h, paste_x, paste_y, crop, lut,
     assert lut.dtype == torch.float32 and lut.shape == (3, 256) and lut.is_contiguous()
     n = 1 + (target_w // crop) * (target_h // crop)
     out = torch.empty(n, 3, crop, crop, device=thumb.device, dtype=dtype)
-    rc = load().omc_anyres_pack(_ptr(thumb), _ptr(resized), resized.shape[1], resized.shape[0], target_w, target_h, paste_x,
-                                paste_y, crop, _ptr(lut), _ptr(out), 1 if dtype == torch.bfloat16 else 0, _stream())
+    rc = load().omc_anyres_pack(thumb, resized, resized.shape[1], resized.shape[0], target_w, target_h, paste_x,
+                                paste_y, crop, lut, out, 1 if dtype == torch.bfloat16 else 0, _stream())
     _check(rc, "omc_anyres_pack")
     return out
 
@@ -529,8 +500,8 @@ def attention(q, k, v, out, cu_seqlens: torch.Tensor, max_seqlen: int, Hq: int, 
     head_dim 128, or 64 (the InternViT-300M tower)."""
     _need_cuda(q, k, v, out, cu_seqlens)
     assert cu_seqlens.dtype == torch.int32
-    rc = load().omc_attention_fwd_hd(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), _ptr(out),
-                                     out.stride(0), _ptr(cu_seqlens), cu_seqlens.numel() - 1, max_seqlen,
+    rc = load().omc_attention_fwd_hd(q, q.stride(0), k, k.stride(0), v, v.stride(0), out,
+                                     out.stride(0), cu_seqlens, cu_seqlens.numel() - 1, max_seqlen,
                                      min(q.shape[0], k.shape[0], v.shape[0], out.shape[0]), Hq, Hkv, head_dim,
                                      1 if causal else 0, scale, _stream())
     _check(rc, "omc_attention_fwd")
@@ -548,8 +519,8 @@ def attention_set_impl(legacy):
 def rope_kv_store(qkv, pos, seq_ids, Hq, Hkv, inv_freq, kv_pool, block_table, page_size):
     _need_cuda(qkv, pos, inv_freq, kv_pool, block_table)
     assert pos.dtype == torch.int32 and block_table.dtype == torch.int32 and inv_freq.dtype == torch.float32
-    rc = load().omc_rope_kv_store(_ptr(qkv), qkv.stride(0), _ptr(pos), _ptr(seq_ids), qkv.shape[0], Hq, Hkv,
-                                  _ptr(inv_freq), _ptr(kv_pool), _ptr(block_table), block_table.shape[1], page_size,
+    rc = load().omc_rope_kv_store(qkv, qkv.stride(0), pos, seq_ids, qkv.shape[0], Hq, Hkv,
+                                  inv_freq, kv_pool, block_table, block_table.shape[1], page_size,
                                   _stream())
     _check(rc, "omc_rope_kv_store")
 
@@ -566,9 +537,9 @@ def decode_attn_workspace(B: int, Hq: int, Hkv: int, splits: int, device) -> tor
 def paged_decode_attn(qkv, inv_freq, kv_pool, block_table, page_size, ctx_lens, Hq, Hkv, splits, scale, out, workspace):
     _need_cuda(qkv, kv_pool, block_table, ctx_lens, out, workspace)
     assert ctx_lens.dtype == torch.int32 and block_table.dtype == torch.int32
-    rc = load().omc_paged_decode_attn(_ptr(qkv), qkv.stride(0), _ptr(inv_freq), _ptr(kv_pool), _ptr(block_table),
-                                      block_table.shape[1], page_size, _ptr(ctx_lens), qkv.shape[0], Hq, Hkv, splits,
-                                      scale, _ptr(out), out.stride(0), _ptr(workspace), _stream())
+    rc = load().omc_paged_decode_attn(qkv, qkv.stride(0), inv_freq, kv_pool, block_table,
+                                      block_table.shape[1], page_size, ctx_lens, qkv.shape[0], Hq, Hkv, splits,
+                                      scale, out, out.stride(0), workspace, _stream())
     _check(rc, "omc_paged_decode_attn")
     return out
 
@@ -579,7 +550,7 @@ def embed_lookup(ids: torch.Tensor, table: torch.Tensor, out: Optional[torch.Ten
     T, C = ids.numel(), table.shape[1]
     if out is None:
         out = torch.empty(T, C, device=table.device, dtype=torch.bfloat16)
-    rc = load().omc_embed_lookup(_ptr(ids), T, _ptr(table), C, _ptr(out), out.stride(0), table.shape[0], _stream())
+    rc = load().omc_embed_lookup(ids, T, table, C, out, out.stride(0), table.shape[0], _stream())
     _check(rc, "omc_embed_lookup")
     return out
 
@@ -599,8 +570,8 @@ def splice(ids: torch.Tensor, seq_offsets: torch.Tensor, table: torch.Tensor, fe
     seq_ids = torch.empty(T_capacity, device=dev, dtype=torch.int32)
     out_off = torch.empty(n_seq + 1, device=dev, dtype=torch.int32)
     ws = torch.empty(S + n_seq + 2, device=dev, dtype=torch.int32)
-    rc = load().omc_splice(_ptr(ids), _ptr(seq_offsets), n_seq, S, image_token, _ptr(table), _ptr(feats), n_img, L, C,
-                           max_len, _ptr(embeds), _ptr(pos_ids), _ptr(seq_ids), _ptr(out_off), _ptr(ws), T_capacity,
+    rc = load().omc_splice(ids, seq_offsets, n_seq, S, image_token, table, feats, n_img, L, C,
+                           max_len, embeds, pos_ids, seq_ids, out_off, ws, T_capacity,
                            table.shape[0], _stream())
     _check(rc, "omc_splice")
     return embeds, pos_ids, seq_ids, out_off
@@ -614,7 +585,7 @@ def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None, workspace: 
         out = torch.empty(B, device=logits.device, dtype=torch.int64)
     if workspace is None:
         workspace = torch.empty(128 * B, device=logits.device, dtype=torch.float32)
-    rc = load_dense().omc_argmax(_ptr(logits), logits.stride(0), B, V, _ptr(out), _ptr(workspace), _stream())
+    rc = load_dense().omc_argmax(logits, logits.stride(0), B, V, out, workspace, _stream())
     _check(rc, "omc_argmax")
     return out
 
@@ -864,22 +835,22 @@ def moe_block(h: torch.Tensor, xn: torch.Tensor, ws: MoeWorkspace, router_w: tor
         if ws.logits is None or ws.logits.shape[1] != W:
             ws.logits = torch.empty(ws.T, W, device=xn.device, dtype=torch.float32)
         gemm(xn, router_cat_w, out=ws.logits[:T], out_f32=True)
-        _check(L.omc_moe_select(_ptr(ws.logits), W, T, E, k, int(norm_topk), 1 if shared_gate_w is not None else 0,
-                                _ptr(ws.topk_ids), _ptr(ws.topk_w), _ptr(ws.shared_gate), _ptr(ws.counts), st), "omc_moe_select")
+        _check(L.omc_moe_select(ws.logits, W, T, E, k, int(norm_topk), 1 if shared_gate_w is not None else 0,
+                                ws.topk_ids, ws.topk_w, ws.shared_gate, ws.counts, st), "omc_moe_select")
     else:
         src = h if norm_w is not None else xn
-        _check(L.omc_moe_route(_ptr(src), src.stride(0), T, C, _ptr(norm_w), eps, _ptr(xn) if norm_w is not None else None,
-                               xn.stride(0), _ptr(router_w), _ptr(shared_gate_w), E, k, int(norm_topk), _ptr(ws.topk_ids),
-                               _ptr(ws.topk_w), _ptr(ws.shared_gate), _ptr(ws.counts), st), "omc_moe_route")
-    _check(L.omc_moe_plan_scatter(_ptr(ws.counts), E, ws.max_tiles, _ptr(ws.seg_start), _ptr(ws.cursor), _ptr(ws.tile_expert),
-                                  _ptr(xn), xn.stride(0), T, C, _ptr(ws.topk_ids), k, _ptr(ws.xperm), C, _ptr(ws.slot_of), st),
+        _check(L.omc_moe_route(src, src.stride(0), T, C, norm_w, eps, xn if norm_w is not None else None,
+                               xn.stride(0), router_w, shared_gate_w, E, k, int(norm_topk), ws.topk_ids,
+                               ws.topk_w, ws.shared_gate, ws.counts, st), "omc_moe_route")
+    _check(L.omc_moe_plan_scatter(ws.counts, E, ws.max_tiles, ws.seg_start, ws.cursor, ws.tile_expert,
+                                  xn, xn.stride(0), T, C, ws.topk_ids, k, ws.xperm, C, ws.slot_of, st),
            "omc_moe_plan_scatter")
     Mc = max_tiles * 128
     hint = min(max_tiles, T * k)
-    _check(L.omc_gemm_bf16_grouped(_ptr(ws.xperm), C, Mc, _ptr(experts_gate_up), C, E, I2, C, _ptr(ws.tile_expert), hint,
-                                   _ptr(ws.aperm), I2 // 2, EPI_SWIGLU, st), "omc_gemm_bf16_grouped")
-    _check(L.omc_gemm_bf16_grouped(_ptr(ws.aperm), I2 // 2, Mc, _ptr(experts_down), I2 // 2, E, C, I2 // 2,
-                                   _ptr(ws.tile_expert), hint, _ptr(ws.yperm), C, EPI_NONE, st), "omc_gemm_bf16_grouped")
+    _check(L.omc_gemm_bf16_grouped(ws.xperm, C, Mc, experts_gate_up, C, E, I2, C, ws.tile_expert, hint,
+                                   ws.aperm, I2 // 2, EPI_SWIGLU, st), "omc_gemm_bf16_grouped")
+    _check(L.omc_gemm_bf16_grouped(ws.aperm, I2 // 2, Mc, experts_down, I2 // 2, E, C, I2 // 2,
+                                   ws.tile_expert, hint, ws.yperm, C, EPI_NONE, st), "omc_gemm_bf16_grouped")
     add_launches(3)
     if defer_combine:
         return h
@@ -895,9 +866,9 @@ def moe_combine(h: torch.Tensor, ws: MoeWorkspace, shared_y: Optional[torch.Tens
     stream meanwhile): h += sum_j w_j * y[slot_j] + sigmoid_gate * shared_y."""
     T, C = h.shape
     k = ws.k
-    _check(load().omc_moe_combine(_ptr(h), h.stride(0), T, C, _ptr(ws.yperm), C, _ptr(ws.slot_of), _ptr(ws.topk_w), k,
-                                  _ptr(shared_y), shared_y.stride(0) if shared_y is not None else C, _ptr(ws.shared_gate),
-                                  _ptr(ssq_out), ssq_parts, _stream()), "omc_moe_combine")
+    _check(load().omc_moe_combine(h, h.stride(0), T, C, ws.yperm, C, ws.slot_of, ws.topk_w, k,
+                                  shared_y, shared_y.stride(0) if shared_y is not None else C, ws.shared_gate,
+                                  ssq_out, ssq_parts, _stream()), "omc_moe_combine")
     add_launches(1 if T * k <= 16 else 2)
     return h
 
@@ -969,8 +940,8 @@ class VitForward:
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.empty(need, device=pixels.device, dtype=torch.uint8)
         out = torch.empty(n, self.tokens, self.desc.proj_hidden, device=pixels.device, dtype=torch.bfloat16)
-        rc = load().omc_vit_forward(ctypes.byref(self.desc), _ptr(pixels), 1 if pixels.dtype == torch.float32 else 0, n,
-                                    self._ws.data_ptr(), _ptr(out), _stream())
+        rc = load().omc_vit_forward(ctypes.byref(self.desc), pixels, 1 if pixels.dtype == torch.float32 else 0, n,
+                                    self._ws.data_ptr(), out, _stream())
         per_layer = 7 + (2 if self.desc.qk_norm else 0) - (2 + (1 if self.desc.qk_norm else 0)) * self.desc.norm_folded
         add_launches(4 + self.desc.norm_folded + self.desc.n_layers * per_layer + 3 - 1)
         _check(rc, "omc_vit_forward")
@@ -998,8 +969,8 @@ def decoder_prefill(layers, final_norm, lm_head, dims, eps, scale, inv_freq, emb
     d.kv_pool, d.kv_layer_stride, d.block_table = kv_pool.data_ptr(), kv_pool.stride(0), block_table.data_ptr()
     ws = torch.empty(load().omc_decoder_prefill_workspace_bytes(ctypes.byref(d), T, n_seq), device=embeds.device, dtype=torch.uint8)
     logits = torch.empty(n_seq, dims[4], device=embeds.device, dtype=torch.float32) if last_rows is not None else None
-    rc = load().omc_decoder_prefill(ctypes.byref(d), _ptr(inv_freq), _ptr(embeds), _ptr(pos_ids), _ptr(seq_ids), _ptr(cu_seqlens),
-                                    n_seq, T, max_len, _ptr(last_rows), ws.data_ptr(), _ptr(logits), 1 if folded is not None else 0,
+    rc = load().omc_decoder_prefill(ctypes.byref(d), inv_freq, embeds, pos_ids, seq_ids, cu_seqlens,
+                                    n_seq, T, max_len, last_rows, ws.data_ptr(), logits, 1 if folded is not None else 0,
                                     _stream())
     add_launches((6 if folded is not None else 8) * n_layers + (1 if folded is not None else 0) + (3 if last_rows is not None else 0) - 1)
     _check(rc, "omc_decoder_prefill")

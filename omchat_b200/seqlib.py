@@ -13,7 +13,8 @@ from typing import Optional
 import torch
 
 from . import lib as _core
-from .lib import OmcError, _need_cuda, _ptr, _stream
+from . import native
+from .lib import OmcError, _need_cuda, _stream
 
 _P, _I, _L, _F = c_void_p, c_int, c_longlong, c_float
 DT_F32, DT_BF16 = 0, 1
@@ -77,7 +78,7 @@ SIGNATURES = {
 _lib = None
 
 
-def load() -> ctypes.CDLL:
+def load() -> native.Entries:
     global _lib
     if _lib is not None:
         return _lib
@@ -87,13 +88,8 @@ def load() -> ctypes.CDLL:
         path = str(build.ensure("seq"))
     if not os.path.exists(path):
         raise OmcError(f"{path} not found (there is no CPU fallback)")
-    lib = ctypes.CDLL(path)
-    for name, (res, args) in SIGNATURES.items():
-        fn = getattr(lib, name)
-        fn.restype = res
-        fn.argtypes = args
-    _lib = lib
-    return lib
+    _lib = native.Entries(ctypes.CDLL(path), SIGNATURES)
+    return _lib
 
 
 def _check(rc: int, what: str):
@@ -139,16 +135,16 @@ def linear(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, *, M: Optional[i
     if gate is not None:
         _need_cuda(gate)
         assert gate.stride(1) == 1 and gate.shape == (M, batch * N) and bias is None and tile_group is None
-        rc = load().omc_linear_gate(_ptr(x), _dt(x), ldx, sx, _ptr(w), _dt(w), ldw, sw, _ptr(out), _dt(out), ldy, sy, M, N, K, batch,
-                                    alpha, act, _ptr(gate), _dt(gate), gate.stride(0), N, _stream())
+        rc = load().omc_linear_gate(x, _dt(x), ldx, sx, w, _dt(w), ldw, sw, out, _dt(out), ldy, sy, M, N, K, batch,
+                                    alpha, act, gate, _dt(gate), gate.stride(0), N, _stream())
     elif bias is not None:
         _need_cuda(bias)
         assert bias.dtype == w.dtype and bias.numel() == N and batch == 1
-        rc = load().omc_linear_bias(_ptr(x), _dt(x), ldx, sx, _ptr(w), _dt(w), ldw, sw, _ptr(out), _dt(out), ldy, sy, M, N, K, batch,
-                                    alpha, act, _ptr(tile_group), group_stride, _ptr(bias), 0, _stream())
+        rc = load().omc_linear_bias(x, _dt(x), ldx, sx, w, _dt(w), ldw, sw, out, _dt(out), ldy, sy, M, N, K, batch,
+                                    alpha, act, tile_group, group_stride, bias, 0, _stream())
     else:
-        rc = load().omc_linear(_ptr(x), _dt(x), ldx, sx, _ptr(w), _dt(w), ldw, sw, _ptr(out), _dt(out), ldy, sy, M, N, K, batch,
-                               alpha, act, _ptr(tile_group), group_stride, _stream())
+        rc = load().omc_linear(x, _dt(x), ldx, sx, w, _dt(w), ldw, sw, out, _dt(out), ldy, sy, M, N, K, batch,
+                               alpha, act, tile_group, group_stride, _stream())
     _check(rc, "omc_linear")
     return out
 
@@ -157,8 +153,8 @@ def embed_scale(ids: torch.Tensor, table: torch.Tensor, scale: float, h32: torch
     _need_cuda(ids, table, h32, xb)
     assert ids.dtype == torch.int32 and h32.dtype == torch.float32 and table.is_contiguous()
     T, C = ids.numel(), table.shape[1]
-    rc = load().omc_embed_scale(_ptr(ids), T, _ptr(table), _dt(table), C, table.shape[0], scale, _ptr(h32), h32.stride(0),
-                                _ptr(xb), _dt(xb), xb.stride(0) if xb is not None else 0, _stream())
+    rc = load().omc_embed_scale(ids, T, table, _dt(table), C, table.shape[0], scale, h32, h32.stride(0),
+                                xb, _dt(xb), xb.stride(0) if xb is not None else 0, _stream())
     _check(rc, "omc_embed_scale")
 
 
@@ -174,7 +170,7 @@ def embed_sinusoid(ids: torch.Tensor, pos: torch.Tensor, table: torch.Tensor, sc
     T, C = ids.numel(), table.shape[1]
     assert ids.dtype == torch.int32 and pos.dtype == torch.int32 and h32.dtype == torch.float32 and table.is_contiguous()
     assert freq.dtype == torch.float64 and freq.is_contiguous() and freq.numel() >= (C + 1) // 2
-    rc = load().omc_embed_sinusoid(_ptr(ids), _ptr(pos), T, _ptr(table), _dt(table), C, table.shape[0], scale, _ptr(freq), _ptr(h32),
+    rc = load().omc_embed_sinusoid(ids, pos, T, table, _dt(table), C, table.shape[0], scale, freq, h32,
                                    h32.stride(0), _stream())
     _check(rc, "omc_embed_sinusoid")
 
@@ -184,7 +180,7 @@ def rms_rows(x: torch.Tensor, w: Optional[torch.Tensor], eps: float, out: torch.
     _need_cuda(x, w, out)
     assert x.dtype == torch.float32 and x.stride(1) == 1 and out.stride(1) == 1
     n = x.shape[1] if n is None else n
-    rc = load().omc_rms_rows(_ptr(x), x.stride(0), _ptr(w), _dt(w), 1 if one_plus else 0, eps, _ptr(out), _dt(out), out.stride(0),
+    rc = load().omc_rms_rows(x, x.stride(0), w, _dt(w), 1 if one_plus else 0, eps, out, _dt(out), out.stride(0),
                              x.shape[0], n, _stream())
     _check(rc, "omc_rms_rows")
     return out
@@ -194,7 +190,7 @@ def norm_residual(y: torch.Tensor, w: torch.Tensor, eps: float, h32: torch.Tenso
     """h32 += y / rms(y) * (1 + w); xb = round(h32)."""
     _need_cuda(y, w, h32, xb)
     assert y.dtype == torch.float32 and h32.dtype == torch.float32
-    rc = load().omc_norm_residual(_ptr(y), y.stride(0), _ptr(w), _dt(w), eps, _ptr(h32), h32.stride(0), _ptr(xb), _dt(xb),
+    rc = load().omc_norm_residual(y, y.stride(0), w, _dt(w), eps, h32, h32.stride(0), xb, _dt(xb),
                                   xb.stride(0) if xb is not None else 0, y.shape[0], y.shape[1], _stream())
     _check(rc, "omc_norm_residual")
 
@@ -204,8 +200,8 @@ def latent_kv_store(dkv: torch.Tensor, r: int, dr: int, w: torch.Tensor, eps: fl
     _need_cuda(dkv, w, cs, pos, slot, block_table, pool)
     assert dkv.dtype == torch.float32 and cs.dtype == torch.float32 and pos.dtype == torch.int32 and slot.dtype == torch.int32
     assert block_table.dtype == torch.int32 and block_table.is_contiguous() and pool.is_contiguous() and pool.shape[-1] == r + dr
-    rc = load().omc_latent_kv_store(_ptr(dkv), dkv.stride(0), dkv.shape[0], r, dr, _ptr(w), _dt(w), eps, _ptr(cs), rot_dims,
-                                    _ptr(pos), _ptr(slot), _ptr(block_table), block_table.shape[1], page_size, _ptr(pool),
+    rc = load().omc_latent_kv_store(dkv, dkv.stride(0), dkv.shape[0], r, dr, w, _dt(w), eps, cs, rot_dims,
+                                    pos, slot, block_table, block_table.shape[1], page_size, pool,
                                     _dt(pool), _stream())
     _check(rc, "omc_latent_kv_store")
 
@@ -219,9 +215,9 @@ def latent_rope_store(dkv: Optional[torch.Tensor], r: int, dr: int, w, eps: floa
     if dkv is not None:
         assert dkv.dtype == torch.float32 and dkv.stride(1) == 1 and w.dtype == pool.dtype == qcat.dtype
         assert block_table.is_contiguous() and pool.is_contiguous() and pool.shape[-1] == r + dr
-    rc = load().omc_latent_rope_store(_ptr(dkv), dkv.stride(0) if dkv is not None else 0, q.shape[0], r, dr, _ptr(w), eps, _ptr(cs), rot_dims,
-                                      1 if rot_halves else 0, _ptr(pos), _ptr(slot), _ptr(block_table), block_table.shape[1], page_size, _ptr(pool), _ptr(q), _dt(q), q.stride(0), H, dn,
-                                      _ptr(qcat), _ptr(qn), _dt(qcat), _stream())
+    rc = load().omc_latent_rope_store(dkv, dkv.stride(0) if dkv is not None else 0, q.shape[0], r, dr, w, eps, cs, rot_dims,
+                                      1 if rot_halves else 0, pos, slot, block_table, block_table.shape[1], page_size, pool, q, _dt(q), q.stride(0), H, dn,
+                                      qcat, qn, _dt(qcat), _stream())
     _check(rc, "omc_latent_rope_store")
 
 
@@ -230,9 +226,9 @@ def moe_plan_scatter_small(counts, experts: int, tile: int, max_tiles: int, seg_
     """moe_plan_tiles + moe_scatter_rows as one single-CTA launch (steps of a few rows). row_w as in moe_scatter_rows."""
     _need_cuda(counts, seg_start, tile_group, x, ids, slot_of, xs, row_w)
     assert x.dtype == xs.dtype
-    rc = load().omc_moe_plan_scatter_small(_ptr(counts), experts, tile, max_tiles, _ptr(seg_start), _ptr(tile_group), _ptr(x), _dt(x),
-                                           x.stride(0), x.shape[0], x.shape[1], _ptr(ids), top, _ptr(slot_of), _ptr(xs), xs.stride(0),
-                                           _ptr(row_w), _stream())
+    rc = load().omc_moe_plan_scatter_small(counts, experts, tile, max_tiles, seg_start, tile_group, x, _dt(x),
+                                           x.stride(0), x.shape[0], x.shape[1], ids, top, slot_of, xs, xs.stride(0),
+                                           row_w, _stream())
     _check(rc, "omc_moe_plan_scatter_small")
 
 
@@ -240,7 +236,7 @@ def rotary_q(q32: torch.Tensor, H: int, dn: int, dr: int, cs: torch.Tensor, rot_
              r: int):
     _need_cuda(q32, cs, pos, qcat)
     assert qcat.is_contiguous() and qcat.shape[-1] == r + dr and q32.stride(1) == 1
-    rc = load().omc_rotary_q(_ptr(q32), _dt(q32), q32.stride(0), q32.shape[0], H, dn, dr, _ptr(cs), rot_dims, _ptr(pos), _ptr(qcat),
+    rc = load().omc_rotary_q(q32, _dt(q32), q32.stride(0), q32.shape[0], H, dn, dr, cs, rot_dims, pos, qcat,
                              _dt(qcat), r, _stream())
     _check(rc, "omc_rotary_q")
 
@@ -258,9 +254,9 @@ def latent_attn(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, block_t
     T, H = qcat.shape[0], qcat.shape[1]
     assert out.dtype == torch.float32 and out.is_contiguous() and qcat.is_contiguous()
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() == H)
-    rc = load().omc_latent_attn(_ptr(qcat), _dt(qcat), T, H, r, dr, _ptr(pool), _dt(pool), _ptr(block_table), block_table.shape[1],
-                                page_size, _ptr(pos), _ptr(slot), _ptr(sink), window, _ptr(gate), gate.stride(0) if gate is not None else 0, scale,
-                                _ptr(out), _stream())
+    rc = load().omc_latent_attn(qcat, _dt(qcat), T, H, r, dr, pool, _dt(pool), block_table, block_table.shape[1],
+                                page_size, pos, slot, sink, window, gate, gate.stride(0) if gate is not None else 0, scale,
+                                out, _stream())
     _check(rc, "omc_latent_attn")
     return out
 
@@ -385,8 +381,8 @@ class DecodeAttnPlan:
         return max(1, min(bucket // 256, 148 // B, LatentAttnPlan.MAX_PARTS))
 
     def fill(self, pos: torch.Tensor, slot: torch.Tensor):
-        rc = load().omc_latent_decode_items(_ptr(pos), _ptr(slot), self.B, self.H, self.parts, self.window, _ptr(self.items),
-                                            _ptr(self.merges), _stream())
+        rc = load().omc_latent_decode_items(pos, slot, self.B, self.H, self.parts, self.window, self.items,
+                                            self.merges, _stream())
         _check(rc, "omc_latent_decode_items")
 
 
@@ -411,9 +407,9 @@ def latent_attn_mma(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, blo
             ws = torch.empty(need, device=qcat.device, dtype=torch.float32)
             _mma_ws[key] = ws
         ws_o, ws_ml = ws[:plan.n_parts * MMA_ROWS * r], ws[plan.n_parts * MMA_ROWS * r:]
-    rc = load().omc_latent_attn_mma_pool(_ptr(qcat), T, H, r, dr, _ptr(pool), pool.numel() // (r + dr), _ptr(block_table), block_table.shape[1], page_size,
-                                         _ptr(plan.items), plan.n_items, plan.max_rows, _ptr(plan.merges), plan.n_merges, _ptr(sink), window, _ptr(gate),
-                                         gate.stride(0) if gate is not None else 0, scale, _ptr(out), _dt(out), _ptr(ws_o), _ptr(ws_ml), _stream())
+    rc = load().omc_latent_attn_mma_pool(qcat, T, H, r, dr, pool, pool.numel() // (r + dr), block_table, block_table.shape[1], page_size,
+                                         plan.items, plan.n_items, plan.max_rows, plan.merges, plan.n_merges, sink, window, gate,
+                                         gate.stride(0) if gate is not None else 0, scale, out, _dt(out), ws_o, ws_ml, _stream())
     _check(rc, "omc_latent_attn_mma")
     if plan.n_merges:
         _core.add_launches(1)
@@ -431,8 +427,8 @@ def router_topk(z: torch.Tensor, e_tot: int, experts: int, top: int, correction:
     assert z.dtype == torch.float32 and ids.dtype == torch.int32 and w.dtype == torch.float32 and counts.dtype == torch.int32
     assert correction is None or correction.dtype == torch.float32
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == e_tot)
-    rc = load().omc_router_topk(_ptr(z), z.stride(0), z.shape[0], e_tot, experts, top, _ptr(correction), _ptr(bias), 1 if renorm else 0, score,
-                                groups, keep, scale, 1 if has_gate else 0, _ptr(ids), _ptr(w), _ptr(gate), _ptr(counts), _stream())
+    rc = load().omc_router_topk(z, z.stride(0), z.shape[0], e_tot, experts, top, correction, bias, 1 if renorm else 0, score,
+                                groups, keep, scale, 1 if has_gate else 0, ids, w, gate, counts, _stream())
     _check(rc, "omc_router_topk")
 
 
@@ -443,7 +439,7 @@ def moe_max_tiles(T: int, top: int, experts: int, tile: int = LINEAR_TILE) -> in
 
 def moe_plan_tiles(counts, experts: int, tile: int, max_tiles: int, seg_start, cursor, tile_group):
     _need_cuda(counts, seg_start, cursor, tile_group)
-    rc = load().omc_moe_plan_tiles(_ptr(counts), experts, tile, max_tiles, _ptr(seg_start), _ptr(cursor), _ptr(tile_group), _stream())
+    rc = load().omc_moe_plan_tiles(counts, experts, tile, max_tiles, seg_start, cursor, tile_group, _stream())
     _check(rc, "omc_moe_plan_tiles")
 
 
@@ -452,8 +448,8 @@ def moe_scatter_rows(x, ids, top: int, experts: int, seg_start, cursor, slot_of,
     _need_cuda(x, ids, seg_start, cursor, slot_of, xs, row_w)
     assert row_w is None or (row_w.dtype == torch.float32 and row_w.is_contiguous())
     assert x.dtype == xs.dtype
-    rc = load().omc_moe_scatter_rows(_ptr(x), _dt(x), x.stride(0), x.shape[0], x.shape[1], _ptr(ids), top, experts, _ptr(seg_start),
-                                     _ptr(cursor), _ptr(slot_of), _ptr(xs), xs.stride(0), _ptr(row_w), _stream())
+    rc = load().omc_moe_scatter_rows(x, _dt(x), x.stride(0), x.shape[0], x.shape[1], ids, top, experts, seg_start,
+                                     cursor, slot_of, xs, xs.stride(0), row_w, _stream())
     _check(rc, "omc_moe_scatter_rows")
 
 
@@ -468,10 +464,10 @@ def moe_combine_depth(ys: Optional[torch.Tensor], slot_of, w: Optional[torch.Ten
     assert x.dtype == torch.float32 and out.dtype == torch.float32 and x.stride(1) == 1 and out.stride(1) == 1
     assert streams is None or (streams.dtype == torch.float32 and streams.stride(2) == 1 and streams.shape[0] >= n_streams)
     assert coef is None or (coef.is_contiguous() and coef.numel() >= n_streams)
-    rc = load().omc_moe_combine_depth(_ptr(ys), ys.stride(0) if ys is not None else 0, _ptr(slot_of), _ptr(w), top, _ptr(x), x.stride(0),
-                                      _ptr(y1), y1.stride(0) if y1 is not None else 0, a1, _ptr(y2), y2.stride(0) if y2 is not None else 0, a2,
-                                      mult, _ptr(streams), streams.stride(0) if streams is not None else 0,
-                                      streams.stride(1) if streams is not None else 0, n_streams, _ptr(coef), _dt(coef), _ptr(out),
+    rc = load().omc_moe_combine_depth(ys, ys.stride(0) if ys is not None else 0, slot_of, w, top, x, x.stride(0),
+                                      y1, y1.stride(0) if y1 is not None else 0, a1, y2, y2.stride(0) if y2 is not None else 0, a2,
+                                      mult, streams, streams.stride(0) if streams is not None else 0,
+                                      streams.stride(1) if streams is not None else 0, n_streams, coef, _dt(coef), out,
                                       out.stride(0), x.shape[0], x.shape[1], _stream())
     _check(rc, "omc_moe_combine_depth")
 
@@ -481,9 +477,9 @@ def moe_combine_norm(ys: Optional[torch.Tensor], slot_of, w, top: int, gate, ysh
     """w_next: xb receives h32 / rms(h32) * (1 + w_next), the next sublayer's normed input, instead of the rounded h32."""
     _need_cuda(ys, slot_of, w, gate, ysh, nw, h32, xb, w_next)
     assert w_next is None or w_next.dtype == nw.dtype
-    rc = load().omc_moe_combine_norm(_ptr(ys), ys.stride(0) if ys is not None else 0, _ptr(slot_of), _ptr(w), top, _ptr(gate),
-                                     _ptr(ysh), ysh.stride(0) if ysh is not None else 0, _ptr(nw), _dt(nw), eps, _ptr(h32),
-                                     h32.stride(0), _ptr(w_next), _ptr(xb), _dt(xb), xb.stride(0) if xb is not None else 0, h32.shape[0],
+    rc = load().omc_moe_combine_norm(ys, ys.stride(0) if ys is not None else 0, slot_of, w, top, gate,
+                                     ysh, ysh.stride(0) if ysh is not None else 0, nw, _dt(nw), eps, h32,
+                                     h32.stride(0), w_next, xb, _dt(xb), xb.stride(0) if xb is not None else 0, h32.shape[0],
                                      h32.shape[1], _stream())
     _check(rc, "omc_moe_combine_norm")
 
@@ -496,8 +492,8 @@ def post_norm_residual(y1: torch.Tensor, w_post: torch.Tensor, eps: float, mult:
     xb = h32 / rms(h32) * (1 + w_next) (w_next None: the rounded h32)."""
     _need_cuda(y1, y2, wa, wb, w_post, h32, w_next, xb)
     assert y1.dtype == torch.float32 and h32.dtype == torch.float32 and y1.stride(1) == 1 and (y2 is None or y2.dtype == torch.float32)
-    rc = load().omc_post_norm_residual(_ptr(y1), y1.stride(0), _ptr(wa), _ptr(y2), y2.stride(0) if y2 is not None else 0, _ptr(wb),
-                                       _ptr(w_post), _dt(w_post), eps, mult, _ptr(h32), h32.stride(0), _ptr(w_next), _ptr(xb), _dt(xb),
+    rc = load().omc_post_norm_residual(y1, y1.stride(0), wa, y2, y2.stride(0) if y2 is not None else 0, wb,
+                                       w_post, _dt(w_post), eps, mult, h32, h32.stride(0), w_next, xb, _dt(xb),
                                        xb.stride(0) if xb is not None else 0, h32.shape[0], h32.shape[1], _stream())
     _check(rc, "omc_post_norm_residual")
 
@@ -516,8 +512,8 @@ def ln_residual(x: torch.Tensor, alpha: float, nw: torch.Tensor, nb: torch.Tenso
 
     def ld(t):
         return t.stride(0) if t is not None else 0
-    rc = load().omc_ln_residual(_ptr(x), ld(x), alpha, _ptr(y), ld(y), _ptr(ys), ld(ys), _ptr(slot_of), _ptr(w), top, _ptr(nw), _ptr(nb), _dt(nw), eps,
-                                _ptr(x_out), ld(x_out), _ptr(xb), _dt(xb), ld(xb), x.shape[0], C, _stream())
+    rc = load().omc_ln_residual(x, ld(x), alpha, y, ld(y), ys, ld(ys), slot_of, w, top, nw, nb, _dt(nw), eps,
+                                x_out, ld(x_out), xb, _dt(xb), ld(xb), x.shape[0], C, _stream())
     _check(rc, "omc_ln_residual")
     return x_out if xb is None else xb
 
@@ -535,8 +531,8 @@ def rms_residual(x: torch.Tensor, nw: Optional[torch.Tensor], eps: float, *, y: 
 
     def ld(t):
         return t.stride(0) if t is not None else 0
-    rc = load().omc_rms_residual(_ptr(x), ld(x), _ptr(y), ld(y), _ptr(ys), ld(ys), _ptr(slot_of), _ptr(w), top, _ptr(nw), _dt(nw), eps, _ptr(x_out),
-                                 ld(x_out), _ptr(xb), _dt(xb), ld(xb), x.shape[0], C, _stream())
+    rc = load().omc_rms_residual(x, ld(x), y, ld(y), ys, ld(ys), slot_of, w, top, nw, _dt(nw), eps, x_out,
+                                 ld(x_out), xb, _dt(xb), ld(xb), x.shape[0], C, _stream())
     _check(rc, "omc_rms_residual")
     return x_out if xb is None else xb
 
@@ -551,8 +547,8 @@ def embed_bigram(ids: torch.Tensor, pos: torch.Tensor, slot: torch.Tensor, table
     assert ids.dtype == pos.dtype == slot.dtype == prev.dtype == torch.int32 and h32.dtype == torch.float32 and table.dtype == bigram.dtype
     assert table.is_contiguous() and bigram.is_contiguous() and bigram.shape[1] == C and prev.is_contiguous()
     assert xb is None or (nw.dtype == table.dtype and nw.numel() == C and xb.stride(1) == 1)
-    rc = load().omc_embed_bigram(_ptr(ids), _ptr(pos), _ptr(slot), T, _ptr(table), _dt(table), C, table.shape[0], _ptr(bigram), buckets,
-                                 mul_prev % buckets, mul_cur % buckets, _ptr(prev), _ptr(nw), eps, _ptr(h32), h32.stride(0), _ptr(xb), _dt(xb),
+    rc = load().omc_embed_bigram(ids, pos, slot, T, table, _dt(table), C, table.shape[0], bigram, buckets,
+                                 mul_prev % buckets, mul_cur % buckets, prev, nw, eps, h32, h32.stride(0), xb, _dt(xb),
                                  xb.stride(0) if xb is not None else 0, 1 if single_rows else 0, _stream())
     _check(rc, "omc_embed_bigram")
     if not single_rows:
@@ -565,8 +561,8 @@ def glu_mul(z: torch.Tensor, n: int, act: int, out: torch.Tensor, limit: float =
     out = g * sigmoid(slope * g) * (u + shift). tile_group: rows of `tile`-row tiles that no expert uses are skipped."""
     _need_cuda(z, out, tile_group)
     assert z.stride(1) == 1 and out.stride(1) == 1 and z.shape[1] >= 2 * n
-    rc = load().omc_glu_mul(_ptr(z), _dt(z), z.stride(0), z.shape[0], n, act, limit, slope, shift, _ptr(out), _dt(out), out.stride(0),
-                            _ptr(tile_group), tile, _stream())
+    rc = load().omc_glu_mul(z, _dt(z), z.stride(0), z.shape[0], n, act, limit, slope, shift, out, _dt(out), out.stride(0),
+                            tile_group, tile, _stream())
     _check(rc, "omc_glu_mul")
     return out
 
@@ -589,8 +585,8 @@ def causal_conv_silu(x: torch.Tensor, w: torch.Tensor, pos: torch.Tensor, slot: 
     assert bias is None or (bias.dtype == w.dtype and bias.numel() == ch and bias.is_contiguous())
     assert pos.dtype == torch.int32 and slot.dtype == torch.int32
     assert taps == 1 or (state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (taps - 1, ch))
-    rc = load().omc_causal_conv(_ptr(x), x.stride(0), x.shape[0], ch, _ptr(w), _ptr(bias), _dt(w), taps, _ptr(pos), _ptr(slot), _ptr(state),
-                                _ptr(y), _dt(y), y.stride(0), act, unit_channels, unit_group, unit_eps, scaled_channels, unit_mult,
+    rc = load().omc_causal_conv(x, x.stride(0), x.shape[0], ch, w, bias, _dt(w), taps, pos, slot, state,
+                                y, _dt(y), y.stride(0), act, unit_channels, unit_group, unit_eps, scaled_channels, unit_mult,
                                 1 if single_rows else 0, _stream())
     _check(rc, "omc_causal_conv")
     if taps > 1 and not single_rows:
@@ -615,9 +611,9 @@ def conv_qk_norm_kv_store(x: torch.Tensor, w: torch.Tensor, pos, slot, state: Op
     assert taps == 1 or (state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (taps - 1, ch))
     assert pool.is_contiguous() and pool.shape[-1] == ch - nq and pool.dtype == q_out.dtype
     assert wq.dtype == wk.dtype == w.dtype and wq.numel() == group and wk.numel() == group
-    rc = load().omc_conv_qk_norm_kv_store(_ptr(x), x.stride(0), x.shape[0], ch, _ptr(w), _dt(w), taps, _ptr(pos), _ptr(slot), _ptr(state),
-                                          nq, nk, group, _ptr(wq), _ptr(wk), eps, _ptr(block_table), block_table.shape[1], page_size,
-                                          _ptr(pool), _ptr(q_out), q_out.stride(0), _dt(pool), 1 if single_rows else 0, _stream())
+    rc = load().omc_conv_qk_norm_kv_store(x, x.stride(0), x.shape[0], ch, w, _dt(w), taps, pos, slot, state,
+                                          nq, nk, group, wq, wk, eps, block_table, block_table.shape[1], page_size,
+                                          pool, q_out, q_out.stride(0), _dt(pool), 1 if single_rows else 0, _stream())
     _check(rc, "omc_conv_qk_norm_kv_store")
     if taps > 1 and not single_rows:
         _core.add_launches(1)
@@ -646,10 +642,10 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
         mode = DECAY_GIVEN_MINUS_ONE if decay_given else DECAY_SIGMOID_POW
     if step_size:
         mode = DECAY_STEP
-    rc = load().omc_linear_state_scan(_ptr(q), q.stride(0), _ptr(k), k.stride(0), _ptr(v), v.stride(0), 1 if silu_in else 0, mode,
-                                      _ptr(decay_const), _ptr(a), a.stride(0) if a is not None else 0, _ptr(A_log), _ptr(dt_bias),
-                                      _ptr(D), _ptr(beta), beta.stride(0) if beta is not None else 0, _ptr(state), _ptr(out), out.stride(0),
-                                      _ptr(row_begin), portions, _ptr(pos), _ptr(slot), q.shape[0], H, G, dim, vdim,
+    rc = load().omc_linear_state_scan(q, q.stride(0), k, k.stride(0), v, v.stride(0), 1 if silu_in else 0, mode,
+                                      decay_const, a, a.stride(0) if a is not None else 0, A_log, dt_bias,
+                                      D, beta, beta.stride(0) if beta is not None else 0, state, out, out.stride(0),
+                                      row_begin, portions, pos, slot, q.shape[0], H, G, dim, vdim,
                                       float(sigmoid_pow or 0.0), out_scale, _stream())
     _check(rc, "omc_linear_state_scan")
     return out
@@ -660,8 +656,8 @@ def gated_rms_rows(x: torch.Tensor, groups: int, n: int, w: torch.Tensor, eps: f
     _need_cuda(x, w, gate, out)
     assert x.dtype == torch.float32 and x.stride(1) == 1 and out.stride(1) == 1 and w.numel() == n
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
-    rc = load().omc_gated_rms_rows(_ptr(x), x.stride(0), x.shape[0], groups, n, _ptr(w), _dt(w), eps, _ptr(gate),
-                                   gate.stride(0) if gate is not None else 0, gate_act, _ptr(out), _dt(out), out.stride(0), _stream())
+    rc = load().omc_gated_rms_rows(x, x.stride(0), x.shape[0], groups, n, w, _dt(w), eps, gate,
+                                   gate.stride(0) if gate is not None else 0, gate_act, out, _dt(out), out.stride(0), _stream())
     _check(rc, "omc_gated_rms_rows")
     return out
 
@@ -671,8 +667,8 @@ def gate_rms_rows(x: torch.Tensor, groups: int, w: torch.Tensor, eps: float, gat
     _need_cuda(x, w, gate, out)
     n = w.numel() // groups
     assert x.dtype == torch.float32 and x.stride(1) == gate.stride(1) == out.stride(1) == 1 and w.numel() == groups * n
-    rc = load().omc_gate_rms_rows(_ptr(x), x.stride(0), x.shape[0], groups, n, _ptr(w), _dt(w), eps, _ptr(gate), _dt(gate), gate.stride(0), gate_act,
-                                  _ptr(out), _dt(out), out.stride(0), _stream())
+    rc = load().omc_gate_rms_rows(x, x.stride(0), x.shape[0], groups, n, w, _dt(w), eps, gate, _dt(gate), gate.stride(0), gate_act,
+                                  out, _dt(out), out.stride(0), _stream())
     _check(rc, "omc_gate_rms_rows")
     return out
 
@@ -691,9 +687,9 @@ def qk_norm_kv_store(q: torch.Tensor, wq: torch.Tensor, k: torch.Tensor, wk: tor
     assert q.dtype == k.dtype == v.dtype == torch.float32 and q.stride(1) == k.stride(1) == v.stride(1) == 1
     assert pool.is_contiguous() and pool.shape[-1] == nk + nv and pool.dtype == q_out.dtype and wq.dtype == wk.dtype
     assert block_table.dtype == torch.int32 and block_table.is_contiguous() and q_out.stride(1) == 1
-    rc = load().omc_qk_norm_kv_store(_ptr(q), q.stride(0), nq, group, _ptr(wq), _ptr(k), k.stride(0), nk, group, _ptr(wk), _dt(wq), _ptr(v), v.stride(0),
-                                     nv, eps, _ptr(cs), head, rot_dims, 1 if rot_halves else 0, q.shape[0], _ptr(pos), _ptr(slot), _ptr(block_table), block_table.shape[1], page_size,
-                                     _ptr(pool), _ptr(q_out), q_out.stride(0), _dt(pool), _stream())
+    rc = load().omc_qk_norm_kv_store(q, q.stride(0), nq, group, wq, k, k.stride(0), nk, group, wk, _dt(wq), v, v.stride(0),
+                                     nv, eps, cs, head, rot_dims, 1 if rot_halves else 0, q.shape[0], pos, slot, block_table, block_table.shape[1], page_size,
+                                     pool, q_out, q_out.stride(0), _dt(pool), _stream())
     _check(rc, "omc_qk_norm_kv_store")
 
 
@@ -711,9 +707,9 @@ def window_attn(q: torch.Tensor, H: int, G: int, d: int, dv: int, pool: torch.Te
     assert q.dtype == pool.dtype and q.stride(1) == 1 and out.stride(1) == 1 and pool.is_contiguous()
     assert pool.shape[-1] == G * (maps * d + dv)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape == (window, H))
-    rc = load().omc_window_attn(_ptr(q), q.stride(0), q.shape[0], H, G, d, dv, maps, _ptr(pool), _dt(pool), _ptr(block_table),
-                                block_table.shape[1], page_size, _ptr(pos), _ptr(slot), window, chunk, keep_first, scale, softcap,
-                                _ptr(dist_bias), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0, gate_act, 1 if gate_heads else 0, _ptr(out),
+    rc = load().omc_window_attn(q, q.stride(0), q.shape[0], H, G, d, dv, maps, pool, _dt(pool), block_table,
+                                block_table.shape[1], page_size, pos, slot, window, chunk, keep_first, scale, softcap,
+                                dist_bias, sink, gate, gate.stride(0) if gate is not None else 0, gate_act, 1 if gate_heads else 0, out,
                                 _dt(out), out.stride(0), _stream())
     _check(rc, "omc_window_attn")
     return out
@@ -759,10 +755,10 @@ def window_attn_mma(q: torch.Tensor, H: int, G: int, d: int, dv: int, pool: torc
     assert pool.is_contiguous() and pool.shape[-1] == G * (maps * d + dv) and block_table.is_contiguous()
     assert items is None or (items.dtype == torch.int32 and items.is_contiguous() and items.shape[1] == 4)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape == (window, H))
-    rc = load().omc_window_attn_mma(_ptr(q), q.stride(0), q.shape[0], H, G, d, dv, maps, _ptr(pool), _ptr(block_table), block_table.shape[1],
-                                    page_size, _ptr(items), items.shape[0] if items is not None else 0, _ptr(pos), _ptr(slot), window, chunk,
-                                    keep_first, scale, softcap, _ptr(dist_bias), _ptr(sink), _ptr(gate), gate.stride(0) if gate is not None else 0,
-                                    gate_act, 1 if gate_heads else 0, _ptr(out), _dt(out), out.stride(0), _stream())
+    rc = load().omc_window_attn_mma(q, q.stride(0), q.shape[0], H, G, d, dv, maps, pool, block_table, block_table.shape[1],
+                                    page_size, items, items.shape[0] if items is not None else 0, pos, slot, window, chunk,
+                                    keep_first, scale, softcap, dist_bias, sink, gate, gate.stride(0) if gate is not None else 0,
+                                    gate_act, 1 if gate_heads else 0, out, _dt(out), out.stride(0), _stream())
     _check(rc, "omc_window_attn_mma")
     return out
 
@@ -781,9 +777,9 @@ def diff_attn_pair(q: torch.Tensor, H: int, G: int, d: int, dv: int, pool: torch
     assert pool.is_contiguous() and pool.shape[-1] == G * (2 * d + dv) and block_table.is_contiguous()
     assert items.dtype == torch.int32 and items.is_contiguous() and items.shape[1] == 4
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
-    rc = load().omc_diff_attn_pair(_ptr(q), q.stride(0), q.shape[0], H, G, d, dv, _ptr(pool), _ptr(block_table), block_table.shape[1],
-                                   page_size, _ptr(items), items.shape[0], window, keep_first, scale, lam, mult, eps, _ptr(gate),
-                                   gate.stride(0) if gate is not None else 0, gate_act, _ptr(out), _dt(out), out.stride(0), _stream())
+    rc = load().omc_diff_attn_pair(q, q.stride(0), q.shape[0], H, G, d, dv, pool, block_table, block_table.shape[1],
+                                   page_size, items, items.shape[0], window, keep_first, scale, lam, mult, eps, gate,
+                                   gate.stride(0) if gate is not None else 0, gate_act, out, _dt(out), out.stride(0), _stream())
     _check(rc, "omc_diff_attn_pair")
     return out
 
@@ -795,8 +791,8 @@ def diff_heads_gate(a: torch.Tensor, H: int, dv: int, lam: float, mult: float, e
     _need_cuda(a, gate, out)
     assert a.dtype == torch.float32 and a.stride(1) == 1 and out.stride(1) == 1 and a.shape[1] >= 2 * H * dv
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
-    rc = load().omc_diff_heads_gate(_ptr(a), a.stride(0), a.shape[0], H, dv, lam, mult, eps, _ptr(gate),
-                                    gate.stride(0) if gate is not None else 0, gate_act, _ptr(out), _dt(out), out.stride(0), _stream())
+    rc = load().omc_diff_heads_gate(a, a.stride(0), a.shape[0], H, dv, lam, mult, eps, gate,
+                                    gate.stride(0) if gate is not None else 0, gate_act, out, _dt(out), out.stride(0), _stream())
     _check(rc, "omc_diff_heads_gate")
     return out
 
@@ -807,7 +803,7 @@ def map_rows(x: torch.Tensor, op: int, A_log: Optional[torch.Tensor] = None, bia
     or MAP_SIGMOID_POW: sigmoid(x + bias[c])^p_exp - 1 (the decay as its distance from 1)."""
     _need_cuda(x, A_log, bias)
     assert x.dtype == torch.float32 and x.stride(1) == 1
-    rc = load().omc_map_rows(_ptr(x), x.stride(0), x.shape[0], x.shape[1], op, _ptr(A_log), _ptr(bias), group, p_exp, _stream())
+    rc = load().omc_map_rows(x, x.stride(0), x.shape[0], x.shape[1], op, A_log, bias, group, p_exp, _stream())
     _check(rc, "omc_map_rows")
     return x
 
@@ -826,9 +822,9 @@ def dyt_conv(x: torch.Tensor, alpha: torch.Tensor, nw: torch.Tensor, nb: torch.T
     assert taps == 1 or (state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (taps - 1, C))
     for t in (y1, y2, x_out):
         assert t is None or (t.dtype == torch.float32 and t.stride(1) == 1)
-    rc = load().omc_dyt_conv(_ptr(x), x.stride(0), _ptr(y1), y1.stride(0) if y1 is not None else 0, a1, _ptr(y2),
-                             y2.stride(0) if y2 is not None else 0, a2, _ptr(x_out), x_out.stride(0) if x_out is not None else 0,
-                             _ptr(alpha), _ptr(nw), _ptr(nb), _ptr(cw), _dt(cw), taps, _ptr(pos), _ptr(slot), _ptr(state), _ptr(u), _dt(u),
+    rc = load().omc_dyt_conv(x, x.stride(0), y1, y1.stride(0) if y1 is not None else 0, a1, y2,
+                             y2.stride(0) if y2 is not None else 0, a2, x_out, x_out.stride(0) if x_out is not None else 0,
+                             alpha, nw, nb, cw, _dt(cw), taps, pos, slot, state, u, _dt(u),
                              u.stride(0), T, C, 1 if single_rows else 0, _stream())
     _check(rc, "omc_dyt_conv")
     if taps > 1 and not single_rows:
@@ -840,7 +836,7 @@ def dyt_rows(x: torch.Tensor, alpha: torch.Tensor, w: torch.Tensor, b: torch.Ten
     """out = tanh(alpha x) w + b."""
     _need_cuda(x, alpha, w, b, out)
     assert x.dtype == torch.float32 and x.stride(1) == 1 and out.stride(1) == 1 and w.dtype == b.dtype and alpha.dtype == torch.float32
-    rc = load().omc_dyt_rows(_ptr(x), x.stride(0), _ptr(alpha), _ptr(w), _ptr(b), _dt(w), _ptr(out), _dt(out), out.stride(0), x.shape[0],
+    rc = load().omc_dyt_rows(x, x.stride(0), alpha, w, b, _dt(w), out, _dt(out), out.stride(0), x.shape[0],
                              x.shape[1], _stream())
     _check(rc, "omc_dyt_rows")
     return out
@@ -850,7 +846,7 @@ def tanh_cap_rows(x: torch.Tensor, cap: float):
     """x <- cap tanh(x / cap), in place (fp32)."""
     _need_cuda(x)
     assert x.dtype == torch.float32 and x.stride(1) == 1
-    rc = load().omc_tanh_cap_rows(_ptr(x), x.stride(0), x.shape[0], x.shape[1], cap, _stream())
+    rc = load().omc_tanh_cap_rows(x, x.stride(0), x.shape[0], x.shape[1], cap, _stream())
     _check(rc, "omc_tanh_cap_rows")
     return x
 
@@ -868,9 +864,9 @@ def selective_scan(x: torch.Tensor, dt: torch.Tensor, dt_bias: torch.Tensor, B: 
         assert t.dtype == torch.float32 and t.is_contiguous()
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (inner, N) and row_begin.dtype == torch.int32
     assert x.stride(1) == 1 and out.stride(1) == 1 and x.shape[1] == inner and B.shape[1] == N and Cm.shape[1] == N
-    rc = load().omc_selective_scan(_ptr(x), _dt(x), x.stride(0), _ptr(dt), dt.stride(0), _ptr(dt_bias), _ptr(B), B.stride(0), _ptr(Cm),
-                                   Cm.stride(0), _ptr(A_log), _ptr(D), _ptr(z), z.stride(0) if z is not None else 0, _ptr(state), _ptr(out),
-                                   _dt(out), out.stride(0), _ptr(row_begin), portions, _ptr(pos), _ptr(slot), inner, N, _stream())
+    rc = load().omc_selective_scan(x, _dt(x), x.stride(0), dt, dt.stride(0), dt_bias, B, B.stride(0), Cm,
+                                   Cm.stride(0), A_log, D, z, z.stride(0) if z is not None else 0, state, out,
+                                   _dt(out), out.stride(0), row_begin, portions, pos, slot, inner, N, _stream())
     _check(rc, "omc_selective_scan")
     return out
 
@@ -887,8 +883,8 @@ def rglru_scan(u: torch.Tensor, g: torch.Tensor, gb: Optional[torch.Tensor], lam
     for t in (lam, gb):
         assert t is None or (t.dtype == torch.float32 and t.is_contiguous())
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (width,) and row_begin.dtype == torch.int32
-    rc = load().omc_rglru_scan(_ptr(u), _dt(u), u.stride(0), _ptr(g), g.stride(0), _ptr(gb), _ptr(lam), _ptr(y), y.stride(0) if y is not None else 0,
-                               _ptr(state), _ptr(out), out.stride(0), _ptr(row_begin), portions, _ptr(pos), _ptr(slot), u.shape[0], width, blocks,
+    rc = load().omc_rglru_scan(u, _dt(u), u.stride(0), g, g.stride(0), gb, lam, y, y.stride(0) if y is not None else 0,
+                               state, out, out.stride(0), row_begin, portions, pos, slot, u.shape[0], width, blocks,
                                decay_scale, _stream())
     _check(rc, "omc_rglru_scan")
     return out
@@ -908,7 +904,7 @@ def pos_qkv_store(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, H: int, G: 
     assert pool.is_contiguous() and pool.shape[-1] == G * (d + dv) and pool.dtype == q_out.dtype and q_out.stride(1) == 1
     assert block_table.dtype == torch.int32 and block_table.is_contiguous()
     assert freq is None or (freq.dtype == torch.float32 and freq.is_contiguous() and freq.numel() >= rot_dims // 2)
-    rc = load().omc_pos_qkv_store(_ptr(q), q.stride(0), H, _ptr(k), k.stride(0), G, d, _ptr(v), v.stride(0), dv, _ptr(freq), rot_dims,
-                                  temp_coef, temp_every, 1 if v_unit else 0, eps, q.shape[0], _ptr(pos), _ptr(slot), _ptr(block_table),
-                                  block_table.shape[1], page_size, _ptr(pool), _ptr(q_out), q_out.stride(0), _dt(pool), _stream())
+    rc = load().omc_pos_qkv_store(q, q.stride(0), H, k, k.stride(0), G, d, v, v.stride(0), dv, freq, rot_dims,
+                                  temp_coef, temp_every, 1 if v_unit else 0, eps, q.shape[0], pos, slot, block_table,
+                                  block_table.shape[1], page_size, pool, q_out, q_out.stride(0), _dt(pool), _stream())
     _check(rc, "omc_pos_qkv_store")
