@@ -43,12 +43,10 @@ __device__ __forceinline__ float norm_rot_value(const float* __restrict__ x, con
   return second ? v * co + o * si : v * co - o * si;
 }
 
-// The same for four neighbouring columns (c, heads, rotated parts and their halves multiples of four).
+// The same for four neighbouring columns (c, heads, rotated parts and their halves multiples of four), which xv and wv hold.
 template <typename TW>
-__device__ __forceinline__ void norm_rot_value4(const float* __restrict__ x, const TW* __restrict__ w, int c, float rstd, const HeadRotation& rot, float (&o)[4]) {
-  float xv[4], wv[4];
-  ld4(x + c, xv);
-  ld4(w + c, wv);
+__device__ __forceinline__ void norm_rot_value4(const float* __restrict__ x, const TW* __restrict__ w, const float (&xv)[4], const float (&wv)[4], int c, float rstd,
+                                                const HeadRotation& rot, float (&o)[4]) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) o[e] = xv[e] * rstd * wv[e];
   if (rot.cs == nullptr) return;
@@ -87,17 +85,47 @@ template <bool VEC, typename TW, typename TD>
 __device__ __forceinline__ void rms_to(const float* __restrict__ x, int n, int group, const TW* __restrict__ w, float eps,
                                        TD* __restrict__ dst, float* red, const HeadRotation& rot) {
   if (VEC && group <= 0) {
+    // A row is read once (3126 rows of 4096 + 2 x 1024 columns: 33 us, 43 with two passes and three barriers): a thread's first pieces of it, and of the weight, wait in registers for the sum (rows wider than that are read again).
+    constexpr int KEEP = 4;
+    const int step = blockDim.x * 4, c0 = threadIdx.x * 4;
+    float xv[KEEP][4], wv[KEEP][4];
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+      if (c0 + i * step < n) ld4(x + c0 + i * step, xv[i]);
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+      if (c0 + i * step < n) ld4(w + c0 + i * step, wv[i]);
     float ss = 0.f;
-    for (int c = threadIdx.x * 4; c < n; c += blockDim.x * 4) {
+    auto add = [&](const float (&v)[4]) { ss = fmaf(v[0], v[0], ss), ss = fmaf(v[1], v[1], ss), ss = fmaf(v[2], v[2], ss), ss = fmaf(v[3], v[3], ss); };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+      if (c0 + i * step < n) add(xv[i]);
+    for (int c = c0 + KEEP * step; c < n; c += step) {
       float v[4];
       ld4(x + c, v);
-      ss = fmaf(v[0], v[0], ss), ss = fmaf(v[1], v[1], ss), ss = fmaf(v[2], v[2], ss), ss = fmaf(v[3], v[3], ss);
+      add(v);
     }
-    ss = block_sum(ss, red);
+    // block_sum for a kernel that needs one: the warps' sums meet behind one barrier, and every warp adds them up
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    ss = seq_warp_sum(ss);
+    if (lane == 0) red[warp] = ss;
+    __syncthreads();
+    ss = seq_warp_sum(lane < (int)(blockDim.x >> 5) ? red[lane] : 0.f);
     const float rstd = 1.f / sqrtf(ss / (float)n + eps);
-    for (int c = threadIdx.x * 4; c < n; c += blockDim.x * 4) {
-      float o[4];
-      norm_rot_value4(x, w, c, rstd, rot, o);
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i) {
+      const int c = c0 + i * step;
+      if (c < n) {
+        float o[4];
+        norm_rot_value4(x, w, xv[i], wv[i], c, rstd, rot, o);
+        st4(dst + c, o);
+      }
+    }
+    for (int c = c0 + KEEP * step; c < n; c += step) {
+      float v[4], u[4], o[4];
+      ld4(x + c, v);
+      ld4(w + c, u);
+      norm_rot_value4(x, w, v, u, c, rstd, rot, o);
       st4(dst + c, o);
     }
     return;
@@ -121,12 +149,12 @@ __device__ __forceinline__ void rms_to(const float* __restrict__ x, int n, int g
   }
 }
 
-// One CTA per row for the queries (blockIdx.y 0), another for keys and values (blockIdx.y 1).
+// One CTA per row for the queries (blockIdx.y 0), another for keys and values (blockIdx.y 1). vec_v: values in pieces of four.
 template <typename TW, typename TC, bool VEC>
 __global__ void __launch_bounds__(256) qk_norm_kv_store_kernel(const float* __restrict__ q, long long ldq, int nq, int q_group,
                                                                const TW* __restrict__ wq, const float* __restrict__ k, long long ldk,
                                                                int nk, int k_group, const TW* __restrict__ wk, const float* __restrict__ v,
-                                                               long long ldv, int nv, float eps, HeadRotation rot, const int32_t* __restrict__ pos,
+                                                               long long ldv, int nv, bool vec_v, float eps, HeadRotation rot, const int32_t* __restrict__ pos,
                                                                const int32_t* __restrict__ slot, const int32_t* __restrict__ block_table,
                                                                int max_pages, int page_size, TC* __restrict__ pool,
                                                                TC* __restrict__ q_out, long long ldqo) {
@@ -140,6 +168,15 @@ __global__ void __launch_bounds__(256) qk_norm_kv_store_kernel(const float* __re
   }
   const int page = block_table[(long long)slot[t] * max_pages + p / page_size];
   TC* dst = pool + ((long long)page * page_size + p % page_size) * (nk + nv);
+  if (VEC && vec_v) {   // under way before the norm's sum is waited for
+    for (int c = threadIdx.x * 4; c < nv; c += blockDim.x * 4) {
+      float o[4];
+      ld4(v + t * ldv + c, o);
+      st4(dst + nk + c, o);
+    }
+    rms_to<VEC>(k + t * ldk, nk, k_group, wk, eps, dst, red, rot);
+    return;
+  }
   rms_to<VEC>(k + t * ldk, nk, k_group, wk, eps, dst, red, rot);
   for (int c = threadIdx.x; c < nv; c += blockDim.x) stf(dst + nk + c, v[t * ldv + c]);
 }
@@ -1097,8 +1134,8 @@ extern "C" int omc_qk_norm_kv_store(const float* q, long long ldq, int nq, int q
                    al16(pool) && al16(q_out) && (rot.cs == nullptr || (al16(cs) && head % 4 == 0 && rot_dims % (rot_halves ? 8 : 4) == 0));
   OMC_DT_SWITCH(w_dt, TW, OMC_DT_SWITCH(dt, TC, {
     auto go = [&](auto kernel) {
-      kernel<<<dim3(T, 2), 256, 0, st>>>(q, ldq, nq, q_group, static_cast<const TW*>(wq), k, ldk, nk, k_group, static_cast<const TW*>(wk), v, ldv, nv, eps, rot,
-                                         pos, slot, block_table, max_pages, page_size, static_cast<TC*>(pool), static_cast<TC*>(q_out), ldqo);
+      kernel<<<dim3(T, 2), 256, 0, st>>>(q, ldq, nq, q_group, static_cast<const TW*>(wq), k, ldk, nk, k_group, static_cast<const TW*>(wk), v, ldv, nv,
+                                         ldv % 4 == 0 && al16(v), eps, rot, pos, slot, block_table, max_pages, page_size, static_cast<TC*>(pool), static_cast<TC*>(q_out), ldqo);
     };
     if (vec) go(qk_norm_kv_store_kernel<TW, TC, true>);
     else go(qk_norm_kv_store_kernel<TW, TC, false>);
