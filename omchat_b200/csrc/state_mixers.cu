@@ -102,41 +102,64 @@ struct ConvUnit {   // unit vectors behind the convolution: the first `channels`
 // TAPS - 1 inputs in registers, so a row of x is read once per tile (plus TAPS - 1 rows in front of it), and nothing goes through
 // shared memory. The same sums of taps as causal_conv_silu_kernel. UNIT: groups that a power of two of lanes of a warp holds are made unit vectors by
 // shuffles among them (every warp is whole: ch is a multiple of 128); causal_conv_silu_kernel, a block of rows in shared memory, is for other
-// groups. 3126 rows of 4096 channels with unit queries and keys of 128: 73 us there, 42 here (2.4 TB/s).
+// groups. Nothing that a tile reads waits for another load of it, except for ring entries. 3126 rows of 4096 channels with unit queries and keys of
+// 128: 73 us there, 40 here (2.6 TB/s; 42 with slots looked up in front of the rows before the tile); 6144 channels: 45 (3.4 TB/s).
 template <typename TW, typename TY, int TAPS, int ROWS, bool UNIT>
 __global__ void __launch_bounds__(128) causal_conv_rows_kernel(const float* __restrict__ x, long long ldx, int T, int ch,
                                                                const TW* __restrict__ w, const TW* __restrict__ bias,
                                                                const int32_t* __restrict__ pos, const int32_t* __restrict__ slot,
                                                                float* __restrict__ state, TY* __restrict__ y, long long ldy, int save_here,
-                                                               int act, ConvUnit unit) {
+                                                               int act, ConvUnit unit, bool vec_w) {
   constexpr int R = TAPS - 1;
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
   if (c >= ch) return;
   const int t0 = blockIdx.x * ROWS, nr = min(ROWS, T - t0);
-  float wv[TAPS][4], b4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-#pragma unroll
-    for (int j = 0; j < TAPS; ++j) wv[j][i] = ldf(w + (long long)(c + i) * TAPS + j);
-    if (bias != nullptr) b4[i] = ldf(bias + c + i);
-  }
+  // everything that does not wait for anything else first: the rows, those in front of them, whose they are, the weights
   float4 xv[ROWS], h[R > 0 ? R : 1];   // h[j]: the input R - j positions back
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) xv[r] = r < nr ? *reinterpret_cast<const float4*>(x + (long long)(t0 + r) * ldx + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-  int prev = -1;   // slot of the row before
+#pragma unroll
+  for (int j = 0; j < R; ++j) h[j] = t0 >= R - j ? *reinterpret_cast<const float4*>(x + (long long)(t0 - R + j) * ldx + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  int sl[R + ROWS];                    // slots of the rows from t0 - R on
+#pragma unroll
+  for (int j = 0; j < R + ROWS; ++j) sl[j] = t0 - R + j >= 0 && j < R + nr ? slot[t0 - R + j] : -1;
+  float wv[TAPS][4], b4[4] = {0.f, 0.f, 0.f, 0.f};
+  if constexpr (TAPS == 4) {
+    if (vec_w) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float u[4];
+        ld4(w + (long long)(c + i) * 4, u);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wv[j][i] = u[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (TAPS != 4 || !vec_w) {
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) wv[j][i] = ldf(w + (long long)(c + i) * TAPS + j);
+    }
+    if (bias != nullptr) b4[i] = ldf(bias + c + i);
+  }
 #pragma unroll
   for (int r = 0; r < ROWS; ++r) {
     if (r < nr) {
-      const int t = t0 + r, s = slot[t], p = pos[t];
-      if (s != prev) {   // first row of the tile, or of another request: the inputs in front come from the step, the ring or are zero
+      const int t = t0 + r, s = sl[R + r], p = pos[t];
+      if (r == 0) {                    // the inputs in front of the tile: rows of the same request, the ring or nothing
 #pragma unroll
         for (int j = 0; j < R; ++j) {
-          const int back = R - j, sp = p - back;
-          const float* q = nullptr;
-          if (sp >= 0) q = (t - back >= 0 && slot[t - back] == s) ? x + (long long)(t - back) * ldx : state + ((long long)s * R + sp % R) * ch;
-          h[j] = q != nullptr ? *reinterpret_cast<const float4*>(q + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const int sp = p - (R - j);
+          if (sp < 0) h[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          else if (sl[j] != s) h[j] = *reinterpret_cast<const float4*>(state + ((long long)s * R + sp % (R > 0 ? R : 1)) * ch + c);
         }
-        prev = s;
+      } else if (s != sl[R + r - 1]) {   // first row of another request
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+          const int sp = p - (R - j);
+          h[j] = sp >= 0 ? *reinterpret_cast<const float4*>(state + ((long long)s * R + sp % (R > 0 ? R : 1)) * ch + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
       }
       float o[4] = {b4[0], b4[1], b4[2], b4[3]};
 #pragma unroll
@@ -707,6 +730,83 @@ __global__ void __launch_bounds__(256) gated_rms_kernel(const float* __restrict_
 }
 
 
+// Both norms for groups that LANES neighbouring lanes hold in PIECES pieces of four columns each (n = 4 LANES PIECES): x and the gate are read once, all
+// of it before anything is waited for, and no two warps meet. FRONT: the gate in front of the norm and a weight for every column of the row, else behind
+// it and one weight of n columns for all groups. 3126 rows: 8 parts of 512 with a bf16 gate in front 38 -> 22 us, 16 groups of 128 with an fp32 gate behind 29 -> 16
+// (a block per part, a warp per group reading single columns twice).
+template <typename TG, typename TW, typename TY, int LANES, int PIECES, bool FRONT>
+__global__ void __launch_bounds__(256) group_rms_kernel(const float* __restrict__ x, long long ldx, int groups, long long total, const TW* __restrict__ w, float eps,
+                                                        const TG* __restrict__ gate, long long ldg, int gate_act, TY* __restrict__ y, long long ldy) {
+  constexpr int N = 4 * LANES * PIECES;
+  const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;   // (row, group)
+  const int lane = threadIdx.x % LANES;
+  const bool live = i < total;
+  const long long t = live ? i / groups : 0;
+  const int c0 = live ? (int)(i - t * groups) * N : 0;
+  float v[PIECES][4], g[PIECES][4], wv[PIECES][4];
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = (p * LANES + lane) * 4;
+    ld4(x + t * ldx + c0 + c, v[p]);
+    if (gate != nullptr) ld4(gate + t * ldg + c0 + c, g[p]);
+  }
+  auto act = [&](float z) { return gate_act == 1 ? silu_f(z) : (gate_act == 2 ? sigmoid_f(z) : z); };
+  if (gate != nullptr) {
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[p][e] = act(g[p][e]);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      if (FRONT) v[p][e] *= g[p][e];
+      ss = fmaf(v[p][e], v[p][e], ss);
+    }
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) ld4(w + (FRONT ? c0 : 0) + (p * LANES + lane) * 4, wv[p]);   // where a gate in front has left its registers
+#pragma unroll
+  for (int m = LANES / 2; m > 0; m >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
+  const float rstd = 1.f / sqrtf(ss / (float)N + eps);
+  if (!live) return;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    float o[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      o[e] = v[p][e] * rstd * wv[p][e];
+      if (!FRONT && gate != nullptr) o[e] *= g[p][e];
+    }
+    st4(y + t * ldy + c0 + (p * LANES + lane) * 4, o);
+  }
+}
+
+// Launches it for the widths it takes (a power of two from 32 to 1024 columns, everything on 16 bytes); false: not one of them.
+template <bool FRONT, typename TG, typename TW, typename TY>
+static bool group_rms(const float* x, long long ldx, int rows, int groups, int n, const TW* w, float eps, const TG* gate, long long ldg, int gate_act, TY* y, long long ldy,
+                      cudaStream_t st) {
+  auto al = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  if (ldx % 4 || (gate != nullptr && ldg % 4) || ldy % 4 || !al(x) || !al(gate) || !al(y) || !al(w)) return false;
+  const long long total = (long long)rows * groups;
+  auto go = [&](auto lanes, auto pieces) {
+    constexpr int L = decltype(lanes)::value, P = decltype(pieces)::value;
+    const long long blocks = (total * L + 255) / 256;
+    if (blocks >= 1ll << 31) return false;
+    group_rms_kernel<TG, TW, TY, L, P, FRONT><<<(unsigned)blocks, 256, 0, st>>>(x, ldx, groups, total, w, eps, gate, ldg, gate_act, y, ldy);
+    return true;
+  };
+  using std::integral_constant;
+  if (n == 32) return go(integral_constant<int, 8>(), integral_constant<int, 1>());
+  if (n == 64) return go(integral_constant<int, 16>(), integral_constant<int, 1>());
+  if (n == 128) return go(integral_constant<int, 32>(), integral_constant<int, 1>());
+  if (n == 256) return go(integral_constant<int, 32>(), integral_constant<int, 2>());
+  if (n == 512) return go(integral_constant<int, 32>(), integral_constant<int, 4>());
+  if (n == 1024) return go(integral_constant<int, 32>(), integral_constant<int, 8>());
+  return false;
+}
+
 // The gate in front of the norm: v = x * act(gate), y = v / sqrt(mean(v^2) + eps) * w with the mean over each of `groups` equal parts of
 // the row and a weight for every column. NT threads per (row, part); a thread keeps its elements in registers (VEC: four neighbours
 // at a time), parts too wide for that are read twice.
@@ -1179,7 +1279,8 @@ extern "C" int omc_causal_conv(const float* x, long long ldx, int T, int ch, con
       const ConvUnit cu{unit_channels, unit ? unit_group / 4 : 0, scaled_channels, unit_eps, unit_mult};
       auto launch = [&](auto kernel, int rows) {
         kernel<<<dim3((T + rows - 1) / rows, b4), 128, 0, st>>>(x, ldx, T, ch, static_cast<const TW*>(w), static_cast<const TW*>(bias), pos, slot, state,
-                                                              static_cast<TY*>(y), ldy, single_rows ? 1 : 0, act == OMC_CONV_SILU ? 1 : 0, cu);
+                                                              static_cast<TY*>(y), ldy, single_rows ? 1 : 0, act == OMC_CONV_SILU ? 1 : 0, cu,
+                                                              reinterpret_cast<uintptr_t>(w) % 16 == 0);
       };
       auto go = [&](auto taps_c) {
         constexpr int TAPS = decltype(taps_c)::value;
@@ -1327,6 +1428,7 @@ extern "C" int omc_gated_rms_rows(const float* x, long long ldx, int rows, int g
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int gy = groups > 8 ? (groups + 7) / 8 : 1;
   OMC_DT_SWITCH(w_dt, TW, OMC_DT_SWITCH(y_dt, TY, {
+    if (group_rms<false>(x, ldx, rows, groups, n, static_cast<const TW*>(w), eps, gate, ldg, gate_act, static_cast<TY*>(y), ldy, st)) return check_launch("omc_gated_rms_rows");
     gated_rms_kernel<TW, TY><<<dim3(rows, gy > 65535 ? 65535 : gy), 256, 0, st>>>(x, ldx, groups, n, static_cast<const TW*>(w), eps,
                                                                                  gate, ldg, gate_act, static_cast<TY*>(y), ldy);
   }))
@@ -1347,6 +1449,8 @@ extern "C" int omc_gate_rms_rows(const float* x, long long ldx, int rows, int gr
   while (threads < 256 && threads * per * 2 < n) threads <<= 1;
   const dim3 grid(rows, groups);
   OMC_DT_SWITCH(gate_dt, TG, OMC_DT_SWITCH(w_dt, TW, OMC_DT_SWITCH(y_dt, TY, {
+    if (group_rms<true>(x, ldx, rows, groups, n, static_cast<const TW*>(w), eps, static_cast<const TG*>(gate), ldg, gate_act, static_cast<TY*>(y), ldy, st))
+      return check_launch("omc_gate_rms_rows");
     if (vec) gate_rms_kernel<TG, TW, TY, true><<<grid, threads, 0, st>>>(x, ldx, n, static_cast<const TW*>(w), eps, static_cast<const TG*>(gate), ldg, gate_act,
                                                                          static_cast<TY*>(y), ldy);
     else gate_rms_kernel<TG, TW, TY, false><<<grid, threads, 0, st>>>(x, ldx, n, static_cast<const TW*>(w), eps, static_cast<const TG*>(gate), ldg, gate_act,
