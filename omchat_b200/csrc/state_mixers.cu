@@ -356,10 +356,10 @@ __device__ __forceinline__ int scan_place(int i) { return (i / DPT) * (DPT + 4) 
 // column, so that keys, queries and per-channel decays are used as they lie in shared memory, and only the numbers that all channels
 // share (the input u of a column, a head's decay) are doubled. What bounds it is the issue of the three (delta: four) packed fma per
 // state pair and token, behind them the latency of a token's chain; so what a token reads first is loaded during the token before it, and
-// the read-out of a chunk is summed over the lanes once at its end, from shared memory, instead of by shuffles in every token. Measured,
-// four portions of 1024, 777, 1024, 301 tokens (before: pairs of columns, a doubled key and a shuffled read-out per token): step sizes, 64
-// heads of 128 x 64: 341 us (501); delta rule, 16 heads of 128 x 128: 368 (513), per-channel decays 435 (560); one token of 32 requests,
-// step sizes: 22 us = 6.1 TB/s (42).
+// the read-out of a chunk is summed over the lanes once at its end, from shared memory, instead of by shuffles in every token. Portions of
+// several tokens at 64 or 128 channels go to scan_rows_kernel below; measured here, 16 heads of 128 x 128, four portions of 1024, 777, 1024, 301
+// tokens with per-channel decays: 435 us (560 with pairs of columns, a doubled key and a shuffled read-out per token); one token of 32 requests, step
+// sizes: 22 us = 6.1 TB/s (42).
 enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
 template <int DPT, int TOK>
 __host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
@@ -683,6 +683,263 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
         for (int c = 0; c < CPT; ++c)
           if (col + c < a.vdim) row[c] = e[j][c];
       }
+    }
+  }
+}
+
+// The same recurrence for portions of several tokens at 64 or 128 key channels, inputs that need no preparation of their own (no silu, per-channel decays given)
+// and 16-byte rows: the same sums in the same order, so the same bits, with what the general kernel spends beside them taken out. There 54 of 124 instructions
+// per token were addresses and bookkeeping, and a stage had three barriers with the decays' exponentials between two of them. Here the widths are constants, a stage is
+// eight tokens without a loop around them, with two barriers, and the decays and step sizes of the next stage are formed in the shadow of this one. A CTA of four warps has
+// CPT columns per group of eight lanes (see the launch). What bounds it: a token's chain through 90 instructions per warp (3.1 cycles each where a scheduler has one
+// warp), with many CTAs the packed fma and the shared-memory reads of keys and queries. Measured in us, the general kernel in brackets: step sizes, 64 heads of
+// 128 x 64, portions of 1024, 777, 1024, 301 tokens 306 (340), 32 x 64 tokens 185 (228), 16 heads, 1100 tokens 149 (195); delta rule, 16 heads of 128 x 128
+// over the same portions 351 (366), 8 x 300 tokens 174 (212), 4 heads, 1100 tokens 255 (299), with per-channel decays 305 (361).
+constexpr int kSrTok = 8, kSrThreads = 128;
+template <int DIM, int COLS, bool CHAN>
+struct ScanRowsStage {
+  static constexpr int PITCH = kScanLanes * (DIM / kScanLanes + 4);
+  float k[kSrTok * PITCH], q[kSrTok * PITCH], g[CHAN ? kSrTok * PITCH : 4], v[kSrTok * COLS];
+  float2 gb[kSrTok];   // a token's decay (or the decay minus one) and its beta or step size
+};
+template <int DIM, int COLS, bool CHAN>
+struct ScanRowsShared {
+  ScanRowsStage<DIM, COLS, CHAN> stage[2];
+  float po[kSrTok * kScanLanes * (COLS + 4)];   // [token][lane][column]: partial read-outs
+};
+
+template <int DIM, int CPT, int KIND, bool CHAN>
+__global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
+  extern __shared__ __align__(16) float sm[];
+  constexpr int COLS = kSrThreads / kScanLanes * CPT;
+  typedef ScanRowsShared<DIM, COLS, CHAN> Shared;
+  typedef ScanRowsStage<DIM, COLS, CHAN> Stage;
+  Shared& sh = *reinterpret_cast<Shared*>(sm);
+  constexpr int DPT = DIM / kScanLanes, DP = DPT / 2, PITCH = Stage::PITCH, OPITCH = COLS + 4;
+  const bool minus1 = KIND == kScanStep || a.decay_mode == 5;
+  const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
+  const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
+  if (r1 <= r0) return;
+  const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
+  const bool in = col < a.vdim;   // a thread's columns all exist or none does
+  const float A = KIND == kScanStep || a.decay_mode == 1 ? expf(a.A_log[h]) : 0.f;
+  const float bias = KIND == kScanStep || a.decay_mode == 1 ? a.dt_bias[h] : 0.f;
+  const float Dh = KIND == kScanStep && a.D != nullptr ? a.D[h] : 0.f;
+  const float gconst = a.decay_mode == 0 ? a.decay_const[h] : 1.f;
+
+  // a thread copies the 16-byte pieces `piece` of tokens tok0, tok0 + STEP, ...
+  constexpr int PIECES = DIM / 4, STEP = kSrThreads / PIECES;
+  const int piece = tid % PIECES, tok0 = tid / PIECES, place = scan_place<DPT>(piece * 4);
+  const float* kp = a.k + (long long)kvh * DIM + piece * 4;
+  const float* qp = a.q + (long long)kvh * DIM + piece * 4;
+  const float* gp = CHAN ? a.a + (long long)h * DIM + piece * 4 : nullptr;
+  constexpr int VP = COLS / 4, PARTS = CHAN ? kSrThreads / (kSrTok * VP) : 1, PL = kScanLanes / PARTS;   // pieces of a token's columns; threads per token and piece of the
+  const int vtok = tid / VP, vcol = tid % VP * 4, otok = tid / (VP * PARTS), opart = tid / VP % PARTS;   // read-out, and lanes that each of them adds up
+  const float* vp = a.v + (long long)h * a.vdim + col0 + vcol;
+  auto issue = [&](int c0, Stage& s) {
+#pragma unroll
+    for (int i = 0; i < kSrTok; i += STEP) {
+      const int tt = tok0 + i;
+      if (c0 + tt < r1) {
+        cp_async16(s.k + tt * PITCH + place, kp + (long long)(c0 + tt) * a.ldk);
+        cp_async16(s.q + tt * PITCH + place, qp + (long long)(c0 + tt) * a.ldq);
+        if (CHAN) cp_async16(s.g + tt * PITCH + place, gp + (long long)(c0 + tt) * a.lda);
+      }
+    }
+    if (vtok < kSrTok && c0 + vtok < r1 && col0 + vcol < a.vdim) cp_async16(s.v + vtok * COLS + vcol, vp + (long long)(c0 + vtok) * a.ldv);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // raw numbers of token c0 + tid, and what the recurrence makes of them
+  float raw_a = 0.f, raw_b = 0.f;
+  auto load_raw = [&](int c0) {
+    const int t = c0 + tid;
+    if (tid < kSrTok && t < r1) {
+      if (KIND == kScanStep || a.decay_mode == 1) raw_a = a.a[(long long)t * a.lda + h];
+      if (KIND == kScanDelta) raw_b = a.beta[(long long)t * a.ldb + h];
+    }
+  };
+  auto put_raw = [&](Stage& s) {
+    if (tid >= kSrTok) return;
+    if (KIND == kScanStep) {
+      const float dt = softplus_f(raw_a + bias);
+      s.gb[tid] = make_float2(expm1f(-A * dt), dt);
+    } else {
+      s.gb[tid] = make_float2(a.decay_mode == 1 ? expf(-A * softplus_f(raw_a + bias)) : gconst, KIND == kScanDelta ? sigmoid_f(raw_b) : 1.f);
+    }
+  };
+
+  issue(r0, sh.stage[0]);
+  load_raw(r0);
+  float* S = a.state + (((long long)a.slot[r0] * a.H + h) * DIM) * a.vdim;
+  f32x2 st[CPT][DP];   // state elements (lane * DPT + 2 r, col + c) and (lane * DPT + 2 r + 1, col + c)
+  const bool fresh = a.pos[r0] == 0;
+#pragma unroll
+  for (int r = 0; r < DP; ++r) {
+    float e[2][CPT];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float* row = S + (long long)(lane * DPT + 2 * r + j) * a.vdim + col;
+      const bool read = !fresh && in;
+      if constexpr (CPT == 1) {
+        e[j][0] = read ? *row : 0.f;
+      } else {
+        const float2 x = read ? *reinterpret_cast<const float2*>(row) : make_float2(0.f, 0.f);
+        e[j][0] = x.x, e[j][1] = x.y;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) st[c][r] = pack2(e[0][c], e[1][c]);
+  }
+  put_raw(sh.stage[0]);
+  load_raw(r0 + kSrTok);
+
+  int at = 0;
+  for (int c0 = r0; c0 < r1; c0 += kSrTok, at ^= 1) {
+    const int n = min(kSrTok, r1 - c0);
+    Stage& s = sh.stage[at];
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // this stage is there; the other one, and the partial read-outs, have been read by all
+    if (c0 + kSrTok < r1) {
+      issue(c0 + kSrTok, sh.stage[at ^ 1]);
+      put_raw(sh.stage[at ^ 1]);
+      load_raw(c0 + 2 * kSrTok);
+    }
+    f32x2 k2[DP];
+    float un[CPT];
+    float2 gb;
+    auto fetch = [&](int tt) {   // what a token reads first, during the token before it
+      const ulonglong2* kr = reinterpret_cast<const ulonglong2*>(s.k + tt * PITCH + lane * (DPT + 4));
+#pragma unroll
+      for (int r = 0; r < DP; r += 2) {
+        const ulonglong2 x = kr[r / 2];
+        k2[r] = x.x, k2[r + 1] = x.y;
+      }
+    };
+    auto fetch_shared = [&](int tt) {
+      const float* p = s.v + tt * COLS + CPT * cg;
+      if constexpr (CPT == 1) {
+        un[0] = *p;
+      } else {
+        const float2 x = *reinterpret_cast<const float2*>(p);
+        un[0] = x.x, un[1] = x.y;
+      }
+      gb = s.gb[tt];
+    };
+    fetch(0);
+    fetch_shared(0);
+    auto token = [&](int tt, int next) {
+      float u[CPT];
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) u[c] = KIND == kScanStep ? un[c] * gb.y : un[c];
+      const float b = gb.y;
+      if constexpr (CHAN) {
+        const ulonglong2* gr = reinterpret_cast<const ulonglong2*>(s.g + tt * PITCH + lane * (DPT + 4));
+#pragma unroll
+        for (int r = 0; r < DP; r += 2) {
+          const ulonglong2 g = gr[r / 2];
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) {
+            st[c][r] = minus1 ? fma2(st[c][r], g.x, st[c][r]) : mul2(st[c][r], g.x);
+            st[c][r + 1] = minus1 ? fma2(st[c][r + 1], g.y, st[c][r + 1]) : mul2(st[c][r + 1], g.y);
+          }
+        }
+      } else {
+        const f32x2 gh = pack2(gb.x, gb.x);
+#pragma unroll
+        for (int r = 0; r < DP; ++r)
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) st[c][r] = minus1 ? fma2(st[c][r], gh, st[c][r]) : mul2(st[c][r], gh);
+      }
+      fetch_shared(next);
+      f32x2 q2[DP];
+      const ulonglong2* qr = reinterpret_cast<const ulonglong2*>(s.q + tt * PITCH + lane * (DPT + 4));
+#pragma unroll
+      for (int r = 0; r < DP; r += 2) {
+        const ulonglong2 x = qr[r / 2];
+        q2[r] = x.x, q2[r + 1] = x.y;
+      }
+      auto columns = [&](const f32x2 (&with)[DP], float (&sum)[CPT]) {   // the general kernel's two chains per column
+        f32x2 x0[CPT], x1[CPT];
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) x0[c] = x1[c] = 0ull;
+#pragma unroll
+        for (int r = 0; r < DP; r += 2)
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) x0[c] = fma2(st[c][r], with[r], x0[c]), x1[c] = fma2(st[c][r + 1], with[r + 1], x1[c]);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) {
+          float w, x, y, z;
+          unpack2(x0[c], w, x);
+          unpack2(x1[c], y, z);
+          sum[c] = (w + y) + (x + z);
+        }
+      };
+      if (KIND == kScanDelta) {
+        float dot[CPT];
+        columns(k2, dot);
+#pragma unroll
+        for (int m = 1; m < kScanLanes; m <<= 1)
+#pragma unroll
+          for (int c = 0; c < CPT; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], m);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) u[c] = b * (u[c] - dot[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < CPT; ++c) {
+        const f32x2 u2 = pack2(u[c], u[c]);
+#pragma unroll
+        for (int r = 0; r < DP; ++r) st[c][r] = fma2(k2[r], u2, st[c][r]);
+      }
+      fetch(next);
+      float o[CPT];
+      columns(q2, o);
+      float* dst = sh.po + (tt * kScanLanes + lane) * OPITCH + CPT * cg;
+      if constexpr (CPT == 1) *dst = o[0];
+      else *reinterpret_cast<float2*>(dst) = make_float2(o[0], o[1]);
+    };
+    if (n == kSrTok) {
+#pragma unroll (CHAN ? 1 : kSrTok)
+      for (int tt = 0; tt < kSrTok; ++tt) token(tt, min(tt + 1, kSrTok - 1));
+    } else {
+#pragma unroll 1
+      for (int tt = 0; tt < n; ++tt) token(tt, min(tt + 1, n - 1));
+    }
+    __syncthreads();   // the partial read-outs are there
+    if (PARTS == 1 && otok >= n) continue;
+    const float* src = sh.po + (otok * kScanLanes + opart * PL) * OPITCH + vcol;
+    float4 x[PL];
+#pragma unroll
+    for (int l = 0; l < PL; ++l) x[l] = *reinterpret_cast<const float4*>(src + l * OPITCH);
+#pragma unroll
+    for (int m = 1; m < PL; m <<= 1)   // the order of the general kernel, through the threads that share a piece: the same bits
+#pragma unroll
+      for (int l = 0; l < PL; l += 2 * m) x[l].x += x[l + m].x, x[l].y += x[l + m].y, x[l].z += x[l + m].z, x[l].w += x[l + m].w;
+    float4 o = x[0];
+#pragma unroll
+    for (int m = VP; m < VP * PARTS; m <<= 1) {
+      o.x += __shfl_xor_sync(0xffffffffu, o.x, m), o.y += __shfl_xor_sync(0xffffffffu, o.y, m);
+      o.z += __shfl_xor_sync(0xffffffffu, o.z, m), o.w += __shfl_xor_sync(0xffffffffu, o.w, m);
+    }
+    if (otok < n && opart == 0 && col0 + vcol < a.vdim) {
+      if (KIND == kScanStep) {
+        const float4 v = *reinterpret_cast<const float4*>(s.v + otok * COLS + vcol);
+        o.x = fmaf(Dh, v.x, o.x), o.y = fmaf(Dh, v.y, o.y), o.z = fmaf(Dh, v.z, o.z), o.w = fmaf(Dh, v.w, o.w);
+      }
+      o.x *= a.out_scale, o.y *= a.out_scale, o.z *= a.out_scale, o.w *= a.out_scale;
+      *reinterpret_cast<float4*>(a.out + (long long)(c0 + otok) * a.ldo + h * a.vdim + col0 + vcol) = o;
+    }
+  }
+  if (!in) return;
+#pragma unroll
+  for (int r = 0; r < DP; ++r) {
+    float e[2][CPT];
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) unpack2(st[c][r], e[0][c], e[1][c]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float* row = S + (long long)(lane * DPT + 2 * r + j) * a.vdim + col;
+      if constexpr (CPT == 1) *row = e[j][0];
+      else *reinterpret_cast<float2*>(row) = make_float2(e[j][0], e[j][1]);
     }
   }
 }
@@ -1383,6 +1640,43 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   // (39 at 32 channels) leave three CTAs to an SM: eight portions of three tokens, 16 heads of 128 x 128, 15.4 / 10.3
   const bool tight = chan && (long long)grid.x * H * portions > 296;
   const bool brief = rows <= 16LL * portions;
+  // portions of several tokens whose inputs are ready: scan_rows_kernel
+  const bool ready = !silu_in && (decay_mode == 0 || decay_mode == 1 || decay_mode == 3 || decay_mode >= 5);
+  if (!one && vec && ready && (dim == 64 || dim == 128) && s.vec_out && s.vec_state) {
+    auto go = [&](auto dim_c, auto cpt_c, auto kind_c, auto chan_c) {
+      constexpr int DIM = decltype(dim_c)::value, CPT = decltype(cpt_c)::value, KIND = decltype(kind_c)::value, COLS = kSrThreads / kScanLanes * CPT;
+      constexpr bool CHAN = decltype(chan_c)::value;
+      static bool attr_done[kMaxDevices] = {};
+      constexpr int smem = (int)sizeof(ScanRowsShared<DIM, COLS, CHAN>);
+      if (!attr_done[cur_device()]) {
+        cudaFuncSetAttribute(scan_rows_kernel<DIM, CPT, KIND, CHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        attr_done[cur_device()] = true;
+      }
+      scan_rows_kernel<DIM, CPT, KIND, CHAN><<<dim3((vdim + COLS - 1) / COLS, H, portions), kSrThreads, smem, st>>>(s);
+      return check_launch("omc_linear_state_scan");
+    };
+    using std::integral_constant;
+    auto kinds = [&](auto dim_c, auto cpt_c) {
+      if (decay_mode == 6) return go(dim_c, cpt_c, integral_constant<int, kScanStep>(), std::false_type());
+      if (beta != nullptr) return go(dim_c, cpt_c, integral_constant<int, kScanDelta>(), std::false_type());
+      return go(dim_c, cpt_c, integral_constant<int, kScanPlain>(), std::false_type());
+    };
+    auto channels = [&](auto dim_c) {
+      typedef integral_constant<int, 1> One;
+      if (beta != nullptr) return go(dim_c, One(), integral_constant<int, kScanDelta>(), std::true_type());
+      return go(dim_c, One(), integral_constant<int, kScanPlain>(), std::true_type());
+    };
+    // 32 columns per CTA once CTAs of 16 would be more than the SMs: alone on an SM the smaller CTA is the faster one (in us, 16 / 32 columns: 16 heads of 128 x
+    // 64, step sizes, 1100 tokens 149 / 162; delta rule 4 of 128 x 128 255 / 269, 4 of 64 x 64 195 / 213), two of them on it never (64 heads 230 / 163).
+    // Per-channel decays take the registers of the larger one: there the general kernel is up to 12 % faster
+    const bool small = (long long)grid.x * H * portions <= 74;
+    typedef integral_constant<int, 1> One;
+    typedef integral_constant<int, 2> Two;
+    if (chan && small)
+      return dim == 64 ? channels(integral_constant<int, 64>()) : channels(integral_constant<int, 128>());
+    if (!chan && dim == 64) return small ? kinds(integral_constant<int, 64>(), One()) : kinds(integral_constant<int, 64>(), Two());
+    if (!chan) return small ? kinds(integral_constant<int, 128>(), One()) : kinds(integral_constant<int, 128>(), Two());
+  }
 #define OMC_SCAN_LAUNCH(DPT, VEC, KIND, CHAN, TOK)                                                                                        \
   do {                                                                                                                                    \
     static bool attr_done[kMaxDevices] = {};                                                                                              \
