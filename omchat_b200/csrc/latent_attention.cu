@@ -236,6 +236,12 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 4 && PER_LANE == 32 ? 6 :
   }
 }
 
+// attention_rows.cu
+bool attn_rows_ok(int rep, int d, int dv, bool values_in_keys, long long ldq, long long ldo, int out_dt, const void* q, const void* pool, const void* out, int row_w, int reach);
+int attn_rows(const float* q, long long ldq, int T, int H, int G, int d, int dv, bool values_in_keys, const float* pool, const int32_t* bt, int max_pages, int page_size,
+              const int32_t* pos, const int32_t* slot, int window, int chunk, float scale, float softcap, const float* bias, const float* sink, const float* gate,
+              long long ldg, int gate_act, int gate_heads, void* out, int out_dt, long long ldo, cudaStream_t st);
+
 }  // namespace omc
 
 using namespace omc;
@@ -300,6 +306,9 @@ extern "C" int omc_latent_attn(const void* qcat, int q_dt, int T, int H, int r, 
   const size_t smem = sizeof(float) * ((size_t)r + dr + (size_t)kLatParts * r + 2 * kLatParts);
   // the widths whose query and four partial outputs fit 48 KB; the eight partial outputs of the widest take up to 64 KB
   if (sizeof(float) * (5 * (size_t)r + dr + 8) > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_latent_attn: rows too wide");
+  if (q_dt == OMC_DT_F32 && pool_dt == OMC_DT_F32 && attn_rows_ok(H, r + dr, r, true, (long long)H * (r + dr), (long long)H * r, OMC_DT_F32, qcat, pool, out, r + dr, window))
+    return attn_rows(static_cast<const float*>(qcat), (long long)H * (r + dr), T, H, 1, r + dr, r, true, static_cast<const float*>(pool), block_table, max_pages, page_size, pos,
+                     slot, window, 1 << 30, scale, 0.f, nullptr, sink, gate, ldg, 2, 1, out, OMC_DT_F32, (long long)H * r, st);
   OMC_DT_SWITCH(q_dt, TQ, OMC_DT_SWITCH(pool_dt, TC, {
     auto go = [&](auto kernel, int warps) {
       if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return check_launch("omc_latent_attn");

@@ -1094,6 +1094,13 @@ __global__ void __launch_bounds__(256) diff_heads_gate_kernel(const float* __res
   }
 }
 
+// attention_rows.cu
+bool attn_rows_ok(int rep, int d, int dv, bool values_in_keys, long long ldq, long long ldo, int out_dt, const void* q, const void* pool, const void* out, int row_w, int reach);
+int attn_rows(const float* q, long long ldq, int T, int H, int G, int d, int dv, bool values_in_keys, const float* pool, const int32_t* bt, int max_pages, int page_size,
+              const int32_t* pos, const int32_t* slot, int window, int chunk, float scale, float softcap, const float* bias, const float* sink, const float* gate,
+              long long ldg, int gate_act, int gate_heads, void* out, int out_dt, long long ldo, cudaStream_t st);
+
+// window_attention_sm100.cu
 bool window_sm100_ok(int H, int G, int d, int dv, int maps, int keep_first, int page_size, int n_items, int window, int chunk, const float* bias, const void* out,
                      long long ldo);
 int window_sm100(const void* q, long long ldq, int T, int H, int G, int d, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
@@ -1158,6 +1165,10 @@ extern "C" int omc_window_attn(const void* q, long long ldq, int T, int H, int G
   const size_t smem = sizeof(float) * ((size_t)d + (size_t)kWinParts * dv + 2 * kWinParts);
   // the widths whose query and four partial outputs fit 48 KB; the eight partial outputs of the widest take up to 52 KB
   if (sizeof(float) * ((size_t)d + 4 * (size_t)dv + 8) > 48 * 1024) return set_error(OMC_ERR_SHAPE, "omc_window_attn: head width too large");
+  if (dt == OMC_DT_F32 && (out_dt == OMC_DT_F32 || out_dt == OMC_DT_BF16) && maps == 1 && keep_first == 0 &&
+      attn_rows_ok(H / G, d, dv, false, ldq, ldo, out_dt, q, pool, out, G * (d + dv), min(window, chunk)))
+    return attn_rows(static_cast<const float*>(q), ldq, T, H, G, d, dv, false, static_cast<const float*>(pool), block_table, max_pages, page_size, pos, slot, window, chunk, scale,
+                     softcap, dist_bias, sink, gate, ldg, gate_act, gate_heads, out, out_dt, ldo, st);
   OMC_DT_SWITCH(dt, TC, OMC_DT_SWITCH(out_dt, TY, {
     auto go = [&](auto kernel, int warps) {
       if (smem > 48 * 1024 && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return check_launch("omc_window_attn");
