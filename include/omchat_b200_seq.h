@@ -124,6 +124,10 @@ int omc_step_wait_failed(void);
  * the count above. */
 int omc_step_wait_selfcheck(int32_t* out, void* stream);
 
+/* The same for a wait of a whole warp, half of whose lanes wait for what has come and half for what never does: out (device, int32 [32]) receives
+ * every lane's answer, 0 for all of them. Adds one to the count above. */
+int omc_step_wait_warp_selfcheck(int32_t* out, void* stream);
+
 /* The work list of a decode-only step, written on the device from pos / slot (one row per request, `parts` <= 64 key ranges each):
  * items int32 [B * parts][8], merges int32 [B][4] (untouched when parts == 1). Lets a CUDA graph replay the step as contexts grow. */
 int omc_latent_decode_items(const int32_t* pos, const int32_t* slot, int B, int H, int parts, int window, int32_t* items,

@@ -246,9 +246,14 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     float l[NC];
 #pragma unroll
     for (int c = 0; c < NC; ++c) l[c] = 0.f;
+    // the lanes of a warp may leave a wait one by one, and accesses to tensor memory are the warp's as a whole; whether the phase came is not asked
+    auto wait_together = [&](uint64_t* bar, uint32_t parity) {
+      wait(bar, parity);
+      __syncwarp();
+    };
     for (int t = 0; t < n_tiles; ++t) {
       const int j0 = k0 + t * kKT, key = j0 + key_lane;
-      wait(&sh->s_full, t & 1);
+      wait_together(&sh->s_full, t & 1);
       tc_fence_after();
       // a tile that every row of the item sees in full needs no mask
       const bool whole = j0 >= kb && j0 + kKT <= k_end && j0 + kKT - 1 <= first_pos && (long long)j0 >= (long long)first_pos + n_tok - a.window;
@@ -365,7 +370,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       }
     }
     ls_softmax_sync();
-    if (n_tiles > 0) wait(&sh->o_done[nm - 1], (n_tiles - 1) & 1);
+    if (n_tiles > 0) wait_together(&sh->o_done[nm - 1], (n_tiles - 1) & 1);
     tc_fence_after();
     for (int m = 0; m < nm; ++m) {
       uint32_t v[NC];

@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kHgThreads) linear_sm100_kernel(const __grid_c
     const int quarter = warp & 3;
     float* slab = reinterpret_cast<float*>(ring) + quarter * 32 * kHgPitch;
     const bool plain = vec_out && a.act == OMC_ACT_NONE && a.bias == nullptr && (a.gate == nullptr || vec_gate);
-    const bool done = wait(&sh->done, 0);
+    const bool done = wait_bounded_warp(&sh->done, 0, report);
     tc_fence_after();
     for (int c = 0; done && c < BN && n0 + c < a.N; c += 64) {
 #pragma unroll
@@ -274,6 +274,23 @@ __global__ void step_wait_selfcheck_kernel(int32_t* out, unsigned int* failed) {
   }
 }
 
+// One warp whose lanes wait for different barriers, the lower half for one whose phase has come, the others for one that nothing arrives at. out: every
+// lane's answer.
+__global__ void step_wait_warp_selfcheck_kernel(int32_t* out, unsigned int* failed) {
+  __shared__ uint64_t come, never;
+  __shared__ uint32_t dead;
+  if (threadIdx.x == 0) {
+    mbar_init(&come, 1);
+    mbar_init(&never, 1);
+    dead = 0u;
+    fence_barrier_init();
+    mbar_arrive(&come);
+  }
+  __syncwarp();
+  const WaitReport report{&dead, &g_linear_failures, failed};
+  out[threadIdx.x] = wait_bounded_warp(threadIdx.x < 16 ? &come : &never, 0, report, 8);
+}
+
 }  // namespace omc
 
 extern "C" int omc_step_wait_failed(void) {
@@ -289,6 +306,14 @@ extern "C" int omc_step_wait_selfcheck(int32_t* out, void* stream) {
   if (const int rc = omc::step_failure_word(&failed); rc != OMC_OK) return rc;
   omc::step_wait_selfcheck_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(out, failed);
   return omc::check_launch("omc_step_wait_selfcheck");
+}
+
+extern "C" int omc_step_wait_warp_selfcheck(int32_t* out, void* stream) {
+  if (out == nullptr) return omc::set_error(OMC_ERR_ARG, "omc_step_wait_warp_selfcheck: bad argument");
+  unsigned int* failed = nullptr;
+  if (const int rc = omc::step_failure_word(&failed); rc != OMC_OK) return rc;
+  omc::step_wait_warp_selfcheck_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(out, failed);
+  return omc::check_launch("omc_step_wait_warp_selfcheck");
 }
 
 extern "C" int omc_step_wait_failures(unsigned int* count) {

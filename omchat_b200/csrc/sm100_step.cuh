@@ -31,6 +31,13 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, con
   }
   return true;
 }
+// A wait of all 32 lanes, with one answer for them all: whether every lane's phase has come. Where a wait gives up, lanes of a warp can see different
+// answers of wait_bounded (a phase that comes at that moment); lanes that then went different ways would leave the others in the next barrier of
+// the warp, or reach tensor memory without them.
+__device__ __forceinline__ bool wait_bounded_warp(uint64_t* bar, uint32_t parity, const WaitReport& r, uint32_t tries = kWaitTries) {
+  const bool come = wait_bounded(bar, parity, r, tries);
+  return __all_sync(0xffffffffu, come);
+}
 // For copies and products that have been issued: none may be under way into shared or tensor memory when the CTA gives these back, so these
 // waits have tries of their own whether or not another wait has given up.
 __device__ __forceinline__ bool drain_bounded(uint64_t* bar, uint32_t parity, const WaitReport& r) {

@@ -209,8 +209,7 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(WinSmA
       const int t = i >> 1, j0 = k0 + t * kWsKeys;
       const bool values = i & 1;
       if (!values) first = (long long)bt[j0 / a.page_size] * a.page_size + j0 % a.page_size;
-      const bool free = wait(values ? &sh->v_empty[t & 1] : &sh->k_empty[t & 1], ((uint32_t)(t >> 1) & 1u) ^ 1u);
-      if (!free) break;
+      if (!wait_bounded_warp(values ? &sh->v_empty[t & 1] : &sh->k_empty[t & 1], ((uint32_t)(t >> 1) & 1u) ^ 1u, report)) break;   // the lanes leave together or not at all
       uint8_t* dst = (values ? vs : ks) + (t & 1) * kTile;
       const bf16_t* src = a.pool + first * W + (values ? a.G + kvh : kvh) * D + c * 8;
 #pragma unroll
@@ -244,11 +243,10 @@ __global__ void __launch_bounds__(kWsThreads, 2) window_attn_sm100_kernel(WinSmA
     const float c1 = CAP ? a.scale / a.softcap * (2.f * kLog2e) : a.scale * kLog2e, c2 = -2.f * a.softcap * kLog2e, cap = a.softcap * kLog2e;
     const float* brow = BIAS ? table + (is_row ? h : 0) * ws_bias_pitch(a.window, rep) + p : nullptr;
     float m_ref = -INFINITY, l = 0.f;
-    // the lanes of a warp may leave a wait one by one, and accesses to tensor memory are the warp's as a whole
+    // the lanes of a warp may leave a wait one by one, and accesses to tensor memory are the warp's as a whole; whether the phase came is not asked
     auto wait_together = [&](uint64_t* bar, uint32_t parity) {
-      const bool come = wait(bar, parity);
+      wait(bar, parity);
       __syncwarp();
-      return come;
     };
     // The output product of the tile before is done. Waited for in front of every arrival that lets the next one start: a wait knows only odd from
     // even, and a warp can be one product behind the others, but never two.

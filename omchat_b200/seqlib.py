@@ -67,6 +67,7 @@ SIGNATURES = {
     "omc_step_wait_failures": (_I, [_P]),
     "omc_step_wait_failed": (_I, []),
     "omc_step_wait_selfcheck": (_I, [_P, _P]),
+    "omc_step_wait_warp_selfcheck": (_I, [_P, _P]),
     "omc_latent_attn_mma": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_latent_decode_items": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
     "omc_router_topk": (_I, [_P, _L, _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P, _P]),

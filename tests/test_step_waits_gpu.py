@@ -37,3 +37,11 @@ def test_a_wait_that_ran_out_is_reported():
                "    except seqlib.OmcError as e:\n        print('ran out' in str(e))\n"
                "z = torch.ones(64, 64, device='cuda'); seqlib.linear(z, z, y); print(y[0, 0].item())\n")
     assert got[:5] == ["0 128.0", "1", "True", "True", "64.0"]
+
+
+def test_the_lanes_of_a_warp_have_one_answer():
+    """Half of them wait for a phase that has come: they too go the way of the others, or the warp's next barrier would wait for ever."""
+    got = _run("out = torch.full((32,), 9, dtype=torch.int32, device='cuda')\n"
+               "print(L.omc_step_wait_warp_selfcheck(out.data_ptr(), torch.cuda.current_stream().cuda_stream), out.tolist() == [0] * 32)\n"
+               "print(L.omc_step_wait_failures(ctypes.byref(n)), n.value)\n")
+    assert got[:2] == ["0 True", "0 1"]
