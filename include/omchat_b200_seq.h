@@ -98,14 +98,15 @@ int omc_latent_attn_mma(const void* qcat, int T, int H, int r, int dr, const voi
                         int page_size, const int32_t* items, int n_items, const int32_t* merges, int n_merges, const float* sink,
                         int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o, float* ws_ml, void* stream);
 
-/* The same with the most rows (n_tok * H) any item has, which may be fewer than 64 (a decode step: H). */
+/* The same with the most rows (n_tok * H) any item has, which may be fewer than 64 (a decode step: H). All three entries run on tcgen05, with both
+ * products transposed and a probability as two bf16 numbers, where r is a multiple of 128 up to 512, dr a multiple of 16 up to 64, page_size a
+ * multiple of 64 and max_rows at most 64; else on mma.sync with one. */
 int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, int dr, const void* pool, const int32_t* block_table, int max_pages,
                              int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
                              const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,
                              float* ws_o, float* ws_ml, void* stream);
 
-/* The same, told how many rows (pages * page_size) the pool has: on tcgen05 with both products transposed where r is a multiple of 128, dr <= 64,
- * page_size a multiple of 64 and max_rows at most 64. pool_rows 0: not known, on mma.sync as the two above. */
+/* The same; pool_rows (pages * page_size) is not needed. */
 int omc_latent_attn_mma_pool(const void* qcat, int T, int H, int r, int dr, const void* pool, long long pool_rows, const int32_t* block_table,
                              int max_pages, int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
                              const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,

@@ -721,8 +721,8 @@ __global__ void latent_decode_items_kernel(const int32_t* __restrict__ pos, cons
 }
 
 // latent_attention_sm100.cu
-bool latent_sm100_ok(int max_rows, int r, int dr, long long pool_rows, int page_size, const void* q, const void* pool);
-int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, long long pool_rows, const int32_t* bt, int max_pages, int page_size,
+bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool);
+int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size,
                  const int32_t* items, int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
                  float* ws_ml, cudaStream_t st);
 
@@ -751,20 +751,20 @@ extern "C" int omc_latent_attn_mma(const void* qcat, int T, int H, int r, int dr
                                    int max_pages, int page_size, const int32_t* items, int n_items, const int32_t* merges,
                                    int n_merges, const float* sink, int window, const float* gate, long long ldg, float scale, void* out,
                                    int out_dt, float* ws_o, float* ws_ml, void* stream) {
-  return omc_latent_attn_mma_pool(qcat, T, H, r, dr, pool, 0, block_table, max_pages, page_size, items, n_items, omc::kMmaRows, merges, n_merges, sink, window,
-                                  gate, ldg, scale, out, out_dt, ws_o, ws_ml, stream);
+  return omc_latent_attn_mma_rows(qcat, T, H, r, dr, pool, block_table, max_pages, page_size, items, n_items, omc::kMmaRows, merges, n_merges, sink, window, gate,
+                                  ldg, scale, out, out_dt, ws_o, ws_ml, stream);
+}
+
+extern "C" int omc_latent_attn_mma_pool(const void* qcat, int T, int H, int r, int dr, const void* pool, long long, const int32_t* block_table,
+                                        int max_pages, int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
+                                        const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,
+                                        float* ws_o, float* ws_ml, void* stream) {
+  return omc_latent_attn_mma_rows(qcat, T, H, r, dr, pool, block_table, max_pages, page_size, items, n_items, max_rows, merges, n_merges, sink, window, gate, ldg,
+                                  scale, out, out_dt, ws_o, ws_ml, stream);
 }
 
 extern "C" int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, int dr, const void* pool, const int32_t* block_table, int max_pages,
                                         int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
-                                        const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,
-                                        float* ws_o, float* ws_ml, void* stream) {
-  return omc_latent_attn_mma_pool(qcat, T, H, r, dr, pool, 0, block_table, max_pages, page_size, items, n_items, max_rows, merges, n_merges, sink, window, gate,
-                                  ldg, scale, out, out_dt, ws_o, ws_ml, stream);
-}
-
-extern "C" int omc_latent_attn_mma_pool(const void* qcat, int T, int H, int r, int dr, const void* pool, long long pool_rows, const int32_t* block_table,
-                                        int max_pages, int page_size, const int32_t* items, int n_items, int max_rows, const int32_t* merges, int n_merges,
                                         const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt,
                                         float* ws_o, float* ws_ml, void* stream) {
   if (window < 1) return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: the window holds at least the row itself");
@@ -788,8 +788,8 @@ extern "C" int omc_latent_attn_mma_pool(const void* qcat, int T, int H, int r, i
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc;
   if (out_dt != OMC_DT_F32 && out_dt != OMC_DT_BF16) return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: unknown output dtype");
-  if (latent_sm100_ok(max_rows, r, dr, pool_rows, page_size, qcat, pool))
-    rc = latent_sm100(qcat, (long long)T * H, H, r, dr, pool, pool_rows, block_table, max_pages, page_size, items, n_items, max_rows, sink, window, gate, ldg, scale,
+  if (latent_sm100_ok(max_rows, r, dr, page_size, qcat, pool))
+    rc = latent_sm100(qcat, (long long)T * H, H, r, dr, pool, block_table, max_pages, page_size, items, n_items, max_rows, sink, window, gate, ldg, scale,
                       out, out_dt, ws_o, ws_ml, st);
   else if (r <= 64) rc = launch_lat_mma<1, 8>(a, out_dt, n_items, smem, st);
   else if (r <= 128) rc = launch_lat_mma<1, 16>(a, out_dt, n_items, smem, st);

@@ -8,9 +8,10 @@
 //     O^T [r, NR]       += V^T P^T        A = the SAME shared-memory tile read MN-major (r / 128 accumulators)   B = P^T
 // which needs (r / 128 + 1) NR columns, lets one staged tile serve both products, and lets a decode step (16 heads of one token) run at
 // N = 16 instead of on a mostly empty row tile.
-//   warp 0       TMA: Q once; per tile the 64-column chunks of two 64-key boxes. The two chunks (the last time with the rotated one) that hold
-//                128 value dimensions share a barrier: scores start with the first pair, and a pair is refilled as soon as the output
-//                product that reads it is done
+//   warps 0, 10  Q once, by TMA; per tile the 64-column chunks of two boxes of 64 keys, by cp.async: the pages alone say where a row lies, and nobody has to
+//                know the rows of the pool (a tensor map of more rows than there are let copies touch what lies behind it). The two chunks (the last
+//                time with the rotated one) that hold 128 value dimensions share a barrier, at which each thread's copies arrive by themselves:
+//                scores start with the first pair, and a pair is refilled as soon as the output product that reads it is done
 //   warp 1       MMA issuer (one thread)
 //   warps 2..9   softmax: thread = one key x half the rows. Maxima over keys are maxima over lanes: a transposing butterfly leaves every
 //                lane with one row's maximum. The reference maximum of a row only moves when it grew by more than 2^8; the output
@@ -19,21 +20,25 @@
 //                together): with one, tiles of 128 keys and longer key ranges gave 1 to 44 % more error than the mma.sync kernel's tiles of 64. Where
 //                Q and the key tile fill shared memory (64 rows, r = 512) half of it takes the places of the rotated chunks, which the scores
 //                have consumed.
-// What bounds it: shared memory holds one key tile, so a tile of 8300 cycles is a load that only the output products overlap (3100), 100 instructions
-// on the tensor pipe (36 for the scores), and one softmax pass over 8192 scores (2200). 16 heads, latents of 512 + 64 (the mma.sync kernel in
-// brackets): portions of 1024, 777, 1024 behind 1024 and 301 rows 253 us = 336 TFLOP/s without the second half of the probabilities (722); 4 x 1024
-// rows of 32 heads 483 us (1136); 2048 rows 196 us (653); a decode step of 32 rows over 700 to 2100 keys, merge included, 31 us (79).
+// What bounds it: shared memory holds one key tile, so a tile of 8000 cycles is a load that only the output products overlap (3100), 100 instructions
+// on the tensor pipe (36 for the scores), and one softmax pass over 8192 scores (2200). 16 heads, latents of 512 + 64 (key tiles by TMA / the mma.sync
+// kernel in brackets): portions of 1024, 777, 1024 behind 1024 and 301 rows 244 us (260 / 722); 4 x 1024 rows of 32 heads 460 us (495 / 1136); 2048 rows
+// 193 us (202 / 653); a decode step of 32 rows over 700 to 2100 keys, merge included, 34 us (33 / 79). By cp.async with a wait and a fence of the load
+// warps in front of every pair: 359, 660, 297 and 52 us.
 #include "sm100_step.cuh"
 
 namespace omc {
 
 constexpr int kKT = 128;                    // keys per tile
 constexpr int kChunkBytes = kKT * 128;      // 64 columns of a key tile
-constexpr int kLsThreads = 320, kLsSoftmax = 256, kLsMaxRows = 64;
+constexpr int kLsSoftmax = 256, kLsLoad = 64, kLsThreads = kLsSoftmax + 32 + kLsLoad, kLsMaxRows = 64;
 
 static __device__ unsigned int g_latent_failures;   // waits that ran out
 
 struct LatSmArgs {
+  const bf16_t* q;        // q_rows rows; with the pool, for the copies by cp.async
+  const bf16_t* pool;
+  long long q_rows;
   const int32_t* bt;
   const int32_t* items;   // as LatMmaArgs of latent_attention.cu
   const float* sink;
@@ -63,6 +68,8 @@ __device__ __forceinline__ float ls_exp2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Arrives (one of the counted arrivals) once the copies that this thread has issued so far are there.
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) { asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory"); }
 __device__ __forceinline__ void ls_softmax_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kLsSoftmax) : "memory"); }
 
 // v[c]: this lane's value of column c. Returns the reduction over the 32 lanes of column lane / (32 / NC) (v is overwritten).
@@ -101,8 +108,7 @@ __device__ __forceinline__ void ls_tmem_st(uint32_t addr, const uint32_t* v) {
 }
 
 template <int NR, typename TO>
-__global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kv,
-                                                                          LatSmArgs a) {
+__global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const __grid_constant__ CUtensorMap tm_q, LatSmArgs a) {
   constexpr int NC = NR / 2;                 // rows per softmax thread
   constexpr int QCHUNK = NR * 128;           // bytes of a 64-column chunk of Q
   extern __shared__ uint8_t ls_raw[];
@@ -111,10 +117,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   uint8_t* base = ls_raw + ((1024u - (smem_u32(ls_raw) & 1023u)) & 1023u);
   uint8_t* qs = base;                        // [nc][NR][128 B]
   uint8_t* ks = base + a.nc * QCHUNK;        // [nc][128][128 B]
-  if (threadIdx.x == 32) {
-    tma_prefetch_desc(&tm_q);
-    tma_prefetch_desc(&tm_kv);
-  }
+  if (threadIdx.x == 32) tma_prefetch_desc(&tm_q);
   const int32_t* it = a.items + blockIdx.x * 8;
   const int first_row = it[0], n_tok = it[1], slot = it[2], first_pos = it[3], kb = it[4], part = it[6];
   const int k_end = min(it[5], first_pos + n_tok), n_rows = n_tok * a.H;
@@ -137,16 +140,37 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
       row[b] = j < k_end ? bt[j / a.page_size] * a.page_size + j % a.page_size : -1;
     }
   };
-  auto load_q = [&](int c, uint64_t* bar) { tma_load_3d(qs + c * QCHUNK, &tm_q, bar, chunk_col(c), first_row * a.H, 0); };
-  auto load_pair = [&](const int (&row)[2], int g, bool again) {   // chunks of barrier g
-    const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
-    const bool q_too = again && a.reload_q && g == nm - 1;
-    mbar_arrive_expect_tx(&sh->full[g], (c1 - 2 * g) * (row[1] >= 0 ? 2 : 1) * (kChunkBytes / 2) + (q_too ? QCHUNK : 0));
-    if (q_too) load_q(a.nc - 1, &sh->full[g]);
+  // The chunks of barrier g by the load warps: eight lanes per 128 bytes of a row, as the 128-byte swizzle has them, eight rows at a time. Rows that are no keys of
+  // this item become zeros: what the cache holds there must not meet a product.
+  static_assert(kLsLoad == 64, "eight rows at a time");
+  const bool loads = warp == 0 || warp == kLsThreads / 32 - 1;
+  const int piece = lane & 7, r0 = (warp == 0 ? lane : lane + 32) >> 3, swizzled = r0 * 128 + ((piece ^ r0) << 4);
+  auto copy_pair = [&](int t, const int (&row)[2], int g) {
+    const int c1 = g == nm - 1 ? a.nc : 2 * g + 2, j = k0 + t * kKT;
+    const long long step = 8LL * a.D;
+    for (int c = 2 * g; c < c1; ++c) {
+      uint8_t* at = ks + c * kChunkBytes + swizzled;
 #pragma unroll
-    for (int b = 0; b < 2; ++b)
-      if (row[b] >= 0)
-        for (int c = 2 * g; c < c1; ++c) tma_load_3d(ks + c * kChunkBytes + b * (kChunkBytes / 2), &tm_kv, &sh->full[g], chunk_col(c), row[b], 0);
+      for (int b = 0; b < 2; ++b, at += kChunkBytes / 2) {
+        const bf16_t* src = a.pool + (long long)(max(row[b], 0) + r0) * a.D + chunk_col(c) + piece * 8;
+        if (j + 64 * b >= kb && j + 64 * b + 64 <= k_end) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) cp_async16(at + i * 1024, src + i * step, true);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int key = j + 64 * b + i * 8 + r0;
+            cp_async16(at + i * 1024, src + i * step, key >= kb && key < k_end);
+          }
+        }
+      }
+    }
+    if (t > 0 && a.reload_q && g == nm - 1) {
+      const bf16_t* src = a.q + ((long long)first_row * a.H + r0) * a.D + chunk_col(a.nc - 1) + piece * 8;
+#pragma unroll
+      for (int i = 0; i < NR / 8; ++i) cp_async16(qs + (a.nc - 1) * QCHUNK + swizzled + i * 1024, src + i * step, (long long)first_row * a.H + r0 + i * 8 < a.q_rows);
+    }
+    cp_async_arrive(&sh->full[g]);           // once this thread's copies so far are there
   };
   if (tid >= 64 && tid < 64 + kLsMaxRows) sh->mref[tid - 64] = -INFINITY;
   if (tid == 0) {
@@ -155,20 +179,24 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
     mbar_init(&sh->p_ready, kLsSoftmax / 32);
     mbar_init(&sh->mma_done, 1);
     for (int m = 0; m < 4; ++m) {
-      mbar_init(&sh->full[m], 1);
+      mbar_init(&sh->full[m], kLsLoad);
       mbar_init(&sh->o_done[m], 1);
     }
     sh->dead = 0u;
     sh->rescale[0] = sh->rescale[1] = 0u;
     fence_barrier_init();
     fence_proxy_async();
-    if (n_tiles > 0) {                       // on their way while tensor memory is allocated
+    if (n_tiles > 0) {
       mbar_arrive_expect_tx(&sh->q_full, a.nc * QCHUNK);
-      for (int c = 0; c < a.nc; ++c) load_q(c, &sh->q_full);
-      int row[2];
-      box_rows(0, row);
-      for (int g = 0; g < nm; ++g) load_pair(row, g, false);
+      for (int c = 0; c < a.nc; ++c) tma_load_3d(qs + c * QCHUNK, &tm_q, &sh->q_full, chunk_col(c), first_row * a.H, 0);
     }
+  }
+  int row[2] = {-1, -1};                     // of the tile that is loaded next
+  if (loads && n_tiles > 0) {                // the first tile is on its way while tensor memory is allocated
+    box_rows(0, row);
+    __syncwarp();
+    asm volatile("bar.sync 2, %0;" ::"n"(kLsLoad) : "memory");   // the barriers are there
+    for (int g = 0; g < nm; ++g) copy_pair(0, row, g);
   }
   if (warp == 1) {
     __syncwarp();
@@ -180,17 +208,18 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   tc_fence_after();
   const uint32_t tmem = sh->tmem, tmem_s = tmem + nm * NR;
 
-  if (warp == 0) {
-    if (lane == 0 && n_tiles > 0) {
-      int t = 0, upto = nm;                  // the copies of tile t have been issued for the first `upto` groups, those of the tile before for the others
-      while (upto == nm && t + 1 < n_tiles) {
-        int row[2];
-        box_rows(++t, row);
-        for (upto = 0; upto < nm && wait(&sh->o_done[upto], (t - 1) & 1); ++upto) load_pair(row, upto, true);
+  if (loads) {
+    bool go = true;
+    for (int t = 1; go && t < n_tiles; ++t) {
+      box_rows(t, row);
+      for (int g = 0; g < nm; ++g) {
+        go = wait_bounded_warp(&sh->o_done[g], (t - 1) & 1, report);
+        if (!go) break;
+        copy_pair(t, row, g);
       }
-      drain(&sh->q_full, 0);          // nothing is on its way any more when this thread leaves
-      for (int g = 0; g < nm; ++g) drain(&sh->full[g], (g < upto ? t : t - 1) & 1);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");   // nothing is on its way any more when these threads leave
+    if (tid == 0 && n_tiles > 0) drain(&sh->q_full, 0);
   } else if (warp == 1) {
     if (elect_one() && n_tiles > 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16_major(128, NR, 0, 0);
@@ -209,6 +238,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
         for (int g = 0; g < nm; ++g) {
           go = wait(&sh->full[g], t & 1);
           if (!go) break;
+          fence_proxy_async();               // what the load warps' copies wrote is seen by the products
           tc_fence_after();
           const int c1 = g == nm - 1 ? a.nc : 2 * g + 2;
           for (int c = 2 * g; c < c1; ++c) {
@@ -275,14 +305,6 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
         }
       };
       load_scores();
-      // rows of the tile that are no keys of this item hold whatever the cache holds there: as values they must not meet a product
-      if (!whole) {                          // eight lanes per row of 128 bytes: a lane per row would meet one bank with all 32
-        for (int i = 0; i < 32; i += 4) {
-          const int row = quarter * 32 + i + (lane >> 3);
-          if (j0 + row < kb || j0 + row >= k_end)
-            for (int c = half; c < a.r >> 6; c += 2) *reinterpret_cast<uint4*>(ks + c * kChunkBytes + row * 128 + (lane & 7) * 16) = make_uint4(0, 0, 0, 0);
-        }
-      }
       const float mx = ls_columns<NC>(s, lane, [](float x, float y) { return fmaxf(x, y); });
       if (lane % (32 / NC) == 0) sh->part[quarter][c0 + lane / (32 / NC)] = mx;
       ls_softmax_sync();
@@ -420,14 +442,14 @@ static int ls_smem(int nr, int r, int D, LatSmArgs* a) {
 }
 
 // Shapes this kernel takes. max_rows: the most rows an item has.
-bool latent_sm100_ok(int max_rows, int r, int dr, long long pool_rows, int page_size, const void* q, const void* pool) {
+bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool) {
   LatSmArgs a;
-  return pool_rows >= 64 && pool_rows <= (1ll << 31) && max_rows <= kLsMaxRows && r % 128 == 0 && r <= 512 && dr <= 64 && dr % 16 == 0 && page_size % 64 == 0 &&
+  return max_rows <= kLsMaxRows && r % 128 == 0 && r <= 512 && dr <= 64 && dr % 16 == 0 && page_size % 64 == 0 &&
          reinterpret_cast<uintptr_t>(q) % 16 == 0 && reinterpret_cast<uintptr_t>(pool) % 16 == 0 && ls_smem(max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64), r, r + dr, &a) > 0;
 }
 
 template <int NR, typename TO>
-static int ls_launch(const CUtensorMap& tq, const CUtensorMap& tk, const LatSmArgs& a, int n_items, int smem, cudaStream_t st) {
+static int ls_launch(const CUtensorMap& tq, const LatSmArgs& a, int n_items, int smem, cudaStream_t st) {
   static bool done[kMaxDevices] = {};
   const int dev = cur_device();
   if (!done[dev]) {
@@ -435,28 +457,27 @@ static int ls_launch(const CUtensorMap& tq, const CUtensorMap& tk, const LatSmAr
     if (e != cudaSuccess) return set_error(OMC_ERR_CUDA, cudaGetErrorString(e));
     done[dev] = true;
   }
-  latent_attn_sm100_kernel<NR, TO><<<n_items, kLsThreads, smem, st>>>(tq, tk, a);
+  latent_attn_sm100_kernel<NR, TO><<<n_items, kLsThreads, smem, st>>>(tq, a);
   return check_launch("omc_latent_attn_mma");
 }
 
-int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, long long pool_rows, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
+int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
                  int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
                  float* ws_ml, cudaStream_t st) {
   const int D = r + dr, nr = max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64);
-  LatSmArgs a{bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D, (D + 63) / 64, {}, false, 0, scale * 1.4426950408889634f, nullptr};
+  LatSmArgs a{static_cast<const bf16_t*>(q), static_cast<const bf16_t*>(pool), q_rows, bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D,
+              (D + 63) / 64, {}, false, 0, scale * 1.4426950408889634f, nullptr};
   const int smem = ls_smem(nr, r, D, &a);
   const int cols = (r / 128 + 1) * nr;
   a.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : (cols <= 256 ? 256 : 512)));
-  CUtensorMap tq, tk;
+  CUtensorMap tq;
   int rc = step_failure_word(&a.failed);
   if (rc == OMC_OK) rc = step_tensor_map(&tq, q, D, q_rows, D, 1, 0, nr);
-  // the rows that there are and no more: a map of 2^31 rows let copies of a pool's last rows touch what lies behind the pool
-  if (rc == OMC_OK) rc = step_tensor_map(&tk, pool, D, pool_rows, D, 1, 0, 64);
   if (rc != OMC_OK) return rc;
   const bool b = out_dt == OMC_DT_BF16;
-  if (nr == 16) return b ? ls_launch<16, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<16, float>(tq, tk, a, n_items, smem, st);
-  if (nr == 32) return b ? ls_launch<32, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<32, float>(tq, tk, a, n_items, smem, st);
-  return b ? ls_launch<64, bf16_t>(tq, tk, a, n_items, smem, st) : ls_launch<64, float>(tq, tk, a, n_items, smem, st);
+  if (nr == 16) return b ? ls_launch<16, bf16_t>(tq, a, n_items, smem, st) : ls_launch<16, float>(tq, a, n_items, smem, st);
+  if (nr == 32) return b ? ls_launch<32, bf16_t>(tq, a, n_items, smem, st) : ls_launch<32, float>(tq, a, n_items, smem, st);
+  return b ? ls_launch<64, bf16_t>(tq, a, n_items, smem, st) : ls_launch<64, float>(tq, a, n_items, smem, st);
 }
 
 int latent_sm100_failures(unsigned int* n) { return cudaMemcpyFromSymbol(n, g_latent_failures, sizeof(*n)) == cudaSuccess ? OMC_OK : OMC_ERR_CUDA; }

@@ -408,7 +408,7 @@ def latent_attn_mma(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, blo
             ws = torch.empty(need, device=qcat.device, dtype=torch.float32)
             _mma_ws[key] = ws
         ws_o, ws_ml = ws[:plan.n_parts * MMA_ROWS * r], ws[plan.n_parts * MMA_ROWS * r:]
-    rc = load().omc_latent_attn_mma_pool(qcat, T, H, r, dr, pool, pool.numel() // (r + dr), block_table, block_table.shape[1], page_size,
+    rc = load().omc_latent_attn_mma_rows(qcat, T, H, r, dr, pool, block_table, block_table.shape[1], page_size,
                                          plan.items, plan.n_items, plan.max_rows, plan.merges, plan.n_merges, sink, window, gate,
                                          gate.stride(0) if gate is not None else 0, scale, out, _dt(out), ws_o, ws_ml, _stream())
     _check(rc, "omc_latent_attn_mma")

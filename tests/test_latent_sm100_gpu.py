@@ -1,5 +1,5 @@
-"""The tcgen05 latent attention (omc_latent_attn_mma_rows where r is a multiple of 128 and pages of 64 rows) against float64: tile edges, portions
-behind a cached prefix, windows that start inside a box, decode steps in key ranges, sinks, gates, rows of the cache that hold no key."""
+"""The tcgen05 latent attention (omc_latent_attn_mma_rows, as seqlib calls it, and the two other entries, where r is a multiple of 128 and pages of 64 rows) against float64: tile edges, portions behind a cached prefix, windows that start inside a box, decode steps in key ranges, sinks, gates,
+rows of the cache that hold no key."""
 import math
 
 import pytest
@@ -173,3 +173,35 @@ def test_steps_of_few_keys_take_the_other_kernel(H, r, portions, window):
         plan = LatentAttention._prompt_plan(plist, H, "cuda", window, tcgen05)
         seqlib.latent_attn_mma(q.cuda(), r, 32, torch.cat(lat).view(-1, 64, D).cuda(), table, 64, plan, None, D ** -0.5, out, window=window)
         assert ((out.double().cpu() - want).abs() <= mag * (2.0 ** (-17 if tcgen05 else -8) + 6e-5) + 1e-6).all(), tcgen05
+
+
+@pytest.fixture(params=["omc_latent_attn_mma", "omc_latent_attn_mma_pool"])
+def other_entry(request, monkeypatch):
+    """seqlib.latent_attn_mma through one of the entries that it does not call itself."""
+    lib = seqlib.load()
+
+    def call(qcat, T, H, r, dr, pool, table, max_pages, page, items, n_items, max_rows, *rest):
+        if request.param == "omc_latent_attn_mma":
+            return lib.omc_latent_attn_mma(qcat, T, H, r, dr, pool, table, max_pages, page, items, n_items, *rest)
+        return lib.omc_latent_attn_mma_pool(qcat, T, H, r, dr, pool, 0, table, max_pages, page, items, n_items, max_rows, *rest)
+    monkeypatch.setattr(lib, "omc_latent_attn_mma_rows", call)
+
+
+@pytest.mark.parametrize("H,r,dr,page,window,portions", [
+    (16, 512, 64, 64, 1 << 30, [(5, 0), (4, 123), (9, 124), (1, 127), (1, 128), (133, 60)]),
+    (32, 512, 48, 128, 100, [(70, 0), (64, 300), (1, 511), (3, 190)]),
+    (5, 128, 16, 192, 1 << 30, [(13, 0), (30, 100)]),
+    (8, 384, 0, 64, 33, [(50, 0), (1, 200)]),
+])
+def test_other_entries_against_float64(other_entry, H, r, dr, page, window, portions):
+    test_against_float64(H, r, dr, page, window, portions, "sink_gate")
+
+
+@pytest.mark.parametrize("H,r,dr,n,first", [(16, 512, 64, 9, 500), (16, 512, 0, 70, 300), (16, 384, 64, 33, 60), (8, 128, 32, 20, 700)])
+@pytest.mark.parametrize("decode", [0, 1, 3])
+def test_other_entries_do_not_round_probabilities(other_entry, H, r, dr, n, first, decode):
+    test_probabilities_are_not_rounded_to_8_bits(H, r, dr, n, first, decode)
+
+
+def test_other_entries_stay_inside_the_pool(other_entry):
+    test_a_pool_that_ends_with_its_mapping(512, 64)
