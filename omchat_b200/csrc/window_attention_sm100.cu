@@ -388,13 +388,13 @@ static int ws_table(bool bias, int window, int rep) { return bias ? (ws_bias_pit
 
 // Shapes this kernel takes (the alignment of the output is what its 16-byte accesses want), where it is the faster one. A CTA of it costs some 5 us before
 // its first tile, so a row has to see enough keys: at widths of 128 from 64 keys on (64 keys 0.52 to 0.93 of the mma.sync kernel's time, 32 keys up to
-// 1.34), at widths of 64, whose tiles are shorter, from 192 on (0.54 to 1.03; 128 keys up to 1.20) or from 64 on where CTAs come in several waves
-// (0.65 to 0.85).
+// 1.34), at widths of 64, whose tiles are shorter, from 192 on (0.54 to 1.03; 128 keys up to 1.20). Steps of several waves of CTAs would gain from 64 keys on
+// there (0.65 to 0.85), but the two kernels round differently, and a request's rows must not depend on what else is in the step.
 bool window_sm100_ok(int H, int G, int d, int dv, int maps, int keep_first, int page_size, int n_items, int window, int chunk, const float* bias, const void* out,
                      long long ldo) {
   const int rep = H / G, reach = window < chunk ? window : chunk;
   return (d == 64 || d == 128) && dv == d && maps == 1 && keep_first == 0 && page_size % kWsKeys == 0 && rep <= 64 && ldo % 8 == 0 &&
-         reinterpret_cast<uintptr_t>(out) % 16 == 0 && reach >= 64 && (d == 128 || reach >= 192 || (long long)n_items * G >= 4 * 148) &&
+         reinterpret_cast<uintptr_t>(out) % 16 == 0 && reach >= (d == 128 ? 64 : 192) &&
          (long long)n_items * G < (1ll << 31) && (bias == nullptr || (window <= 16384 && ws_smem(d, ws_table(true, window, rep)) <= 220 * 1024));
 }
 

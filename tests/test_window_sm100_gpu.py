@@ -117,6 +117,25 @@ def test_requests_do_not_meet():
         assert (out[a:b].double() - want[a:b]).abs().max() < 1e-3
 
 
+@pytest.mark.parametrize("d,window", [(64, 64), (64, 128), (64, 191), (64, 192), (128, 63), (128, 64)])     # either side of the line to the mma.sync kernel
+def test_a_request_does_not_depend_on_the_others_of_the_step(d, window):
+    """Alone, and beside so many others that the CTAs come in several waves: the same bits."""
+    H, G = 8, 8
+    gen = torch.Generator().manual_seed(window)
+    rows, pool, table, q, plan = _inputs([(97, 150)] + [(64, 200)] * 80, H, G, d, 64, gen)
+    scale, outs = d ** -0.5, []
+    for some in (plan[:1], plan):
+        n = some[-1][0] + some[-1][1]
+        items = seqlib.window_attn_items(some, H // G, "cuda")
+        assert (items.shape[0] * G >= 4 * 148) == (len(some) > 1)
+        outs.append(torch.empty(n, H * d, device="cuda"))
+        seqlib.window_attn_mma(q[:n].cuda(), H, G, d, d, pool.cuda(), table.cuda(), 64, items, None, None, window, scale, 0.0, None, outs[-1])
+    assert torch.equal(outs[0], outs[1][:97])
+    want, mag = _oracle(rows, q, plan, H, G, d, window, seqlib.WINDOW_ALL, scale, 0.0, None, None, None, 0, False)
+    # as test_against_float64; on mma.sync one bf16 number per probability, in the sums above and below the line
+    assert ((outs[1].double() - want).abs() <= mag * (2.0 ** -13 + 2.0 ** -8) + 1e-30).all()
+
+
 def test_the_largest_probability_takes_no_rounding():
     """128 keys of one score, then one whose probability is 128.49 times theirs: as two bf16 numbers relative to either maximum it is exact to 2^-17."""
     import math
