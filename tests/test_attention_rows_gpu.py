@@ -74,3 +74,42 @@ def test_latent_rows(H, r, dr, window):
         pr = torch.softmax(torch.cat([q[t].double() @ k.T * scale, sink.double()[:, None]], 1), 1)[:, :n - lo]
         f = torch.sigmoid(gate[t].double())[:, None]
         assert ((out[t].double().cpu() - pr @ k[:, :r] * f).abs() <= _err(r + dr, scale) * (pr @ k[:, :r].abs()) * f + 1e-6).all(), n
+
+
+@pytest.mark.parametrize("window", [63, 64, seqlib.WINDOW_ALL])       # fewer than 64 keys: the plain kernel
+def test_one_query_head_per_key_head(window):
+    test_window_rows(8, 8, 64, 64, False, window, seqlib.WINDOW_ALL)
+    test_window_rows(3, 3, 64, 128, True, window, seqlib.WINDOW_ALL)
+    test_latent_rows(1, 128, 64, window)
+
+
+MANY = (1, 16, 31, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 160, 257, 300)
+
+
+@pytest.mark.parametrize("window,chunk", [(seqlib.WINDOW_ALL, seqlib.WINDOW_ALL), (32, seqlib.WINDOW_ALL), (64, seqlib.WINDOW_ALL), (200, 70)])
+@pytest.mark.parametrize("H,G,d,dv,bf16", [(8, 1, 64, 64, False), (14, 2, 128, 128, False), (9, 1, 96, 256, True), (6, 2, 36, 100, False), (4, 2, 32, 64, True), (8, 8, 64, 64, False),
+                                           (0, 1, 320, 256, False), (0, 1, 576, 512, False)])
+def test_few_rows_and_many_give_the_same_bits(H, G, d, dv, bf16, window, chunk):
+    """Two heads to a CTA and several tiles to a stage, or all heads and one tile: by the number of rows. H 0: latents, of d columns in all."""
+    gen = torch.Generator().manual_seed(d + dv + min(window, 999))
+    latent, H = H == 0, H or 16
+    rows, pool, table = _paged(MANY, d if latent else G * (d + dv), gen)
+    q, sink, gate = torch.randn(len(MANY), H * d, generator=gen), torch.randn(H, generator=gen).cuda(), torch.randn(len(MANY), H, generator=gen)
+    bias = torch.randn(window, H, generator=gen).cuda() if window < 999 else None
+
+    def run(of):
+        pos, slot = torch.tensor([MANY[i] - 1 for i in of], dtype=torch.int32).cuda(), torch.tensor(of, dtype=torch.int32).cuda()
+        out = torch.empty(len(of), H * dv, device="cuda", dtype=torch.bfloat16 if bf16 else torch.float32)
+        if latent:
+            seqlib.latent_attn(q[of].cuda().view(len(of), H, d), dv, d - dv, pool, table, PAGE, pos, slot, sink, d ** -0.5, out.view(len(of), H, dv), window=min(window, chunk),
+                               gate=gate[of].cuda())
+        else:
+            seqlib.window_attn(q[of].cuda(), H, G, d, dv, pool, table, PAGE, pos, slot, window, d ** -0.5, 4.0, bias, out, sink=sink, gate=gate[of].cuda(), gate_act=2, chunk=chunk,
+                               gate_heads=True)
+        return out
+    order = list(range(len(MANY)))
+    many = run(order * 20)
+    assert torch.isfinite(many).all()
+    for i in (order[:1], order[4:6], order[-2:], order[8:12]):                # few rows: the CTAs of each of these run in one wave
+        assert len(i) * G * -(-H // G // 2) <= 148 < 20 * len(MANY) * G
+        assert torch.equal(run(i), many[i[0]:i[-1] + 1])
