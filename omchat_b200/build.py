@@ -102,9 +102,9 @@ def build_component(name: str, force: bool = False, verbose: bool = False) -> Pa
 CALL_LIB, CALL_SOURCE = LIBDIR / "omc_call.so", CSRC / "call.cpp"
 
 
-def ensure_call(force: bool = False) -> Path | None:
+def ensure_call(force: bool = False, compile: bool = True) -> Path | None:
     """The compiled calls of native.py (host code, a few seconds of g++), built first if missing, older than the source or made for another interpreter or torch; None
-    where there is neither a built one nor a compiler with Python's headers."""
+    where there is neither a built one nor a compiler with Python's headers, or none is built and `compile` is off."""
     import sysconfig
 
     import torch
@@ -116,7 +116,7 @@ def ensure_call(force: bool = False) -> Path | None:
     if not force and CALL_LIB.exists() and stamp.exists() and stamp.read_text() == digest:
         return CALL_LIB
     gxx = shutil.which("g++")
-    if gxx is None or not os.path.exists(os.path.join(include, "Python.h")):
+    if not compile or gxx is None or not os.path.exists(os.path.join(include, "Python.h")):
         return None
     LIBDIR.mkdir(exist_ok=True)
     tmp = CALL_LIB.with_suffix(f".so.tmp{os.getpid()}")

@@ -3,6 +3,7 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+import warnings
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -19,29 +20,29 @@ class Pointer:
         return c_void_p.from_param(v.data_ptr() if isinstance(v, torch.Tensor) else v)
 
 
-def _load():
-    from . import build
-    path = build.ensure_call()
-    if path is None:
-        return None
-    spec = importlib.util.spec_from_file_location("omc_call", path)
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
-    return module
+_module, _tried, _error = None, False, RuntimeError
 
 
-_module, _tried = None, False
-
-
-def module():
-    """The compiled calls, or None where there are none (no compiler or headers): ctypes then."""
+def module(compile: bool = True):
+    """The compiled calls, or None where there are none (no compiler or headers): ctypes then, several times slower per call. One that does not compile or load is
+    said, once. compile False: as far as it is built already."""
     global _module, _tried
-    if not _tried:
+    if _module is None and not _tried:
+        _tried = compile
         try:
-            _module = _load()
-        except (OSError, ImportError, RuntimeError):
-            _module = None
-        _tried = True
+            from . import build
+            path = build.ensure_call(compile=compile)
+            if path is not None:
+                spec = importlib.util.spec_from_file_location("omc_call", path)
+                loaded = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(loaded)
+                loaded.set_error_type(_error)
+                _module = loaded
+        except (OSError, ImportError, RuntimeError) as e:
+            _tried = True
+            lines = [line.strip() for line in str(e).splitlines() if line.strip()] or [type(e).__name__]
+            reason = next((line for line in lines if "error:" in line), lines[-1])
+            warnings.warn(f"omchat_b200: the compiled calls could not be built or loaded, every call goes through ctypes (slower): {reason}", RuntimeWarning, stacklevel=2)
     return _module
 
 
@@ -69,12 +70,16 @@ class Entries:
 def need_cuda(error: type):
     """A function of tensors (or None) that raises `error` for one that is not on the current GPU. Every kernel is launched on the current stream of the CURRENT
     device: a tensor living on another GPU would be dereferenced there (illegal access or silent peer traffic), so that is an error, not a convention."""
-    native = module()
+    global _error
+    _error = error
+    native = module(compile=False)            # nothing is compiled while the package is imported
     if native is not None:
         native.set_error_type(error)
         return native.need_cuda
 
     def check(*ts):
+        if _module is not None:               # compiled meanwhile
+            return _module.need_cuda(*ts)
         cur: Optional[int] = None
         for t in ts:
             if t is None:
