@@ -688,11 +688,12 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
 }
 
 // The same recurrence for portions of several tokens at 64 or 128 key channels, inputs that need no preparation of their own (no silu, per-channel decays given)
-// and 16-byte rows: the same sums in the same order, so the same bits, with what the general kernel spends beside them taken out. There 54 of 124 instructions
-// per token were addresses and bookkeeping, and a stage had three barriers with the decays' exponentials between two of them. Here the widths are constants, a stage is
+// and 16-byte rows: the same sums in the same order, so the same bits, with what the general kernel spends beside them taken out (addresses and
+// bookkeeping per token, a third barrier per stage, the decays' exponentials between two of them). Here the widths are constants, a stage is
 // eight tokens without a loop around them, with two barriers, and the decays and step sizes of the next stage are formed in the shadow of this one. A CTA of four warps has
-// CPT columns per group of eight lanes (see the launch). What bounds it: a token's chain through 90 instructions per warp (3.1 cycles each where a scheduler has one
-// warp), with many CTAs the packed fma and the shared-memory reads of keys and queries. Measured in us, the general kernel in brackets: step sizes, 64 heads of
+// CPT columns per group of eight lanes (see the launch). What bounds it: a token's chain through 92 instructions per warp (step sizes; delta rule 135), some three
+// cycles each where a scheduler has one warp (4 heads, 1100 tokens: 440 cycles per token), with many CTAs the packed fma (58 % of the pipe's cycles) and the shared-memory
+// reads of keys and queries (74 % of the data path's). Measured in us, the general kernel in brackets: step sizes, 64 heads of
 // 128 x 64, portions of 1024, 777, 1024, 301 tokens 306 (340), 32 x 64 tokens 185 (228), 16 heads, 1100 tokens 149 (195); delta rule, 16 heads of 128 x 128
 // over the same portions 351 (366), 8 x 300 tokens 174 (212), 4 heads, 1100 tokens 255 (299), with per-channel decays 305 (361).
 constexpr int kSrTok = 8, kSrThreads = 128;

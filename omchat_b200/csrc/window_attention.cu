@@ -85,7 +85,8 @@ template <bool VEC, typename TW, typename TD>
 __device__ __forceinline__ void rms_to(const float* __restrict__ x, int n, int group, const TW* __restrict__ w, float eps,
                                        TD* __restrict__ dst, float* red, const HeadRotation& rot) {
   if (VEC && group <= 0) {
-    // A row is read once (3126 rows of 4096 + 2 x 1024 columns: 33 us, 43 with two passes and three barriers): a thread's first pieces of it, and of the weight, wait in registers for the sum (rows wider than that are read again).
+    // A row is read once: a thread's first pieces of it, and of the weight, wait in registers for the sum (rows wider than that are read again). 3126 rows of
+    // 4096 + 2 x 1024 columns: 33 us, 43 with two passes and three barriers.
     constexpr int KEEP = 4;
     const int step = blockDim.x * 4, c0 = threadIdx.x * 4;
     float xv[KEEP][4], wv[KEEP][4];

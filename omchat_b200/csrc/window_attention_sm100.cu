@@ -12,13 +12,15 @@
 //   warps 5, 6   keys and values by cp.async, two tiles each
 // The bias lies in shared memory by head and distance, in base-2 units with the soft cap's constant added: a row walks its tile at fixed offsets
 // from one address, and the rows of a warp (consecutive tokens, heads a bank offset apart) meet different banks.
-// Two CTAs share an SM and hide each other's waits. What bounds it with a soft cap is the exponential unit (three operations per score, 16 per cycle and SM:
-// 1536 cycles per tile) and the chain of a tile behind it; two threads per row were slower without a cap (12 to 27 %: one more barrier per tile) and no
+// Two CTAs share an SM and hide each other's waits. What bounds it is the chain of a tile, at two softmax warps per scheduler: with a soft cap (three operations of the
+// exponential unit per score, 16 per cycle and SM: 1536 cycles per tile) that unit is busy 42 % of the time, issue slots 43 %, tensor pipe 19 %. Two threads per row were slower without a cap (12 to 27 %: one more barrier per tile) and no
 // faster with one. Head fastest and the later items first in the grid: portions end with their items of few keys (103 us with the items fastest).
 // Measured, mma.sync kernel in brackets: 32 heads on 8 key/value heads of 128, portions of 1024, 777, 1024 behind 1024 and 301 rows, window 512, cap and
 // bias: 89 us (270); 4 x 2048 rows behind 2048, causal: 667 us = 618 TFLOP/s (2880).
 // Keys and values come by cp.async and not by TMA: boxes addressed through a block table, every one of them inside the pool, gave illegal accesses with
 // a tensor map that claimed more rows than the pool has, and once with one that did not, for no reason that was found.
+// A value that is not a finite number reaches every row of a CTA that has its key, also those of earlier tokens (0 x infinity in the output product; on mma.sync the
+// rows of one item, here of two).
 #include <type_traits>
 
 #include "sm100_step.cuh"
