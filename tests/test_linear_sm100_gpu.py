@@ -59,3 +59,25 @@ def test_gates_that_do_not_come_in_pairs_use_the_precise_exponential(N, pad, gat
     err = (y.double() / (K * torch.sigmoid(g.double())) - 1).abs()
     # the product is exact; two units of the last place for the exponential, half of one for the sum, the quotient and their effect on it
     assert err.max() <= 4 * 2.0 ** -23, float(err.max())
+
+
+@pytest.mark.parametrize("N,K,batch,M", [(512, 64, 8, 3100), (128, 192, 8, 12900), (64, 64, 6, 25700)])   # six and eight tiles of 256, 128 and 64 columns per CTA
+@pytest.mark.parametrize("gated", [False, True])
+def test_a_cta_walks_over_many_tiles(N, K, batch, M, gated):
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x, w = (torch.randn(*s, generator=gen, device="cuda").to(BF16) for s in ((M, batch * K), (batch, N, K)))
+    g = torch.randn(M, batch * N, generator=gen, device="cuda").to(BF16) if gated else None
+    if gated:      # gates of no finite value: shut, open, undefined
+        g[0, :3] = torch.tensor([-torch.inf, torch.inf, torch.nan], device="cuda")
+        g[-1, -3:] = torch.tensor([-torch.inf, torch.inf, torch.nan], device="cuda")
+    y = torch.empty(M, batch * N, dtype=BF16, device="cuda")
+    seqlib.linear(x, w, y, M=M, N=N, K=K, ldx=batch * K, sx=K, ldw=K, sw=N * K, ldy=batch * N, sy=N, batch=batch, gate=g)
+    for b in range(batch):
+        cols = slice(b * N, (b + 1) * N)
+        xs, ws = x[:, b * K:(b + 1) * K].double(), w[b].double()
+        want, mag = xs @ ws.T, xs.abs() @ ws.abs().T
+        if gated:
+            want, mag = want * torch.sigmoid(g[:, cols].double()), mag * torch.sigmoid(g[:, cols].double())
+        bound = mag * (K * 2.0 ** -23 + 2.0 ** -20) + want.abs() * 2.0 ** -8 + 1e-30   # as above
+        ok = (y[:, cols].double() - want).abs() <= bound
+        assert (ok | (want.isnan() & y[:, cols].isnan())).all(), b
