@@ -386,6 +386,9 @@ __device__ __forceinline__ void w_mma_bf16(float (&c)[4], uint32_t a0, uint32_t 
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void w_cp_async16_or_zero(uint32_t dst, const void* src, bool there) {   // zeros, and nothing read, unless `there`
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
 __device__ __forceinline__ void w_cp_async16(uint32_t dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
@@ -433,8 +436,10 @@ struct WinMmaArgs {
 
 // Decode: items of one token whose query heads per key/value head fit one 16-row tile. The keys are dealt to the CTA's warps in tiles of
 // 32; every warp stages its own tile, works on it alone and keeps a partial (max, sum, output), and the partials meet in shared memory at the
-// end. One warp walking all tiles was bound by its own instructions, 7 us per 64 keys: 32 rows x 4 key/value heads of 128 + 128 over
-// up to 512 keys 20 us (60). How many warps: win_decode_warps.
+// end. One warp walking all tiles was bound by its own instructions, 7 us per 64 keys, and so is each of the eight: the copies of a tile, with a division
+// and a branch per 16 bytes, were two thirds of them. Now a lane's piece of a row is fixed and a copy five instructions, and the next tile's keys and values are
+// on their way as soon as their places are free: 32 rows x 4 key/value heads of 128 + 128 over up to 512 keys 16 us (20; one warp 60), 64 x 8 heads 59 (74), 256 x 8
+// heads 148 (194). How many warps: win_decode_warps.
 constexpr int kWdWarps = 8, kWdKeys = 32, kWdRows = 16;
 template <int NV, typename TO>
 __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMmaArgs a) {
@@ -467,30 +472,53 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
   const int nv = dv >> 3;
   constexpr float kLog2e = 1.4426950408889634f;
   const float inv_cap = a.softcap > 0.f ? 1.f / a.softcap : 0.f;
+  // Keys and values of a tile are copies of their own: the next tile's keys are on their way from the scores on, its values from the products on. A lane
+  // copies one piece of a key, or, where rows are narrow, of every kpr-th key; rows behind the end are zeros
+  auto tile = [&](int kt, int& j0, int& j_end) {
+    j0 = kt < kept_tiles ? kt * kWdKeys : k_begin + (kt - kept_tiles) * kWdKeys, j_end = kt < kept_tiles ? kept_end : k_end;
+  };
+  auto row_of = [&](int kt) {   // the row of the pool that lane's key lies in
+    int j0, j_end;
+    tile(kt, j0, j_end);
+    const int j = j0 + lane;
+    return kt < n_tiles && j < j_end ? bt[j / a.page_size] * a.page_size + j % a.page_size : -1;
+  };
+  struct Lane { int keys, sub, c; bool works; };   // keys per round; the one of them that a lane copies a piece of, and which piece
+  auto lane_of = [&](int chunks) {
+    const int keys = max(1, 32 / chunks), sub = lane / chunks;
+    return Lane{keys, sub, (lane - sub * chunks) * 8, sub < keys};
+  };
+  auto copy = [&](int rows, const Lane& l, const bf16_t* base, uint32_t to, int pitch) {
+    const bf16_t* src = base + l.c;
+    uint32_t dst = to + (l.sub * pitch + l.c) * 2;
+    const uint32_t step = l.keys * pitch * 2;
+#pragma unroll 4
+    for (int key = l.sub; key - l.sub < kWdKeys; key += l.keys, dst += step) {
+      const int row = __shfl_sync(0xffffffffu, rows, key & 31);
+      if (l.works && key < kWdKeys) w_cp_async16_or_zero(dst, src + (row >= 0 ? (long long)row * roww : 0), row >= 0);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const Lane kl = lane_of(qchunks), vl = lane_of(vchunks);
+  const uint32_t kto = wsmem_u32(Ks), vto = wsmem_u32(Vs);
+  const bf16_t* kbase = a.pool + (kvh * a.maps + mp) * d;
+  const bf16_t* vbase = a.pool + a.G * a.maps * d + kvh * dv;
+  int mine = row_of(warp);
+  if (warp < n_tiles) copy(mine, kl, kbase, kto, pq), copy(mine, vl, vbase, vto, pv);
   __syncthreads();
   for (int kt = warp; kt < n_tiles; kt += warps) {
-    const int j0 = kt < kept_tiles ? kt * kWdKeys : k_begin + (kt - kept_tiles) * kWdKeys, j_end = kt < kept_tiles ? kept_end : k_end;
-    {
-      const int j = j0 + lane;
-      const int mine = j < j_end ? bt[j / a.page_size] * a.page_size + j % a.page_size : -1;   // the row of the pool that lane's key lies in
-      for (int e = lane; e < kWdKeys * pieces; e += 32) {   // the same number of rounds for every lane
-        const int key = e / pieces, c = e - key * pieces, row = __shfl_sync(0xffffffffu, mine, key);
-        bf16_t* dst = c < qchunks ? Ks + key * pq + c * 8 : Vs + key * pv + (c - qchunks) * 8;
-        if (row >= 0) {
-          const bf16_t* src = a.pool + (long long)row * roww + (c < qchunks ? (kvh * a.maps + mp) * d + c * 8 : a.G * a.maps * d + kvh * dv + (c - qchunks) * 8);
-          w_cp_async16(wsmem_u32(dst), src);
-        } else {
-          *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-        }
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncwarp();
-    }
+    int j0, j_end;
+    tile(kt, j0, j_end);
+    const bool more = kt + warps < n_tiles;
+    mine = row_of(kt + warps);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncwarp();
     float s[4][4];
 #pragma unroll
     for (int n = 0; n < 4; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
     const uint32_t q_base = wsmem_u32(Qs + ((lane & 7) + 8 * ((lane >> 3) & 1)) * pq + 8 * (lane >> 4));
     const uint32_t k_base = wsmem_u32(Ks + ((lane & 7) + 8 * (lane >> 4)) * pq + 8 * ((lane >> 3) & 1));
+#pragma unroll 4
     for (int kk = 0; kk < d; kk += 16) {
       uint32_t a0, a1, a2, a3;
       w_ldsm_x4(q_base + kk * 2, a0, a1, a2, a3);
@@ -502,6 +530,8 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
         w_mma_bf16(s[2 * n2 + 1], a0, a1, a2, a3, b2, b3);
       }
     }
+    __syncwarp();   // every lane is done with the keys
+    if (more) copy(mine, kl, kbase, kto, pq);
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
@@ -545,6 +575,9 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
     l1 = l1 * c1 + rs1;
 #pragma unroll
     for (int j = 0; j < NV; ++j) o[j][0] *= c0, o[j][1] *= c0, o[j][2] *= c1, o[j][3] *= c1;
+    if (more) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
     const uint32_t v_base = wsmem_u32(Vs + ((lane & 7) + 8 * ((lane >> 3) & 1)) * pv + 8 * (lane >> 4));
 #pragma unroll
     for (int kb16 = 0; kb16 < 2; ++kb16) {
@@ -559,7 +592,8 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
         }
       }
     }
-    __syncwarp();   // every lane is done with the tile
+    __syncwarp();   // ... and with the values
+    if (more) copy(mine, vl, vbase, vto, pv);
   }
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
   l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
@@ -1187,9 +1221,9 @@ extern "C" int omc_window_attn(const void* q, long long ldq, int T, int H, int G
 
 // Warps of a decode CTA. Eight finish a CTA soonest, and take more than half an SM's shared memory at widths of 128 (two such CTAs fit at 64): right
 // while every CTA runs in the first wave. Beyond that four, of which three CTAs share an SM: short contexts are then a matter of CTAs, each some
-// 9 us from its first load to its last store. 128 + 128 columns, us at 8 / 4 / 2 warps (one warp of 64 threads per CTA in brackets): 256 CTAs over
-// 16 keys 19 / 11 / 12 (12), over 512 37 / 35 / 59 (104); 2048 CTAs over 16 keys 123 / 45 / 30 (49), over 512 257 / 176 / 199 (301); 128 CTAs over
-// 512 20 / 32 / 58 (55).
+// 8 us from its first load to its last store. 128 + 128 columns, us at 8 / 4 / 2 warps: 256 CTAs over 16 keys 17 / 9 / 10, over 512 31 / 28 / 48; 2048 CTAs
+// over 16 keys 113 / 41 / 29, over 512 210 / 145 / 159; 128 CTAs over 512 16 / 26 / 49. 64 + 64 columns: 256 CTAs over 512 keys 13 / 17 / 27, 512 CTAs
+// 24 / 21 / 30, over 16 14 / 7 / 8.
 static int win_decode_warps(long long ctas, size_t smem_of_eight) {
   const int fit = smem_of_eight + 2048 <= 113 * 1024 ? 2 : 1;   // 1 KB of its own and 1 KB of the system's per CTA; 128 registers allow two as well
   return ctas <= 148LL * fit ? 8 : 4;
