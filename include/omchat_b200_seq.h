@@ -134,6 +134,16 @@ int omc_step_wait_warp_selfcheck(int32_t* out, void* stream);
 int omc_latent_decode_items(const int32_t* pos, const int32_t* slot, int B, int H, int parts, int window, int32_t* items,
                             int32_t* merges, void* stream);
 
+/* Work lists of prompt portions, in two calls of one thread: the first builds the list on the host and leaves its counts, the second fetches it. portions (host):
+ * int32 [n_portions][4], first row, rows, slot, first position of each request's consecutive rows.
+ * omc_latent_plan: the list of omc_latent_attn_mma; tiles of `tok` tokens; while there are fewer than target_ctas / 2 of them their keys are cut into up to max_parts
+ * ranges of at least min_keys, multiples of row_tile. counts (host): items, merges, partial results, tokens of the largest item; 8 items + 4 merges words.
+ * omc_window_plan: the list of omc_window_attn_mma; tiles also end where a chunk of positions does, where row_tile <= chunk < no_chunk. counts[0]: items of 4 words.
+ * omc_plan_words: the n words of the list built last on the calling thread, to host memory or, on `stream`, to the device (as parameters of kernels). */
+int omc_latent_plan(const int32_t* portions, int n_portions, int H, int tok, int target_ctas, int min_keys, int max_parts, int row_tile, int window, int32_t* counts);
+int omc_window_plan(const int32_t* portions, int n_portions, int tok, int row_tile, int chunk, int no_chunk, int32_t* counts);
+int omc_plan_words(int32_t* to, int n, int on_device, void* stream);
+
 /* Router with score correction and identity experts. z fp32 [T, ldz]: logits of E_tot = experts + identity outputs, and, when
  * has_gate, one more column: the shared expert's gate logit. s = softmax(z[:E_tot] + bias) (bias fp32 [E_tot] or NULL);
  * choice = s + correction (fp32 [E_tot] or NULL); the `top` largest choices (ties: lowest index) -> ids int32 [T, top];

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+from array import array
 from ctypes import c_char_p, c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -21,6 +22,7 @@ DT_F32, DT_BF16 = 0, 1
 ACT_NONE, ACT_RELU2, ACT_GELU_TANH, ACT_GELU_ERF, ACT_CLAMP_SWISH, ACT_SILU = 0, 1, 2, 3, 4, 5
 ROUTER_SOFTMAX, ROUTER_SIGMOID = 0, 1
 CONV_LINEAR, CONV_SILU = 0, 1
+PLAN_LAUNCH_WORDS = 8000  # of a work list that one launch brings to the device (csrc/plans.cu)
 LINEAR_TILE = 64  # rows per tile of omc_linear's tile -> group table
 
 SIGNATURES = {
@@ -69,6 +71,9 @@ SIGNATURES = {
     "omc_step_wait_selfcheck": (_I, [_P, _P]),
     "omc_step_wait_warp_selfcheck": (_I, [_P, _P]),
     "omc_latent_attn_mma": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
+    "omc_latent_plan": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _I, _P]),
+    "omc_window_plan": (_I, [_P, _I, _I, _I, _I, _I, _P]),
+    "omc_plan_words": (_I, [_P, _I, _I, _P]),
     "omc_latent_decode_items": (_I, [_P, _P, _I, _I, _I, _I, _P, _P, _P]),
     "omc_router_topk": (_I, [_P, _L, _I, _I, _I, _I, _P, _P, _I, _I, _I, _I, _F, _I, _P, _P, _P, _P, _P]),
     "omc_moe_plan_tiles": (_I, [_P, _I, _I, _I, _P, _P, _P, _P]),
@@ -277,6 +282,35 @@ def latent_attn_tcgen05_ok(H: int, r: int, dr: int, page_size: int) -> bool:
     return H <= MMA_ROWS and r % 128 == 0 and 0 < r <= 512 and dr <= 64 and dr % 16 == 0 and page_size % 64 == 0
 
 
+def _portion_words(portions):
+    """Portions as int32 words (an array that must live as long as its address is used), and how many there are."""
+    words = array("i")
+    n = 0
+    for p in portions:
+        words.extend(p)
+        n += 1
+    if len(words) != 4 * n:
+        raise OmcError("a portion is (first row, rows, slot, first position)")
+    return words, n
+
+
+def _check_host(rc: int, what: str):   # a call that launches nothing
+    if rc != 0:
+        raise OmcError(f"{what} failed ({rc}): {load().omc_last_error().decode(errors='replace')}")
+
+
+def _plan_words(n: int, device) -> torch.Tensor:
+    """The list that this thread has built last: int32 [n] on `device`."""
+    device = torch.device(device)
+    here = device.type == "cuda" and device.index in (None, torch.cuda.current_device())
+    out = torch.empty(n, dtype=torch.int32, device=device if here else "cpu")
+    _check_host(load().omc_plan_words(out, n, 1 if here else 0, _stream() if here else None), "omc_plan_words")
+    if here:
+        _core.add_launches(-(-n // PLAN_LAUNCH_WORDS))
+        return out
+    return out.to(device)
+
+
 class LatentAttnPlan:
     """Work list of one step for one head count (omc_latent_attn_mma): items, merge groups and the partial-result workspace.
     portions: host list of (first_row, n_rows, slot, first_pos) - the consecutive rows of each request in the packed batch.
@@ -285,18 +319,16 @@ class LatentAttnPlan:
 
     MAX_PARTS = 64  # key ranges one merge group may have (csrc/latent_attention.cu: kMergeMaxParts)
 
-    FEW_TILES = 24  # up to here a loop builds the lists sooner than array arithmetic, some 60 calls of a microsecond or two: 5 rows 18 us (120)
-
     def __init__(self, portions, H: int, device, target_ctas: int = 296, min_keys: int = 128, window: int = WINDOW_ALL, mma_sync: bool = False):
-        portions, tok = list(portions), max(1, MMA_ROWS // H)
-        base = sum(-(-n // tok) for _, n, _, _ in portions)                 # row tiles
-        build = self._by_loop if base <= self.FEW_TILES else self._by_arrays
-        numbers, self.n_items, self.n_merges, self.n_parts = build(portions, H, tok, base, target_ctas, min_keys, window)
-        self.max_rows = max((min(tok, n) for _, n, _, _ in portions), default=1) * H   # (token, head) pairs of the largest item
-        if mma_sync:    # whatever the shapes
-            self.max_rows = MMA_ROWS + 1
-        buf = torch.as_tensor(numbers, dtype=torch.int32).pin_memory().to(device, non_blocking=True)
-        self.items = buf[:self.n_items * 8]
+        tok = max(1, MMA_ROWS // H)
+        words, n = _portion_words(portions)
+        counts = array("i", (0, 0, 0, 0))
+        _check_host(load().omc_latent_plan(words.buffer_info()[0], n, H, tok, target_ctas, min_keys, self.MAX_PARTS, MMA_ROWS, window, counts.buffer_info()[0]),
+                    "omc_latent_plan")
+        self.n_items, self.n_merges, self.n_parts, most = counts
+        self.max_rows = MMA_ROWS + 1 if mma_sync else most * H   # (token, head) pairs of the largest item; mma_sync: the kernel for whatever shapes
+        buf = _plan_words(self.n_items * 8 + self.n_merges * 4, device)
+        self.items = buf[:self.n_items * 8] if self.n_merges else buf
         self.merges = buf[self.n_items * 8:] if self.n_merges else None
 
     @classmethod
@@ -325,7 +357,7 @@ class LatentAttnPlan:
 
     @classmethod
     def _by_arrays(cls, portions, H, tok, base, target_ctas, min_keys, window):
-        """The same lists."""
+        """The same lists by array arithmetic. Both say in Python what omc_latent_plan builds."""
         import numpy as np
         por = np.array(portions, dtype=np.int64).reshape(-1, 4)
         tiles = -(-por[:, 1] // tok)                                    # row tiles per portion
@@ -725,22 +757,10 @@ def window_attn_items(portions, rep: int, device, chunk: int = WINDOW_ALL) -> to
     """Work list of omc_window_attn_mma for one step: portions [(first_row, n_rows, slot, first_pos)] cut into tiles of 64 // rep
     tokens (rep = query heads per key/value head) -> int32 [n_items, 4] on the device. Tiles also end where a chunk does (a tile across
     the edge would walk the keys of both chunks), unless chunks are shorter than a key tile."""
-    import numpy as np
-    tok = MMA_ROWS // rep
-    parts = []
-    if MMA_ROWS <= chunk < WINDOW_ALL:
-        cut = []
-        for first_row, n, slot, p0 in portions:
-            while n > 0:
-                m = min(n, chunk - p0 % chunk)
-                cut.append((first_row, m, slot, p0))
-                first_row, n, p0 = first_row + m, n - m, p0 + m
-        portions = cut
-    for first_row, n, slot, p0 in portions:
-        st = np.arange(0, n, tok, dtype=np.int32)
-        parts.append(np.stack([first_row + st, np.minimum(tok, n - st), np.full_like(st, slot), p0 + st], axis=1))
-    flat = torch.from_numpy(np.concatenate(parts, axis=0).astype(np.int32))
-    return flat.pin_memory().to(device, non_blocking=True) if torch.device(device).type == "cuda" else flat
+    words, n = _portion_words(portions)
+    counts = array("i", (0,))
+    _check_host(load().omc_window_plan(words.buffer_info()[0], n, MMA_ROWS // rep, MMA_ROWS, chunk, WINDOW_ALL, counts.buffer_info()[0]), "omc_window_plan")
+    return _plan_words(counts[0] * 4, device).view(-1, 4)
 
 
 def window_attn_mma(q: torch.Tensor, H: int, G: int, d: int, dv: int, pool: torch.Tensor, block_table: torch.Tensor, page_size: int,

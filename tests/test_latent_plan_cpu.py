@@ -3,7 +3,7 @@ import random
 
 import pytest
 
-from omchat_b200.seqlib import MMA_ROWS, WINDOW_ALL, LatentAttnPlan
+from omchat_b200.seqlib import MMA_ROWS, WINDOW_ALL, LatentAttnPlan, window_attn_items
 
 
 def _portions(rng):
@@ -44,3 +44,34 @@ def test_the_loop_and_the_arrays_build_the_same_lists(seed):
     for i in range(n_merges):
         qrow, rows, part, n = numbers[8 * n_items + 4 * i:8 * n_items + 4 * i + 4]
         assert rows <= MMA_ROWS and 1 <= n <= LatentAttnPlan.MAX_PARTS and all(parts[part + j] * H == qrow for j in range(n))
+
+
+@pytest.mark.parametrize("seed", range(40))
+def test_the_library_builds_the_lists_of_the_loop(seed):
+    rng = random.Random(1000 + seed)
+    portions, H = _portions(rng), rng.choice([1, 3, 8, 16, 33, 64])
+    target, min_keys, window = rng.choice([2, 148, 296]), rng.choice([64, 128, 256]), rng.choice([1, 33, 256, 1024, WINDOW_ALL])
+    tok = MMA_ROWS // H
+    base = sum(-(-n // tok) for _, n, _, _ in portions)
+    numbers, n_items, n_merges, n_parts = LatentAttnPlan._by_loop(portions, H, tok, base, target, min_keys, window)
+    plan = LatentAttnPlan(portions, H, "cpu", target_ctas=target, min_keys=min_keys, window=window)
+    assert (plan.n_items, plan.n_merges, plan.n_parts) == (n_items, n_merges, n_parts)
+    assert plan.items.tolist() + (plan.merges.tolist() if plan.merges is not None else []) == list(numbers)
+    assert plan.max_rows == max((min(tok, n) for _, n, _, _ in portions), default=1) * H
+
+
+@pytest.mark.parametrize("seed", range(20))
+def test_windowed_items_cover_every_row_once_and_end_where_chunks_do(seed):
+    rng = random.Random(seed)
+    portions, rep, chunk = _portions(rng), rng.choice([1, 3, 4, 64]), rng.choice([33, 64, 100, 512, WINDOW_ALL])
+    items = window_attn_items(portions, rep, "cpu", chunk).tolist()
+    tok, want = MMA_ROWS // rep, []
+    for first_row, n, slot, p0 in portions:
+        row = 0
+        while row < n:
+            m = min(tok, n - row)
+            if MMA_ROWS <= chunk < WINDOW_ALL:       # tiles count from the portion's or the chunk's begin
+                m = min(m, chunk - (p0 + row) % chunk)
+            want.append([first_row + row, m, slot, p0 + row])
+            row += m
+    assert items == want
