@@ -30,7 +30,7 @@ LIBDIR = PKG / "_lib"
 LIB = LIBDIR / "libomchat_b200.so"
 SEQ_LIB = LIBDIR / "libomchat_b200_seq.so"
 SOURCES = ["capi.cu", "gemm_sm100.cu", "gemm_skinny.cu", "gemm_stream.cu", "gemv.cu", "rowops.cu", "attention.cu", "attention_sm100.cu", "decode_mega.cu", "preprocess.cu", "model_capi.cu", "moe.cu"]
-SEQ_SOURCES = ["attention_rows.cu", "capi.cu", "linear_any.cu", "linear_sm100.cu", "rownorm32.cu", "latent_attention.cu", "latent_attention_sm100.cu", "plans.cu", "router_moe.cu", "state_mixers.cu", "window_attention.cu", "window_attention_sm100.cu"]
+SEQ_SOURCES = ["attention_rows.cu", "capi.cu", "linear_any.cu", "linear_sm100.cu", "rownorm32.cu", "latent_attention.cu", "latent_attention_sm100.cu", "plans.cu", "router_moe.cu", "scan_chunk.cu", "state_mixers.cu", "window_attention.cu", "window_attention_sm100.cu"]
 DENSE_LIB = LIBDIR / "libomchat_b200_dense.so"
 DENSE_SOURCES = ["capi.cu", "gemm_sm100.cu", "gemm_skinny.cu", "rowops.cu", "moe.cu"]  # a subset of SOURCES that links on its own
 BASE_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xptxas", "-v"]

@@ -1,0 +1,73 @@
+// What the kernels of the linear-state recurrence share (state_mixers.cu describes it): their arguments, packed fp32 pairs, asynchronous copies.
+#pragma once
+#include "seq_common.cuh"
+
+namespace omc {
+
+__device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
+__device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
+
+struct ScanArgs {
+  const float* q;      // [T, ldq]: head g of kv_heads at columns g * dim
+  const float* k;
+  const float* v;      // [T, ldv]: head h at columns h * vdim
+  long long ldq, ldk, ldv;
+  int silu_in;         // q, k, v pass silu on the way in
+  int decay_mode;      // 0: decay_const[h]; 1: a[t, h]; 2: a[t, h * dim + i]  (1, 2: g = exp(-exp(A_log[h]) softplus(a + dt_bias))); 3: g = a[t, h * dim + i];
+                       // 4: g = sigmoid(a[t, h * dim + i] + dt_bias[h * dim + i])^decay_pow; 5: a[t, h * dim + i] holds g - 1
+                       // (4 and 5 apply the decay as S + (g - 1) S); 6: dt = softplus(a[t, h] + dt_bias[h]), g = exp(-exp(A_log[h]) dt),
+                       // u = dt v, o = S^T q + D[h] v (the decay as S + expm1(.) S)
+  float decay_pow;     // mode 4
+  float out_scale;     // o_t = out_scale * S^T q_t (a query scale, applied to the read-out)
+  const float* decay_const;
+  const float* a;
+  long long lda;
+  const float* A_log;    // fp32 [H]
+  const float* dt_bias;  // fp32 [H] (modes 1, 6) or [H * dim] (mode 2)
+  const float* D;        // fp32 [H] (mode 6) or NULL
+  const float* beta;     // raw [T, ldb]: beta = sigmoid; NULL: no delta correction (u = v)
+  long long ldb;
+  float* state;          // [slots][H][dim][vdim]
+  float* out;            // [T, ldo]
+  long long ldo;
+  const int32_t* row_begin;  // [P + 1] first row of every portion
+  const int32_t* pos;
+  const int32_t* slot;
+  int H, G, dim, vdim;
+  bool vec_state, vec_out;   // a thread's columns of the state / four outputs as one access
+  int long_from;             // portions of this many rows and more are scan_chunk_kernel's, the others the token-by-token kernels' (0: all of them are theirs)
+};
+
+__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));
+}
+__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));
+}
+
+// Packed fp32 pairs (sm_100: one instruction, two IEEE fp32 operations): the recurrence's state lives in such pairs.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
+constexpr int kScanLong = 64;   // rows from which a portion goes eight tokens at a time
+// The launch of scan_chunk.cu for the portions of at least a.long_from rows: the delta rule or per-channel decays (decay modes 0 and 1 with beta, 3, 5), 64 or 128 key
+// channels, inputs that need no preparation of their own, 16-byte rows of k, q, v, decays, outputs and states. Returns check_launch's code.
+int launch_scan_chunk(const ScanArgs& a, int rows, int portions, cudaStream_t st);
+
+}  // namespace omc

@@ -8,8 +8,9 @@
 // A portion that starts at position 0 starts from a zero state, so a slot needs no clearing when it is handed to a new request.
 // Everything here is fp32: state, decays and their logarithms, softplus / exponentials, step sizes, unit norms.
 //
-// The recurrence is evaluated token by token in every case - prompt portions and single decoded tokens run the same
-// instructions in the same order, which makes the result independent of how a prompt is cut. Its parallelism is over the
+// The recurrence is evaluated token by token - prompt portions and single decoded tokens run the same instructions
+// in the same order - except in portions of 64 rows and more of the delta rule or with a decay per key channel, which scan_chunk.cu takes eight tokens at a time: the
+// same sums in another order. The result does not depend on how a prompt is cut but in these last bits. Its parallelism is over the
 // independent COLUMNS of S: column j of a head's state only ever meets v[:, j], so a CTA owns 32 columns of one head of one
 // portion; a thread holds an eighth of the state elements of TWO neighbouring columns as packed fp32 pairs (one fma.rn.f32x2 serves
 // both columns, and a key or query value read from shared memory is used twice), and the eight lanes of a column pair finish the
@@ -18,13 +19,11 @@
 // Recurrences whose channels carry one or a few states of their own (selective scan, gated linear recurrent unit) follow below.
 #include <type_traits>
 
-#include "seq_common.cuh"
+#include "scan_args.cuh"
 
 namespace omc {
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
-__device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
-__device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 // sigmoid(z)^p - 1 = expm1(p * log sigmoid(z)), log sigmoid(z) = -softplus(-z). The decay is kept as its distance from 1: rounded to
 // fp32 itself, a decay close to 1 loses most of the digits of 1 - decay, and the state multiplies by it once per token.
 __device__ __forceinline__ float sigmoid_pow_m1_f(float z, float p) { return expm1f(-p * softplus_f(-z)); }
@@ -284,61 +283,6 @@ __global__ void __launch_bounds__(256) conv_state_save_kernel(const float* __res
 // ---- linear-state recurrence ----------------------------------------------------------------------------------------------
 constexpr int kScanLanes = 8, kScanGroups = 16, kScanThreads = kScanLanes * kScanGroups, kScanCpt = 2;
 
-struct ScanArgs {
-  const float* q;      // [T, ldq]: head g of kv_heads at columns g * dim
-  const float* k;
-  const float* v;      // [T, ldv]: head h at columns h * vdim
-  long long ldq, ldk, ldv;
-  int silu_in;         // q, k, v pass silu on the way in
-  int decay_mode;      // 0: decay_const[h]; 1: a[t, h]; 2: a[t, h * dim + i]  (1, 2: g = exp(-exp(A_log[h]) softplus(a + dt_bias))); 3: g = a[t, h * dim + i];
-                       // 4: g = sigmoid(a[t, h * dim + i] + dt_bias[h * dim + i])^decay_pow; 5: a[t, h * dim + i] holds g - 1
-                       // (4 and 5 apply the decay as S + (g - 1) S); 6: dt = softplus(a[t, h] + dt_bias[h]), g = exp(-exp(A_log[h]) dt),
-                       // u = dt v, o = S^T q + D[h] v (the decay as S + expm1(.) S)
-  float decay_pow;     // mode 4
-  float out_scale;     // o_t = out_scale * S^T q_t (a query scale, applied to the read-out)
-  const float* decay_const;
-  const float* a;
-  long long lda;
-  const float* A_log;    // fp32 [H]
-  const float* dt_bias;  // fp32 [H] (modes 1, 6) or [H * dim] (mode 2)
-  const float* D;        // fp32 [H] (mode 6) or NULL
-  const float* beta;     // raw [T, ldb]: beta = sigmoid; NULL: no delta correction (u = v)
-  long long ldb;
-  float* state;          // [slots][H][dim][vdim]
-  float* out;            // [T, ldo]
-  long long ldo;
-  const int32_t* row_begin;  // [P + 1] first row of every portion
-  const int32_t* pos;
-  const int32_t* slot;
-  int H, G, dim, vdim;
-  bool vec_state, vec_out;   // a thread's columns of the state / four outputs as one access
-};
-
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));
-}
-__device__ __forceinline__ void cp_async16(float* dst, const float* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));
-}
-
-// Packed fp32 pairs (sm_100: one instruction, two IEEE fp32 operations): the recurrence's state lives in such pairs.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 // Shared-memory place of key channel i: lane l = i / DPT owns DPT consecutive channels (read as float4), and a gap of four floats
 // between the lanes' blocks moves them to different banks (the eight float4 reads of a quarter warp, at strides of 12, 20 or 36 floats, fall on different banks).
 template <int DPT>
@@ -360,7 +304,6 @@ __device__ __forceinline__ int scan_place(int i) { return (i / DPT) * (DPT + 4) 
 // several tokens at 64 or 128 channels go to scan_rows_kernel below; measured here, 16 heads of 128 x 128, four portions of 1024, 777, 1024, 301
 // tokens with per-channel decays: 435 us (560 with pairs of columns, a doubled key and a shuffled read-out per token); one token of 32 requests, step
 // sizes: 22 us = 6.1 TB/s (42).
-enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
 template <int DPT, int TOK>
 __host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
   return TOK * kScanLanes * (DPT + 4) * (chan ? 3 : 2) + TOK * cols + 2 * (TOK < 4 ? 4 : TOK);
@@ -380,7 +323,7 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
   const int h = blockIdx.y, kvh = h / (a.H / a.G);
   const int col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
-  if (r1 <= r0) return;
+  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
   // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
   // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
   const int tid = threadIdx.x, lane = WIDE ? tid / kScanGroups : tid & (kScanLanes - 1), cg = WIDE ? tid % kScanGroups : tid / kScanLanes;
@@ -720,7 +663,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
   const bool minus1 = KIND == kScanStep || a.decay_mode == 5;
   const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
-  if (r1 <= r0) return;
+  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
   const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
   const bool in = col < a.vdim;   // a thread's columns all exist or none does
   const float A = KIND == kScanStep || a.decay_mode == 1 ? expf(a.A_log[h]) : 0.f;
@@ -1624,7 +1567,7 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   if (dim > 256) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: key width above 256");
   if (portions > 65535 || H > 65535) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: more than 65535 portions or heads");
   ScanArgs s{q, k, v, ldq, ldk, ldv, silu_in, decay_mode, decay_pow, out_scale, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo,
-             row_begin, pos, slot, H, G, dim, vdim, false, false};
+             row_begin, pos, slot, H, G, dim, vdim, false, false, 0};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int dpt = dim <= 32 ? 4 : (dim <= 64 ? 8 : (dim <= 128 ? 16 : 32));   // key channels per thread: dim / 8 lanes, rounded up to a float4
   const bool chan = decay_mode >= 2 && decay_mode <= 5;
@@ -1644,6 +1587,11 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   // portions of several tokens whose inputs are ready: scan_rows_kernel
   const bool ready = !silu_in && (decay_mode == 0 || decay_mode == 1 || decay_mode == 3 || decay_mode >= 5);
   if (!one && vec && ready && (dim == 64 || dim == 128) && s.vec_out && s.vec_state) {
+    if (rows >= kScanLong && (chan || (beta != nullptr && decay_mode <= 1))) {   // long portions: scan_chunk_kernel; whichever are left, the kernels below
+      s.long_from = kScanLong;
+      const int rc = launch_scan_chunk(s, rows, portions, st);
+      if (rc != OMC_OK || portions == 1) return rc;
+    }
     auto go = [&](auto dim_c, auto cpt_c, auto kind_c, auto chan_c) {
       constexpr int DIM = decltype(dim_c)::value, CPT = decltype(cpt_c)::value, KIND = decltype(kind_c)::value, COLS = kSrThreads / kScanLanes * CPT;
       constexpr bool CHAN = decltype(chan_c)::value;

@@ -1,0 +1,109 @@
+"""The recurrence's kernel for long portions (64 rows and more of the delta rule or with per-channel decays): against float64 over whole and ragged stages of eight tokens
+and column counts, beside short portions that keep the bits of single tokens, from a fresh state and one that is carried on."""
+import pytest
+import torch
+
+from omchat_b200 import seqlib
+
+pytestmark = pytest.mark.gpu
+KINDS = ["delta", "delta_const", "given", "given_plain", "given_minus_one"]
+
+
+def _i32(x):
+    return torch.tensor(x, dtype=torch.int32, device="cuda")
+
+
+class Case:
+    def __init__(self, kind, H, G, dim, vdim, lens, first):
+        gen = torch.Generator().manual_seed(H * dim + vdim)
+        rn = lambda *s: torch.randn(*s, generator=gen).cuda()  # noqa: E731
+        self.kind, self.H, self.G, self.dim, self.vdim, self.lens, self.first = kind, H, G, dim, vdim, lens, first
+        T = sum(lens)
+        self.q, self.v = rn(T, G * dim) * dim ** -0.5, rn(T, H * vdim)
+        self.k = torch.nn.functional.normalize(rn(T, G, dim), dim=-1).reshape(T, -1).contiguous()
+        self.a, self.beta, self.A_log, self.dtb = rn(T, H * dim if "given" in kind else H), rn(T, H), rn(H) - 1, rn(H) - 1
+        self.const = torch.sigmoid(rn(H) + 2)
+        if "given" in kind:
+            self.a = torch.sigmoid(self.a + 3) - (1.0 if kind == "given_minus_one" else 0.0)
+        self.starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
+        self.S0 = rn(len(lens), H, dim, vdim) if first else torch.zeros(len(lens), H, dim, vdim, device="cuda")
+
+    def run(self, rows=slice(None), lens=None, slots=None, S=None, first=None):
+        lens = self.lens if lens is None else lens
+        slots = range(len(lens)) if slots is None else slots
+        S = self.S0.clone() if S is None else S
+        first = self.first if first is None else first
+        kw = {"delta": dict(a=self.a[rows], A_log=self.A_log, dt_bias=self.dtb, beta=self.beta[rows]), "delta_const": dict(decay_const=self.const, beta=self.beta[rows], out_scale=0.5),
+              "given": dict(a=self.a[rows], beta=self.beta[rows], channel_decay=True, decay_given=True),
+              "given_plain": dict(a=self.a[rows], channel_decay=True, decay_given=True),
+              "given_minus_one": dict(a=self.a[rows], channel_decay=True, decay_given=True, sigmoid_pow=1.0)}[self.kind]
+        out = torch.empty(sum(lens), self.H * self.vdim, device="cuda")
+        begin = _i32([sum(lens[:i]) for i in range(len(lens) + 1)])
+        pos, slot = _i32([first + p for n in lens for p in range(n)]), _i32([s for s, n in zip(slots, lens) for _ in range(n)])
+        seqlib.linear_state_scan(self.q[rows], self.k[rows], self.v[rows], S, out, begin, len(lens), pos, slot, self.H, self.G, self.dim, self.vdim, **kw)
+        return out, S
+
+    def exact(self):
+        d = lambda x: x.double()  # noqa: E731
+        H, dim = self.H, self.dim
+        q, k = (d(x).view(-1, self.G, dim).repeat_interleave(H // self.G, 1) for x in (self.q, self.k))
+        v, b = d(self.v).view(-1, H, self.vdim), torch.sigmoid(d(self.beta))
+        if self.kind == "delta":
+            g = torch.exp(-torch.exp(d(self.A_log)) * torch.nn.functional.softplus(d(self.a) + d(self.dtb), threshold=1e9))[..., None]
+        elif self.kind == "delta_const":
+            g = d(self.const)[None, :, None].expand(len(v), H, 1)
+        else:
+            g = (d(self.a) + (1.0 if self.kind == "given_minus_one" else 0.0)).view(-1, H, dim)
+        S, out = d(self.S0), torch.empty_like(v)
+        for i, n in enumerate(self.lens):
+            for t in range(self.starts[i], self.starts[i] + n):
+                S[i] *= g[t][..., None]
+                u = v[t] if self.kind in ("given_plain", "given_minus_one") else b[t][:, None] * (v[t] - torch.einsum("hdv,hd->hv", S[i], k[t]))
+                S[i] += k[t][..., None] * u[:, None]
+                out[t] = torch.einsum("hdv,hd->hv", S[i], q[t])
+        return out.reshape(len(v), -1) * (0.5 if self.kind == "delta_const" else 1.0), S
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("H,G,vdim", [(3, 1, 20), (2, 2, 132), (4, 2, 64)])
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("first", [0, 5])
+def test_long_portions_are_as_exact_as_fp32_sums(kind, H, G, dim, vdim, first):
+    c = Case(kind, H, G, dim, vdim, [64, 9, 71, 130], first)
+    out, S = c.run()
+    want, Sw = c.exact()
+    # sums of dim + 8 products, a rounding of the state by a decay per stage: a few units of 2^-24 of the largest terms, which 2-norms see as about one
+    assert _rel(out, want) < 5e-7 and _rel(S, Sw) < 5e-7, (_rel(out, want), _rel(S, Sw))
+    # the short portion beside them: the bits of one token at a time; a long one alone: the bits it has in company
+    S1 = c.S0.clone()
+    for t in range(9):
+        one, _ = c.run(slice(64 + t, 65 + t), [1], [1], S1, first + t)
+        assert torch.equal(one[0], out[64 + t])
+    assert torch.equal(S1[1], S[1])
+    alone, S2 = c.run(slice(73, 144), [71], [2])
+    assert torch.equal(alone, out[73:144]) and torch.equal(S2[2], S[2])
+
+
+@pytest.mark.parametrize("kind", ["delta", "given", "given_plain"])
+def test_what_is_not_finite_reaches_no_earlier_token_and_no_other_column(kind):
+    c = Case(kind, 2, 1, 128, 64, [75], 0)
+    clean, _ = c.run()
+    c.v[37, 5], c.v[61, 70] = torch.inf, torch.nan
+    out, S = c.run()
+    out, clean = out.view(75, 2, 64), clean.view(75, 2, 64)
+    hit = torch.zeros(75, 2, 64, dtype=torch.bool, device="cuda")
+    hit[37:, 0, 5] = hit[61:, 1, 6] = True
+    assert torch.equal(out[~hit], clean[~hit]) and not torch.isfinite(out[hit]).any()
+    assert torch.isfinite(S).all(2).view(-1).sum() == 2 * 64 - 2
+
+
+def test_many_portions_of_which_few_are_long():
+    lens = [3] * 140 + [64, 200, 1]      # more portions than a CTA sorts by length
+    c = Case("delta", 2, 1, 64, 36, lens, 0)
+    out, S = c.run()
+    want, Sw = c.exact()
+    assert _rel(out, want) < 5e-7 and _rel(S, Sw) < 5e-7
