@@ -4,7 +4,15 @@
 
 namespace omc {
 
-__device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
+// x / y for y >= 1: the reciprocal with one Newton step, within a unit of the last place, in five instructions without a branch (a division that serves every exponent takes
+// ten, and a call where its operands are small)
+__device__ __forceinline__ float over(float x, float y) {
+  y = y > 8e37f ? 8e37f : y;   // its reciprocal is a normal number; NaN stays NaN
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  return x * fmaf(r, fmaf(-y, r, 1.f), r);
+}
+__device__ __forceinline__ float sigmoid_f(float z) { return over(1.f, 1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 struct ScanArgs {

@@ -23,7 +23,7 @@
 
 namespace omc {
 
-__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
+__device__ __forceinline__ float silu_f(float z) { return over(z, 1.f + expf(-z)); }
 // sigmoid(z)^p - 1 = expm1(p * log sigmoid(z)), log sigmoid(z) = -softplus(-z). The decay is kept as its distance from 1: rounded to
 // fp32 itself, a decay close to 1 loses most of the digits of 1 - decay, and the state multiplies by it once per token.
 __device__ __forceinline__ float sigmoid_pow_m1_f(float z, float p) { return expm1f(-p * softplus_f(-z)); }
@@ -102,7 +102,8 @@ struct ConvUnit {   // unit vectors behind the convolution: the first `channels`
 // shared memory. The same sums of taps as causal_conv_silu_kernel. UNIT: groups that a power of two of lanes of a warp holds are made unit vectors by
 // shuffles among them (every warp is whole: ch is a multiple of 128); causal_conv_silu_kernel, a block of rows in shared memory, is for other
 // groups. Nothing that a tile reads waits for another load of it, except for ring entries. 3126 rows of 4096 channels with unit queries and keys of
-// 128: 73 us there, 40 here (2.6 TB/s; 42 with slots looked up in front of the rows before the tile); 6144 channels: 45 (3.4 TB/s).
+// 128: 73 us there, 34 here (3.0 TB/s; 40 with a division in the activation, 42 with slots looked up in front of the rows before the tile); 6144 channels: 37
+// (4.1 TB/s; 45 with a division). What bounds it: half of the cycles the activation's instructions, otherwise the rows.
 template <typename TW, typename TY, int TAPS, int ROWS, bool UNIT>
 __global__ void __launch_bounds__(128) causal_conv_rows_kernel(const float* __restrict__ x, long long ldx, int T, int ch,
                                                                const TW* __restrict__ w, const TW* __restrict__ bias,
@@ -933,7 +934,7 @@ __global__ void __launch_bounds__(256) gated_rms_kernel(const float* __restrict_
 
 // Both norms for groups that LANES neighbouring lanes hold in PIECES pieces of four columns each (n = 4 LANES PIECES): x and the gate are read once, all
 // of it before anything is waited for, and no two warps meet. FRONT: the gate in front of the norm and a weight for every column of the row, else behind
-// it and one weight of n columns for all groups. 3126 rows: 8 parts of 512 with a bf16 gate in front 38 -> 22 us, 16 groups of 128 with an fp32 gate behind 29 -> 16
+// it and one weight of n columns for all groups. 3126 rows: 8 parts of 512 with a bf16 gate in front 38 -> 19 us (22 with a division in the gate), 16 groups of 128 with an fp32 gate behind 29 -> 15
 // (a block per part, a warp per group reading single columns twice).
 template <typename TG, typename TW, typename TY, int LANES, int PIECES, bool FRONT>
 __global__ void __launch_bounds__(256) group_rms_kernel(const float* __restrict__ x, long long ldx, int groups, long long total, const TW* __restrict__ w, float eps,
