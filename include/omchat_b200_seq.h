@@ -134,6 +134,12 @@ int omc_step_wait_warp_selfcheck(int32_t* out, void* stream);
 int omc_latent_decode_items(const int32_t* pos, const int32_t* slot, int B, int H, int parts, int window, int32_t* items,
                             int32_t* merges, void* stream);
 
+/* omc_latent_attn_mma for a step of one row per request, which needs no work list: row t at position pos[t] of slot[t], its keys in `parts` <= 64 ranges (ws_o / ws_ml
+ * as for T * parts partial results). For the shapes of the tcgen05 kernel; the same bits as with the list of omc_latent_decode_items. */
+int omc_latent_attn_decode(const void* qcat, int T, int H, int r, int dr, const void* pool, const int32_t* block_table, int max_pages, int page_size,
+                           const int32_t* pos, const int32_t* slot, int parts, const float* sink, int window, const float* gate, long long ldg, float scale,
+                           void* out, int out_dt, float* ws_o, float* ws_ml, void* stream);
+
 /* Work lists of prompt portions, in two calls of one thread: the first builds the list on the host and leaves its counts, the second fetches it. portions (host):
  * int32 [n_portions][4], first row, rows, slot, first position of each request's consecutive rows.
  * omc_latent_plan: the list of omc_latent_attn_mma; tiles of `tok` tokens; while there are fewer than target_ctas / 2 of them their keys are cut into up to max_parts

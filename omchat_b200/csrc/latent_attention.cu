@@ -13,6 +13,7 @@
 //                        an optional sink term exp(sink_h) that only enlarges the denominator
 // Rows of a step are addressed by (slot, position): a row sees cache entries 0..position of its slot, whether they were written
 // by this step or by earlier ones, so portions of prompts and single decoded tokens are the same case.
+#include "latent_decode.cuh"
 #include "seq_common.cuh"
 
 namespace omc {
@@ -756,14 +757,15 @@ __global__ void __launch_bounds__(128 * VS) latent_attn_mma_kernel(LatMmaArgs a)
 // four parts' loads in flight per thread (a warp that walked parts and columns one load at a time spent 70 us on latency).
 constexpr int kMergeMaxParts = 64;
 template <typename TO>
-__global__ void __launch_bounds__(128) latent_attn_merge_kernel(const int32_t* __restrict__ merges, const float* __restrict__ ws_o,
+__global__ void __launch_bounds__(128) latent_attn_merge_kernel(const int32_t* __restrict__ merges, int parts, const float* __restrict__ ws_o,
                                                                 const float* __restrict__ ws_ml, const float* __restrict__ sink,
                                                                 const float* __restrict__ gate, long long ldg, int H, int r,
                                                                 TO* __restrict__ out) {
   __shared__ float s_f[kMergeMaxParts];
   __shared__ float s_inv;
-  const int32_t* mg = merges + blockIdx.x * 4;
-  const int qrow0 = mg[0], n_rows = mg[1], part0 = mg[2], n_parts = mg[3];
+  const int32_t* mg = merges + blockIdx.x * 4;   // NULL: one row per request in `parts` ranges
+  const int b = blockIdx.x, qrow0 = merges != nullptr ? mg[0] : b * H, n_rows = merges != nullptr ? mg[1] : H, part0 = merges != nullptr ? mg[2] : b * parts,
+            n_parts = merges != nullptr ? mg[3] : parts;
   const int row = blockIdx.y;
   if (row >= n_rows) return;
   if (threadIdx.x < 32) {
@@ -804,22 +806,22 @@ __global__ void __launch_bounds__(128) latent_attn_merge_kernel(const int32_t* _
 }
 
 // Work list of a decode-only step written on the device (so that the step can be replayed from a CUDA graph while the contexts
-// grow): row b at position pos[b] sees the last min(pos[b] + 1, window) keys, cut into `parts` ranges of whole 64-key tiles (ranges past the end stay
-// empty and contribute nothing to the merge).
+// grow). Ranges past the end stay empty and contribute nothing to the merge.
 __global__ void latent_decode_items_kernel(const int32_t* __restrict__ pos, const int32_t* __restrict__ slot, int B, int H, int parts, int window,
                                            int32_t* __restrict__ items, int32_t* __restrict__ merges) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= B * parts) return;
   const int b = i / parts, j = i - b * parts;
-  const int keys = pos[b] + 1, low = max(0, keys - window);
-  const int span = ((keys - low + parts - 1) / parts + kMmaKeys - 1) / kMmaKeys * kMmaKeys;
+  static_assert(kMmaKeys == 64, "");
+  int from, to;
+  latent_decode_range(pos[b], window, parts, j, from, to);
   int32_t* it = items + (long long)i * 8;
   it[0] = b;
   it[1] = 1;
   it[2] = slot[b];
   it[3] = pos[b];
-  it[4] = min(low + j * span, keys);
-  it[5] = min(low + (j + 1) * span, keys);
+  it[4] = from;
+  it[5] = to;
   it[6] = parts > 1 ? i : -1;
   it[7] = 0;
   if (j == 0 && parts > 1) {
@@ -834,8 +836,8 @@ __global__ void latent_decode_items_kernel(const int32_t* __restrict__ pos, cons
 // latent_attention_sm100.cu
 bool latent_sm100_ok(int max_rows, int r, int dr, int page_size, const void* q, const void* pool);
 int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size,
-                 const int32_t* items, int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
-                 float* ws_ml, cudaStream_t st);
+                 const int32_t* items, const LatentDecodeRows& rows, int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale,
+                 void* out, int out_dt, float* ws_o, float* ws_ml, cudaStream_t st);
 
 template <int VS, int NV, typename TO>
 static int launch_lat_mma_t(const LatMmaArgs& a, int n_items, size_t smem, cudaStream_t st) {
@@ -854,6 +856,13 @@ template <int VS, int NV>
 static int launch_lat_mma(const LatMmaArgs& a, int out_dt, int n_items, size_t smem, cudaStream_t st) {
   if (out_dt == OMC_DT_BF16) return launch_lat_mma_t<VS, NV, bf16_t>(a, n_items, smem, st);
   return launch_lat_mma_t<VS, NV, float>(a, n_items, smem, st);
+}
+
+static int launch_lat_merge(const int32_t* merges, int parts, int n, int rows, const float* ws_o, const float* ws_ml, const float* sink, const float* gate, long long ldg, int H,
+                            int r, void* out, int out_dt, cudaStream_t st) {
+  if (out_dt == OMC_DT_BF16) latent_attn_merge_kernel<bf16_t><<<dim3(n, rows), 128, 0, st>>>(merges, parts, ws_o, ws_ml, sink, gate, ldg, H, r, static_cast<bf16_t*>(out));
+  else latent_attn_merge_kernel<float><<<dim3(n, rows), 128, 0, st>>>(merges, parts, ws_o, ws_ml, sink, gate, ldg, H, r, static_cast<float*>(out));
+  return check_launch("omc_latent_attn_merge");
 }
 
 }  // namespace omc
@@ -884,6 +893,7 @@ extern "C" int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, i
     return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: bad argument");
   if (r <= 0 || r % 16 != 0 || r > 512 || dr < 0 || dr % 16 != 0 || H > kMmaRows)
     return set_error(OMC_ERR_SHAPE, "omc_latent_attn_mma: latent width a multiple of 16 up to 512, rotated width a multiple of 16, at most 64 heads");
+  if (reinterpret_cast<uintptr_t>(qcat) % 16 || reinterpret_cast<uintptr_t>(pool) % 16) return set_error(OMC_ERR_SHAPE, "omc_latent_attn_mma: queries and cached rows lie on 16-byte boundaries");
   if (n_items == 0) return OMC_OK;
   const int D = r + dr;
   const size_t extra = r > 128 ? kPairBytes : 0;  // several warps per row group exchange probabilities
@@ -900,18 +910,30 @@ extern "C" int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, i
   int rc;
   if (out_dt != OMC_DT_F32 && out_dt != OMC_DT_BF16) return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: unknown output dtype");
   if (latent_sm100_ok(max_rows, r, dr, page_size, qcat, pool))
-    rc = latent_sm100(qcat, (long long)T * H, H, r, dr, pool, block_table, max_pages, page_size, items, n_items, max_rows, sink, window, gate, ldg, scale,
+    rc = latent_sm100(qcat, (long long)T * H, H, r, dr, pool, block_table, max_pages, page_size, items, LatentDecodeRows{}, n_items, max_rows, sink, window, gate, ldg, scale,
                       out, out_dt, ws_o, ws_ml, st);
   else if (r <= 64) rc = launch_lat_mma<1, 8>(a, out_dt, n_items, smem, st);
   else if (r <= 128) rc = launch_lat_mma<1, 16>(a, out_dt, n_items, smem, st);
   else if (r <= 256) rc = launch_lat_mma<2, 16>(a, out_dt, n_items, smem, st);
   else rc = launch_lat_mma<4, 16>(a, out_dt, n_items, smem, st);  // 16 warps: four per row group, 128 value columns and 16 keys each
   if (rc != OMC_OK || n_merges == 0) return rc;
-  if (out_dt == OMC_DT_BF16)
-    latent_attn_merge_kernel<bf16_t><<<dim3(n_merges, kMmaRows), 128, 0, st>>>(merges, ws_o, ws_ml, sink, gate, ldg, H, r, static_cast<bf16_t*>(out));
-  else
-    latent_attn_merge_kernel<float><<<dim3(n_merges, kMmaRows), 128, 0, st>>>(merges, ws_o, ws_ml, sink, gate, ldg, H, r, static_cast<float*>(out));
-  return check_launch("omc_latent_attn_merge");
+  return launch_lat_merge(merges, 1, n_merges, max_rows < kMmaRows ? max_rows : kMmaRows, ws_o, ws_ml, sink, gate, ldg, H, r, out, out_dt, st);
+}
+
+extern "C" int omc_latent_attn_decode(const void* qcat, int T, int H, int r, int dr, const void* pool, const int32_t* block_table, int max_pages, int page_size,
+                                      const int32_t* pos, const int32_t* slot, int parts, const float* sink, int window, const float* gate, long long ldg, float scale,
+                                      void* out, int out_dt, float* ws_o, float* ws_ml, void* stream) {
+  if (qcat == nullptr || pool == nullptr || block_table == nullptr || pos == nullptr || slot == nullptr || out == nullptr || T < 0 || H <= 0 || page_size <= 0 || max_pages <= 0 ||
+      parts < 1 || parts > kMergeMaxParts || window < 1 || (parts > 1 && (ws_o == nullptr || ws_ml == nullptr)) || (out_dt != OMC_DT_F32 && out_dt != OMC_DT_BF16))
+    return set_error(OMC_ERR_ARG, "omc_latent_attn_decode: bad argument");
+  if (r <= 0 || r > 512 || H > kMmaRows || !latent_sm100_ok(H, r, dr, page_size, qcat, pool) || (long long)T * parts > 0x7fffffff)
+    return set_error(OMC_ERR_SHAPE, "omc_latent_attn_decode: shape not supported (omc_latent_attn_mma takes others)");
+  if (T == 0) return OMC_OK;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int rc = latent_sm100(qcat, (long long)T * H, H, r, dr, pool, block_table, max_pages, page_size, nullptr, LatentDecodeRows{pos, slot, parts}, T * parts, H, sink, window, gate,
+                              ldg, scale, out, out_dt, ws_o, ws_ml, st);
+  if (rc != OMC_OK || parts == 1) return rc;
+  return launch_lat_merge(nullptr, parts, T, H, ws_o, ws_ml, sink, gate, ldg, H, r, out, out_dt, st);
 }
 
 extern "C" int omc_latent_decode_items(const int32_t* pos, const int32_t* slot, int B, int H, int parts, int window, int32_t* items,

@@ -25,6 +25,7 @@
 // kernel in brackets): portions of 1024, 777, 1024 behind 1024 and 301 rows 244 us (260 / 722); 4 x 1024 rows of 32 heads 460 us (495 / 1136); 2048 rows
 // 193 us (202 / 653); a decode step of 32 rows over 700 to 2100 keys, merge included, 34 us (33 / 79). By cp.async with a wait and a fence of the load
 // warps in front of every pair: 359, 660, 297 and 52 us.
+#include "latent_decode.cuh"
 #include "sm100_step.cuh"
 
 namespace omc {
@@ -40,7 +41,10 @@ struct LatSmArgs {
   const bf16_t* pool;
   long long q_rows;
   const int32_t* bt;
-  const int32_t* items;   // as LatMmaArgs of latent_attention.cu
+  const int32_t* items;   // as LatMmaArgs of latent_attention.cu; NULL: one row per request, at (slot, pos), in `parts` ranges of its keys
+  const int32_t* pos;
+  const int32_t* slot;
+  int parts;
   const float* sink;
   void* out;
   float* ws_o;
@@ -118,9 +122,19 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_attn_sm100_kernel(const 
   uint8_t* qs = base;                        // [nc][NR][128 B]
   uint8_t* ks = base + a.nc * QCHUNK;        // [nc][128][128 B]
   if (threadIdx.x == 32) tma_prefetch_desc(&tm_q);
-  const int32_t* it = a.items + blockIdx.x * 8;
-  const int first_row = it[0], n_tok = it[1], slot = it[2], first_pos = it[3], kb = it[4], part = it[6];
-  const int k_end = min(it[5], first_pos + n_tok), n_rows = n_tok * a.H;
+  int first_row, n_tok = 1, slot, first_pos, kb, k_end, part;
+  if (a.items != nullptr) {
+    const int32_t* it = a.items + blockIdx.x * 8;
+    first_row = it[0], n_tok = it[1], slot = it[2], first_pos = it[3], kb = it[4], part = it[6];
+    k_end = min(it[5], first_pos + n_tok);
+  } else {
+    first_row = blockIdx.x / a.parts;
+    const int i = blockIdx.x - first_row * a.parts;
+    slot = a.slot[first_row], first_pos = a.pos[first_row];
+    latent_decode_range(first_pos, a.window, a.parts, i, kb, k_end);
+    part = a.parts > 1 ? (int)blockIdx.x : -1;
+  }
+  const int n_rows = n_tok * a.H;
   const int k0 = kb & ~63;                   // boxes of 64 keys start where pages may
   const int n_tiles = k_end > kb ? (k_end - k0 + kKT - 1) / kKT : 0;
   const int nm = a.r >> 7;                   // 128-dimension tiles of the output
@@ -462,10 +476,10 @@ static int ls_launch(const CUtensorMap& tq, const LatSmArgs& a, int n_items, int
 }
 
 int latent_sm100(const void* q, long long q_rows, int H, int r, int dr, const void* pool, const int32_t* bt, int max_pages, int page_size, const int32_t* items,
-                 int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
+                 const LatentDecodeRows& rows, int n_items, int max_rows, const float* sink, int window, const float* gate, long long ldg, float scale, void* out, int out_dt, float* ws_o,
                  float* ws_ml, cudaStream_t st) {
   const int D = r + dr, nr = max_rows <= 16 ? 16 : (max_rows <= 32 ? 32 : 64);
-  LatSmArgs a{static_cast<const bf16_t*>(q), static_cast<const bf16_t*>(pool), q_rows, bt, items, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D,
+  LatSmArgs a{static_cast<const bf16_t*>(q), static_cast<const bf16_t*>(pool), q_rows, bt, items, rows.pos, rows.slot, rows.parts, sink, out, ws_o, ws_ml, gate, ldg, window, max_pages, page_size, H, r, D,
               (D + 63) / 64, {}, false, 0, scale * 1.4426950408889634f, nullptr};
   const int smem = ls_smem(nr, r, D, &a);
   const int cols = (r / 128 + 1) * nr;

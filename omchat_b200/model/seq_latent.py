@@ -40,7 +40,7 @@ class RotaryTables:
 class LatentAttention:
     """Chooses the kernel and keeps the work lists. `plans` describes one step and collects its lists: {"portions": [...]} as the host
     knows the batch, {"decode_parts": n} or {"decode_keys": n} for a step of one row per request (the lists are then written on the
-    device, in buffers that live as long as this object, so that a captured graph may use them), or None: the plain kernel."""
+    device, in buffers that live as long as this object, so that a captured graph may use them; the tcgen05 kernel needs none), or None: the plain kernel."""
 
     def __init__(self, device, dtype: torch.dtype):
         self.device, self.dtype = device, dtype
@@ -61,11 +61,14 @@ class LatentAttention:
             else:
                 keys = min(window, plans["decode_keys"]) if "decode_keys" in plans else 0
                 parts = plans["decode_parts"] if "decode_parts" in plans else self._decode_parts(T, keys, tcgen05)
-                key = (T, H, parts, window)
-                plan = self._decode_plans.get(key)
-                if plan is None:
-                    plan = self._decode_plans[key] = seqlib.DecodeAttnPlan(T, H, parts, self.device, window=window)
-                plan.fill(pos, slot)
+                if tcgen05:
+                    plan = seqlib.DecodeRows(pos, slot, T, H, parts, window)
+                else:
+                    key = (T, H, parts, window)
+                    plan = self._decode_plans.get(key)
+                    if plan is None:
+                        plan = self._decode_plans[key] = seqlib.DecodeAttnPlan(T, H, parts, self.device, window=window)
+                    plan.fill(pos, slot)
             plans[(H, window, tcgen05)] = plan
         return plan
 

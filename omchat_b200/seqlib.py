@@ -71,6 +71,7 @@ SIGNATURES = {
     "omc_step_wait_selfcheck": (_I, [_P, _P]),
     "omc_step_wait_warp_selfcheck": (_I, [_P, _P]),
     "omc_latent_attn_mma": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _I, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
+    "omc_latent_attn_decode": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _I, _P, _P, _I, _P, _I, _P, _L, _F, _P, _I, _P, _P, _P]),
     "omc_latent_plan": (_I, [_P, _I, _I, _I, _I, _I, _I, _I, _I, _P]),
     "omc_window_plan": (_I, [_P, _I, _I, _I, _I, _I, _P]),
     "omc_plan_words": (_I, [_P, _I, _I, _P]),
@@ -419,6 +420,16 @@ class DecodeAttnPlan:
         _check(rc, "omc_latent_decode_items")
 
 
+class DecodeRows:
+    """A decode-only step of B rows for the tcgen05 kernel, which finds a row's key ranges from pos and slot by itself: no list, and nothing that outlives the step."""
+
+    def __init__(self, pos: torch.Tensor, slot: torch.Tensor, B: int, H: int, parts: int, window: int = WINDOW_ALL):
+        self.pos, self.slot, self.B, self.H, self.parts, self.window = pos, slot, B, H, parts, window
+        self.n_items, self.max_rows = B * parts, H
+        self.n_merges = B if parts > 1 else 0
+        self.n_parts = B * parts if parts > 1 else 0
+
+
 _mma_ws = {}
 
 
@@ -426,7 +437,8 @@ def latent_attn_mma(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, blo
                     plan: LatentAttnPlan, sink: Optional[torch.Tensor], scale: float, out: torch.Tensor, window: int = WINDOW_ALL,
                     gate: Optional[torch.Tensor] = None):
     """latent_attn on the tensor cores; the plan was made for the same window."""
-    _need_cuda(qcat, pool, block_table, plan.items, sink, out, gate)
+    rows = isinstance(plan, DecodeRows)
+    _need_cuda(qcat, pool, block_table, plan.pos if rows else plan.items, sink, out, gate)
     assert gate is None or (gate.dtype == torch.float32 and gate.stride(1) == 1)
     T, H = qcat.shape[0], qcat.shape[1]
     assert qcat.dtype == torch.bfloat16 and pool.dtype == torch.bfloat16
@@ -440,6 +452,14 @@ def latent_attn_mma(qcat: torch.Tensor, r: int, dr: int, pool: torch.Tensor, blo
             ws = torch.empty(need, device=qcat.device, dtype=torch.float32)
             _mma_ws[key] = ws
         ws_o, ws_ml = ws[:plan.n_parts * MMA_ROWS * r], ws[plan.n_parts * MMA_ROWS * r:]
+    if rows:
+        assert T == plan.B and plan.H == H and plan.pos.dtype == plan.slot.dtype == torch.int32 and plan.pos.is_contiguous() and plan.slot.is_contiguous()
+        rc = load().omc_latent_attn_decode(qcat, T, H, r, dr, pool, block_table, block_table.shape[1], page_size, plan.pos, plan.slot, plan.parts, sink, window, gate,
+                                           gate.stride(0) if gate is not None else 0, scale, out, _dt(out), ws_o, ws_ml, _stream())
+        _check(rc, "omc_latent_attn_decode")
+        if plan.n_merges:
+            _core.add_launches(1)
+        return out
     rc = load().omc_latent_attn_mma_rows(qcat, T, H, r, dr, pool, block_table, block_table.shape[1], page_size,
                                          plan.items, plan.n_items, plan.max_rows, plan.merges, plan.n_merges, sink, window, gate,
                                          gate.stride(0) if gate is not None else 0, scale, out, _dt(out), ws_o, ws_ml, _stream())
