@@ -43,6 +43,7 @@ struct ScanArgs {
   const int32_t* slot;
   int H, G, dim, vdim;
   bool vec_state, vec_out;   // a thread's columns of the state / four outputs as one access
+  int portions;              // P, where the CTAs take portions in the order of their lengths, the longest first; 0: in their own order
   int long_from;             // portions of this many rows and more are scan_chunk_kernel's, the others the token-by-token kernels' (0: all of them are theirs)
 };
 
@@ -51,6 +52,27 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
 }
 __device__ __forceinline__ void cp_async16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));
+}
+
+// The portion whose length has the block's rank z, longest first (of up to as many portions as the block has threads): a long chain that starts last would run alone at the end.
+// scratch: shared memory of that many words, free again behind it.
+__device__ __forceinline__ int scan_portion(const int32_t* row_begin, int portions, int z, int* scratch) {
+  const int p = threadIdx.x;
+  if (p < portions) scratch[p] = row_begin[p + 1] - row_begin[p];
+  __syncthreads();
+  bool mine = false;
+  if (p < portions) {
+    const int n = scratch[p];
+    int before = 0;
+    for (int o = 0; o < portions; ++o) before += scratch[o] > n || (scratch[o] == n && o < p);
+    mine = before == z;
+  }
+  __syncthreads();
+  if (mine) scratch[0] = p;
+  __syncthreads();
+  const int found = scratch[0];
+  __syncthreads();
+  return found;
 }
 
 // Packed fp32 pairs (sm_100: one instruction, two IEEE fp32 operations): the recurrence's state lives in such pairs.

@@ -91,26 +91,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
   constexpr int CPT = kScCpt, LANES = Shared::LANES, COLS = Shared::COLS, WC = Shared::WC, XP = Shared::XP;
   constexpr bool DELTA = KIND == kScanDelta, HALVES = LANES == 16;
 
-  // longest portions first: the CTA of rank z in that order takes its portion (in their own order where they are more than the threads)
-  int portion = blockIdx.z;
-  if (portions > 1 && portions <= kScThreads) {
-    int* len = reinterpret_cast<int*>(sm);
-    const int p = threadIdx.x;
-    if (p < portions) len[p] = a.row_begin[p + 1] - a.row_begin[p];
-    __syncthreads();
-    bool mine = false;
-    if (p < portions) {
-      const int n = len[p];
-      int before = 0;
-      for (int o = 0; o < portions; ++o) before += len[o] > n || (len[o] == n && o < p);
-      mine = before == (int)blockIdx.z;
-    }
-    __syncthreads();
-    if (mine) len[0] = p;
-    __syncthreads();
-    portion = len[0];
-    __syncthreads();
-  }
+  const int portion = portions > 1 && portions <= kScThreads ? scan_portion(a.row_begin, portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1], stages = (r1 - r0 + kScTok - 1) / kScTok;
   if (r1 - r0 < a.long_from) return;
   const int h = blockIdx.y, col0 = blockIdx.x * COLS;

@@ -638,8 +638,8 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
 // CPT columns per group of eight lanes (see the launch). What bounds it: a token's chain through 92 instructions per warp (step sizes; delta rule 135), some three
 // cycles each where a scheduler has one warp (4 heads, 1100 tokens: 440 cycles per token), with many CTAs the packed fma (58 % of the pipe's cycles) and the shared-memory
 // reads of keys and queries (74 % of the data path's). Measured in us, the general kernel in brackets: step sizes, 64 heads of
-// 128 x 64, portions of 1024, 777, 1024, 301 tokens 306 (340), 32 x 64 tokens 185 (228), 16 heads, 1100 tokens 149 (195); delta rule, 16 heads of 128 x 128
-// over the same portions 351 (366), 8 x 300 tokens 174 (212), 4 heads, 1100 tokens 255 (299), with per-channel decays 305 (361).
+// 128 x 64, portions of 1024, 777, 1024, 301 tokens 292 (340), 32 x 64 tokens 154 (228), 16 heads, 1100 tokens 149 (195). Long portions of the delta rule and with
+// per-channel decays are scan_chunk.cu's.
 constexpr int kSrTok = 8, kSrThreads = 128;
 template <int DIM, int COLS, bool CHAN>
 struct ScanRowsStage {
@@ -663,7 +663,8 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
   constexpr int DPT = DIM / kScanLanes, DP = DPT / 2, PITCH = Stage::PITCH, OPITCH = COLS + 4;
   const bool minus1 = KIND == kScanStep || a.decay_mode == 5;
   const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
-  const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
+  const int portion = a.portions > 1 ? scan_portion(a.row_begin, a.portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
+  const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1];
   if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
   const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
   const bool in = col < a.vdim;   // a thread's columns all exist or none does
@@ -727,6 +728,9 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
       const bool read = !fresh && in;
       if constexpr (CPT == 1) {
         e[j][0] = read ? *row : 0.f;
+      } else if constexpr (CPT == 4) {
+        const float4 x = read ? *reinterpret_cast<const float4*>(row) : make_float4(0.f, 0.f, 0.f, 0.f);
+        e[j][0] = x.x, e[j][1] = x.y, e[j][2] = x.z, e[j][3] = x.w;
       } else {
         const float2 x = read ? *reinterpret_cast<const float2*>(row) : make_float2(0.f, 0.f);
         e[j][0] = x.x, e[j][1] = x.y;
@@ -764,6 +768,9 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
       const float* p = s.v + tt * COLS + CPT * cg;
       if constexpr (CPT == 1) {
         un[0] = *p;
+      } else if constexpr (CPT == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(p);
+        un[0] = x.x, un[1] = x.y, un[2] = x.z, un[3] = x.w;
       } else {
         const float2 x = *reinterpret_cast<const float2*>(p);
         un[0] = x.x, un[1] = x.y;
@@ -840,6 +847,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
       columns(q2, o);
       float* dst = sh.po + (tt * kScanLanes + lane) * OPITCH + CPT * cg;
       if constexpr (CPT == 1) *dst = o[0];
+      else if constexpr (CPT == 4) *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1], o[2], o[3]);
       else *reinterpret_cast<float2*>(dst) = make_float2(o[0], o[1]);
     };
     if (n == kSrTok) {
@@ -884,6 +892,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
     for (int j = 0; j < 2; ++j) {
       float* row = S + (long long)(lane * DPT + 2 * r + j) * a.vdim + col;
       if constexpr (CPT == 1) *row = e[j][0];
+      else if constexpr (CPT == 4) *reinterpret_cast<float4*>(row) = make_float4(e[j][0], e[j][1], e[j][2], e[j][3]);
       else *reinterpret_cast<float2*>(row) = make_float2(e[j][0], e[j][1]);
     }
   }
@@ -1568,7 +1577,7 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   if (dim > 256) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: key width above 256");
   if (portions > 65535 || H > 65535) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: more than 65535 portions or heads");
   ScanArgs s{q, k, v, ldq, ldk, ldv, silu_in, decay_mode, decay_pow, out_scale, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo,
-             row_begin, pos, slot, H, G, dim, vdim, false, false, 0};
+             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int dpt = dim <= 32 ? 4 : (dim <= 64 ? 8 : (dim <= 128 ? 16 : 32));   // key channels per thread: dim / 8 lanes, rounded up to a float4
   const bool chan = decay_mode >= 2 && decay_mode <= 5;
@@ -1593,6 +1602,8 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
       const int rc = launch_scan_chunk(s, rows, portions, st);
       if (rc != OMC_OK || portions == 1) return rc;
     }
+    // chains of hundreds of tokens, more CTAs than SMs: the longest portions first (32 heads of 128 x 64, portions of 1024, 777, 1024, 301 tokens: 197, in their own order 224)
+    if (portions > 1 && portions <= kSrThreads && rows >= 128LL * portions && (long long)grid.x * H * portions > 148) s.portions = portions;
     auto go = [&](auto dim_c, auto cpt_c, auto kind_c, auto chan_c) {
       constexpr int DIM = decltype(dim_c)::value, CPT = decltype(cpt_c)::value, KIND = decltype(kind_c)::value, COLS = kSrThreads / kScanLanes * CPT;
       constexpr bool CHAN = decltype(chan_c)::value;
@@ -1624,6 +1635,18 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
     typedef integral_constant<int, 2> Two;
     if (chan && small)
       return dim == 64 ? channels(integral_constant<int, 64>()) : channels(integral_constant<int, 128>());
+    // 64 columns per CTA, four per thread, where such CTAs are many: half the shared-memory reads per column, which bound it then, but longer chains of a token, which do where
+    // CTAs are few (in us, 32 / 64 columns: 64 heads of 128 x 64, 4 x 700 tokens 267 / 235, 32 x 64 184 / 154, 3 x 500 150 / 169; 80 heads, 3 x 600 230 / 203; 128 heads,
+    // 8 x 400 517 / 427). Not where the last half of the columns would be empty (96: 181 / 205)
+    const int blocks = (vdim + 63) / 64;
+    if (!chan && beta == nullptr && (vdim + 31) / 32 == 2 * blocks && (long long)blocks * H * portions >= 240) {
+      typedef integral_constant<int, 4> Four;
+      auto plain = [&](auto dim_c) {
+        if (decay_mode == 6) return go(dim_c, Four(), integral_constant<int, kScanStep>(), std::false_type());
+        return go(dim_c, Four(), integral_constant<int, kScanPlain>(), std::false_type());
+      };
+      return dim == 64 ? plain(integral_constant<int, 64>()) : plain(integral_constant<int, 128>());
+    }
     if (!chan && dim == 64) return small ? kinds(integral_constant<int, 64>(), One()) : kinds(integral_constant<int, 64>(), Two());
     if (!chan) return small ? kinds(integral_constant<int, 128>(), One()) : kinds(integral_constant<int, 128>(), Two());
   }
