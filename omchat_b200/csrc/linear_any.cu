@@ -161,10 +161,11 @@ __global__ void __launch_bounds__(NT) linear_tile_kernel(LinearArgs a) {
 // 1024 at a time into shared memory, all of them in one go; thread (p, c) sums chunk c of the columns p and p + 4 for every row, and
 // the chunks' sums are added by one thread per output. A pitch of 68 floats per chunk puts the chunks on different
 // banks. 3 x 6144 x 2048 in fp32: 19 us = 2.6 TB/s of W (the tile kernel before: 145), 3 x 4096 x 1024 10 (76).
-constexpr int kRowsCols = 8, kRowsChunks = 16, kRowsPitch = kRowsChunks * (kLinChunk + 4), kRowsThreads = 64;
+constexpr int kRowsCols = 8;
 
-template <typename TX, typename TW, typename TY, int MR, bool VEC>
-__global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(LinearArgs a) {
+template <typename TX, typename TW, typename TY, int MR, bool VEC, int CHUNKS>   // 16; 32: twice the threads, and sums of up to 2048 terms without a second load behind the first
+__global__ void __launch_bounds__(4 * CHUNKS) linear_rows_kernel(LinearArgs a) {
+  constexpr int kRowsChunks = CHUNKS, kRowsPitch = CHUNKS * (kLinChunk + 4), kRowsThreads = 4 * CHUNKS;
   extern __shared__ __align__(16) float lin_sm[];   // W [8][pitch] | X [MR][pitch] | chunk sums [8][MR][16 + 1]
   float* ws = lin_sm;
   float* xs = ws + kRowsCols * kRowsPitch;
@@ -173,7 +174,7 @@ __global__ void __launch_bounds__(kRowsThreads) linear_rows_kernel(LinearArgs a)
   const TX* X = static_cast<const TX*>(a.X) + (long long)blockIdx.z * a.sx;
   const TW* W = static_cast<const TW*>(a.W) + (long long)blockIdx.z * a.sw;
   TY* Y = static_cast<TY*>(a.Y) + (long long)blockIdx.z * a.sy;
-  const int tid = threadIdx.x, c = tid & (kRowsChunks - 1), p = tid >> 4;
+  const int tid = threadIdx.x, c = tid % kRowsChunks, p = tid / kRowsChunks;
   const int out_n = tid & (kRowsCols - 1), out_m = tid / kRowsCols;   // the output whose chunks this thread adds
   float total = 0.f;
   for (int k0 = 0; k0 < a.K; k0 += kRowsChunks * kLinChunk) {
@@ -365,14 +366,21 @@ static int allow_smem(Kernel* kernel, int smem, bool (&done)[kMaxDevices]) {
   return OMC_OK;
 }
 
+template <typename TX, typename TW, typename TY, int MR, bool VEC, int CHUNKS>
+static int launch_rows(const LinearArgs& a, const dim3& grid, cudaStream_t st) {
+  constexpr int smem = ((kRowsCols + MR) * CHUNKS * (kLinChunk + 4) + kRowsCols * MR * (CHUNKS + 1)) * 4;
+  static bool done[kMaxDevices] = {};
+  if (int rc = allow_smem(linear_rows_kernel<TX, TW, TY, MR, VEC, CHUNKS>, smem, done); rc != OMC_OK) return rc;
+  linear_rows_kernel<TX, TW, TY, MR, VEC, CHUNKS><<<grid, 4 * CHUNKS, smem, st>>>(a);
+  return check_launch("omc_linear");
+}
+// Sums of more than 1024 terms whose CTAs run in one wave have all of their terms under way at once: 3 x 1024 x 2048 8.5 -> 6.4 us, 8 x 1024 x 2048 10.5 -> 8.4, 100 x 77 x 4096
+// 15.1 -> 11.5. With more CTAs than that the smaller ones, of which four share an SM, are as fast (3 x 4096 x 2048 14.2).
 template <typename TX, typename TW, typename TY, int MR, bool VEC>
 static int launch_rows(const LinearArgs& a, int batch, cudaStream_t st) {
-  constexpr int smem = ((kRowsCols + MR) * kRowsPitch + kRowsCols * MR * (kRowsChunks + 1)) * 4;
-  static bool done[kMaxDevices] = {};
-  if (int rc = allow_smem(linear_rows_kernel<TX, TW, TY, MR, VEC>, smem, done); rc != OMC_OK) return rc;
   const dim3 grid((a.N + kRowsCols - 1) / kRowsCols, (a.M + MR - 1) / MR, batch);
-  linear_rows_kernel<TX, TW, TY, MR, VEC><<<grid, kRowsThreads, smem, st>>>(a);
-  return check_launch("omc_linear");
+  if (a.K > 1024 && (long long)grid.x * grid.y * batch <= (MR == 4 ? 296 : 148)) return launch_rows<TX, TW, TY, MR, VEC, 32>(a, grid, st);
+  return launch_rows<TX, TW, TY, MR, VEC, 16>(a, grid, st);
 }
 
 template <typename TX, typename TW, typename TY, bool VEC, int NT>
