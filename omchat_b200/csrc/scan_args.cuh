@@ -45,7 +45,28 @@ struct ScanArgs {
   bool vec_state, vec_out;   // a thread's columns of the state / four outputs as one access
   int portions;              // P, where the CTAs take portions in the order of their lengths, the longest first; 0: in their own order
   int long_from;             // portions of this many rows and more are scan_chunk_kernel's, the others the token-by-token kernels' (0: all of them are theirs)
+  int beside;                // 1, 2: the first and the second of the two kernels that share the portions of a step; 0: alone
 };
+
+// The two kernels of a step write different portions and slots, so the second may run beside the first: the first lets it start as soon as all of its own CTAs have, and the
+// second ends behind the first, whose end nothing else would wait for. One CTA does that; all of them would keep their place on an SM.
+__device__ __forceinline__ void scan_begin(const ScanArgs& a) {
+  if (a.beside == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void scan_end(const ScanArgs& a) {
+  if (a.beside == 2 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+int scan_launch(void (*kernel)(Params...), dim3 grid, int threads, int smem, cudaStream_t st, const ScanArgs& a, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr, cfg.numAttrs = a.beside == 2 ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kernel, a, args...);
+  return check_launch("omc_linear_state_scan");
+}
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src));

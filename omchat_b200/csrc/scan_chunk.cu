@@ -81,6 +81,30 @@ __device__ __forceinline__ float sum8_over_warp(const float (&x)[8], int lane) {
   return s + __shfl_xor_sync(0xffffffffu, s, 1);
 }
 
+// The z-th portion of at least `least` rows, of any number of portions; -1: they are fewer. scratch: shared memory of nine words, free again behind it.
+static __device__ int scan_long_portion(const int32_t* row_begin, int portions, int least, int z, int* scratch) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid / 32;
+  for (int p0 = 0; p0 < portions; p0 += 2 * kScThreads) {
+    const int p = p0 + tid;
+    const bool is = p < portions && row_begin[p + 1] - row_begin[p] >= least;
+    const int n = __syncthreads_count(is);
+    if (z < n) {
+      const unsigned these = __ballot_sync(0xffffffffu, is);
+      if (lane == 0) scratch[warp] = __popc(these);
+      __syncthreads();
+      int before = __popc(these & ((1u << lane) - 1));
+      for (int w = 0; w < warp; ++w) before += scratch[w];
+      if (is && before == z) scratch[8] = p;
+      __syncthreads();
+      const int found = scratch[8];
+      __syncthreads();
+      return found;
+    }
+    z -= n;
+  }
+  return -1;
+}
+
 template <int DIM, int KIND, bool CHAN>
 __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs a, int portions) {
   typedef ScanChunkShared<DIM, KIND, CHAN> Shared;
@@ -91,9 +115,16 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
   constexpr int CPT = kScCpt, LANES = Shared::LANES, COLS = Shared::COLS, WC = Shared::WC, XP = Shared::XP;
   constexpr bool DELTA = KIND == kScanDelta, HALVES = LANES == 16;
 
-  const int portion = portions > 1 && portions <= kScThreads ? scan_portion(a.row_begin, portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
+  int portion = 0;
+  if (portions > kScThreads) {
+    portion = scan_long_portion(a.row_begin, portions, a.long_from, blockIdx.z, reinterpret_cast<int*>(sm));
+    if (portion < 0) return;
+  } else if (portions > 1) {
+    portion = scan_portion(a.row_begin, portions, blockIdx.z, reinterpret_cast<int*>(sm));
+  }
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1], stages = (r1 - r0 + kScTok - 1) / kScTok;
   if (r1 - r0 < a.long_from) return;
+  scan_begin(a);   // not before: CTAs without a portion would still be there when the other kernel's are spread over the SMs (3 x 63 tokens 27 -> 35 us)
   const int h = blockIdx.y, col0 = blockIdx.x * COLS;
   const bool minus1 = CHAN && a.decay_mode == 5;
   auto meet = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };   // once per stage, both halves
@@ -455,8 +486,7 @@ int launch_scan_chunk(const ScanArgs& a, int rows, int portions, cudaStream_t st
   using std::integral_constant;
   const bool chan = a.decay_mode == 3 || a.decay_mode == 5;
   if (a.long_from <= 0 || (!chan && (a.beta == nullptr || a.decay_mode > 1)) || (a.dim != 64 && a.dim != 128)) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: not a recurrence of the kernel for long portions");
-  // in the order of their lengths only so many portions can be long ones
-  const int most = portions <= kScThreads && rows / a.long_from < portions ? rows / a.long_from : portions;
+  const int most = rows / a.long_from < portions ? rows / a.long_from : portions;   // only so many portions can be long ones
   auto go = [&](auto dim_c, auto kind_c, auto chan_c) {
     constexpr int DIM = decltype(dim_c)::value, KIND = decltype(kind_c)::value;
     constexpr bool CHAN = decltype(chan_c)::value;
@@ -467,16 +497,14 @@ int launch_scan_chunk(const ScanArgs& a, int rows, int portions, cudaStream_t st
       cudaFuncSetAttribute(scan_chunk_kernel<DIM, KIND, CHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
       attr_done[cur_device()] = true;
     }
-    scan_chunk_kernel<DIM, KIND, CHAN><<<dim3((a.vdim + Shared::COLS - 1) / Shared::COLS, a.H, most), 2 * kScThreads, smem, st>>>(a, portions);
+    return scan_launch(scan_chunk_kernel<DIM, KIND, CHAN>, dim3((a.vdim + Shared::COLS - 1) / Shared::COLS, a.H, most), 2 * kScThreads, smem, st, a, portions);
   };
   auto kinds = [&](auto dim_c) {
-    if (!chan) go(dim_c, integral_constant<int, kScanDelta>(), std::false_type());
-    else if (a.beta != nullptr) go(dim_c, integral_constant<int, kScanDelta>(), std::true_type());
-    else go(dim_c, integral_constant<int, kScanPlain>(), std::true_type());
+    if (!chan) return go(dim_c, integral_constant<int, kScanDelta>(), std::false_type());
+    if (a.beta != nullptr) return go(dim_c, integral_constant<int, kScanDelta>(), std::true_type());
+    return go(dim_c, integral_constant<int, kScanPlain>(), std::true_type());
   };
-  if (a.dim == 128) kinds(integral_constant<int, 128>());
-  else kinds(integral_constant<int, 64>());
-  return check_launch("omc_linear_state_scan");
+  return a.dim == 128 ? kinds(integral_constant<int, 128>()) : kinds(integral_constant<int, 64>());
 }
 
 }  // namespace omc

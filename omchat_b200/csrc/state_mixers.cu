@@ -324,7 +324,7 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
   const int h = blockIdx.y, kvh = h / (a.H / a.G);
   const int col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
-  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
+  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return scan_end(a);
   // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
   // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
   const int tid = threadIdx.x, lane = WIDE ? tid / kScanGroups : tid & (kScanLanes - 1), cg = WIDE ? tid % kScanGroups : tid / kScanLanes;
@@ -629,6 +629,7 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
       }
     }
   }
+  scan_end(a);
 }
 
 // The same recurrence for portions of several tokens at 64 or 128 key channels, inputs that need no preparation of their own (no silu, per-channel decays given)
@@ -665,7 +666,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
   const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
   const int portion = a.portions > 1 ? scan_portion(a.row_begin, a.portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1];
-  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
+  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return scan_end(a);
   const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
   const bool in = col < a.vdim;   // a thread's columns all exist or none does
   const float A = KIND == kScanStep || a.decay_mode == 1 ? expf(a.A_log[h]) : 0.f;
@@ -1577,7 +1578,7 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   if (dim > 256) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: key width above 256");
   if (portions > 65535 || H > 65535) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: more than 65535 portions or heads");
   ScanArgs s{q, k, v, ldq, ldk, ldv, silu_in, decay_mode, decay_pow, out_scale, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo,
-             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0};
+             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0, 0};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int dpt = dim <= 32 ? 4 : (dim <= 64 ? 8 : (dim <= 128 ? 16 : 32));   // key channels per thread: dim / 8 lanes, rounded up to a float4
   const bool chan = decay_mode >= 2 && decay_mode <= 5;
@@ -1596,60 +1597,56 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   const bool brief = rows <= 16LL * portions;
   // portions of several tokens whose inputs are ready: scan_rows_kernel
   const bool ready = !silu_in && (decay_mode == 0 || decay_mode == 1 || decay_mode == 3 || decay_mode >= 5);
-  if (!one && vec && ready && (dim == 64 || dim == 128) && s.vec_out && s.vec_state) {
-    if (rows >= kScanLong && (chan || (beta != nullptr && decay_mode <= 1))) {   // long portions: scan_chunk_kernel; whichever are left, the kernels below
-      s.long_from = kScanLong;
-      const int rc = launch_scan_chunk(s, rows, portions, st);
-      if (rc != OMC_OK || portions == 1) return rc;
-    }
-    // chains of hundreds of tokens, more CTAs than SMs: the longest portions first (32 heads of 128 x 64, portions of 1024, 777, 1024, 301 tokens: 197, in their own order 224)
-    if (portions > 1 && portions <= kSrThreads && rows >= 128LL * portions && (long long)grid.x * H * portions > 148) s.portions = portions;
-    auto go = [&](auto dim_c, auto cpt_c, auto kind_c, auto chan_c) {
-      constexpr int DIM = decltype(dim_c)::value, CPT = decltype(cpt_c)::value, KIND = decltype(kind_c)::value, COLS = kSrThreads / kScanLanes * CPT;
-      constexpr bool CHAN = decltype(chan_c)::value;
-      static bool attr_done[kMaxDevices] = {};
-      constexpr int smem = (int)sizeof(ScanRowsShared<DIM, COLS, CHAN>);
-      if (!attr_done[cur_device()]) {
-        cudaFuncSetAttribute(scan_rows_kernel<DIM, CPT, KIND, CHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        attr_done[cur_device()] = true;
-      }
-      scan_rows_kernel<DIM, CPT, KIND, CHAN><<<dim3((vdim + COLS - 1) / COLS, H, portions), kSrThreads, smem, st>>>(s);
-      return check_launch("omc_linear_state_scan");
-    };
-    using std::integral_constant;
-    auto kinds = [&](auto dim_c, auto cpt_c) {
-      if (decay_mode == 6) return go(dim_c, cpt_c, integral_constant<int, kScanStep>(), std::false_type());
-      if (beta != nullptr) return go(dim_c, cpt_c, integral_constant<int, kScanDelta>(), std::false_type());
-      return go(dim_c, cpt_c, integral_constant<int, kScanPlain>(), std::false_type());
-    };
-    auto channels = [&](auto dim_c) {
-      typedef integral_constant<int, 1> One;
-      if (beta != nullptr) return go(dim_c, One(), integral_constant<int, kScanDelta>(), std::true_type());
-      return go(dim_c, One(), integral_constant<int, kScanPlain>(), std::true_type());
-    };
-    // 32 columns per CTA once CTAs of 16 would be more than the SMs: alone on an SM the smaller CTA is the faster one (in us, 16 / 32 columns: 16 heads of 128 x
-    // 64, step sizes, 1100 tokens 149 / 162; delta rule 4 of 128 x 128 255 / 269, 4 of 64 x 64 195 / 213), two of them on it never (64 heads 230 / 163).
-    // Per-channel decays take the registers of the larger one: there the general kernel is up to 12 % faster
-    const bool small = (long long)grid.x * H * portions <= 74;
-    typedef integral_constant<int, 1> One;
-    typedef integral_constant<int, 2> Two;
-    if (chan && small)
-      return dim == 64 ? channels(integral_constant<int, 64>()) : channels(integral_constant<int, 128>());
-    // 64 columns per CTA, four per thread, where such CTAs are many: half the shared-memory reads per column, which bound it then, but longer chains of a token, which do where
-    // CTAs are few (in us, 32 / 64 columns: 64 heads of 128 x 64, 4 x 700 tokens 267 / 235, 32 x 64 184 / 154, 3 x 500 150 / 169; 80 heads, 3 x 600 230 / 203; 128 heads,
-    // 8 x 400 517 / 427). Not where the last half of the columns would be empty (96: 181 / 205)
-    const int blocks = (vdim + 63) / 64;
-    if (!chan && beta == nullptr && (vdim + 31) / 32 == 2 * blocks && (long long)blocks * H * portions >= 240) {
-      typedef integral_constant<int, 4> Four;
-      auto plain = [&](auto dim_c) {
-        if (decay_mode == 6) return go(dim_c, Four(), integral_constant<int, kScanStep>(), std::false_type());
-        return go(dim_c, Four(), integral_constant<int, kScanPlain>(), std::false_type());
+  const bool several = !one && vec && ready && (dim == 64 || dim == 128) && s.vec_out && s.vec_state;
+  auto tokens = [&]() -> int {   // token by token
+    if (several) {
+      // chains of hundreds of tokens, more CTAs than SMs: the longest portions first (32 heads of 128 x 64, portions of 1024, 777, 1024, 301 tokens: 197, in their own order 224)
+      if (portions > 1 && portions <= kSrThreads && rows >= 128LL * portions && (long long)grid.x * H * portions > 148) s.portions = portions;
+      auto go = [&](auto dim_c, auto cpt_c, auto kind_c, auto chan_c) {
+        constexpr int DIM = decltype(dim_c)::value, CPT = decltype(cpt_c)::value, KIND = decltype(kind_c)::value, COLS = kSrThreads / kScanLanes * CPT;
+        constexpr bool CHAN = decltype(chan_c)::value;
+        static bool attr_done[kMaxDevices] = {};
+        constexpr int smem = (int)sizeof(ScanRowsShared<DIM, COLS, CHAN>);
+        if (!attr_done[cur_device()]) {
+          cudaFuncSetAttribute(scan_rows_kernel<DIM, CPT, KIND, CHAN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+          attr_done[cur_device()] = true;
+        }
+        return scan_launch(scan_rows_kernel<DIM, CPT, KIND, CHAN>, dim3((vdim + COLS - 1) / COLS, H, portions), kSrThreads, smem, st, s);
       };
-      return dim == 64 ? plain(integral_constant<int, 64>()) : plain(integral_constant<int, 128>());
+      using std::integral_constant;
+      auto kinds = [&](auto dim_c, auto cpt_c) {
+        if (decay_mode == 6) return go(dim_c, cpt_c, integral_constant<int, kScanStep>(), std::false_type());
+        if (beta != nullptr) return go(dim_c, cpt_c, integral_constant<int, kScanDelta>(), std::false_type());
+        return go(dim_c, cpt_c, integral_constant<int, kScanPlain>(), std::false_type());
+      };
+      auto channels = [&](auto dim_c) {
+        typedef integral_constant<int, 1> One;
+        if (beta != nullptr) return go(dim_c, One(), integral_constant<int, kScanDelta>(), std::true_type());
+        return go(dim_c, One(), integral_constant<int, kScanPlain>(), std::true_type());
+      };
+      // 32 columns per CTA once CTAs of 16 would be more than the SMs: alone on an SM the smaller CTA is the faster one (in us, 16 / 32 columns: 16 heads of 128 x
+      // 64, step sizes, 1100 tokens 149 / 162; delta rule 4 of 128 x 128 255 / 269, 4 of 64 x 64 195 / 213), two of them on it never (64 heads 230 / 163).
+      // Per-channel decays take the registers of the larger one: there the general kernel is up to 12 % faster
+      const bool small = (long long)grid.x * H * portions <= 74;
+      typedef integral_constant<int, 1> One;
+      typedef integral_constant<int, 2> Two;
+      if (chan && small)
+        return dim == 64 ? channels(integral_constant<int, 64>()) : channels(integral_constant<int, 128>());
+      // 64 columns per CTA, four per thread, where such CTAs are many: half the shared-memory reads per column, which bound it then, but longer chains of a token, which do where
+      // CTAs are few (in us, 32 / 64 columns: 64 heads of 128 x 64, 4 x 700 tokens 267 / 235, 32 x 64 184 / 154, 3 x 500 150 / 169; 80 heads, 3 x 600 230 / 203; 128 heads,
+      // 8 x 400 517 / 427). Not where the last half of the columns would be empty (96: 181 / 205)
+      const int blocks = (vdim + 63) / 64;
+      if (!chan && beta == nullptr && (vdim + 31) / 32 == 2 * blocks && (long long)blocks * H * portions >= 240) {
+        typedef integral_constant<int, 4> Four;
+        auto plain = [&](auto dim_c) {
+          if (decay_mode == 6) return go(dim_c, Four(), integral_constant<int, kScanStep>(), std::false_type());
+          return go(dim_c, Four(), integral_constant<int, kScanPlain>(), std::false_type());
+        };
+        return dim == 64 ? plain(integral_constant<int, 64>()) : plain(integral_constant<int, 128>());
+      }
+      if (!chan && dim == 64) return small ? kinds(integral_constant<int, 64>(), One()) : kinds(integral_constant<int, 64>(), Two());
+      if (!chan) return small ? kinds(integral_constant<int, 128>(), One()) : kinds(integral_constant<int, 128>(), Two());
     }
-    if (!chan && dim == 64) return small ? kinds(integral_constant<int, 64>(), One()) : kinds(integral_constant<int, 64>(), Two());
-    if (!chan) return small ? kinds(integral_constant<int, 128>(), One()) : kinds(integral_constant<int, 128>(), Two());
-  }
 #define OMC_SCAN_LAUNCH(DPT, VEC, KIND, CHAN, TOK)                                                                                        \
   do {                                                                                                                                    \
     static bool attr_done[kMaxDevices] = {};                                                                                              \
@@ -1658,7 +1655,7 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
       cudaFuncSetAttribute(linear_state_scan_kernel<DPT, VEC, KIND, CHAN, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);       \
       attr_done[cur_device()] = true;                                                                                                     \
     }                                                                                                                                     \
-    linear_state_scan_kernel<DPT, VEC, KIND, CHAN, TOK><<<grid, kScanThreads, smem, st>>>(s);                                             \
+    return scan_launch(linear_state_scan_kernel<DPT, VEC, KIND, CHAN, TOK>, grid, kScanThreads, smem, st, s);                              \
   } while (0)
 #define OMC_SCAN_KIND(DPT, VEC, TOK)                                                      \
   do {                                                                                    \
@@ -1674,17 +1671,28 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
     else if (vec) OMC_SCAN_KIND(DPT, true, TOK); \
     else OMC_SCAN_KIND(DPT, false, TOK);        \
   } while (0)
-  if (dpt == 4 && brief) OMC_SCAN_DPT(4, 8);
-  else if (dpt == 4) OMC_SCAN_DPT(4, 16);
-  else if (dpt == 8 && brief) OMC_SCAN_DPT(8, 8);
-  else if (dpt == 8) OMC_SCAN_DPT(8, 16);
-  else if (dpt == 16 && (tight || brief)) OMC_SCAN_DPT(16, 8);
-  else if (dpt == 16) OMC_SCAN_DPT(16, 16);
-  else OMC_SCAN_DPT(32, 8);
+    if (dpt == 4 && brief) OMC_SCAN_DPT(4, 8);
+    else if (dpt == 4) OMC_SCAN_DPT(4, 16);
+    else if (dpt == 8 && brief) OMC_SCAN_DPT(8, 8);
+    else if (dpt == 8) OMC_SCAN_DPT(8, 16);
+    else if (dpt == 16 && (tight || brief)) OMC_SCAN_DPT(16, 8);
+    else if (dpt == 16) OMC_SCAN_DPT(16, 16);
+    else OMC_SCAN_DPT(32, 8);
 #undef OMC_SCAN_DPT
 #undef OMC_SCAN_KIND
 #undef OMC_SCAN_LAUNCH
-  return check_launch("omc_linear_state_scan");
+  };
+  // long portions of the delta rule and with per-channel decays: scan_chunk_kernel; whichever are left, the kernels above
+  if (!several || rows < kScanLong || !(chan || (beta != nullptr && decay_mode <= 1))) return tokens();
+  s.long_from = kScanLong;
+  if (portions == 1) return launch_scan_chunk(s, rows, portions, st);
+  // The long chains first, the others beside them. In us, all token by token / one kernel behind the other / beside: 500 + 16 x 1 tokens of 16 heads of 128 x 128 131 / 97 / 90, with
+  // decays per channel 195 / 113 / 101 (152 with the short ones first); 65 + 31 x 1 tokens 29 / 36 / 25; 100, 50, 50, 50 33 / 46 / 31. The host does not know the lengths: where no
+  // portion is long, the first kernel is empty and costs 1.2 on the device (8 x 8 tokens 9.3 / 10.5).
+  s.beside = 1;
+  if (const int rc = launch_scan_chunk(s, rows, portions, st); rc != OMC_OK) return rc;
+  s.beside = 2;
+  return tokens();
 }
 
 extern "C" int omc_gated_rms_rows(const float* x, long long ldx, int rows, int groups, int n, const void* w, int w_dt, float eps,

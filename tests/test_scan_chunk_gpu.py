@@ -107,3 +107,17 @@ def test_many_portions_of_which_few_are_long():
     out, S = c.run()
     want, Sw = c.exact()
     assert _rel(out, want) < 5e-7 and _rel(S, Sw) < 5e-7
+
+
+@pytest.mark.parametrize("kind", ["delta", "given"])
+@pytest.mark.parametrize("lens", [[3] * 128 + [70, 1, 64] + [2] * 170 + [97], [1] * 40 + [200], [5] * 24])   # more portions than a CTA orders, two kernels side by side, none long
+def test_long_portions_among_many_short_ones(kind, lens):
+    c = Case(kind, 4, 2, 64, 64, lens, 3)
+    out, S = c.run()
+    for rep in range(3):     # a kernel behind it sees the ends of both
+        again, S2 = c.run()
+        assert torch.equal(again.clone(), out) and torch.equal(S2.clone(), S)
+    for i in {0, len(lens) // 2, len(lens) - 1} | {i for i, n in enumerate(lens) if n >= 64}:
+        rows = slice(c.starts[i], c.starts[i + 1])
+        o1, S1 = c.run(rows, [lens[i]], [i])
+        assert torch.equal(o1, out[rows]) and torch.equal(S1[i], S[i]), i
