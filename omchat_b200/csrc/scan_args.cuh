@@ -5,11 +5,12 @@
 namespace omc {
 
 // x / y for y >= 1: the reciprocal with one Newton step, within a unit of the last place, in five instructions without a branch (a division that serves every exponent takes
-// ten, and a call where its operands are small)
+// ten, and a call where its operands are small). y and its reciprocal are normal numbers, so .ftz gives the same bits without the scaling of small ones (convolution of
+// 3126 x 6144 37 -> 35 us, gated norms of 3126 x 4096 19.5 -> 18.1)
 __device__ __forceinline__ float over(float x, float y) {
   y = y > 8e37f ? 8e37f : y;   // its reciprocal is a normal number; NaN stays NaN
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
   return x * fmaf(r, fmaf(-y, r, 1.f), r);
 }
 __device__ __forceinline__ float sigmoid_f(float z) { return over(1.f, 1.f + expf(-z)); }
