@@ -102,8 +102,8 @@ struct ConvUnit {   // unit vectors behind the convolution: the first `channels`
 // shared memory. The same sums of taps as causal_conv_silu_kernel. UNIT: groups that a power of two of lanes of a warp holds are made unit vectors by
 // shuffles among them (every warp is whole: ch is a multiple of 128); causal_conv_silu_kernel, a block of rows in shared memory, is for other
 // groups. Nothing that a tile reads waits for another load of it, except for ring entries. 3126 rows of 4096 channels with unit queries and keys of
-// 128: 73 us there, 34 here (3.0 TB/s; 40 with a division in the activation, 42 with slots looked up in front of the rows before the tile); 6144 channels: 37
-// (4.1 TB/s; 45 with a division). What bounds it: half of the cycles the activation's instructions, otherwise the rows.
+// 128: 73 us there, 29 here (3.5 TB/s; 40 with a division in the activation, 42 with slots looked up in front of the rows before the tile); 6144 channels: 33
+// (4.6 TB/s; 45 with a division). What bounds it: half of the cycles the activation's instructions, otherwise the rows.
 template <typename TW, typename TY, int TAPS, int ROWS, bool UNIT>
 __global__ void __launch_bounds__(128) causal_conv_rows_kernel(const float* __restrict__ x, long long ldx, int T, int ch,
                                                                const TW* __restrict__ w, const TW* __restrict__ bias,
@@ -1495,9 +1495,10 @@ extern "C" int omc_causal_conv(const float* x, long long ldx, int T, int ch, con
                                                               reinterpret_cast<uintptr_t>(w) % 16 == 0);
       };
       auto go = [&](auto taps_c) {
-        constexpr int TAPS = decltype(taps_c)::value;
-        if (T >= 256 && unit) launch(causal_conv_rows_kernel<TW, TY, TAPS, kConvRows, true>, kConvRows);
-        else if (T >= 256) launch(causal_conv_rows_kernel<TW, TY, TAPS, kConvRows, false>, kConvRows);
+        // four rows keep more warps on an SM than eight, whose thread reads its weights less often: with weights of 16 bits 33 and 35 us, of 32 bits 37 and 35 (3126 x 6144)
+        constexpr int TAPS = decltype(taps_c)::value, ROWS = sizeof(TW) == 2 ? 4 : 8;
+        if (T >= 256 && unit) launch(causal_conv_rows_kernel<TW, TY, TAPS, ROWS, true>, ROWS);
+        else if (T >= 256) launch(causal_conv_rows_kernel<TW, TY, TAPS, ROWS, false>, ROWS);
         else if (unit) launch(causal_conv_rows_kernel<TW, TY, TAPS, 1, true>, 1);
         else launch(causal_conv_rows_kernel<TW, TY, TAPS, 1, false>, 1);
       };

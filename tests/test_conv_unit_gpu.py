@@ -41,3 +41,29 @@ def test_unit_groups(ch, group, unit, scaled, taps, ydt):
         # a few roundings of values of order one (taps, silu, sum of squares, quotient), then the output's own
         assert ((got - want).abs() <= 4e-6 * (1 + want.abs()) + (want.abs() * 2.0 ** -8 if ydt == torch.bfloat16 else 0)).all()
         at += n
+
+
+@pytest.mark.parametrize("T", [256, 259, 263, 700])
+@pytest.mark.parametrize("unit", [0, 64])
+def test_tiles_of_four_and_eight_rows_agree(T, unit):
+    """Weights of 16 bits take tiles of four rows, of 32 bits tiles of eight; the ring is written beside the end of the convolution and read by the next one."""
+    gen = torch.Generator().manual_seed(T)
+    x = torch.randn(2 * T, 512, generator=gen).cuda()
+    w = torch.randn(512, 4, generator=gen).to(torch.bfloat16).cuda()
+    lens = [T - 11, 2, 9]
+    slot = torch.tensor([i for i, n in enumerate(lens) for _ in range(n)], dtype=torch.int32).cuda()
+    pos = torch.tensor([p for n in lens for p in range(n)], dtype=torch.int32).cuda()
+    after = pos + torch.tensor(lens, dtype=torch.int32).cuda()[slot.long()]
+    kw = dict(unit_channels=256, unit_group=unit, unit_eps=1e-6, scaled_channels=128, unit_mult=0.5) if unit else {}
+    got = []
+    for wt in (w, w.float()):
+        state, y = torch.full((3, 3, 512), float("nan"), device="cuda"), torch.empty(2 * T, 512, device="cuda")
+        seqlib.causal_conv_silu(x[:T], wt, pos, slot, state, y[:T], **kw)
+        seqlib.causal_conv_silu(x[T:], wt, after, slot, state, y[T:], **kw)
+        got.append((y, state))
+    assert torch.isfinite(got[0][0]).all() and torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    whole = torch.empty(2 * lens[0], 512, device="cuda")     # the first request in one go
+    rows = torch.cat([x[:lens[0]], x[T:T + lens[0]]])
+    n = torch.arange(2 * lens[0], dtype=torch.int32).cuda()
+    seqlib.causal_conv_silu(rows, w, n, torch.zeros_like(n), torch.full((1, 3, 512), float("nan"), device="cuda"), whole, **kw)
+    assert torch.equal(torch.cat([got[0][0][:lens[0]], got[0][0][T:T + lens[0]]]), whole)
