@@ -50,13 +50,17 @@ struct ScanArgs {
 };
 
 // The two kernels of a step write different portions and slots, so the second may run beside the first: the first lets it start as soon as all of its own CTAs have, and the
-// second ends behind the first, whose end nothing else would wait for. One CTA does that; all of them would keep their place on an SM.
+// second ends behind the first, whose end nothing else would wait for: what comes next on the stream waits for the second alone. One CTA does that, on whichever way it goes
+// out (so the wait is a destructor's); all of them would keep their place on an SM.
 __device__ __forceinline__ void scan_begin(const ScanArgs& a) {
   if (a.beside == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-__device__ __forceinline__ void scan_end(const ScanArgs& a) {
-  if (a.beside == 2 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
-}
+struct ScanEnd {
+  const ScanArgs& a;
+  __device__ __forceinline__ ~ScanEnd() {
+    if (a.beside == 2 && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+};
 template <typename... Params, typename... Args>
 int scan_launch(void (*kernel)(Params...), dim3 grid, int threads, int smem, cudaStream_t st, const ScanArgs& a, Args... args) {
   cudaLaunchConfig_t cfg{};

@@ -324,6 +324,7 @@ __host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
 }
 template <int DPT, bool VEC, int KIND, bool CHAN, int TOK>   // CHAN: one decay per key channel
 __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 32 ? 4 : 7) : 0) linear_state_scan_kernel(ScanArgs a) {
+  const ScanEnd end{a};
   extern __shared__ __align__(16) float sm[];
   constexpr int PITCH = kScanLanes * (DPT + 4), CPT = kScanCpt, COLS = kScanGroups * CPT, DP = DPT / 2;
   constexpr int OPITCH = COLS + 4;           // a lane's partial read-outs of one token
@@ -337,7 +338,7 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
   const int h = blockIdx.y, kvh = h / (a.H / a.G);
   const int col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
-  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return scan_end(a);
+  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
   // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
   // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
   const int tid = threadIdx.x, lane = WIDE ? tid / kScanGroups : tid & (kScanLanes - 1), cg = WIDE ? tid % kScanGroups : tid / kScanLanes;
@@ -642,7 +643,6 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
       }
     }
   }
-  scan_end(a);
 }
 
 // The same recurrence for portions of several tokens at 64 or 128 key channels, inputs that need no preparation of their own (no silu, per-channel decays given)
@@ -669,6 +669,7 @@ struct ScanRowsShared {
 
 template <int DIM, int CPT, int KIND, bool CHAN>
 __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
+  const ScanEnd end{a};
   extern __shared__ __align__(16) float sm[];
   constexpr int COLS = kSrThreads / kScanLanes * CPT;
   typedef ScanRowsShared<DIM, COLS, CHAN> Shared;
@@ -679,7 +680,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
   const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
   const int portion = a.portions > 1 ? scan_portion(a.row_begin, a.portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1];
-  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return scan_end(a);
+  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
   const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
   const bool in = col < a.vdim;   // a thread's columns all exist or none does
   const float A = KIND == kScanStep || a.decay_mode == 1 ? expf(a.A_log[h]) : 0.f;

@@ -28,19 +28,24 @@ class Case:
         self.starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
         self.S0 = rn(len(lens), H, dim, vdim) if first else torch.zeros(len(lens), H, dim, vdim, device="cuda")
 
-    def run(self, rows=slice(None), lens=None, slots=None, S=None, first=None):
+    def prepared(self, rows=slice(None), lens=None, slots=None, first=None):
+        """The call with everything on the device: nothing but the launches is left."""
         lens = self.lens if lens is None else lens
         slots = range(len(lens)) if slots is None else slots
-        S = self.S0.clone() if S is None else S
         first = self.first if first is None else first
         kw = {"delta": dict(a=self.a[rows], A_log=self.A_log, dt_bias=self.dtb, beta=self.beta[rows]), "delta_const": dict(decay_const=self.const, beta=self.beta[rows], out_scale=0.5),
               "given": dict(a=self.a[rows], beta=self.beta[rows], channel_decay=True, decay_given=True),
               "given_plain": dict(a=self.a[rows], channel_decay=True, decay_given=True),
               "given_minus_one": dict(a=self.a[rows], channel_decay=True, decay_given=True, sigmoid_pow=1.0)}[self.kind]
-        out = torch.empty(sum(lens), self.H * self.vdim, device="cuda")
         begin = _i32([sum(lens[:i]) for i in range(len(lens) + 1)])
         pos, slot = _i32([first + p for n in lens for p in range(n)]), _i32([s for s, n in zip(slots, lens) for _ in range(n)])
-        seqlib.linear_state_scan(self.q[rows], self.k[rows], self.v[rows], S, out, begin, len(lens), pos, slot, self.H, self.G, self.dim, self.vdim, **kw)
+        q, k, v = self.q[rows], self.k[rows], self.v[rows]
+        return lambda out, S: seqlib.linear_state_scan(q, k, v, S, out, begin, len(lens), pos, slot, self.H, self.G, self.dim, self.vdim, **kw)
+
+    def run(self, rows=slice(None), lens=None, slots=None, S=None, first=None):
+        S = self.S0.clone() if S is None else S
+        out = torch.empty(sum(self.lens if lens is None else lens), self.H * self.vdim, device="cuda")
+        self.prepared(rows, lens, slots, first)(out, S)
         return out, S
 
     def exact(self):
@@ -114,10 +119,37 @@ def test_many_portions_of_which_few_are_long():
 def test_long_portions_among_many_short_ones(kind, lens):
     c = Case(kind, 4, 2, 64, 64, lens, 3)
     out, S = c.run()
-    for rep in range(3):     # a kernel behind it sees the ends of both
-        again, S2 = c.run()
-        assert torch.equal(again.clone(), out) and torch.equal(S2.clone(), S)
     for i in {0, len(lens) // 2, len(lens) - 1} | {i for i, n in enumerate(lens) if n >= 64}:
         rows = slice(c.starts[i], c.starts[i + 1])
         o1, S1 = c.run(rows, [lens[i]], [i])
         assert torch.equal(o1, out[rows]) and torch.equal(S1[i], S[i]), i
+
+
+@pytest.mark.parametrize("kind,H,dim", [("delta", 4, 128), ("delta", 2, 64), ("given", 2, 64), ("given", 32, 128), ("given_minus_one", 32, 64)])   # 32 heads: the general kernel has the short ones
+@pytest.mark.parametrize("lens", [[1, 2000], [9, 64, 1], [1] * 8 + [2000], [1500, 1]])   # a short portion is the second kernel's first: one of its CTAs waits all the same
+@pytest.mark.parametrize("graph", [False, True])
+def test_what_follows_a_step_sees_the_ends_of_both_kernels(kind, H, dim, lens, graph):
+    c = Case(kind, H, 1, dim, 64, lens, 3)
+    want, Sw = c.run()
+    torch.cuda.synchronize()
+    scan, out, S = c.prepared(), torch.empty_like(want), torch.empty_like(Sw)
+    out2, S2 = torch.empty_like(want), torch.empty_like(Sw)
+
+    def step():     # copies right behind the scan read what they see then
+        scan(out, S)
+        out2.copy_(out)
+        S2.copy_(S)
+
+    if graph:
+        side = torch.cuda.Stream()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=side):
+            step()
+    for _ in range(3):
+        S.copy_(c.S0)
+        for x in (out, out2, S2):
+            x.fill_(torch.nan)
+        torch.cuda.synchronize()
+        g.replay() if graph else step()
+        torch.cuda.synchronize()
+        assert torch.equal(out2, want) and torch.equal(S2, Sw)
