@@ -177,10 +177,10 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
         if (DELTA) raw_b = a.beta[(long long)t * a.ldb + h];
       }
     };
-    auto put_raw = [&](int c0, int block) {   // a token behind the end decays nothing; its zero rows enter nothing
+    auto put_raw = [&](int c0, int block) {   // a token behind the end decays nothing (however large A is); its zero rows enter nothing
       const bool there = c0 + wl < r1;
-      const float x = logs && there ? softplus_f(raw_a + bias) : 0.f;
-      sh.la[(block & 1) * 32 + wl] = product ? (there ? gconst : 1.f) : -A * x;
+      const float none = product ? 1.f : 0.f;
+      sh.la[(block & 1) * 32 + wl] = there ? (product ? gconst : (logs ? -A * softplus_f(raw_a + bias) : 0.f)) : none;
       if (DELTA) sh.w[(block & 1) * 32 + wl] = sigmoid_f(raw_b);
     };
     // What the tokens of a stage have among themselves: warp w forms the products of tokens w and 7 - w with those up to them (nine each, the lanes over the channels)

@@ -153,3 +153,15 @@ def test_what_follows_a_step_sees_the_ends_of_both_kernels(kind, H, dim, lens, g
         g.replay() if graph else step()
         torch.cuda.synchronize()
         assert torch.equal(out2, want) and torch.equal(S2, Sw)
+
+
+@pytest.mark.parametrize("n", [75, 72])     # a ragged last stage, and a whole one
+def test_heads_that_forget_at_once(n):
+    c = Case("delta", 2, 1, 128, 64, [n], 5)
+    c.A_log[1] = 90.0     # its exponential is an infinity: a decay of zero
+    out, S = c.run()
+    S1 = c.S0.clone()
+    single = torch.cat([c.run(slice(t, t + 1), [1], [0], S1, 5 + t)[0] for t in range(n)])
+    assert torch.isfinite(single).all() and torch.isfinite(out).all() and torch.isfinite(S).all()
+    # each form is within 5e-7 of float64 (above), so the two are within twice that of each other
+    assert _rel(out, single.double()) < 1e-6 and _rel(S, S1.double()) < 1e-6
