@@ -46,8 +46,15 @@ struct ScanArgs {
   bool vec_state, vec_out;   // a thread's columns of the state / four outputs as one access
   int portions;              // P, where the CTAs take portions in the order of their lengths, the longest first; 0: in their own order
   int long_from;             // portions of this many rows and more are scan_chunk_kernel's, the others the token-by-token kernels' (0: all of them are theirs)
+  int rows;                  // the host's number of rows, by which scan_chunk_kernel has been launched
   int beside;                // 1, 2: the first and the second of the two kernels that share the portions of a step; 0: alone
 };
+
+// Whether a portion of n rows is scan_chunk_kernel's, for which the host has launched CTAs for rows / long_from portions: if row_begin has more rows than the host was told of,
+// there may be more long portions than that, and the token-by-token kernels take them all.
+__device__ __forceinline__ bool scan_is_long(const ScanArgs& a, int portions, int n) {
+  return a.long_from > 0 && n >= a.long_from && a.row_begin[portions] - a.row_begin[0] <= a.rows;
+}
 
 // The two kernels of a step write different portions and slots, so the second may run beside the first: the first lets it start as soon as all of its own CTAs have, and the
 // second ends behind the first, whose end nothing else would wait for: what comes next on the stream waits for the second alone. One CTA does that, on whichever way it goes

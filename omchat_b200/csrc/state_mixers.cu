@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
   const int h = blockIdx.y, kvh = h / (a.H / a.G);
   const int col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
-  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
+  if (r1 <= r0 || scan_is_long(a, gridDim.z, r1 - r0)) return;
   // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
   // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
   const int tid = threadIdx.x, lane = WIDE ? tid / kScanGroups : tid & (kScanLanes - 1), cg = WIDE ? tid % kScanGroups : tid / kScanLanes;
@@ -680,7 +680,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
   const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
   const int portion = a.portions > 1 ? scan_portion(a.row_begin, a.portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1];
-  if (r1 <= r0 || (a.long_from > 0 && r1 - r0 >= a.long_from)) return;
+  if (r1 <= r0 || scan_is_long(a, gridDim.z, r1 - r0)) return;
   const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
   const bool in = col < a.vdim;   // a thread's columns all exist or none does
   const float A = KIND == kScanStep || a.decay_mode == 1 ? expf(a.A_log[h]) : 0.f;
@@ -1593,7 +1593,7 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   if (dim > 256) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: key width above 256");
   if (portions > 65535 || H > 65535) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: more than 65535 portions or heads");
   ScanArgs s{q, k, v, ldq, ldk, ldv, silu_in, decay_mode, decay_pow, out_scale, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo,
-             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0, 0};
+             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0, rows, 0};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int dpt = dim <= 32 ? 4 : (dim <= 64 ? 8 : (dim <= 128 ? 16 : 32));   // key channels per thread: dim / 8 lanes, rounded up to a float4
   const bool chan = decay_mode >= 2 && decay_mode <= 5;
@@ -1699,8 +1699,11 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
   };
   // long portions of the delta rule and with per-channel decays: scan_chunk_kernel; whichever are left, the kernels above
   if (!several || rows < kScanLong || !(chan || (beta != nullptr && decay_mode <= 1))) return tokens();
+  if (portions == 1) {   // alone: what row_begin has is this kernel's, however few rows (a padded buffer)
+    s.long_from = 1, s.rows = 0x7fffffff;
+    return launch_scan_chunk(s, rows, portions, st);
+  }
   s.long_from = kScanLong;
-  if (portions == 1) return launch_scan_chunk(s, rows, portions, st);
   // The long chains first, the others beside them. In us, all token by token / one kernel behind the other / beside: 500 + 16 x 1 tokens of 16 heads of 128 x 128 131 / 97 / 90, with
   // decays per channel 195 / 113 / 101 (152 with the short ones first); 65 + 31 x 1 tokens 29 / 36 / 25; 100, 50, 50, 50 33 / 46 / 31. The host does not know the lengths: where no
   // portion is long, the first kernel is empty and costs 1.2 on the device (8 x 8 tokens 9.3 / 10.5).

@@ -165,3 +165,15 @@ def test_heads_that_forget_at_once(n):
     assert torch.isfinite(single).all() and torch.isfinite(out).all() and torch.isfinite(S).all()
     # each form is within 5e-7 of float64 (above), so the two are within twice that of each other
     assert _rel(out, single.double()) < 1e-6 and _rel(S, S1.double()) < 1e-6
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("lens,rows", [([40], 100), ([1], 64), ([100, 3, 80], 70), ([100, 3, 80], 183), ([30, 64, 9], 200)])   # rows of the tensors: more than the portions have, fewer, as many
+def test_what_is_computed_is_a_matter_of_row_begin(kind, lens, rows):
+    n = sum(lens)
+    c = Case(kind, 2, 1, 64, 36, lens + [max(rows - n, 1)], 5)
+    out, S = torch.full((len(c.q), 2 * 36), torch.nan, device="cuda"), c.S0.clone()
+    c.prepared(slice(0, rows), lens)(out, S)
+    want, Sw = c.exact()
+    assert _rel(out[:n], want[:n]) < 5e-7 and _rel(S[:-1], Sw[:-1]) < 5e-7
+    assert out[n:].isnan().all() and torch.equal(S[-1], c.S0[-1])
