@@ -5,10 +5,11 @@
 // Warp 0: TMA (three-dimensional maps: K, rows, batch; edges arrive as zeros), as far ahead as the ring goes. Warp 1: MMA issuer, into one of two accumulators.
 // The others: epilogue, thread = row; gates are asked for before the accumulator is waited for. The K terms of an output are added in one order whatever
 // the tile, so a row's result does not depend on M.
-// What bounds it: bytes (103 MB from L2 and 26 MB of output and gate in 19 us) behind 8 us of set-up, first load and last epilogue; before, one tile per CTA and two CTAs per SM, a tile's
+// What bounds it: bytes (103 MB from L2 and 26 MB of output and gate in 19 to 21 us) behind 8 us of set-up, first load and last epilogue; before, one tile per CTA and two CTAs per SM, a tile's
 // load (2.9 us) and epilogue (4.3, with a gate 11.5: fp32 slabs read with two-way bank conflicts, gates asked for behind the accumulator, divisions of 10
-// instructions) followed one another. 3126 rows x 16 heads, us (before): 128 -> 512 18.6 (39.5); 512 -> 128 with a gate per element 18.6 (45.0); 1338 rows without
+// instructions) followed one another. 3126 rows x 16 heads, us (before): 128 -> 512 18.6 (39.5); 512 -> 128 with a gate per element 20.7 (45.0; 26.8 with the quotients as plain divisions); 1338 rows without
 // a gate 12.4 (31.0), 11.1 (18.6); 300 rows 8.2 (10.5), 10.4 (12.5); 94 rows 8.6 (10.5), 10.4 (19.6); 1 row 7.9 (8.0), 8.8 (8.9).
+#include "fp32_pairs.cuh"
 #include "linear_args.cuh"
 #include "sm100_step.cuh"
 
@@ -52,13 +53,18 @@ __device__ __forceinline__ void hg_gates(const LinearArgs& a, const uint4 (&g)[2
     z[0] = g0.x, z[1] = g0.y, z[2] = g1.x, z[3] = g1.y, z[4] = g2.x, z[5] = g2.y, z[6] = g3.x, z[7] = g3.y;
   }
 }
-// x / y for y >= 1: the reciprocal with one Newton step, within a unit of the last place (what the exponential in y is off by is more) and without the branches of a
-// division that serves every exponent, which took longer than the product's other instructions and a call for every zero
-__device__ __forceinline__ float hg_divide(float x, float y) {
-  y = y > 1e38f ? 1e38f : y;   // NaN stays NaN
-  float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return x * fmaf(r, fmaf(-y, r, 1.f), r);
+// f[e] / y[e], y >= 1 behind a gate, the bits of a division: by quotients2 unless one of the eight is out of its range
+__device__ __forceinline__ void hg_divide(float (&f)[8], const float (&y)[8]) {
+  float most = fabsf(f[0]), least = most, top = y[0];
+#pragma unroll
+  for (int e = 1; e < 8; ++e) most = fmaxf(most, fabsf(f[e])), least = fminf(least, fabsf(f[e])), top = fmaxf(top, y[e]);
+  if (most <= 0x1p100f && least >= 0x1p-60f && top <= 0x1p62f) {
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) quotients2(-f[e], -f[e + 1], y[e], y[e + 1], f[e], f[e + 1]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) f[e] /= y[e];
+  }
 }
 __device__ __forceinline__ void hg_store(float* y, const float (&f)[8]) {
   reinterpret_cast<float4*>(y)[0] = make_float4(f[0], f[1], f[2], f[3]);
@@ -233,7 +239,8 @@ __global__ void __launch_bounds__(64 + 32 * hg_epilogue(BN)) linear_sm100_kernel
               if (a.gate != nullptr) {
                 hg_gates(a, gate[j], z);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = hg_divide(f[e], 1.f + __expf(-z[e]));   // as at the edges: bits do not depend on the tile
+                for (int e = 0; e < 8; ++e) z[e] = 1.f + __expf(-z[e]);   // as at the edges: bits do not depend on the tile
+                hg_divide(f, z);
               }
               hg_store(y + (long long)(j * 4) * a.ldy, f);
             }
@@ -262,7 +269,7 @@ __global__ void __launch_bounds__(64 + 32 * hg_epilogue(BN)) linear_sm100_kernel
                 z[e] = e >= left ? 0.f : (a.gate_dt == OMC_DT_F32 ? static_cast<const float*>(a.gate)[at + e] : ldf(static_cast<const bf16_t*>(a.gate) + at + e));
             }
 #pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = hg_divide(f[e], 1.f + (pair_gate && n + (e | 1) < a.N ? __expf(-z[e]) : expf(-z[e])));
+            for (int e = 0; e < 8; ++e) f[e] /= 1.f + (pair_gate && n + (e | 1) < a.N ? __expf(-z[e]) : expf(-z[e]));
           }
           TY* y = static_cast<TY*>(a.Y) + (long long)b * a.sy + (long long)mr * a.ldy + n;
           if (vec_out && left == 8) {

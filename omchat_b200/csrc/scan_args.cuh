@@ -1,19 +1,27 @@
-// What the kernels of the linear-state recurrence share (state_mixers.cu describes it): their arguments, packed fp32 pairs, asynchronous copies.
+// What the kernels of the linear-state recurrence share (state_mixers.cu describes it): their arguments, activations, asynchronous copies.
 #pragma once
+#include "fp32_pairs.cuh"
 #include "seq_common.cuh"
 
 namespace omc {
 
-// x / y for y >= 1: the reciprocal with one Newton step, within a unit of the last place, in five instructions without a branch (a division that serves every exponent takes
-// ten, and a call where its operands are small). y and its reciprocal are normal numbers, so .ftz gives the same bits without the scaling of small ones (convolution of
-// 3126 x 6144 37 -> 35 us, gated norms of 3126 x 4096 19.5 -> 18.1)
-__device__ __forceinline__ float over(float x, float y) {
-  y = y > 8e37f ? 8e37f : y;   // its reciprocal is a normal number; NaN stays NaN
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-  return x * fmaf(r, fmaf(-y, r, 1.f), r);
+__device__ __forceinline__ float sigmoid_f(float z) { return 1.f / (1.f + expf(-z)); }
+__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
+// The same bits for four numbers at once: a division serves every exponent, in some ten instructions with a branch each, which these functions' callers wait for. Where a number
+// is further from zero than 44 (or infinite) all four are divided.
+template <bool SILU>
+__device__ __forceinline__ void sigmoid4(float (&z)[4]) {
+  float y[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) y[e] = 1.f + expf(-z[e]);
+  if (fmaxf(fmaxf(fabsf(z[0]), fabsf(z[1])), fmaxf(fabsf(z[2]), fabsf(z[3]))) <= 44.f) {
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) quotients2(SILU ? -z[e] : -1.f, SILU ? -z[e + 1] : -1.f, y[e], y[e + 1], z[e], z[e + 1]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) z[e] = (SILU ? z[e] : 1.f) / y[e];
+  }
 }
-__device__ __forceinline__ float sigmoid_f(float z) { return over(1.f, 1.f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
 struct ScanArgs {
@@ -106,25 +114,6 @@ __device__ __forceinline__ int scan_portion(const int32_t* row_begin, int portio
   const int found = scratch[0];
   __syncthreads();
   return found;
-}
-
-// Packed fp32 pairs (sm_100: one instruction, two IEEE fp32 operations): the recurrence's state lives in such pairs.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
 }
 
 enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };

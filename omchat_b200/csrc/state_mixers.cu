@@ -23,7 +23,6 @@
 
 namespace omc {
 
-__device__ __forceinline__ float silu_f(float z) { return over(z, 1.f + expf(-z)); }
 // sigmoid(z)^p - 1 = expm1(p * log sigmoid(z)), log sigmoid(z) = -softplus(-z). The decay is kept as its distance from 1: rounded to
 // fp32 itself, a decay close to 1 loses most of the digits of 1 - decay, and the state multiplies by it once per token.
 __device__ __forceinline__ float sigmoid_pow_m1_f(float z, float p) { return expm1f(-p * softplus_f(-z)); }
@@ -102,8 +101,8 @@ struct ConvUnit {   // unit vectors behind the convolution: the first `channels`
 // shared memory. The same sums of taps as causal_conv_silu_kernel. UNIT: groups that a power of two of lanes of a warp holds are made unit vectors by
 // shuffles among them (every warp is whole: ch is a multiple of 128); causal_conv_silu_kernel, a block of rows in shared memory, is for other
 // groups. Nothing that a tile reads waits for another load of it, except for ring entries. 3126 rows of 4096 channels with unit queries and keys of
-// 128: 73 us there, 29 here (3.5 TB/s; 40 with a division in the activation, 42 with slots looked up in front of the rows before the tile); 6144 channels: 33
-// (4.6 TB/s; 45 with a division). What bounds it: half of the cycles the activation's instructions, otherwise the rows.
+// 128: 73 us there, 31 here (3.3 TB/s; 34 with plain divisions in the activation, 42 with slots looked up in front of the rows before the tile); 6144 channels: 37
+// (4.2 TB/s; 40 with plain divisions). What bounds it: half of the cycles the activation's instructions, otherwise the rows.
 template <typename TW, typename TY, int TAPS, int ROWS, bool UNIT>
 __global__ void __launch_bounds__(128) causal_conv_rows_kernel(const float* __restrict__ x, long long ldx, int T, int ch,
                                                                const TW* __restrict__ w, const TW* __restrict__ bias,
@@ -168,10 +167,7 @@ __global__ void __launch_bounds__(128) causal_conv_rows_kernel(const float* __re
         const float4 v = j < R ? h[j < R ? j : 0] : xv[r];
         o[0] = fmaf(wv[j][0], v.x, o[0]), o[1] = fmaf(wv[j][1], v.y, o[1]), o[2] = fmaf(wv[j][2], v.z, o[2]), o[3] = fmaf(wv[j][3], v.w, o[3]);
       }
-      if (act) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o[i] = silu_f(o[i]);
-      }
+      if (act) sigmoid4<true>(o);
       if (UNIT) {
         float ss = fmaf(o[0], o[0], fmaf(o[1], o[1], fmaf(o[2], o[2], o[3] * o[3])));
         for (int m = 1; m < unit.lanes; m <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, m);
@@ -958,10 +954,11 @@ __global__ void __launch_bounds__(256) gated_rms_kernel(const float* __restrict_
 
 // Both norms for groups that LANES neighbouring lanes hold in PIECES pieces of four columns each (n = 4 LANES PIECES): x and the gate are read once, all
 // of it before anything is waited for, and no two warps meet. FRONT: the gate in front of the norm and a weight for every column of the row, else behind
-// it and one weight of n columns for all groups. 3126 rows: 8 parts of 512 with a bf16 gate in front 38 -> 19 us (22 with a division in the gate), 16 groups of 128 with an fp32 gate behind 29 -> 15
+// it and one weight of n columns for all groups. 3126 rows: 8 parts of 512 with a bf16 gate in front 38 -> 18 us (22 with plain divisions in the gate; 20 without the bound on
+// registers, which the quotients' rare way out takes), 16 groups of 128 with an fp32 gate behind 29 -> 14 (16)
 // (a block per part, a warp per group reading single columns twice).
 template <typename TG, typename TW, typename TY, int LANES, int PIECES, bool FRONT>
-__global__ void __launch_bounds__(256) group_rms_kernel(const float* __restrict__ x, long long ldx, int groups, long long total, const TW* __restrict__ w, float eps,
+__global__ void __launch_bounds__(256, FRONT && PIECES == 4 ? 5 : 0) group_rms_kernel(const float* __restrict__ x, long long ldx, int groups, long long total, const TW* __restrict__ w, float eps,
                                                         const TG* __restrict__ gate, long long ldg, int gate_act, TY* __restrict__ y, long long ldy) {
   constexpr int N = 4 * LANES * PIECES;
   const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;   // (row, group)
@@ -976,12 +973,12 @@ __global__ void __launch_bounds__(256) group_rms_kernel(const float* __restrict_
     ld4(x + t * ldx + c0 + c, v[p]);
     if (gate != nullptr) ld4(gate + t * ldg + c0 + c, g[p]);
   }
-  auto act = [&](float z) { return gate_act == 1 ? silu_f(z) : (gate_act == 2 ? sigmoid_f(z) : z); };
-  if (gate != nullptr) {
+  if (gate != nullptr && gate_act != 0) {
 #pragma unroll
-    for (int p = 0; p < PIECES; ++p)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) g[p][e] = act(g[p][e]);
+    for (int p = 0; p < PIECES; ++p) {
+      if (gate_act == 1) sigmoid4<true>(g[p]);
+      else sigmoid4<false>(g[p]);
+    }
   }
   float ss = 0.f;
 #pragma unroll
@@ -1509,7 +1506,7 @@ extern "C" int omc_causal_conv(const float* x, long long ldx, int T, int ch, con
                                                               reinterpret_cast<uintptr_t>(w) % 16 == 0);
       };
       auto go = [&](auto taps_c) {
-        // four rows keep more warps on an SM than eight, whose thread reads its weights less often: with weights of 16 bits 33 and 35 us, of 32 bits 37 and 35 (3126 x 6144)
+        // four rows keep more warps on an SM than eight, whose thread reads its weights less often: with weights of 16 bits 38 and 39 us, of 32 bits 38 and 35 (3126 x 6144)
         constexpr int TAPS = decltype(taps_c)::value, ROWS = sizeof(TW) == 2 ? 4 : 8;
         if (T >= 256 && unit) launch(causal_conv_rows_kernel<TW, TY, TAPS, ROWS, true>, ROWS);
         else if (T >= 256) launch(causal_conv_rows_kernel<TW, TY, TAPS, ROWS, false>, ROWS);
