@@ -133,16 +133,19 @@ __global__ void __launch_bounds__(128) latent_rope_store4_kernel(const float* __
                                                                  const int32_t* __restrict__ slot, const int32_t* __restrict__ block_table, int max_pages, int page_size,
                                                                  T* __restrict__ pool, const TQ* __restrict__ q, long long ldq, int H, int dn, T* __restrict__ qcat, T* __restrict__ qn) {
   __shared__ float red[4];
-  constexpr int KEEP = 4;              // pieces of 512 columns that wait in registers
+  constexpr int KEEP = 4, SQUARES = 4;   // pieces of 512 columns that wait in registers; columns of a thread whose squares do
   const int t = blockIdx.x, tid = threadIdx.x, p = pos[t], half = rot_dims >> 1, D = r + dr;
   const float* csr = cs + (long long)p * rot_dims;
   const float* row = dkv + (long long)t * ld;
   const bool latent = blockIdx.y == 0;   // on short steps the heads are spread over blockIdx.y
   const int per = (H + gridDim.y - 1) / gridDim.y, h0 = blockIdx.y * per, nh = min(per, H - h0), heads = max(nh, 0) + (latent ? 1 : 0);
-  float x[KEEP][4];
+  float x[KEEP][4], first[SQUARES];
 #pragma unroll
   for (int i = 0; i < KEEP; ++i)
     if (latent && (tid + i * 128) * 4 < r) ld4(row + (tid + i * 128) * 4, x[i]);
+#pragma unroll
+  for (int i = 0; i < SQUARES; ++i)
+    if (latent && tid + i * 128 < r) first[i] = row[tid + i * 128];
   const int page = block_table[(long long)slot[t] * max_pages + p / page_size];
   T* dst = pool + ((long long)page * page_size + p % page_size) * D;
   // a unit: four pairs (u, v) of a head, or of the latent row as head H
@@ -195,20 +198,16 @@ __global__ void __launch_bounds__(128) latent_rope_store4_kernel(const float* __
     }
   }
   if (!latent) return;
+  // the sum over every 128th column, as column by column: a row has the same bits whichever of the two kernels it takes
   float ss = 0.f;
-  auto add = [&](const float (&v)[4]) { ss = fmaf(v[0], v[0], ss), ss = fmaf(v[1], v[1], ss), ss = fmaf(v[2], v[2], ss), ss = fmaf(v[3], v[3], ss); };
 #pragma unroll
-  for (int i = 0; i < KEEP; ++i)
-    if ((tid + i * 128) * 4 < r) add(x[i]);
-  for (int c = (tid + KEEP * 128) * 4; c < r; c += 512) {
-    float v[4];
-    ld4(row + c, v);
-    add(v);
-  }
+  for (int i = 0; i < SQUARES; ++i)
+    if (tid + i * 128 < r) ss = fmaf(first[i], first[i], ss);
+  for (int c = tid + SQUARES * 128; c < r; c += 128) ss = fmaf(row[c], row[c], ss);
   ss = seq_warp_sum(ss);
   if ((tid & 31) == 0) red[tid >> 5] = ss;
   __syncthreads();
-  const float rstd = 1.f / sqrtf(((red[0] + red[1]) + (red[2] + red[3])) / (float)r + eps);
+  const float rstd = 1.f / sqrtf(((red[0] + red[2]) + (red[1] + red[3])) / (float)r + eps);
   auto put = [&](int c, const float (&v)[4]) {
     float u[4], o[4];
     ld4(w + c, u);

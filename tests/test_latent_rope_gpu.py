@@ -48,3 +48,24 @@ def test_rows_and_queries_against_float64(dt, qdt, keep, r, dr, rot, H, dn, T, h
     assert ((qcat[..., r:].double() - wq).abs() <= wq.abs() * (eps + 2e-6) + 2e-6).all() and (qcat[..., :r] == 7.0).all()
     if keep:
         assert torch.equal(qn.view(T, H, dn), q3[..., :dn].to(dt))
+
+
+@pytest.mark.parametrize("dt,qdt", [(BF16, F32), (BF16, BF16), (F32, F32)])
+@pytest.mark.parametrize("r,dr,rot,H,dn", [(512, 64, 64, 16, 128), (2052, 40, 8, 3, 4), (64, 32, 0, 33, 128), (256, 64, 32, 5, 64), (1200, 64, 48, 2, 32)])
+@pytest.mark.parametrize("T", [7, 65])
+@pytest.mark.parametrize("halves", [False, True])
+def test_rows_have_the_same_bits_on_and_off_the_grid(dt, qdt, r, dr, rot, H, dn, T, halves):
+    gen = torch.Generator(device="cuda").manual_seed(r + T)
+    rn = lambda *s: torch.randn(*s, generator=gen, device="cuda")  # noqa: E731
+    row, q, w = rn(T, r + dr), rn(T, H * (dn + dr)).to(qdt), (1 + 0.2 * rn(r)).to(dt)
+    angle = rn(128, max(1, rot // 2))
+    cs = torch.stack([angle.cos(), angle.sin()], -1).contiguous()
+    pos, slot, table = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (list(range(3, 3 + T)), [0] * T, [[1, 0]]))
+    got = []
+    for off in (0, 1):      # rows off 16 bytes go column by column
+        dkv = torch.zeros(T, r + dr + 4, device="cuda")[:, off:off + r + dr]
+        dkv.copy_(row)
+        pool, qcat, qn = torch.zeros(2, 64, r + dr, device="cuda", dtype=dt), torch.zeros(T, H, r + dr, device="cuda", dtype=dt), torch.empty(T, H * dn, device="cuda", dtype=dt)
+        seqlib.latent_rope_store(dkv, r, dr, w, 1e-6, cs, rot, pos, slot, table, 64, pool, q, H, dn, qcat, qn=qn, rot_halves=halves)
+        got.append((pool, qcat, qn))
+    assert all(torch.equal(a, b) for a, b in zip(*got))
