@@ -310,6 +310,12 @@ int omc_linear_state_scan(const float* q, long long ldq, const float* k, long lo
                           const float* dt_bias, const float* D, const float* beta, long long ldb, float* state, float* out, long long ldo,
                           const int32_t* row_begin, int portions, const int32_t* pos, const int32_t* slot, int rows, int H, int G,
                           int dim, int vdim, float decay_pow, float out_scale, void* stream);
+/* The same where the host knows of a number of rows, `longest`, that no portion has more of: without long portions there is nothing to launch for them. */
+int omc_linear_state_scan_longest(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, int silu_in,
+                                  int decay_mode, const float* decay_const, const float* a, long long lda, const float* A_log,
+                                  const float* dt_bias, const float* D, const float* beta, long long ldb, float* state, float* out, long long ldo,
+                                  const int32_t* row_begin, int portions, const int32_t* pos, const int32_t* slot, int rows, int longest, int H, int G,
+                                  int dim, int vdim, float decay_pow, float out_scale, void* stream);
 
 /* y[t, g * n + c] = x[t, g * n + c] / sqrt(mean_c(x[t, g * n + :]^2) + eps) * w[c] * act(gate[t, g * n + c]) for g < groups.
  * gate fp32 or NULL; gate_act 0: as is, 1: silu, 2: sigmoid. w [n] of w_dt, y of y_dt. */

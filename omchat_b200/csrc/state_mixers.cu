@@ -1581,6 +1581,15 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
                                      const float* A_log, const float* dt_bias, const float* D, const float* beta, long long ldb, float* state,
                                      float* out, long long ldo, const int32_t* row_begin, int portions, const int32_t* pos,
                                      const int32_t* slot, int rows, int H, int G, int dim, int vdim, float decay_pow, float out_scale, void* stream) {
+  return omc_linear_state_scan_longest(q, ldq, k, ldk, v, ldv, silu_in, decay_mode, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo, row_begin, portions, pos,
+                                       slot, rows, rows, H, G, dim, vdim, decay_pow, out_scale, stream);
+}
+
+extern "C" int omc_linear_state_scan_longest(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv,
+                                             int silu_in, int decay_mode, const float* decay_const, const float* a, long long lda,
+                                             const float* A_log, const float* dt_bias, const float* D, const float* beta, long long ldb, float* state,
+                                             float* out, long long ldo, const int32_t* row_begin, int portions, const int32_t* pos, const int32_t* slot, int rows, int longest,
+                                             int H, int G, int dim, int vdim, float decay_pow, float out_scale, void* stream) {
   if (q == nullptr || k == nullptr || v == nullptr || state == nullptr || out == nullptr || row_begin == nullptr || pos == nullptr ||
       slot == nullptr || portions < 0 || H <= 0 || G <= 0 || H % G || dim <= 0 || vdim <= 0 || decay_mode < 0 || decay_mode > 6 ||
       (decay_mode == 0 && decay_const == nullptr) || (decay_mode != 0 && a == nullptr) || (decay_mode == 6 && beta != nullptr) || (D != nullptr && decay_mode != 6) ||
@@ -1695,15 +1704,16 @@ extern "C" int omc_linear_state_scan(const float* q, long long ldq, const float*
 #undef OMC_SCAN_LAUNCH
   };
   // long portions of the delta rule and with per-channel decays: scan_chunk_kernel; whichever are left, the kernels above
-  if (!several || rows < kScanLong || !(chan || (beta != nullptr && decay_mode <= 1))) return tokens();
+  // (every portion has a row at least, so that none can have more than what is left)
+  if (!several || longest < kScanLong || rows - portions + 1 < kScanLong || !(chan || (beta != nullptr && decay_mode <= 1))) return tokens();
   if (portions == 1) {   // alone: what row_begin has is this kernel's, however few rows (a padded buffer)
     s.long_from = 1, s.rows = 0x7fffffff;
     return launch_scan_chunk(s, rows, portions, st);
   }
   s.long_from = kScanLong;
   // The long chains first, the others beside them. In us, all token by token / one kernel behind the other / beside: 500 + 16 x 1 tokens of 16 heads of 128 x 128 131 / 97 / 90, with
-  // decays per channel 195 / 113 / 101 (152 with the short ones first); 65 + 31 x 1 tokens 29 / 36 / 25; 100, 50, 50, 50 33 / 46 / 31. The host does not know the lengths: where no
-  // portion is long, the first kernel is empty and costs 1.2 on the device (8 x 8 tokens 9.3 / 10.5).
+  // decays per channel 195 / 113 / 101 (152 with the short ones first); 65 + 31 x 1 tokens 29 / 36 / 25; 100, 50, 50, 50 33 / 46 / 31. Where no portion is
+  // long the first kernel is empty and costs 1.2 on the device (8 x 8 tokens 9.3 / 10.5), so the host says how long they are at most.
   s.beside = 1;
   if (const int rc = launch_scan_chunk(s, rows, portions, st); rc != OMC_OK) return rc;
   s.beside = 2;

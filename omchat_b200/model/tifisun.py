@@ -284,7 +284,7 @@ class TifisunDecoder:
         return dense_linear(x, w, out_dtype, tensor_gemm=self.tensor_gemm, act=act, bias=bias)
 
     # ---- mixers: compute-dtype rows [T, C] -> fp32 [T, C] (two tensors for the parallel mixer)
-    def _delta(self, li: int, xb, pos, slot, cache: PagedStateCache, row_begin, n_portions: int):
+    def _delta(self, li: int, xb, pos, slot, cache: PagedStateCache, row_begin, n_portions: int, longest: Optional[int] = None):
         m: DeltaRuleSpec = self.cfg.layers[li].mixer
         mw: DeltaW = self.w.layers[li].mix
         st = cache.states[li]
@@ -306,7 +306,7 @@ class TifisunDecoder:
             seqlib.map_rows(a, seqlib.MAP_DECAY, mw.A_log, mw.dt_bias, d)
         seqlib.linear_state_scan(qkv[:, :nqk], qkv[:, nqk:2 * nqk], qkv[:, 2 * nqk:], st["S"], o, row_begin, n_portions, pos, slot, H, G, d, dv,
                                  a=a, A_log=mw.A_log, dt_bias=mw.dt_bias, channel_decay=m.channel_decay, beta=z[:, mw.cols["beta"]],
-                                 decay_given=prep)
+                                 decay_given=prep, longest=longest)
         on = torch.empty(T, H * dv, device=dev, dtype=self.dtype)
         seqlib.gated_rms_rows(o, H, dv, mw.norm, self.eps, gate, seqlib.GATE_SIGMOID if m.channel_decay else seqlib.GATE_SILU, on)
         return self._linear(on, mw.o, f32)
@@ -387,6 +387,7 @@ class TifisunDecoder:
         # work lists of the tensor-core attention kernel, built once per step and head grouping; without the host's view of the
         # batch (portions) the plain kernel runs
         plans = {"portions": None} if one_row_each else ({"portions": list(portions)} if portions is not None else None)
+        longest = max((p[1] for p in portions), default=0) if portions is not None else None
         layers, mult = self.w.layers, self.cfg.residual_mult
         h32 = torch.empty(T, self.C, device=dev, dtype=f32)
         xb = torch.empty(T, self.C, device=dev, dtype=self.dtype)
@@ -398,7 +399,7 @@ class TifisunDecoder:
             after_mixer = lw.norm2 if lw.mlp is not None else nxt
             xb_out = xb if (lw.mlp is not None or not last) else None
             if isinstance(self.cfg.layers[li].mixer, DeltaRuleSpec):
-                y = self._delta(li, xb, pos, slot, cache, row_begin, n_portions)
+                y = self._delta(li, xb, pos, slot, cache, row_begin, n_portions, longest)
                 seqlib.post_norm_residual(y, lw.norm1b, self.eps, mult, h32, after_mixer, xb_out)
             else:
                 yl, yr = self._parallel(li, xb, pos, slot, cache, row_begin, n_portions, plans)

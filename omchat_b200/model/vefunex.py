@@ -351,7 +351,8 @@ class VefunexDecoder(GraphedDecodeMixin):
         if prep:
             seqlib.map_rows(a, seqlib.MAP_SIGMOID_POW, bias=mw.a2_b, p_exp=1.0 / m.tau)
         seqlib.linear_state_scan(z[:, c["q"]], z[:, c["k"]], z[:, c["v"]], cache.states[li]["S"], o, ctx["row_begin"], ctx["n_portions"], pos, slot,
-                                 H, H, d, dv, a=a, dt_bias=mw.a2_b, decay_given=prep, sigmoid_pow=1.0 / m.tau, out_scale=d ** -0.5)
+                                 H, H, d, dv, a=a, dt_bias=mw.a2_b, decay_given=prep, sigmoid_pow=1.0 / m.tau, out_scale=d ** -0.5,
+                                 longest=ctx["longest"])
         on = torch.empty(T, H * dv, device=dev, dtype=self.dtype)
         seqlib.gated_rms_rows(o, H, dv, mw.norm, self.eps, z[:, c["g"]], seqlib.GATE_SILU, on)
         return self._linear(on, mw.o, f32)
@@ -383,6 +384,7 @@ class VefunexDecoder(GraphedDecodeMixin):
             portions = None
         row_begin, n_portions = portion_starts(self, T, slot, portions, one_row_each)
         ctx = {"cache": cache, "pos": pos, "slot": slot, "row_begin": row_begin, "n_portions": n_portions, "single": n_portions == T,
+               "longest": max((p[1] for p in portions), default=0) if portions is not None else None,
                # work lists of the tensor-core attention kernel, built once per step and head grouping; without the host's view of
                # the batch (portions) the plain kernel runs
                "plans": {"portions": None} if one_row_each else ({"portions": list(portions)} if portions is not None else None)}

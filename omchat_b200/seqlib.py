@@ -43,6 +43,7 @@ SIGNATURES = {
     "omc_moe_combine_depth": (_I, [_P, _L, _P, _P, _I, _P, _L, _P, _L, _F, _P, _L, _F, _F, _P, _L, _L, _I, _P, _I, _P, _L, _I, _I, _P]),
     "omc_conv_qk_norm_kv_store": (_I, [_P, _L, _I, _I, _P, _I, _I, _P, _P, _P, _I, _I, _I, _P, _P, _F, _P, _I, _I, _P, _P, _L, _I, _I, _P]),
     "omc_linear_state_scan": (_I, [_P, _L, _P, _L, _P, _L, _I, _I, _P, _P, _L, _P, _P, _P, _P, _L, _P, _P, _L, _P, _I, _P, _P, _I, _I, _I, _I, _I, _F, _F, _P]),
+    "omc_linear_state_scan_longest": (_I, [_P, _L, _P, _L, _P, _L, _I, _I, _P, _P, _L, _P, _P, _P, _P, _L, _P, _P, _L, _P, _I, _P, _P, _I, _I, _I, _I, _I, _I, _F, _F, _P]),
     "omc_map_rows": (_I, [_P, _L, _I, _I, _I, _P, _P, _I, _F, _P]),
     "omc_gated_rms_rows": (_I, [_P, _L, _I, _I, _I, _P, _I, _F, _P, _L, _I, _P, _I, _L, _P]),
     "omc_gate_rms_rows": (_I, [_P, _L, _I, _I, _I, _P, _I, _F, _P, _I, _L, _I, _P, _I, _L, _P]),
@@ -677,12 +678,12 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
                       decay_const: Optional[torch.Tensor] = None, a: Optional[torch.Tensor] = None, A_log: Optional[torch.Tensor] = None,
                       dt_bias: Optional[torch.Tensor] = None, channel_decay: bool = False, beta: Optional[torch.Tensor] = None,
                       decay_given: bool = False, sigmoid_pow: Optional[float] = None, out_scale: float = 1.0, step_size: bool = False,
-                      D: Optional[torch.Tensor] = None):
+                      D: Optional[torch.Tensor] = None, longest: Optional[int] = None):
     """The recurrence of omc_linear_state_scan; q / k / v / a / beta are fp32 2-D tensors or column slices of one.
     decay_given: `a` [T, H * dim] already holds the per-channel decays (map_rows(..., MAP_DECAY / MAP_SIGMOID_POW)).
     sigmoid_pow: the decay of key channel i is sigmoid(a[t, i] + dt_bias[i])^sigmoid_pow (with decay_given: `a` holds that decay
     minus one). out_scale multiplies the read-out. step_size: dt = softplus(a + dt_bias) is the decay's exponent (times exp(A_log)) AND
-    what v enters the state with; D [H]: D v is added to the read-out."""
+    what v enters the state with; D [H]: D v is added to the read-out. longest: rows that no portion has more of, where the host knows."""
     _need_cuda(q, k, v, state, out, row_begin, pos, slot, decay_const, a, A_log, dt_bias, beta, D)
     assert step_size or D is None
     for t in (q, k, v, out, a, beta):
@@ -695,11 +696,11 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
         mode = DECAY_GIVEN_MINUS_ONE if decay_given else DECAY_SIGMOID_POW
     if step_size:
         mode = DECAY_STEP
-    rc = load().omc_linear_state_scan(q, q.stride(0), k, k.stride(0), v, v.stride(0), 1 if silu_in else 0, mode,
-                                      decay_const, a, a.stride(0) if a is not None else 0, A_log, dt_bias,
-                                      D, beta, beta.stride(0) if beta is not None else 0, state, out, out.stride(0),
-                                      row_begin, portions, pos, slot, q.shape[0], H, G, dim, vdim,
-                                      float(sigmoid_pow or 0.0), out_scale, _stream())
+    rc = load().omc_linear_state_scan_longest(q, q.stride(0), k, k.stride(0), v, v.stride(0), 1 if silu_in else 0, mode,
+                                              decay_const, a, a.stride(0) if a is not None else 0, A_log, dt_bias,
+                                              D, beta, beta.stride(0) if beta is not None else 0, state, out, out.stride(0),
+                                              row_begin, portions, pos, slot, q.shape[0], q.shape[0] if longest is None else longest, H, G, dim, vdim,
+                                              float(sigmoid_pow or 0.0), out_scale, _stream())
     _check(rc, "omc_linear_state_scan")
     return out
 

@@ -28,7 +28,7 @@ class Case:
         self.starts = [sum(lens[:i]) for i in range(len(lens) + 1)]
         self.S0 = rn(len(lens), H, dim, vdim) if first else torch.zeros(len(lens), H, dim, vdim, device="cuda")
 
-    def prepared(self, rows=slice(None), lens=None, slots=None, first=None):
+    def prepared(self, rows=slice(None), lens=None, slots=None, first=None, longest=None):
         """The call with everything on the device: nothing but the launches is left."""
         lens = self.lens if lens is None else lens
         slots = range(len(lens)) if slots is None else slots
@@ -40,7 +40,7 @@ class Case:
         begin = _i32([sum(lens[:i]) for i in range(len(lens) + 1)])
         pos, slot = _i32([first + p for n in lens for p in range(n)]), _i32([s for s, n in zip(slots, lens) for _ in range(n)])
         q, k, v = self.q[rows], self.k[rows], self.v[rows]
-        return lambda out, S: seqlib.linear_state_scan(q, k, v, S, out, begin, len(lens), pos, slot, self.H, self.G, self.dim, self.vdim, **kw)
+        return lambda out, S: seqlib.linear_state_scan(q, k, v, S, out, begin, len(lens), pos, slot, self.H, self.G, self.dim, self.vdim, longest=longest, **kw)
 
     def run(self, rows=slice(None), lens=None, slots=None, S=None, first=None):
         S = self.S0.clone() if S is None else S
@@ -177,3 +177,14 @@ def test_what_is_computed_is_a_matter_of_row_begin(kind, lens, rows):
     want, Sw = c.exact()
     assert _rel(out[:n], want[:n]) < 5e-7 and _rel(S[:-1], Sw[:-1]) < 5e-7
     assert out[n:].isnan().all() and torch.equal(S[-1], c.S0[-1])
+
+
+@pytest.mark.parametrize("kind", ["delta", "given"])
+@pytest.mark.parametrize("lens", [[8] * 8, [3] * 32, [63, 2], [64, 2], [40] * 2 + [90], [64, 0, 5]])
+def test_what_the_host_knows_of_lengths_changes_no_bits(kind, lens):
+    c = Case(kind, 3, 1, 64, 36, lens, 2)
+    want, Sw = c.run()
+    for longest in (max(lens), max(lens) + 70):
+        out, S = torch.full_like(want, torch.nan), c.S0.clone()
+        c.prepared(longest=longest)(out, S)
+        assert torch.equal(out, want) and torch.equal(S, Sw)
