@@ -892,8 +892,8 @@ extern "C" int omc_latent_attn_mma_rows(const void* qcat, int T, int H, int r, i
     return set_error(OMC_ERR_ARG, "omc_latent_attn_mma: bad argument");
   if (r <= 0 || r % 16 != 0 || r > 512 || dr < 0 || dr % 16 != 0 || H > kMmaRows)
     return set_error(OMC_ERR_SHAPE, "omc_latent_attn_mma: latent width a multiple of 16 up to 512, rotated width a multiple of 16, at most 64 heads");
-  if (reinterpret_cast<uintptr_t>(qcat) % 16 || reinterpret_cast<uintptr_t>(pool) % 16) return set_error(OMC_ERR_SHAPE, "omc_latent_attn_mma: queries and cached rows lie on 16-byte boundaries");
   if (n_items == 0) return OMC_OK;
+  if (reinterpret_cast<uintptr_t>(qcat) % 16 || reinterpret_cast<uintptr_t>(pool) % 16) return set_error(OMC_ERR_SHAPE, "omc_latent_attn_mma: queries and cached rows lie on 16-byte boundaries");
   const int D = r + dr;
   const size_t extra = r > 128 ? kPairBytes : 0;  // several warps per row group exchange probabilities
   size_t smem = (size_t)(kMmaRows + 2 * kMmaKeys) * (D + 8) * sizeof(bf16_t) + extra;

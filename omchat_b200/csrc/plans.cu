@@ -119,7 +119,7 @@ extern "C" int omc_latent_plan(const int32_t* portions, int n_portions, int H, i
 }
 
 extern "C" int omc_window_plan(const int32_t* portions, int n_portions, int tok, int row_tile, int chunk, int no_chunk, int32_t* counts) {
-  if ((portions == nullptr && n_portions > 0) || counts == nullptr || n_portions < 0 || tok <= 0 || row_tile <= 0 || chunk <= 0)
+  if ((portions == nullptr && n_portions > 0) || counts == nullptr || n_portions < 0 || tok <= 0 || row_tile <= 0)
     return set_error(OMC_ERR_ARG, "omc_window_plan: bad argument");
   try {
     window_list(portions, n_portions, tok, row_tile, chunk, no_chunk, last_list);

@@ -286,14 +286,10 @@ def latent_attn_tcgen05_ok(H: int, r: int, dr: int, page_size: int) -> bool:
 
 def _portion_words(portions):
     """Portions as int32 words (an array that must live as long as its address is used), and how many there are."""
-    words = array("i")
-    n = 0
-    for p in portions:
-        words.extend(p)
-        n += 1
-    if len(words) != 4 * n:
-        raise OmcError("a portion is (first row, rows, slot, first position)")
-    return words, n
+    words = []
+    for first_row, n_rows, slot, first_pos in portions:
+        words += first_row, n_rows, slot, first_pos
+    return array("i", words), len(words) // 4
 
 
 def _check_host(rc: int, what: str):   # a call that launches nothing
@@ -325,7 +321,8 @@ class LatentAttnPlan:
         tok = max(1, MMA_ROWS // H)
         words, n = _portion_words(portions)
         counts = array("i", (0, 0, 0, 0))
-        _check_host(load().omc_latent_plan(words.buffer_info()[0], n, H, tok, target_ctas, min_keys, self.MAX_PARTS, MMA_ROWS, window, counts.buffer_info()[0]),
+        _check_host(load().omc_latent_plan(words.buffer_info()[0], n, H, tok, target_ctas, min_keys, self.MAX_PARTS, MMA_ROWS, min(window, WINDOW_ALL),
+                                           counts.buffer_info()[0]),
                     "omc_latent_plan")
         self.n_items, self.n_merges, self.n_parts, most = counts
         self.max_rows = MMA_ROWS + 1 if mma_sync else most * H   # (token, head) pairs of the largest item; mma_sync: the kernel for whatever shapes
@@ -780,7 +777,7 @@ def window_attn_items(portions, rep: int, device, chunk: int = WINDOW_ALL) -> to
     the edge would walk the keys of both chunks), unless chunks are shorter than a key tile."""
     words, n = _portion_words(portions)
     counts = array("i", (0,))
-    _check_host(load().omc_window_plan(words.buffer_info()[0], n, MMA_ROWS // rep, MMA_ROWS, chunk, WINDOW_ALL, counts.buffer_info()[0]), "omc_window_plan")
+    _check_host(load().omc_window_plan(words.buffer_info()[0], n, MMA_ROWS // rep, MMA_ROWS, min(chunk, WINDOW_ALL), WINDOW_ALL, counts.buffer_info()[0]), "omc_window_plan")
     return _plan_words(counts[0] * 4, device).view(-1, 4)
 
 

@@ -3,7 +3,7 @@ import random
 
 import pytest
 
-from omchat_b200.seqlib import MMA_ROWS, WINDOW_ALL, LatentAttnPlan, window_attn_items
+from omchat_b200.seqlib import MMA_ROWS, WINDOW_ALL, LatentAttnPlan, load, window_attn_items
 
 
 def _portions(rng):
@@ -75,3 +75,22 @@ def test_windowed_items_cover_every_row_once_and_end_where_chunks_do(seed):
             want.append([first_row + row, m, slot, p0 + row])
             row += m
     assert items == want
+
+
+def test_what_lists_take_and_refuse():
+    portions = [(0, 100, 0, 5), (100, 3, 1, 2000)]
+    plain = window_attn_items(portions, 4, "cpu").tolist()
+    for chunk in (-3, 0, 33, 1 << 40):       # no chunks, or shorter ones than a key tile
+        assert window_attn_items(portions, 4, "cpu", chunk).tolist() == plain
+    assert LatentAttnPlan(portions, 8, "cpu", window=1 << 40).items.tolist() == LatentAttnPlan(portions, 8, "cpu").items.tolist()
+    assert LatentAttnPlan([], 8, "cpu").n_items == 0
+    for odd in ([(0, 1, 2)], [(0, 1, 2), (0, 1, 2, 3, 4)]):
+        with pytest.raises(ValueError):
+            window_attn_items(odd, 4, "cpu")
+        with pytest.raises(ValueError):
+            LatentAttnPlan(odd, 8, "cpu")
+
+
+def test_a_list_without_items_asks_nothing_of_addresses():
+    call = lambda n: load().omc_latent_attn_mma_rows(8, 0, 16, 512, 64, 8, 16, 1, 64, 16, n, 64, None, 0, None, 1, None, 0, 1.0, 16, 1, None, None, None)  # noqa: E731
+    assert call(0) == 0 and call(1) != 0     # with one the addresses are refused: rows are read by 16 bytes
