@@ -40,7 +40,7 @@ static long long div_up(long long a, long long b) { return (a + b - 1) / b; }
 struct LatentItem {
   int32_t v[8];
 };
-// The lists of LatentAttnPlan (seqlib.py, whose loop builds the same): items of 8 words, those with the most keys first, then merges of 4.
+// The lists of LatentAttnPlan (seqlib.py): items of 8 words, those with the most keys first, then merges of 4.
 static void latent_lists(const int32_t* portions, int n_portions, int H, int tok, int target_ctas, int min_keys, int max_parts, int row_tile, long long window,
                          std::vector<int32_t>& out, int32_t (&counts)[4]) {
   std::vector<LatentItem> items;

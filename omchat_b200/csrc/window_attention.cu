@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kWdWarps * 32) window_attn_decode_kernel(WinMm
   bf16_t* Vs = Ks + kWdKeys * pq;
   const int t = blockIdx.x, slot = a.slot[t], p = a.pos[t];
   const int kvh = blockIdx.y / a.maps, mp = blockIdx.y - kvh * a.maps, rep = a.H / a.G;
-  const int qchunks = d >> 3, vchunks = dv >> 3, pieces = qchunks + vchunks;
+  const int qchunks = d >> 3, vchunks = dv >> 3;
   for (int i = tid; i < kWdRows * qchunks; i += blockDim.x) {
     const int row = i / qchunks, c = i - row * qchunks;
     *reinterpret_cast<uint4*>(Qs + row * pq + c * 8) =

@@ -330,60 +330,6 @@ class LatentAttnPlan:
         self.items = buf[:self.n_items * 8] if self.n_merges else buf
         self.merges = buf[self.n_items * 8:] if self.n_merges else None
 
-    @classmethod
-    def _by_loop(cls, portions, H, tok, base, target_ctas, min_keys, window):
-        items, merges, part = [], [], 0
-        for first_row, n, slot, p0 in portions:
-            for start in range(0, n, tok):
-                ntok, first = min(tok, n - start), p0 + start
-                low = max(0, first - window + 1)                            # first key the tile's first row sees
-                keys = first + ntok - low                                   # ... up to the end of what its last row sees
-                want = 1
-                if base < target_ctas // 2:
-                    want = max(1, min(-(-keys // min_keys), -(-target_ctas // base), cls.MAX_PARTS))
-                if want == 1:
-                    items.append((first_row + start, ntok, slot, first, low, low + keys, -1, 0))
-                    continue
-                span = -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS        # keys per part, a multiple of 64
-                ends = [min(keys, at + span) for at in range(0, keys, span)]
-                merges += [(first_row + start) * H, ntok * H, part, len(ends)]
-                for i, end in enumerate(ends):
-                    items.append((first_row + start, ntok, slot, first, low + i * span, low + end, part + i, 0))
-                part += len(ends)
-        # the items with the most keys first: with 148 running at a time a long one at the end would run alone
-        items.sort(key=lambda it: it[4] - it[5])
-        return [x for it in items for x in it] + merges, len(items), len(merges) // 4, part
-
-    @classmethod
-    def _by_arrays(cls, portions, H, tok, base, target_ctas, min_keys, window):
-        """The same lists by array arithmetic. Both say in Python what omc_latent_plan builds."""
-        import numpy as np
-        por = np.array(portions, dtype=np.int64).reshape(-1, 4)
-        tiles = -(-por[:, 1] // tok)                                    # row tiles per portion
-        of = np.repeat(np.arange(len(por)), tiles)
-        start = (np.arange(base) - np.repeat(np.cumsum(tiles) - tiles, tiles)) * tok
-        ntok, first = np.minimum(tok, por[of, 1] - start), por[of, 3] + start
-        low = np.maximum(0, first - window + 1)
-        keys = first + ntok - low
-        want = np.ones_like(keys)
-        if base < target_ctas // 2:
-            want = np.clip(np.minimum(-(-keys // min_keys), -(-target_ctas // max(base, 1))), 1, cls.MAX_PARTS)
-        cut = want > 1
-        span = np.where(cut, -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS, np.maximum(keys, 1))
-        n = np.where(cut, -(-keys // span), 1)
-        it = np.repeat(np.arange(base), n)
-        j = np.arange(len(it)) - np.repeat(np.cumsum(n) - n, n)
-        n_cut = np.where(cut, n, 0)
-        part0 = np.cumsum(n_cut) - n_cut
-        items = np.empty((len(it), 8), dtype=np.int32)
-        items[:, 0], items[:, 1], items[:, 2], items[:, 3] = (por[of, 0] + start)[it], ntok[it], por[of, 2][it], first[it]
-        items[:, 4] = low[it] + j * span[it]
-        items[:, 5] = low[it] + np.minimum(keys[it], (j + 1) * span[it])
-        items[:, 6], items[:, 7] = np.where(cut[it], part0[it] + j, -1), 0
-        items = items[np.argsort(items[:, 4] - items[:, 5], kind="stable")]
-        merges = np.stack([(por[of, 0] + start) * H, ntok * H, part0, n], axis=1)[cut].astype(np.int32)
-        return np.concatenate([items.reshape(-1), merges.reshape(-1)]), len(items), len(merges), int(n_cut.sum())
-
 
 class DecodeAttnPlan:
     """Work list of a decode-only step of B rows with static device buffers: `fill(pos, slot)` rewrites it on the device each step

@@ -1,4 +1,4 @@
-"""The work lists of omc_latent_attn_mma: the loop and the array arithmetic build the same numbers, and these cover every key of every row once."""
+"""The work lists of omc_latent_attn_mma and omc_window_attn_mma: the library builds what a loop in Python says, and that covers every key of every row once."""
 import random
 
 import pytest
@@ -15,17 +15,41 @@ def _portions(rng):
     return out
 
 
-@pytest.mark.parametrize("seed", range(60))
-def test_the_loop_and_the_arrays_build_the_same_lists(seed):
+def _lists(portions, H, tok, base, target_ctas, min_keys, window):
+    """items of eight numbers and merges of four in one list, and how many items, merges and partial results."""
+    items, merges, part = [], [], 0
+    for first_row, n, slot, p0 in portions:
+        for start in range(0, n, tok):
+            ntok, first = min(tok, n - start), p0 + start
+            low = max(0, first - window + 1)                            # first key the tile's first row sees
+            keys = first + ntok - low                                   # ... up to the end of what its last row sees
+            want = 1
+            if base < target_ctas // 2:
+                want = max(1, min(-(-keys // min_keys), -(-target_ctas // base), LatentAttnPlan.MAX_PARTS))
+            if want == 1:
+                items.append((first_row + start, ntok, slot, first, low, low + keys, -1, 0))
+                continue
+            span = -(-(-(-keys // want)) // MMA_ROWS) * MMA_ROWS        # keys per part, a multiple of 64
+            ends = [min(keys, at + span) for at in range(0, keys, span)]
+            merges += [(first_row + start) * H, ntok * H, part, len(ends)]
+            for i, end in enumerate(ends):
+                items.append((first_row + start, ntok, slot, first, low + i * span, low + end, part + i, 0))
+            part += len(ends)
+    items.sort(key=lambda it: it[4] - it[5])    # those with the most keys first
+    return [x for it in items for x in it] + merges, len(items), len(merges) // 4, part
+
+
+def _case(seed):
     rng = random.Random(seed)
     portions, H = _portions(rng), rng.choice([1, 3, 8, 16, 33, 64])
     target, min_keys, window = rng.choice([2, 148, 296]), rng.choice([64, 128, 256]), rng.choice([1, 33, 256, 1024, WINDOW_ALL])
     tok = MMA_ROWS // H
-    base = sum(-(-n // tok) for _, n, _, _ in portions)
-    a = LatentAttnPlan._by_loop(portions, H, tok, base, target, min_keys, window)
-    b = LatentAttnPlan._by_arrays(portions, H, tok, base, target, min_keys, window)
-    assert list(a[0]) == b[0].tolist() and a[1:] == b[1:]
-    numbers, n_items, n_merges, n_parts = a
+    return portions, H, tok, target, min_keys, window, _lists(portions, H, tok, sum(-(-n // tok) for _, n, _, _ in portions), target, min_keys, window)
+
+
+@pytest.mark.parametrize("seed", range(60))
+def test_the_lists_cover_every_key_of_every_row_once(seed):
+    portions, H, tok, _, _, window, (numbers, n_items, n_merges, n_parts) = _case(seed)
     seen, parts = {}, {}
     for i in range(n_items):
         row, ntok, slot, first, lo, hi, part, zero = numbers[8 * i:8 * i + 8]
@@ -48,12 +72,7 @@ def test_the_loop_and_the_arrays_build_the_same_lists(seed):
 
 @pytest.mark.parametrize("seed", range(40))
 def test_the_library_builds_the_lists_of_the_loop(seed):
-    rng = random.Random(1000 + seed)
-    portions, H = _portions(rng), rng.choice([1, 3, 8, 16, 33, 64])
-    target, min_keys, window = rng.choice([2, 148, 296]), rng.choice([64, 128, 256]), rng.choice([1, 33, 256, 1024, WINDOW_ALL])
-    tok = MMA_ROWS // H
-    base = sum(-(-n // tok) for _, n, _, _ in portions)
-    numbers, n_items, n_merges, n_parts = LatentAttnPlan._by_loop(portions, H, tok, base, target, min_keys, window)
+    portions, H, tok, target, min_keys, window, (numbers, n_items, n_merges, n_parts) = _case(1000 + seed)
     plan = LatentAttnPlan(portions, H, "cpu", target_ctas=target, min_keys=min_keys, window=window)
     assert (plan.n_items, plan.n_merges, plan.n_parts) == (n_items, n_merges, n_parts)
     assert plan.items.tolist() + (plan.merges.tolist() if plan.merges is not None else []) == list(numbers)
