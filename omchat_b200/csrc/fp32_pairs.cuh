@@ -22,7 +22,7 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
   return d;
 }
 
-// x[i] / y[i] for neg[i] = -x[i], 1 <= y <= 2^64 and x zero or of a magnitude from 2^-60 to 2^100, rounded as a division is (P. Markstein, Computation of elementary functions on
+// x[i] / y[i] for neg[i] = -x[i], 1 <= y <= 2^64 and x zero or of a magnitude from 2^-60 to 2^100 (smaller too where y is 2, as behind exp(-x)), rounded as a division is (P. Markstein, Computation of elementary functions on
 // the IBM RISC System/6000 processor, IBM J. Res. Dev. 34, 1990): a reciprocal with one Newton step, the quotient, and its remainder, which an fma has exactly. NaN in, NaN
 // out. For pairs without one sign to turn: with R = -1 / y, q = -x R, and x / y = q + R (y q - x).
 __device__ __forceinline__ void quotients2(float neg0, float neg1, float y0, float y1, float& q0, float& q1) {

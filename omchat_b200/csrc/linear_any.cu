@@ -157,16 +157,16 @@ __global__ void __launch_bounds__(NT) linear_tile_kernel(LinearArgs a) {
   }
 }
 
-// Few rows: what counts is how many bytes of W are on their way. A CTA of 64 threads owns 8 columns and up to MR rows and brings K terms
-// 1024 at a time into shared memory, all of them in one go; thread (p, c) sums chunk c of the columns p and p + 4 for every row, and
-// the chunks' sums are added by one thread per output. A pitch of 68 floats per chunk puts the chunks on different
+// Few rows: what counts is how many bytes of W are on their way. A CTA owns 8 columns and up to MR rows and brings CHUNKS chunks of 64 terms at a time into
+// shared memory, all of them in one go (16: 1024 terms and 64 threads; 32: 2048 and 128, for sums that long in few CTAs, see the launch); thread (p, c) sums chunk c of the
+// columns p and p + 4 for every row, and the chunks' sums are added by one thread per output, in one order whatever CHUNKS. A pitch of 68 floats per chunk puts the chunks on different
 // banks. 3 x 6144 x 2048 in fp32: 19 us = 2.6 TB/s of W (the tile kernel before: 145), 3 x 4096 x 1024 10 (76).
 constexpr int kRowsCols = 8;
 
-template <typename TX, typename TW, typename TY, int MR, bool VEC, int CHUNKS>   // 16; 32: twice the threads, and sums of up to 2048 terms without a second load behind the first
+template <typename TX, typename TW, typename TY, int MR, bool VEC, int CHUNKS>
 __global__ void __launch_bounds__(4 * CHUNKS) linear_rows_kernel(LinearArgs a) {
   constexpr int kRowsChunks = CHUNKS, kRowsPitch = CHUNKS * (kLinChunk + 4), kRowsThreads = 4 * CHUNKS;
-  extern __shared__ __align__(16) float lin_sm[];   // W [8][pitch] | X [MR][pitch] | chunk sums [8][MR][16 + 1]
+  extern __shared__ __align__(16) float lin_sm[];   // W [8][pitch] | X [MR][pitch] | chunk sums [8][MR][CHUNKS + 1]
   float* ws = lin_sm;
   float* xs = ws + kRowsCols * kRowsPitch;
   float* part = xs + MR * kRowsPitch;

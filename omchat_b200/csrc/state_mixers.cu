@@ -11,11 +11,11 @@
 // The recurrence is evaluated token by token - prompt portions and single decoded tokens run the same instructions
 // in the same order - except in portions of 64 rows and more of the delta rule or with a decay per key channel, which scan_chunk.cu takes eight tokens at a time: the
 // same sums in another order. The result does not depend on how a prompt is cut but in these last bits. Its parallelism is over the
-// independent COLUMNS of S: column j of a head's state only ever meets v[:, j], so a CTA owns 32 columns of one head of one
-// portion; a thread holds an eighth of the state elements of TWO neighbouring columns as packed fp32 pairs (one fma.rn.f32x2 serves
-// both columns, and a key or query value read from shared memory is used twice), and the eight lanes of a column pair finish the
-// two dot products of a token with three shuffles each. Tokens are staged 16 at a time in shared memory by cp.async, one chunk ahead of the one being
-// computed (decays, sigmoid and silu applied in place on arrival), so the sequential loop touches registers and shared memory only.
+// independent COLUMNS of S: column j of a head's state only ever meets v[:, j], so a CTA owns 16, 32 or 64 columns of one head of one
+// portion; a thread holds an eighth of the state elements of one, two or four neighbouring columns as packed fp32 pairs of key channels (a key or query value read from shared
+// memory is used for each of its columns), and the eight lanes of a column finish the
+// two dot products of a token with three shuffles each. Tokens are staged 8 or 16 at a time in shared memory by cp.async, one stage ahead of the one being
+// computed (decays, sigmoid and silu applied on arrival), so the sequential loop touches registers and shared memory only.
 // Recurrences whose channels carry one or a few states of their own (selective scan, gated linear recurrent unit) follow below.
 #include <type_traits>
 
