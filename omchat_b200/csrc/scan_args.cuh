@@ -118,7 +118,7 @@ __device__ __forceinline__ int scan_portion(const int32_t* row_begin, int portio
 
 enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
 constexpr int kScanLong = 64;   // rows from which a portion goes eight tokens at a time
-// The launch of scan_chunk.cu for the portions of at least a.long_from rows: the delta rule or per-channel decays (decay modes 0 and 1 with beta, 3, 5), 64 or 128 key
+// The launch of scan_chunk.cu for the portions of at least a.long_from rows: the delta rule or per-channel decays (decay modes 1 with beta, 3, 5), 64 or 128 key
 // channels, inputs that need no preparation of their own, 16-byte rows of k, q, v, decays, outputs and states. Returns check_launch's code.
 int launch_scan_chunk(const ScanArgs& a, int rows, int portions, cudaStream_t st);
 

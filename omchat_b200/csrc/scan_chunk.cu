@@ -10,9 +10,11 @@
 // One half of a CTA has the state (32 elements a thread: 4 columns x 8 channels), the other fetches the inputs and forms what a stage's tokens have among
 // themselves, one stage ahead. What bounds it: a stage's chain through some 600 instructions of the one warp that a scheduler has for the state (1.3 us, of which
 // the eight-lane sums of the products are a half); with several CTAs per SM shared memory's data path.
-// Measured in us (token by token in brackets): delta rule, 16 heads of 128 x 128, portions of 1024, 777, 1024, 301 tokens 256 (351), 4 heads, 1100 tokens 182
-// (256), 4 heads of 64 x 64 172 (196), 64 tokens 17 (19) and 15 (15); decays per channel over the same 278 (433), 208 (306), 184 (251), 17 (22) and 15 (19). Error of
-// output and state against 64 bits 0.6 to 1.3 of the other kernels'. With step sizes, or one decay per head and no delta rule, a token's chain is short enough
+// Measured in us (token by token in brackets): delta rule, 16 heads of 128 x 128, portions of 1024, 777, 1024, 301 tokens 250 (351), 4 heads, 1100 tokens 177
+// (256), 4 heads of 64 x 64 172 (196), 64 tokens 17 (19) and 15 (15); decays per channel over the same 279 (433), 201 (306), 184 (251), 17 (22) and 15 (19). Error of
+// output and state against 64 bits (2-norm) 0.5 to 1.0 of token by token, as what a stage's tokens take out of and add to one another is summed by itself before it meets the larger
+// numbers from the state (1.02 to 1.10 for decays per channel with the delta rule otherwise) and a channel's G_8 is two numbers (with one, its rounding in decays that hardly change
+// is the same in every stage: 2.5 to 6.5 at decays from 0.99 to 0.9999). Decays that never change stay token by token. With step sizes, or one decay per head and no delta rule, a token's chain is short enough
 // that this gains nothing with few CTAs (16 heads of 128 x 64, 1100 tokens: 154, 148), so they stay where they were. The same in mma.sync products of three
 // bf16 parts (as exact as fp32 fma where leading products are added in fp32) took 8100 instructions per 16 tokens and 64 columns, most of them splits: 286 (256).
 #include <type_traits>
@@ -35,13 +37,14 @@ struct ScanChunkShared {
   };
   struct Ready {                               // what a stage's tokens have among themselves
     float p[kScTok * 12], kk[DELTA ? kScTok * 12 : 4];   // [t][s]: (G_t / G_s) q_t . k_s, (G_t / G_s) k_t . k_s
-    float qh[CHAN ? kScTok * DIM : 4], kh[CHAN && DELTA ? kScTok * DIM : 4], kt[CHAN ? kScTok * DIM : 4], gl[CHAN ? DIM : 4];   // G_t q_t, G_t k_t, (G_8 / G_s) k_s, G_8
-    float gy[kScTok], r[kScTok], all[4];       // G_t, G_8 / G_s, G_8; by channel: with minus1 less one
+    float qh[CHAN ? kScTok * DIM : 4], kh[CHAN && DELTA ? kScTok * DIM : 4], kt[CHAN ? kScTok * DIM : 4];   // G_t q_t, G_t k_t, (G_8 / G_s) k_s
+    float gl[CHAN ? DIM : 4], gr[CHAN ? DIM : 4];   // G_8, with minus1 less one, and what its rounding leaves: in decays that stay the same that would be the same in every stage and add up
+    float gy[kScTok], r[kScTok], all[4];       // G_t, G_8 / G_s, G_8
   };
   Stage stage[kScRing];
   Ready ready[2];
-  float la[64], w[64];                         // tokens of two blocks of 32: log decays (decay_mode 0: decays), beta
-  float r[DELTA ? kScWarps * kScTok * XP : 4], u[DELTA ? kScWarps * kScTok * XP : 4];   // [warp][token][column]
+  float la[64], w[64];                         // tokens of two blocks of 32: log decays, beta
+  alignas(16) float r[DELTA ? kScWarps * kScTok * XP : 4], u[DELTA ? kScWarps * kScTok * XP : 4];   // [warp][token][column]
 };
 
 __device__ __forceinline__ void cp_async16_or_zero(float* dst, const float* src, bool there) {
@@ -134,8 +137,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
     // ---- the half that fetches and prepares: stages i + 2 and i + 3 are on their way and stage i + 1 is prepared while stage i is computed
     asm volatile("setmaxnreg.dec.sync.aligned.u32 88;");
     const int tid = threadIdx.x - kScThreads, wl = tid & 31, warp = tid / 32, kvh = h / (a.H / a.G);
-    const bool product = a.decay_mode == 0, logs = a.decay_mode == 1;
-    const float A = logs ? expf(a.A_log[h]) : 0.f, bias = logs ? a.dt_bias[h] : 0.f, gconst = product ? a.decay_const[h] : 1.f;
+    const float A = CHAN ? 0.f : expf(a.A_log[h]), bias = CHAN ? 0.f : a.dt_bias[h];
     constexpr int PIECES = DIM / 4, STEP_T = kScThreads / PIECES, VP = COLS / 4, STEP_V = kScThreads / VP;
     static_assert(kScThreads % VP == 0, "");
     const int piece = tid % PIECES * 4, tok0 = tid / PIECES, vtok = tid / VP, vcol = tid % VP * 4;
@@ -173,14 +175,13 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
     auto load_raw = [&](int c0) {
       const int t = c0 + wl;
       if (t < r1) {
-        if (logs) raw_a = a.a[(long long)t * a.lda + h];
+        if (!CHAN) raw_a = a.a[(long long)t * a.lda + h];
         if (DELTA) raw_b = a.beta[(long long)t * a.ldb + h];
       }
     };
     auto put_raw = [&](int c0, int block) {   // a token behind the end decays nothing (however large A is); its zero rows enter nothing
       const bool there = c0 + wl < r1;
-      const float none = product ? 1.f : 0.f;
-      sh.la[(block & 1) * 32 + wl] = there ? (product ? gconst : (logs ? -A * softplus_f(raw_a + bias) : 0.f)) : none;
+      if (!CHAN) sh.la[(block & 1) * 32 + wl] = there ? -A * softplus_f(raw_a + bias) : 0.f;
       if (DELTA) sh.w[(block & 1) * 32 + wl] = sigmoid_f(raw_b);
     };
     // What the tokens of a stage have among themselves: warp w forms the products of tokens w and 7 - w with those up to them (nine each, the lanes over the channels)
@@ -219,12 +220,12 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
       }
       float la[kScTok];
       if (!CHAN) ld_cols(la, sh.la + (stage & 7) * kScTok);
-      auto between = [&](int lo, int hi) {   // the decays of tokens lo .. hi - 1, as their product or the sum of their logarithms
-        float x = product ? 1.f : 0.f;
+      auto between = [&](int lo, int hi) {   // the product of the decays of tokens lo .. hi - 1
+        float x = 0.f;
 #pragma unroll
         for (int i = 0; i < kScTok; ++i)
-          if (i >= lo && i < hi) x = product ? x * la[i] : x + la[i];
-        return x;
+          if (i >= lo && i < hi) x += la[i];
+        return expf(x);
       };
       float x8q[8], x8k[8];
 #pragma unroll
@@ -236,10 +237,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
         const bool first = j <= warp;
         const int from = first ? warp - j : 8 - j, t = first ? warp : 7 - warp;
         float ratio = 1.f;
-        if (!CHAN) {
-          ratio = between(from + 1, t + 1);
-          if (!product) ratio = expf(ratio);
-        }
+        if (!CHAN) ratio = between(from + 1, t + 1);
         if ((wl & 3) == 0 || wl == 1) {
           r.p[t * 12 + from] = (wl == 1 ? q9 : q8) * ratio;
           if (DELTA) r.kk[t * 12 + from] = (wl == 1 ? k9 : k8) * ratio;
@@ -247,37 +245,44 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
       }
       if (!CHAN) {
         if (tid < kScTok) {
-          const float gy = between(0, tid + 1), gr = between(tid + 1, kScTok);
-          r.gy[tid] = product ? gy : expf(gy);
-          r.r[tid] = product ? gr : expf(gr);
+          r.gy[tid] = between(0, tid + 1);
+          r.r[tid] = between(tid + 1, kScTok);
         } else if (tid == 32) {
-          const float x = between(0, kScTok);
-          r.all[0] = product ? x : expf(x);
+          r.all[0] = between(0, kScTok);
         }
       } else {
         // a channel per thread (64 channels: half of the threads go forward, half backward)
         const int i = tid % DIM;
-        float g[kScTok];
+        float x[kScTok], gl, gr;
 #pragma unroll
-        for (int t = 0; t < kScTok; ++t) g[t] = t < n ? s.g[t * DIM + i] : (minus1 ? 0.f : 1.f);
+        for (int t = 0; t < kScTok; ++t) x[t] = t < n ? s.g[t * DIM + i] : (minus1 ? 0.f : 1.f);
+        if (minus1) {   // (1 + a) (1 + b) - 1
+          auto both = [](double a, double b) { return fma(a, b, a) + b; };
+          const double all = both(both(both(x[0], x[1]), both(x[2], x[3])), both(both(x[4], x[5]), both(x[6], x[7])));
+          gl = (float)all, gr = (float)(all - (double)gl);
+#pragma unroll
+          for (int t = 0; t < kScTok; ++t) x[t] += 1.f;
+        }
+        // their products by halves: at most four roundings each instead of seven
+        const float x01 = x[0] * x[1], x23 = x[2] * x[3], x45 = x[4] * x[5], x67 = x[6] * x[7], x03 = x01 * x23, x47 = x45 * x67;
+        if (!minus1) {   // a product's rounding is an fma's; those of its factors come along
+          auto rest = [](float a, float b, float ab, float ra, float rb) { return fmaf(a, b, -ab) + fmaf(a, rb, ra * b); };
+          const float r03 = rest(x01, x23, x03, fmaf(x[0], x[1], -x01), fmaf(x[2], x[3], -x23)), r47 = rest(x45, x67, x47, fmaf(x[4], x[5], -x45), fmaf(x[6], x[7], -x67));
+          gl = x03 * x47, gr = rest(x03, x47, gl, r03, r47);
+        }
         if (DIM == kScThreads || tid < DIM) {
-          float G = 1.f, m = 0.f;
+          const float G[kScTok] = {x[0], x01, x01 * x[2], x03, x03 * x[4], x03 * x45, x03 * (x45 * x[6]), x03 * x47};
 #pragma unroll
           for (int t = 0; t < kScTok; ++t) {
-            G *= minus1 ? 1.f + g[t] : g[t];
-            if (minus1) m = fmaf(m, g[t], m) + g[t];
-            r.qh[t * DIM + i] = s.q[t * DIM + i] * G;
-            if (DELTA) r.kh[t * DIM + i] = s.k[t * DIM + i] * G;
+            r.qh[t * DIM + i] = s.q[t * DIM + i] * G[t];
+            if (DELTA) r.kh[t * DIM + i] = s.k[t * DIM + i] * G[t];
           }
-          r.gl[i] = minus1 ? m : G;
+          r.gl[i] = gl, r.gr[i] = gr;
         }
         if (DIM == kScThreads || tid >= DIM) {
-          float R = 1.f;
+          const float R[kScTok] = {x[1] * (x23 * x47), x23 * x47, x[3] * x47, x47, x[5] * x67, x67, x[7], 1.f};
 #pragma unroll
-          for (int t = kScTok - 1; t >= 0; --t) {
-            r.kt[t * DIM + i] = s.k[t * DIM + i] * R;
-            R *= minus1 ? 1.f + g[t] : g[t];
-          }
+          for (int t = 0; t < kScTok; ++t) r.kt[t * DIM + i] = s.k[t * DIM + i] * R[t];
         }
       }
     };
@@ -385,10 +390,10 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
       for (int c = 0; c < CW; ++c) d[c] = CHAN ? v[c] - d[c] : fmaf(-gy, d[c], v[c]);
       st_cols(sh.r + (warp * kScTok + l7) * XP + wcol + half * H2, d);
       __syncwarp();
-      if (wl < WC) {   // a column per lane: u token by token, each taken out of those behind it at once
+      if (wl < WC) {   // a column per lane: u token by token; what earlier ones take out of a token is added up by itself, with the roundings of its own smaller numbers
         const float* rp = sh.r + warp * kScTok * XP + wl;
         float* up = sh.u + warp * kScTok * XP + wl;
-        float x[kScTok], w[kScTok], kk[kScTok][kScTok];
+        float x[kScTok], w[kScTok], kk[kScTok][kScTok], out_of[kScTok] = {};
 #pragma unroll
         for (int t = 0; t < kScTok; ++t) x[t] = rp[t * XP];
         ld_cols(w, sh.w + (i & 7) * kScTok);
@@ -401,28 +406,26 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
           }
 #pragma unroll
         for (int t = 0; t < kScTok; ++t) {
-          const float u = t < n ? w[t] * x[t] : 0.f;   // nothing of the state comes back through a row behind the end
+          const float u = t < n ? w[t] * (x[t] - out_of[t]) : 0.f;   // nothing of the state comes back through a row behind the end
           up[t * XP] = u;
 #pragma unroll
-          for (int f = t + 1; f < kScTok; ++f) x[f] = fmaf(-kk[f][t], u, x[f]);
+          for (int f = t + 1; f < kScTok; ++f) out_of[f] = fmaf(kk[f][t], u, out_of[f]);
         }
       }
     }
     dots(CHAN ? r.qh : s.q, o);
     if (DELTA) __syncwarp();
-    if (!CHAN)
-#pragma unroll
-      for (int c = 0; c < CW; ++c) o[c] *= gy;
+    float own[CW] = {};   // what the stage's tokens bring
 
     // the state and the read-out with what the stage's tokens bring
     if constexpr (CHAN) {
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
-        const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(r.gl + x * (DIM / 2) + 4 * lane);
+        const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(r.gl + x * (DIM / 2) + 4 * lane), rest = *reinterpret_cast<const ulonglong2*>(r.gr + x * (DIM / 2) + 4 * lane);
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
-          st[c][2 * x] = minus1 ? fma2(st[c][2 * x], g.x, st[c][2 * x]) : mul2(st[c][2 * x], g.x);
-          st[c][2 * x + 1] = minus1 ? fma2(st[c][2 * x + 1], g.y, st[c][2 * x + 1]) : mul2(st[c][2 * x + 1], g.y);
+          st[c][2 * x] = fma2(st[c][2 * x], g.x, minus1 ? fma2(st[c][2 * x], rest.x, st[c][2 * x]) : mul2(st[c][2 * x], rest.x));
+          st[c][2 * x + 1] = fma2(st[c][2 * x + 1], g.y, minus1 ? fma2(st[c][2 * x + 1], rest.y, st[c][2 * x + 1]) : mul2(st[c][2 * x + 1], rest.y));
         }
       }
     } else {
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
       for (int c = 0; c < H2; ++c) x[c] = xa[c], x[H2 + c] = xb[c];
 #pragma unroll
       for (int c = 0; c < CW; ++c)
-        if (f <= l7) o[c] = fmaf(pr[f], x[c], o[c]);
+        if (f <= l7) own[c] = fmaf(pr[f], x[c], own[c]);
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
         const float y = CHAN ? x[c] : x[c] * rf;
@@ -459,7 +462,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
       }
     }
 #pragma unroll
-    for (int c = 0; c < CW; ++c) o[c] *= a.out_scale;
+    for (int c = 0; c < CW; ++c) o[c] = (CHAN ? o[c] + own[c] : fmaf(o[c], gy, own[c])) * a.out_scale;
     if (c0 + l7 < r1) {
       float* dst = a.out + (long long)(c0 + l7) * a.ldo + (long long)h * a.vdim + colA;
       if (inA) st_cols(dst, o);
@@ -485,7 +488,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
 int launch_scan_chunk(const ScanArgs& a, int rows, int portions, cudaStream_t st) {
   using std::integral_constant;
   const bool chan = a.decay_mode == 3 || a.decay_mode == 5;
-  if (a.long_from <= 0 || (!chan && (a.beta == nullptr || a.decay_mode > 1)) || (a.dim != 64 && a.dim != 128)) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: not a recurrence of the kernel for long portions");
+  if (a.long_from <= 0 || (!chan && (a.beta == nullptr || a.decay_mode != 1)) || (a.dim != 64 && a.dim != 128)) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: not a recurrence of the kernel for long portions");
   const int most = rows / a.long_from < portions ? rows / a.long_from : portions;   // only so many portions can be long ones
   auto go = [&](auto dim_c, auto kind_c, auto chan_c) {
     constexpr int DIM = decltype(dim_c)::value, KIND = decltype(kind_c)::value;

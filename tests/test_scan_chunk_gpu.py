@@ -188,3 +188,21 @@ def test_what_the_host_knows_of_lengths_changes_no_bits(kind, lens):
         out, S = torch.full_like(want, torch.nan), c.S0.clone()
         c.prepared(longest=longest)(out, S)
         assert torch.equal(out, want) and torch.equal(S, Sw)
+
+
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("same", [False, True])     # decays that differ from token to token; each channel's (head's) the same in all, close to one: errors that do not cancel
+def test_eight_at_a_time_are_no_less_exact_than_one(kind, dim, same):
+    c = Case(kind, 8, 4, dim, 64, [1000], 3)
+    if same and "given" in kind:
+        c.a = (0.998 + 0.001 * torch.rand(1, c.a.shape[1], device="cuda")).expand(1000, -1).contiguous() - (1.0 if kind == "given_minus_one" else 0.0)
+    elif same:
+        c.a, c.A_log, c.const = c.a[:1].expand(1000, -1).contiguous(), c.A_log - 6, 1 - 0.002 * torch.rand(8, device="cuda")
+    want, Sw = c.exact()
+    out, S = c.run()
+    S1, outs = c.S0.clone(), []
+    for lo in range(0, 1000, 50):     # portions this short go token by token
+        outs.append(c.run(slice(lo, lo + 50), [50], [0], S1, 3 + lo)[0])
+    # the same number of roundings or fewer; 2-norms of half a million errors, which scatter by a few parts in a thousand
+    assert _rel(out, want) < 1.03 * _rel(torch.cat(outs), want) and _rel(S, Sw) < 1.03 * _rel(S1, Sw)
