@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(2 * kScThreads, 2) scan_chunk_kernel(ScanArgs 
     portion = scan_portion(a.row_begin, portions, blockIdx.z, reinterpret_cast<int*>(sm));
   }
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1], stages = (r1 - r0 + kScTok - 1) / kScTok;
-  if (!scan_is_long(a, portions, r1 - r0)) return;
+  if (!scan_is_long(a, r1 - r0)) return;
   scan_begin(a);   // not before: CTAs without a portion would still be there when the other kernel's are spread over the SMs (3 x 63 tokens 27 -> 35 us)
   const int h = blockIdx.y, col0 = blockIdx.x * COLS;
   const bool minus1 = CHAN && a.decay_mode == 5;

@@ -320,7 +320,8 @@ __host__ __device__ constexpr int scan_stage_floats(bool chan, int cols) {
 }
 template <int DPT, bool VEC, int KIND, bool CHAN, int TOK>   // CHAN: one decay per key channel
 __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 32 ? 4 : 7) : 0) linear_state_scan_kernel(ScanArgs a) {
-  const ScanEnd end{a};
+  constexpr bool LONG = CHAN || KIND == kScanDelta;   // long portions may be scan_chunk_kernel's
+  if (LONG && scan_only_waits(a)) return;
   extern __shared__ __align__(16) float sm[];
   constexpr int PITCH = kScanLanes * (DPT + 4), CPT = kScanCpt, COLS = kScanGroups * CPT, DP = DPT / 2;
   constexpr int OPITCH = COLS + 4;           // a lane's partial read-outs of one token
@@ -334,7 +335,7 @@ __global__ void __launch_bounds__(kScanThreads, TOK == 1 && DPT >= 16 ? (DPT == 
   const int h = blockIdx.y, kvh = h / (a.H / a.G);
   const int col0 = blockIdx.x * COLS;
   const int r0 = a.row_begin[blockIdx.z], r1 = a.row_begin[blockIdx.z + 1];
-  if (r1 <= r0 || scan_is_long(a, gridDim.z, r1 - r0)) return;
+  if (r1 <= r0 || (LONG && scan_is_long(a, r1 - r0))) return;
   // a decode step is a matter of reading and writing the states: there neighbouring threads take neighbouring columns (128 bytes of a row
   // of the state), and the lanes' sums meet in shared memory; otherwise the lanes of a column group are neighbours and meet by shuffles
   const int tid = threadIdx.x, lane = WIDE ? tid / kScanGroups : tid & (kScanLanes - 1), cg = WIDE ? tid % kScanGroups : tid / kScanLanes;
@@ -665,7 +666,8 @@ struct ScanRowsShared {
 
 template <int DIM, int CPT, int KIND, bool CHAN>
 __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
-  const ScanEnd end{a};
+  constexpr bool LONG = CHAN || KIND == kScanDelta;   // long portions may be scan_chunk_kernel's
+  if (LONG && scan_only_waits(a)) return;
   extern __shared__ __align__(16) float sm[];
   constexpr int COLS = kSrThreads / kScanLanes * CPT;
   typedef ScanRowsShared<DIM, COLS, CHAN> Shared;
@@ -676,7 +678,7 @@ __global__ void __launch_bounds__(kSrThreads) scan_rows_kernel(ScanArgs a) {
   const int h = blockIdx.y, kvh = h / (a.H / a.G), col0 = blockIdx.x * COLS;
   const int portion = a.portions > 1 ? scan_portion(a.row_begin, a.portions, blockIdx.z, reinterpret_cast<int*>(sm)) : blockIdx.z;
   const int r0 = a.row_begin[portion], r1 = a.row_begin[portion + 1];
-  if (r1 <= r0 || scan_is_long(a, gridDim.z, r1 - r0)) return;
+  if (r1 <= r0 || (LONG && scan_is_long(a, r1 - r0))) return;
   const int tid = threadIdx.x, lane = tid & (kScanLanes - 1), cg = tid / kScanLanes, col = col0 + CPT * cg;
   const bool in = col < a.vdim;   // a thread's columns all exist or none does
   const float A = KIND == kScanStep || a.decay_mode == 1 ? expf(a.A_log[h]) : 0.f;
@@ -1599,7 +1601,7 @@ extern "C" int omc_linear_state_scan_longest(const float* q, long long ldq, cons
   if (dim > 256) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: key width above 256");
   if (portions > 65535 || H > 65535) return set_error(OMC_ERR_SHAPE, "omc_linear_state_scan: more than 65535 portions or heads");
   ScanArgs s{q, k, v, ldq, ldk, ldv, silu_in, decay_mode, decay_pow, out_scale, decay_const, a, lda, A_log, dt_bias, D, beta, ldb, state, out, ldo,
-             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0, rows, 0};
+             row_begin, pos, slot, H, G, dim, vdim, false, false, 0, 0, rows, portions, 0};
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int dpt = dim <= 32 ? 4 : (dim <= 64 ? 8 : (dim <= 128 ? 16 : 32));   // key channels per thread: dim / 8 lanes, rounded up to a float4
   const bool chan = decay_mode >= 2 && decay_mode <= 5;
@@ -1711,6 +1713,7 @@ extern "C" int omc_linear_state_scan_longest(const float* q, long long ldq, cons
     s.long_from = 1, s.rows = 0x7fffffff;
     return launch_scan_chunk(s, rows, portions, st);
   }
+  if (portions == 65535) return tokens();   // no room in the grid for the layer that waits
   s.long_from = kScanLong;
   // The long chains first, the others beside them. In us, all token by token / one kernel behind the other / beside: 500 + 16 x 1 tokens of 16 heads of 128 x 128 131 / 97 / 90, with
   // decays per channel 195 / 113 / 101 (152 with the short ones first); 65 + 31 x 1 tokens 29 / 36 / 25; 100, 50, 50, 50 33 / 46 / 31. Where no portion is
