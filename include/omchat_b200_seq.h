@@ -303,7 +303,7 @@ int omc_conv_qk_norm_kv_store(const float* x, long long ldx, int T, int ch, cons
  * position 0 starts from S = 0. rows: the number of rows over all portions; the kernel and how much is staged at a time are chosen by it, which rows are done is a matter of
  * row_begin alone. dim <= 256. Tokens are processed one after the other, and a portion has the same bits however a prompt is cut, but in one case: with one decay per token and head
  * and beta (mode 1) or given decays per channel (3, 5), dim 64 or 128, no silu_in, vdim and all leading dimensions multiples of four and everything on 16-byte boundaries, portions
- * of 64 rows and more go eight tokens at a time: the same fp32 sums in another order. A portion that is alone in its call goes by `rows` there; and if row_begin has more rows than
+ * of 64 rows and more (per channel 32) go eight tokens at a time: the same fp32 sums in another order. A portion that is alone in its call goes by `rows` there; and if row_begin has more rows than
  * `rows` says, all portions go token by token. */
 int omc_linear_state_scan(const float* q, long long ldq, const float* k, long long ldk, const float* v, long long ldv, int silu_in,
                           int decay_mode, const float* decay_const, const float* a, long long lda, const float* A_log,

@@ -115,7 +115,11 @@ __device__ __forceinline__ int scan_portion(const int32_t* row_begin, int portio
 }
 
 enum { kScanPlain = 0, kScanDelta = 1, kScanStep = 2 };
-constexpr int kScanLong = 64;   // rows from which a portion goes eight tokens at a time
+// Rows from which a portion goes eight tokens at a time: with decays per channel, and per head with the delta rule. A stage's overhead is gained back behind 15 to 35 tokens (per
+// head 28 at 128 channels, 59 at 64). Where a step's portions lie on both sides of the line and CTAs are many its two kernels run one behind the other, so the line is low where it can
+// be: 16 heads of 128 x 128 channels, portions of 64, 64 and 4 x 40 rows 1.56 of token by token with the line at 64 rows, 0.96 at 32; 32 heads, 64, 43, 30 rows 1.68 and 1.32, 8 x
+// 40 rows 1.04 and 1.08. Per head 16 x 48 rows of 16 heads would take 1.16 of it with the line at 48; 64 and 63 rows take 1.42 with it at 64 (20 us).
+constexpr int kScanLongChannel = 32, kScanLongHead = 64;
 // The launch of scan_chunk.cu for the portions of at least a.long_from rows: the delta rule or per-channel decays (decay modes 1 with beta, 3, 5), 64 or 128 key
 // channels, inputs that need no preparation of their own, 16-byte rows of k, q, v, decays, outputs and states. Returns check_launch's code.
 int launch_scan_chunk(const ScanArgs& a, int rows, int portions, cudaStream_t st);

@@ -9,7 +9,7 @@
 // Everything here is fp32: state, decays and their logarithms, softplus / exponentials, step sizes, unit norms.
 //
 // The recurrence is evaluated token by token - prompt portions and single decoded tokens run the same instructions
-// in the same order - except in portions of 64 rows and more of the delta rule or with a decay per key channel, which scan_chunk.cu takes eight tokens at a time: the
+// in the same order - except in portions of 64 rows and more of the delta rule, of 32 and more with a decay per key channel, which scan_chunk.cu takes eight tokens at a time: the
 // same sums in another order. The result does not depend on how a prompt is cut but in these last bits. Its parallelism is over the
 // independent COLUMNS of S: column j of a head's state only ever meets v[:, j], so a CTA owns 16, 32 or 64 columns of one head of one
 // portion; a thread holds an eighth of the state elements of one, two or four neighbouring columns as packed fp32 pairs of key channels (a key or query value read from shared
@@ -1708,13 +1708,14 @@ extern "C" int omc_linear_state_scan_longest(const float* q, long long ldq, cons
   // long portions of the delta rule and with per-channel decays: scan_chunk_kernel; whichever are left, the kernels above. Not decays that are the same in every token: the error of
   // a product of eight of them, always the same too, would add up from stage to stage (1.0 to 1.25 of token by token after 1000 tokens)
   // (every portion has a row at least, so that none can have more than what is left)
-  if (!several || longest < kScanLong || rows - portions + 1 < kScanLong || !(chan || (beta != nullptr && decay_mode == 1))) return tokens();
+  const int long_from = chan ? kScanLongChannel : kScanLongHead;
+  if (!several || longest < long_from || rows - portions + 1 < long_from || !(chan || (beta != nullptr && decay_mode == 1))) return tokens();
   if (portions == 1) {   // alone: what row_begin has is this kernel's, however few rows (a padded buffer)
     s.long_from = 1, s.rows = 0x7fffffff;
     return launch_scan_chunk(s, rows, portions, st);
   }
   if (portions == 65535) return tokens();   // no room in the grid for the layer that waits
-  s.long_from = kScanLong;
+  s.long_from = long_from;
   // The long chains first, the others beside them. In us, all token by token / one kernel behind the other / beside: 500 + 16 x 1 tokens of 16 heads of 128 x 128 131 / 97 / 90, with
   // decays per channel 195 / 113 / 101 (152 with the short ones first); 65 + 31 x 1 tokens 29 / 36 / 25; 100, 50, 50, 50 33 / 46 / 31. Where no portion is
   // long the first kernel is empty and costs 1.2 on the device (8 x 8 tokens 9.3 / 10.5), so the host says how long they are at most.

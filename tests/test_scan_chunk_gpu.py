@@ -1,4 +1,4 @@
-"""The recurrence's kernel for long portions (64 rows and more of the delta rule or with per-channel decays): against float64 over whole and ragged stages of eight tokens
+"""The recurrence's kernel for long portions (64 rows and more of the delta rule, 32 with per-channel decays): against float64 over whole and ragged stages of eight tokens
 and column counts, beside short portions that keep the bits of single tokens, from a fresh state and one that is carried on."""
 import pytest
 import torch
@@ -180,7 +180,7 @@ def test_what_is_computed_is_a_matter_of_row_begin(kind, lens, rows):
 
 
 @pytest.mark.parametrize("kind", ["delta", "given"])
-@pytest.mark.parametrize("lens", [[8] * 8, [3] * 32, [63, 2], [64, 2], [40] * 2 + [90], [64, 0, 5]])
+@pytest.mark.parametrize("lens", [[8] * 8, [3] * 32, [63, 2], [64, 2], [40] * 2 + [90], [64, 0, 5], [31] * 3, [32, 31]])
 def test_what_the_host_knows_of_lengths_changes_no_bits(kind, lens):
     c = Case(kind, 3, 1, 64, 36, lens, 2)
     want, Sw = c.run()
@@ -202,7 +202,25 @@ def test_eight_at_a_time_are_no_less_exact_than_one(kind, dim, same):
     want, Sw = c.exact()
     out, S = c.run()
     S1, outs = c.S0.clone(), []
-    for lo in range(0, 1000, 50):     # portions this short go token by token
-        outs.append(c.run(slice(lo, lo + 50), [50], [0], S1, 3 + lo)[0])
+    for lo in range(0, 1000, 20):     # portions this short go token by token
+        outs.append(c.run(slice(lo, lo + 20), [20], [0], S1, 3 + lo)[0])
     # the same number of roundings or fewer; 2-norms of half a million errors, which scatter by a few parts in a thousand
     assert _rel(out, want) < 1.03 * _rel(torch.cat(outs), want) and _rel(S, Sw) < 1.03 * _rel(S1, Sw)
+
+
+@pytest.mark.parametrize("kind,line", [("delta", 64), ("given", 32), ("given_plain", 32), ("given_minus_one", 32)])
+def test_a_portion_has_the_same_bits_in_any_company(kind, line):
+    """On both sides of the line between the kernels, and whoever else is in the step."""
+    lens = [line, line - 1, line + 1, line - 7, 1, 150]
+    c = Case(kind, 4, 2, 128, 64, lens, 3)
+    out, S = c.run()
+    want, Sw = c.exact()
+    assert _rel(out, want) < 5e-7 and _rel(S, Sw) < 5e-7
+    for i, n in enumerate(lens):
+        rows = slice(c.starts[i], c.starts[i + 1])
+        o1, S1 = c.run(rows, [n], [i])
+        assert torch.equal(o1, out[rows]) and torch.equal(S1[i], S[i]), i
+        if n < line:     # token by token
+            S2 = c.S0.clone()
+            single = torch.cat([c.run(slice(rows.start + t, rows.start + t + 1), [1], [i], S2, 3 + t)[0] for t in range(n)])
+            assert torch.equal(single, o1) and torch.equal(S2[i], S1[i]), i
