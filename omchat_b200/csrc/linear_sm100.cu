@@ -7,8 +7,9 @@
 // the tile, so a row's result does not depend on M.
 // What bounds it: bytes (103 MB from L2 and 26 MB of output and gate in 19 to 21 us) behind 8 us of set-up, first load and last epilogue; before, one tile per CTA and two CTAs per SM, a tile's
 // load (2.9 us) and epilogue (4.3, with a gate 11.5: fp32 slabs read with two-way bank conflicts, gates asked for behind the accumulator, divisions of 10
-// instructions) followed one another. 3126 rows x 16 heads, us (before): 128 -> 512 18.6 (39.5); 512 -> 128 with a gate per element 20.7 (45.0; 26.8 with the quotients as plain divisions); 1338 rows without
-// a gate 12.4 (31.0), 11.1 (18.6); 300 rows 8.2 (10.5), 10.4 (12.5); 94 rows 8.6 (10.5), 10.4 (19.6); 1 row 7.9 (8.0), 8.8 (8.9).
+// instructions) followed one another. 3126 rows x 16 heads, us (before): 128 -> 512 19.3 (39.5); 512 -> 128 with a gate per element 20.6 (45.0; 26.8 with the quotients as plain divisions); 1338 rows without
+// a gate 12.4 (31.0), 10.4 (18.6); 300 rows 7.6 (10.5), 10.3 (12.5); 94 rows 7.8 (10.5), 9.4 (19.6); 1 row 7.7 (8.0), 8.4 (8.9). 206 shapes of 1 to 3000 rows, 1 to 32 problems, 64 to 2048 terms
+// and 64 to 4096 columns: 0.64 of the time before on average, 1.05 at most.
 #include "fp32_pairs.cuh"
 #include "linear_args.cuh"
 #include "sm100_step.cuh"
@@ -74,9 +75,12 @@ __device__ __forceinline__ void hg_store(bf16_t* y, const float (&f)[8]) {
   *reinterpret_cast<uint4*>(y) = make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
 }
 
+// The tiles of a launch and how many of them a CTA has, and their division: a CTA places its first tile, and every copy in its ring, in front of the first load, where divisions by
+// numbers known at run time took 0.7 us
 struct HgTiles {
-  int n, m, batch;   // tiles along N and M, problems
-  int stages;
+  int n, m, each, more;        // tiles along N and M; tiles of every CTA, CTAs that have one more
+  uint32_t by_n, by_m;         // ceil(2^32 / n), ceil(2^32 / m): exact for fewer than 2^16 tiles; 0 for more
+  __device__ __forceinline__ static int over(int t, int d, uint32_t by) { return d == 1 ? t : (by != 0 ? (int)__umulhi((uint32_t)t, by) : t / d); }
 };
 
 template <int BN, typename TY>
@@ -88,11 +92,12 @@ __global__ void __launch_bounds__(64 + 32 * hg_epilogue(BN)) linear_sm100_kernel
   __shared__ HgShared shared;
   HgShared* sh = &shared;
   uint8_t* ring = hg_raw + ((1024u - (smem_u32(hg_raw) & 1023u)) & 1023u);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nk = (a.K + kHgBK - 1) / kHgBK, stages = tiles.stages;
-  const int total = tiles.n * tiles.m * tiles.batch, mine = (total - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // this CTA's: blockIdx.x, + gridDim.x, ...
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nk = (a.K + kHgBK - 1) / kHgBK;
+  constexpr int stages = hg_stages(BN);
+  const int mine = tiles.each + ((int)blockIdx.x < tiles.more);   // this CTA's tiles: blockIdx.x, + gridDim.x, ...
   auto place = [&](int i, int& n0, int& m0, int& b) {
-    const int t = blockIdx.x + i * gridDim.x, row = t / tiles.n;
-    n0 = (t - row * tiles.n) * BN, b = row / tiles.m, m0 = (row - b * tiles.m) * kHgBM;
+    const int t = blockIdx.x + i * gridDim.x, row = HgTiles::over(t, tiles.n, tiles.by_n);
+    n0 = (t - row * tiles.n) * BN, b = HgTiles::over(row, tiles.m, tiles.by_m), m0 = (row - b * tiles.m) * kHgBM;
   };
   const WaitReport report{&sh->dead, &g_linear_failures, failed};
   auto wait = [&](uint64_t* bar, uint32_t parity) { return wait_bounded(bar, parity, report); };
@@ -137,8 +142,11 @@ __global__ void __launch_bounds__(64 + 32 * hg_epilogue(BN)) linear_sm100_kernel
   const uint32_t tmem = sh->tmem;
   if (warp == 0) {
     if (lane == 0) {
-      int at = ahead, kb = ahead % nk, i = ahead / nk;
-      if (at < mine * nk) place(i, n0, m0, b);
+      int at = ahead, kb = ahead, i = 0;
+      if (at < mine * nk) {
+        for (; kb >= nk; kb -= nk) ++i;
+        place(i, n0, m0, b);
+      }
       for (; at < mine * nk && wait(&sh->empty[at % stages], (at / stages - 1) & 1); ++at, ++kb) {
         if (kb == nk) kb = 0, place(++i, n0, m0, b);
         load(kb, at);
@@ -180,11 +188,12 @@ __global__ void __launch_bounds__(64 + 32 * hg_epilogue(BN)) linear_sm100_kernel
       place(i, n0, m0, b);
       const int left_rows = a.M - m0 - quarter * 32, r0 = lane >> 3;   // of this warp's 32; the first of the eight that a thread brings out
       const long long m = m0 + quarter * 32 + r0;
-      auto whole = [&](int c) { return plain && left_rows > 0 && n0 + c + 64 <= a.N; };   // no branch between the loads and the stores of its 8 x 4 rows
+      // no branch between the loads and the stores of its 8 x 4 rows; a row's end lies between two threads' columns, or behind the piece
+      auto whole = [&](int c) { return plain && left_rows > 0 && (n0 + c + 64 <= a.N || (a.N & 7) == 0); };
       uint4 gate[8][2];
       auto gates = [&](int c) {
         if (a.gate == nullptr || !whole(c)) return;
-        const long long at = m * a.ldg + (long long)b * a.sg + n0 + c + (lane & 7) * 8;
+        const long long at = m * a.ldg + (long long)b * a.sg + min(n0 + c + (lane & 7) * 8, a.N - 8);
 #pragma unroll
         for (int j = 0; j < 8; ++j) hg_gates_load(a, at + (long long)(min(r0 + j * 4, left_rows - 1) - r0) * a.ldg, gate[j]);
       };
@@ -223,17 +232,18 @@ __global__ void __launch_bounds__(64 + 32 * hg_epilogue(BN)) linear_sm100_kernel
         const int n = n0 + c + (lane & 7) * 8, left = min(8, a.N - n);
         const bf16_t* bias = a.bias != nullptr ? static_cast<const bf16_t*>(a.bias) + b * a.sbias : nullptr;
         if (whole(c)) {
+          const int rows_here = left > 0 ? left_rows : 0;
           TY* y = static_cast<TY*>(a.Y) + (long long)b * a.sy + m * a.ldy + n;
           if (round_first) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
               const uint4 o = *reinterpret_cast<const uint4*>(slab + (r0 + j * 4) * kHgPitch16 + (lane & 7) * 4);
-              if (r0 + j * 4 < left_rows) *reinterpret_cast<uint4*>(y + (long long)(j * 4) * a.ldy) = o;
+              if (r0 + j * 4 < rows_here) *reinterpret_cast<uint4*>(y + (long long)(j * 4) * a.ldy) = o;
             }
           } else {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              if (r0 + j * 4 >= left_rows) break;
+              if (r0 + j * 4 >= rows_here) break;
               float f[8], z[8];
               hg_row(slab + (r0 + j * 4) * kHgPitch, lane & 7, a.alpha, f);
               if (a.gate != nullptr) {
@@ -316,19 +326,25 @@ static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
   const bool vec_out = aligned(a.Y) && a.ldy % ye == 0 && a.sy % ye == 0, vec_gate = aligned(a.gate) && a.ldg % ge == 0 && a.sg % ge == 0;
   // the hardware exponential for gates that come in pairs on 8-byte boundaries, the precise one for those at odd strides and an odd last column
   const bool pair_gate = a.ldg % 2 == 0 && a.sg % 2 == 0 && reinterpret_cast<uintptr_t>(a.gate) % 8 == 0;
-  const HgTiles tiles{(a.N + BN - 1) / BN, (a.M + kHgBM - 1) / kHgBM, batch, hg_stages(BN)};
+  HgTiles tiles{(a.N + BN - 1) / BN, (a.M + kHgBM - 1) / kHgBM, 0, 0, 0, 0};
   const long long total = (long long)tiles.n * tiles.m * batch;
   if (total > 0x7fffffffLL - 148) return set_error(OMC_ERR_SHAPE, "omc_linear: too many tiles");
-  linear_sm100_kernel<BN, TY><<<(int)(total < 148 ? total : 148), 64 + 32 * hg_epilogue(BN), smem, st>>>(tx, tw, a, tiles, a.sx == 0, a.sw == 0, vec_out, vec_gate, pair_gate, failed);
+  const int ctas = (int)(total < 148 ? total : 148);
+  tiles.each = (int)(total / ctas), tiles.more = (int)(total % ctas);
+  if (total < 1 << 16) tiles.by_n = (uint32_t)(((1ull << 32) + tiles.n - 1) / tiles.n), tiles.by_m = (uint32_t)(((1ull << 32) + tiles.m - 1) / tiles.m);
+  linear_sm100_kernel<BN, TY><<<ctas, 64 + 32 * hg_epilogue(BN), smem, st>>>(tx, tw, a, tiles, a.sx == 0, a.sw == 0, vec_out, vec_gate, pair_gate, failed);
   return check_launch("omc_linear");
 }
 
 template <typename TY>
 static int hg_launch_typed(const LinearArgs& a, int batch, cudaStream_t st) {
-  // the widest tile that still gives every SM a CTA (steps of few rows are a matter of CTAs, not of reuse)
-  const long long rows = (a.M + kHgBM - 1) / kHgBM;
-  if (a.N > 128 && rows * ((a.N + 255) / 256) * batch >= 148) return hg_launch<256, TY>(a, batch, st);
-  if (a.N > 64 && rows * ((a.N + 127) / 128) * batch >= 148) return hg_launch<128, TY>(a, batch, st);
+  // Tiles of 64, 128 and 256 columns take 4 : 5 : 8, and CTAs walk over them in waves of 148. 71 rows x 16, 128 -> 1024: 256 tiles of 64 10.3 us, 128 of 128 7.8, 64 of 256 10.4; 302 x 8,
+  // 128 -> 1024: 384 14.1, 192 12.2, 96 10.5; 282 x 16, 256 -> 1024 with gates: 768 24.4, 384 18.6, 192 20.0; 388 x 32, 512 -> 96: 256 20.3, 128 13.2
+  const long long rows = (long long)((a.M + kHgBM - 1) / kHgBM) * batch;
+  auto cost = [&](int bn, int each) { return (rows * ((a.N + bn - 1) / bn) + 147) / 148 * each; };
+  const long long of64 = cost(64, 4), of128 = a.N > 64 ? cost(128, 5) : of64, of256 = a.N > 128 ? cost(256, 8) : of64;
+  if (of256 < of64 && of256 < of128) return hg_launch<256, TY>(a, batch, st);
+  if (of128 < of64) return hg_launch<128, TY>(a, batch, st);
   return hg_launch<64, TY>(a, batch, st);
 }
 

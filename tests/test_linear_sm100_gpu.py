@@ -81,3 +81,17 @@ def test_a_cta_walks_over_many_tiles(N, K, batch, M, gated):
         bound = mag * (K * 2.0 ** -23 + 2.0 ** -20) + want.abs() * 2.0 ** -8 + 1e-30   # as above
         ok = (y[:, cols].double() - want).abs() <= bound
         assert (ok | (want.isnan() & y[:, cols].isnan())).all(), b
+
+
+@pytest.mark.parametrize("M,batch", [(131200, 64), (130900, 64), (40, 65535)])    # 65600 tiles, 65472 (the last that are placed by a multiplication), a tile per problem
+def test_many_tiles_find_their_places(M, batch):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    N, K = 72, 64
+    x, w = (torch.randn(*s, generator=gen, device="cuda").to(BF16) for s in ((M, K), (batch, N, K)))
+    y = torch.full((M, batch * N), 7.0, dtype=BF16, device="cuda")
+    seqlib.linear(x, w, y, M=M, N=N, K=K, ldx=K, sx=0, ldw=K, sw=N * K, ldy=batch * N, sy=N, batch=batch)
+    rows = torch.cat([torch.arange(0, M, max(1, M // 40), device="cuda"), torch.tensor([M - 1], device="cuda")])
+    want = torch.einsum("mk,bnk->mbn", x[rows].double(), w.double())
+    bound = torch.einsum("mk,bnk->mbn", x[rows].double().abs(), w.double().abs()) * (K * 2.0 ** -23) + want.abs() * 2.0 ** -8
+    assert ((y[rows].view(-1, batch, N).double() - want).abs() <= bound).all()
+    assert not (y[:, ::61] == 7.0).all(1).any()
