@@ -339,7 +339,7 @@ static int hg_launch(const LinearArgs& a, int batch, cudaStream_t st) {
 template <typename TY>
 static int hg_launch_typed(const LinearArgs& a, int batch, cudaStream_t st) {
   // Tiles of 64, 128 and 256 columns take 4 : 5 : 8, and CTAs walk over them in waves of 148. 71 rows x 16, 128 -> 1024: 256 tiles of 64 10.3 us, 128 of 128 7.8, 64 of 256 10.4; 302 x 8,
-  // 128 -> 1024: 384 14.1, 192 12.2, 96 10.5; 282 x 16, 256 -> 1024 with gates: 768 24.4, 384 18.6, 192 20.0; 388 x 32, 512 -> 96: 256 20.3, 128 13.2
+  // 128 -> 1024: 384 14.1, 192 12.2, 96 10.5; 282 x 16, 256 -> 1024 with gates: 768 24.4, 384 18.6, 192 20.0
   const long long rows = (long long)((a.M + kHgBM - 1) / kHgBM) * batch;
   auto cost = [&](int bn, int each) { return (rows * ((a.N + bn - 1) / bn) + 147) / 148 * each; };
   const long long of64 = cost(64, 4), of128 = a.N > 64 ? cost(128, 5) : of64, of256 = a.N > 128 ? cost(256, 8) : of64;
